@@ -374,13 +374,19 @@ struct CsrOp {
 };
 
 // ============================================================================
-// reductions: RED_GRID blocks write partials; consumers reduce them in a
+// reductions: red_blocks(n) blocks write partials; consumers reduce them in a
 // fixed order (deterministic for a given n)
 // ============================================================================
-// Warp sum into lane 0.  Only the lanes that feed lane 0 add (16, 8, 4, 2, 1
-// of them): lane 0 does the same additions in the same order as a full
-// butterfly, with a fifth of the FP64 work, which is what GB300's FP64 pipe
-// is short of.
+// Blocks of a reduction over n rows: RED_GRID, or one thread per row where
+// that takes fewer.  The rows of a thread are the same either way and the
+// blocks left out would add exact zeros, so the sums do not depend on it; a
+// fixed RED_GRID made the small systems pay for 912 blocks' reductions and
+// tickets (k_fg_mdot<double> at 3816 rows: 33 us, of which 15 blocks had rows).
+inline int red_blocks(int64_t n) {
+    return (int)std::min<int64_t>(RED_GRID, (n + RED_BLOCK - 1) / RED_BLOCK);
+}
+
+// Warp sum into lane 0: the tree x[l] += x[l + 16], then + 8, 4, 2, 1.
 __device__ __forceinline__ double warp_sum_to_lane0(double x) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -396,38 +402,69 @@ __device__ __forceinline__ float warp_sum_to_lane0(float x) {
     return x;
 }
 
+// The warp sums of D values (D a power of two up to 32) at once.  While more
+// than one value is left, the two halves of the warp split the values
+// between them: at each step a lane keeps half of its values and adds what
+// its partner at distance o holds of them, so D values take
+// D - 1 + 5 - log2(D) adds instead of 5 D.  An FP64 instruction holds this
+// GPU's FP64 pipe for the whole warp however few lanes want its result, and
+// the shuffle adds bounded the multi-dot kernels (eight dots: 9 adds, 40
+// before).  Every value is summed over the same tree as warp_sum_to_lane0's
+// (each addition's operands at most exchanged): the same bits.  Returns value
+// `which` in the lanes that hold it (all lanes of a group of 32 / D; the
+// group's first lane is 32 / D * which).
+template <int D, typename V>
+__device__ __forceinline__ V warp_sums(V (&v)[D], int& which) {
+    const int lane = threadIdx.x & 31;
+    which = 0;
+#pragma unroll
+    for (int o = 16, m = D; o > 0; o >>= 1) {
+        if (m > 1) {
+            const bool up = lane & o;
+            m >>= 1;
+#pragma unroll
+            for (int q = 0; q < m; ++q) {
+                const V send = up ? v[q] : v[q + m], keep = up ? v[q + m] : v[q];
+                v[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+            which = 2 * which + (up ? 1 : 0);
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
+    }
+    return v[0];
+}
+
 // per-block partial sums of D values into part[d * RED_GRID + block]; the
 // values may be float (warp sums in FP32, block sum in FP64) or double
 template <int D, typename V>
 __device__ __forceinline__ void block_partials(V (&v)[D], double* __restrict__ part) {
-    __shared__ double sh[D][RED_BLOCK / 32];
+    constexpr int W = RED_BLOCK / 32;  // warps: the block sum is a tree over W lanes
+    __shared__ double sh[D][W];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-        const V x = warp_sum_to_lane0(v[d]);
-        if (lane == 0) sh[d][w] = (double)x;
-    }
+    int which;
+    const V x = warp_sums<D, V>(v, which);
+    if (lane == 32 / D * which) sh[which][w] = (double)x;
     __syncthreads();
-    if (threadIdx.x < 32) {
+    if (threadIdx.x < ((D * W + 31) / 32) * 32) {  // W lanes per value
+        const int d = threadIdx.x / W;
+        double y = d < D ? sh[d][threadIdx.x % W] : 0.0;
 #pragma unroll
-        for (int d = 0; d < D; ++d) {
-            double x = (lane < RED_BLOCK / 32) ? sh[d][lane] : 0.0;
-            x = warp_sum_to_lane0(x);
-            if (lane == 0) part[d * RED_GRID + blockIdx.x] = x;
-        }
+        for (int o = W / 2; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+        if (d < D && threadIdx.x % W == 0) part[d * RED_GRID + blockIdx.x] = y;
     }
 }
 
-// every block reduces the partials itself (fixed order): no finalize launch
+// the sums of the nb blocks' partials, in every thread of the calling block
 template <int D>
-__device__ __forceinline__ void reduce_partials(const double* __restrict__ part, double (&out)[D]) {
+__device__ __forceinline__ void reduce_partials(const double* __restrict__ part, int nb, double (&out)[D]) {
     __shared__ double sh[D][RED_BLOCK / 32];
     __shared__ double res[D];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
     for (int d = 0; d < D; ++d) {
         double x = 0.0;
-        for (int k = threadIdx.x; k < RED_GRID; k += blockDim.x) x += __ldcg(part + d * RED_GRID + k);
+        for (int k = threadIdx.x; k < nb; k += blockDim.x) x += __ldcg(part + d * RED_GRID + k);
         x = warp_sum_to_lane0(x);
         if (lane == 0) sh[d][w] = x;
     }
@@ -466,9 +503,9 @@ __global__ void __launch_bounds__(RED_BLOCK) k_bicg_init(int64_t n, Op A, const 
     block_partials<2>(acc, part);
 }
 
-__global__ void k_bicg_setup(const double* __restrict__ part, Scalars* sc, double tol, int rel_r0) {
+__global__ void k_bicg_setup(const double* __restrict__ part, int nb, Scalars* sc, double tol, int rel_r0) {
     double v[2];
-    reduce_partials<2>(part, v);
+    reduce_partials<2>(part, nb, v);
     if (threadIdx.x == 0) {
         sc->rr = v[0];
         sc->rho = v[0];
@@ -486,9 +523,9 @@ __global__ void k_bicg_setup(const double* __restrict__ part, Scalars* sc, doubl
 
 // restart after a breakdown: k_bicg_init has set r = rhat = p = b - A x from
 // the current iterate; the target, iteration count and best residual carry on
-__global__ void k_bicg_restart(const double* __restrict__ part, Scalars* sc) {
+__global__ void k_bicg_restart(const double* __restrict__ part, int nb, Scalars* sc) {
     double v[2];
-    reduce_partials<2>(part, v);
+    reduce_partials<2>(part, nb, v);
     if (threadIdx.x == 0) {
         sc->rr = v[0];
         sc->rho = v[0];
@@ -515,7 +552,7 @@ __device__ __forceinline__ bool finish_partials(double (&v)[D], double* __restri
     __syncthreads();
     if (!last) return false;
     __threadfence();
-    reduce_partials<D>(part, tot);
+    reduce_partials<D>(part, (int)gridDim.x, tot);
     if (threadIdx.x == 0) *ticket = 0u;
     return true;
 }
@@ -661,10 +698,10 @@ __global__ void __launch_bounds__(RED_BLOCK) k_resid(int64_t n, Op A, const T* _
 }
 
 // cycle start: beta = ||r||; v0 = r/beta; g = beta e1; ctl: j = 0, cycle_done
-__global__ void k_fg_start(const double* __restrict__ part, Scalars* sc, double* Hd, FgLayout F, int first,
+__global__ void k_fg_start(const double* __restrict__ part, int nb, Scalars* sc, double* Hd, FgLayout F, int first,
                            double tol, int rel_r0) {
     double v[2];
-    reduce_partials<2>(part, v);
+    reduce_partials<2>(part, nb, v);
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         const double beta = sqrt(v[0]);
         if (first) {
@@ -724,14 +761,14 @@ __global__ void __launch_bounds__(RED_BLOCK) k_fg_mdot(int64_t n, const T* __res
 }
 
 // h(0..j) = reduced dots (added to column j of H on the second pass)
-__global__ void k_fg_hcol(const double* __restrict__ part, double* Hd, FgLayout F, int j, int accumulate,
+__global__ void k_fg_hcol(const double* __restrict__ part, int nb, double* Hd, FgLayout F, int j, int accumulate,
                           const Scalars* __restrict__ sc) {
     if (fg_skip(sc)) return;
     // one warp per dot, fixed order
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int i = w; i <= j; i += nw) {
         double x = 0.0;
-        for (int k = lane; k < RED_GRID; k += 32) x += part[(int64_t)i * RED_GRID + k];
+        for (int k = lane; k < nb; k += 32) x += part[(int64_t)i * RED_GRID + k];
         x = warp_sum_to_lane0(x);
         if (lane == 0) {
             Hd[F.hc(i)] = x;
@@ -761,13 +798,13 @@ __global__ void __launch_bounds__(RED_BLOCK) k_fg_maxpy(int64_t n, const T* __re
 }
 
 // h(j+1,j) = ||w||; Givens; residual estimate; cycle/convergence control
-__device__ void fg_givens(const double* __restrict__ part, Scalars* sc, double* Hd, FgLayout F, int j) {
+__device__ void fg_givens(const double* __restrict__ part, int nb, Scalars* sc, double* Hd, FgLayout F, int j) {
     // the column and the earlier rotations are staged in shared memory by
     // all threads; one thread then applies the rotations (a serial chain
     // that would otherwise wait on global memory at every step)
     __shared__ double hcol[FG_MAXM + 1], csv[FG_MAXM], snv[FG_MAXM];
     double v[1];
-    reduce_partials<1>(part, v);
+    reduce_partials<1>(part, nb, v);
     const int t = threadIdx.x;
     for (int i = t; i <= j; i += blockDim.x) hcol[i] = Hd[F.H(i, j)];
     for (int i = t; i < j; i += blockDim.x) {
@@ -811,9 +848,9 @@ __device__ void fg_givens(const double* __restrict__ part, Scalars* sc, double* 
 
 // `mirror` (pinned host memory, optional) receives the scalars after this
 // iteration, whether it ran or was skipped
-__global__ void k_fg_givens(const double* __restrict__ part, Scalars* sc, double* Hd, FgLayout F, int j,
+__global__ void k_fg_givens(const double* __restrict__ part, int nb, Scalars* sc, double* Hd, FgLayout F, int j,
                             Scalars* mirror) {
-    if (!fg_skip(sc)) fg_givens(part, sc, Hd, F, j);
+    if (!fg_skip(sc)) fg_givens(part, nb, sc, Hd, F, j);
     if (mirror && threadIdx.x == 0) *mirror = *sc;
 }
 
@@ -949,10 +986,10 @@ int graph_run(Ctx* c, const void* k0, const void* k1, const void* k2, int64_t n,
 template <typename Op, typename T>
 int run_bicgstab(Ctx* c, int64_t n, const Op& A, Work<T> w, double tol, int rel_r0, int maxit, int* iters,
                  double* rr_out, T* xbest = nullptr) {
-    const int G = RED_GRID, B = RED_BLOCK;
+    const int G = red_blocks(n), B = RED_BLOCK;
     k_bicg_init<Op, T><<<G, B, 0, c->stream>>>(n, A, w.x, w.b, w.r, w.rh, w.p, c->part);
     BSC_LAUNCH(c);
-    k_bicg_setup<<<1, B, 0, c->stream>>>(c->part, c->sc, tol, rel_r0);
+    k_bicg_setup<<<1, B, 0, c->stream>>>(c->part, G, c->sc, tol, rel_r0);
     BSC_LAUNCH(c);
     if (xbest) BSC_CUDA(c, cudaMemcpyAsync(xbest, w.x, sizeof(T) * n, cudaMemcpyDeviceToDevice, c->stream));
     // the first SpMV of every batch is bracketed by events (recorded into the
@@ -993,7 +1030,7 @@ int run_bicgstab(Ctx* c, int64_t n, const Op& A, Work<T> w, double tol, int rel_
             ++restarts;
             k_bicg_init<Op, T><<<G, B, 0, c->stream>>>(n, A, w.x, w.b, w.r, w.rh, w.p, c->part);
             BSC_LAUNCH(c);
-            k_bicg_restart<<<1, B, 0, c->stream>>>(c->part, c->sc);
+            k_bicg_restart<<<1, B, 0, c->stream>>>(c->part, G, c->sc);
             BSC_LAUNCH(c);
             c->launches += 2;
             continue;
@@ -1047,14 +1084,14 @@ int run_bicgstab(Ctx* c, int64_t n, const Op& A, Work<T> w, double tol, int rel_
 template <typename Op, typename T>
 int run_fgmres(Ctx* c, int64_t n, const Op& A, Work<T> w, double tol, int rel_r0, int maxit, int m, int* iters,
                double* rr_out) {
-    const int G = RED_GRID, B = RED_BLOCK;
+    const int G = red_blocks(n), B = RED_BLOCK;
     FgLayout F{m};
     int first = 1;
     T* wv = w.t;
     for (;;) {
         k_resid<Op, T><<<G, B, 0, c->stream>>>(n, A, w.x, w.b, w.r, c->part);
         BSC_LAUNCH(c);
-        k_fg_start<<<1, B, 0, c->stream>>>(c->part, c->sc, c->Hd, F, first, tol, rel_r0);
+        k_fg_start<<<1, B, 0, c->stream>>>(c->part, G, c->sc, c->Hd, F, first, tol, rel_r0);
         BSC_LAUNCH(c);
         first = 0;
         int rc = fetch_scalars(c);
@@ -1067,11 +1104,11 @@ int run_fgmres(Ctx* c, int64_t n, const Op& A, Work<T> w, double tol, int rel_r0
             k_fg_spmv<Op, T><<<G, B, 0, c->stream>>>(n, A, w.V, wv, j, c->sc);
             for (int pass = 0; pass < 2; ++pass) {
                 k_fg_mdot<T><<<G, B, 0, c->stream>>>(n, w.V, wv, j, c->part, c->sc);
-                k_fg_hcol<<<1, 1024, 0, c->stream>>>(c->part, c->Hd, F, j, pass, c->sc);
+                k_fg_hcol<<<1, 1024, 0, c->stream>>>(c->part, G, c->Hd, F, j, pass, c->sc);
                 k_fg_maxpy<T><<<G, B, 0, c->stream>>>(n, w.V, wv, j, c->Hd, F, pass, c->part, c->sc);
                 c->launches += 3;
             }
-            k_fg_givens<<<1, B, 0, c->stream>>>(c->part, c->sc, c->Hd, F, j, nullptr);
+            k_fg_givens<<<1, B, 0, c->stream>>>(c->part, G, c->sc, c->Hd, F, j, nullptr);
             k_fg_next<T><<<G, B, 0, c->stream>>>(n, wv, w.V, j, c->sc);
             c->launches += 3;
         }
@@ -1104,9 +1141,9 @@ __global__ void __launch_bounds__(RED_BLOCK) k_ir_resid(int64_t n, EllOp<double>
     block_partials<2>(acc, part);
 }
 
-__global__ void k_ir_norms(const double* __restrict__ part, double* out) {
+__global__ void k_ir_norms(const double* __restrict__ part, int nb, double* out) {
     double v[2];
-    reduce_partials<2>(part, v);
+    reduce_partials<2>(part, nb, v);
     if (threadIdx.x == 0) {
         out[0] = sqrt(v[0]);
         out[1] = sqrt(v[1]);
@@ -1163,7 +1200,7 @@ int fetch_outer(Ctx* c) {
 // costs its iterations; x converges to the FP64 system's solution.
 int run_fgmres_ir(Ctx* c, int64_t n, bsc_solve_info* si) {
     const bsc_params& P = c->P;
-    const int G = RED_GRID, B = RED_BLOCK;
+    const int G = red_blocks(n), B = RED_BLOCK;
     const int rel_r0 = P.tol_mode == BSC_TOL_REL_R0;
     const int m = c->ir_m;
     const FgLayout F{m};
@@ -1176,7 +1213,7 @@ int run_fgmres_ir(Ctx* c, int64_t n, bsc_solve_info* si) {
     for (;;) {
         k_resid<EllOp<double>, double><<<G, B, 0, c->stream>>>(n, A, x, c->b, c->r, c->part);
         BSC_LAUNCH(c);
-        k_fg_start<<<1, B, 0, c->stream>>>(c->part, c->sc2, c->Hd, F, first, P.tol, rel_r0);
+        k_fg_start<<<1, B, 0, c->stream>>>(c->part, G, c->sc2, c->Hd, F, first, P.tol, rel_r0);
         BSC_LAUNCH(c);
         first = 0;
         int rc = fetch_outer(c);
@@ -1203,10 +1240,10 @@ int run_fgmres_ir(Ctx* c, int64_t n, bsc_solve_info* si) {
             k_spmv_z<<<G, B, 0, c->stream>>>(n, A, zj, w, c->sc2);
             for (int pass = 0; pass < 2; ++pass) {
                 k_fg_mdot<double><<<G, B, 0, c->stream>>>(n, c->V, w, j, c->part, c->sc2);
-                k_fg_hcol<<<1, 1024, 0, c->stream>>>(c->part, c->Hd, F, j, pass, c->sc2);
+                k_fg_hcol<<<1, 1024, 0, c->stream>>>(c->part, G, c->Hd, F, j, pass, c->sc2);
                 k_fg_maxpy<double><<<G, B, 0, c->stream>>>(n, c->V, w, j, c->Hd, F, pass, c->part, c->sc2);
             }
-            k_fg_givens<<<1, B, 0, c->stream>>>(c->part, c->sc2, c->Hd, F, j, nullptr);
+            k_fg_givens<<<1, B, 0, c->stream>>>(c->part, G, c->sc2, c->Hd, F, j, nullptr);
             k_fg_next<double><<<G, B, 0, c->stream>>>(n, w, c->V, j, c->sc2);
             c->launches += 11;
             BSC_CUDA(c, cudaGetLastError());
@@ -1223,7 +1260,7 @@ int run_fgmres_ir(Ctx* c, int64_t n, bsc_solve_info* si) {
     double* norms = c->Hd + F.size();
     k_resid<EllOp<double>, double><<<G, B, 0, c->stream>>>(n, A, x, c->b, c->r, c->part);
     BSC_LAUNCH(c);
-    k_ir_norms<<<1, B, 0, c->stream>>>(c->part, norms);
+    k_ir_norms<<<1, B, 0, c->stream>>>(c->part, G, norms);
     BSC_LAUNCH(c);
     double nrm[2];
     BSC_CUDA(c, cudaMemcpyAsync(nrm, norms, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -1307,7 +1344,7 @@ int fg_cycle(Ctx* c, int m, int budget, Scalars* h, int* iters, Q queue) {
 // estimate and reports the true residual of the returned pressure.
 int run_fgmres_mg(Ctx* c, int64_t n, bsc_solve_info* si) {
     const bsc_params& P = c->P;
-    const int G = RED_GRID, B = RED_BLOCK;
+    const int G = red_blocks(n), B = RED_BLOCK;
     const int rel_r0 = P.tol_mode == BSC_TOL_REL_R0;
     Mg& mg = c->mg;
     const int m = mg.m;
@@ -1321,7 +1358,7 @@ int run_fgmres_mg(Ctx* c, int64_t n, bsc_solve_info* si) {
     for (;;) {
         k_resid<EllOp<double>, double><<<G, B, 0, c->stream>>>(n, A, x, c->b, c->r, c->part);
         BSC_LAUNCH(c);
-        k_fg_start<<<1, B, 0, c->stream>>>(c->part, c->sc2, c->Hd, F, first, P.tol, rel_r0);
+        k_fg_start<<<1, B, 0, c->stream>>>(c->part, G, c->sc2, c->Hd, F, first, P.tol, rel_r0);
         BSC_LAUNCH(c);
         first = 0;
         if ((rc = fetch_outer(c))) return rc;
@@ -1349,9 +1386,9 @@ int run_fgmres_mg(Ctx* c, int64_t n, bsc_solve_info* si) {
                 // iteration at 846k rows (their last block has a quarter of
                 // k_fg_hcol's warps)
                 k_fg_mdot<double><<<G, B, 0, c->stream>>>(n, V, w, j, c->part, c->sc2);
-                k_fg_hcol<<<1, 1024, 0, c->stream>>>(c->part, c->Hd, F, j, 0, c->sc2);
+                k_fg_hcol<<<1, 1024, 0, c->stream>>>(c->part, G, c->Hd, F, j, 0, c->sc2);
                 k_fg_maxpy<double><<<G, B, 0, c->stream>>>(n, V, w, j, c->Hd, F, 1, c->part, c->sc2);
-                k_fg_givens<<<1, B, 0, c->stream>>>(c->part, c->sc2, c->Hd, F, j, mirror);
+                k_fg_givens<<<1, B, 0, c->stream>>>(c->part, G, c->sc2, c->Hd, F, j, mirror);
                 k_fg_next<double><<<G, B, 0, c->stream>>>(n, w, V, j, c->sc2);
                 if (c->prof_iter) record_event(c, c->ev_it[5]);
                 c->launches += 6;
@@ -1370,7 +1407,7 @@ int run_fgmres_mg(Ctx* c, int64_t n, bsc_solve_info* si) {
     double* norms = c->Hd + F.size();
     k_resid<EllOp<double>, double><<<G, B, 0, c->stream>>>(n, A, x, c->b, c->r, c->part);
     BSC_LAUNCH(c);
-    k_ir_norms<<<1, B, 0, c->stream>>>(c->part, norms);
+    k_ir_norms<<<1, B, 0, c->stream>>>(c->part, G, norms);
     BSC_LAUNCH(c);
     double nrm[2];
     BSC_CUDA(c, cudaMemcpyAsync(nrm, norms, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -1452,7 +1489,7 @@ __global__ void __launch_bounds__(RED_BLOCK) k_fgf_mdot(int64_t n, const T* __re
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int i = wp; i <= j; i += nw) {
         double x = 0.0;
-        for (int k = lane; k < RED_GRID; k += 32) x += __ldcg(part + (int64_t)i * RED_GRID + k);
+        for (int k = lane; k < (int)gridDim.x; k += 32) x += __ldcg(part + (int64_t)i * RED_GRID + k);
         x = warp_sum_to_lane0(x);
         if (lane == 0) {
             Hd[F.hc(i)] = x;
@@ -1495,7 +1532,7 @@ __global__ void __launch_bounds__(RED_BLOCK) k_fgf_maxpy_givens(int64_t n, const
     __syncthreads();
     if (!last) return;
     __threadfence();
-    fg_givens(part, sc, Hd, F, j);
+    fg_givens(part, (int)gridDim.x, sc, Hd, F, j);
     __syncthreads();
     if (threadIdx.x == 0) {
         *ticket = 0u;
@@ -1539,7 +1576,7 @@ __global__ void k_ir_addz(int64_t n, double* __restrict__ x, const float* __rest
 
 int run_fgmres_ir_mg(Ctx* c, int64_t n, bsc_solve_info* si) {
     const bsc_params& P = c->P;
-    const int G = RED_GRID, B = RED_BLOCK;
+    const int G = red_blocks(n), B = RED_BLOCK;
     const int rel_r0 = P.tol_mode == BSC_TOL_REL_R0;
     Mg& mg = c->mg;
     const int m = mg.m;
@@ -1556,7 +1593,7 @@ int run_fgmres_ir_mg(Ctx* c, int64_t n, bsc_solve_info* si) {
     for (;;) {
         k_resid<EllOp<double>, double><<<G, B, 0, c->stream>>>(n, A, x, c->b, c->r, c->part);
         BSC_LAUNCH(c);
-        k_fg_start<<<1, B, 0, c->stream>>>(c->part, c->sc2, c->Hd, F, first, P.tol, rel_r0);
+        k_fg_start<<<1, B, 0, c->stream>>>(c->part, G, c->sc2, c->Hd, F, first, P.tol, rel_r0);
         BSC_LAUNCH(c);
         first = 0;
         if ((rc = fetch_outer(c))) return rc;
@@ -1567,7 +1604,7 @@ int run_fgmres_ir_mg(Ctx* c, int64_t n, bsc_solve_info* si) {
         // inner: A d = r in FP32 from d = 0, one FGMRES(m) cycle
         k_d2f<<<G, B, 0, c->stream>>>(n, c->r, rf);
         k_norm2f<<<G, B, 0, c->stream>>>(n, rf, c->part);
-        k_fg_start<<<1, B, 0, c->stream>>>(c->part, c->sc, c->Hd, F, 1, inner_tol, 1);
+        k_fg_start<<<1, B, 0, c->stream>>>(c->part, G, c->sc, c->Hd, F, 1, inner_tol, 1);
         k_fgf_v0<<<G, B, 0, c->stream>>>(n, rf, V, c->sc);
         c->launches += 4;
         mg.skip = c->sc;
@@ -1608,7 +1645,7 @@ int run_fgmres_ir_mg(Ctx* c, int64_t n, bsc_solve_info* si) {
     double* norms = c->Hd + F.size();
     k_resid<EllOp<double>, double><<<G, B, 0, c->stream>>>(n, A, x, c->b, c->r, c->part);
     BSC_LAUNCH(c);
-    k_ir_norms<<<1, B, 0, c->stream>>>(c->part, norms);
+    k_ir_norms<<<1, B, 0, c->stream>>>(c->part, G, norms);
     BSC_LAUNCH(c);
     double nrm[2];
     BSC_CUDA(c, cudaMemcpyAsync(nrm, norms, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -1653,9 +1690,9 @@ int op_ppe_solve(Ctx* c, bsc_solve_info* info) {
             rc = run_bicgstab<EllOp<double>, double>(c, n, A, w, P.tol, rel_r0, P.maxit, &iters, &rr);
         if (rc && rc != BSC_E_BREAKDOWN) return rc;
         // true residual of the returned pressure
-        k_resid<EllOp<double>, double><<<RED_GRID, RED_BLOCK, 0, c->stream>>>(n, A, c->S.p, c->b, c->r, c->part);
+        k_resid<EllOp<double>, double><<<red_blocks(n), RED_BLOCK, 0, c->stream>>>(n, A, c->S.p, c->b, c->r, c->part);
         BSC_LAUNCH(c);
-        k_ir_norms<<<1, RED_BLOCK, 0, c->stream>>>(c->part, c->Hd + FgLayout{c->fg_m}.size());
+        k_ir_norms<<<1, RED_BLOCK, 0, c->stream>>>(c->part, red_blocks(n), c->Hd + FgLayout{c->fg_m}.size());
         BSC_LAUNCH(c);
         double nrm[2];
         BSC_CUDA(c, cudaMemcpyAsync(nrm, c->Hd + FgLayout{c->fg_m}.size(), 2 * sizeof(double), cudaMemcpyDeviceToHost,
@@ -1691,10 +1728,10 @@ int csr_solve_device(Ctx* c, int32_t n, const int32_t* rp, const int32_t* col, c
                  ? run_fgmres<CsrOp, double>(c, n, A, w, P.tol, rel_r0, P.maxit, c->fg_m, &iters, &rr)
                  : run_bicgstab<CsrOp, double>(c, n, A, w, P.tol, rel_r0, P.maxit, &iters, &rr);
     if (rc) return rc;
-    k_resid<CsrOp, double><<<RED_GRID, RED_BLOCK, 0, c->stream>>>(n, A, x, b, work, c->part);
+    k_resid<CsrOp, double><<<red_blocks(n), RED_BLOCK, 0, c->stream>>>(n, A, x, b, work, c->part);
     BSC_LAUNCH(c);
     double* norms = c->Hd + FgLayout{c->fg_m}.size();
-    k_ir_norms<<<1, RED_BLOCK, 0, c->stream>>>(c->part, norms);
+    k_ir_norms<<<1, RED_BLOCK, 0, c->stream>>>(c->part, red_blocks(n), norms);
     BSC_LAUNCH(c);
     double nrm[2];
     BSC_CUDA(c, cudaMemcpyAsync(nrm, norms, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
