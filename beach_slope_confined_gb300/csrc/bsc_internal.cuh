@@ -429,6 +429,7 @@ int op_piston(Ctx* c);
 int op_comp_pos(Ctx* c);
 // pairs.cu
 int op_neighbour(Ctx* c);
+int op_neighbour_lists(Ctx* c);  // nbr and cnt only
 int op_freesurf(Ctx* c);
 int op_effpor(Ctx* c);
 int op_eddyvis(Ctx* c);

@@ -1,5 +1,6 @@
-// sph_kernel.cuh -- the smoothing kernel W(r) and its gradient factor, shared
-// by the pair operators (pairs.cu) and the salinity flux (scalar.cu).
+// sph_kernel.cuh -- the smoothing kernel W(r), its gradient factor and the
+// FP32 pre-test of the pair searches, shared by the pair operators (pairs.cu),
+// the salinity flux (scalar.cu) and the WCSPH step (wcsph.cu).
 #pragma once
 
 #include "bsc_internal.cuh"
@@ -40,6 +41,20 @@ __device__ __forceinline__ R kern_w(const KParams& K, R r) {
     if (q < (R)1) return A * ((R)4 - (R)6 * q * q + (R)3 * q * q * q) + B * (q * q * q - (R)6 * q + (R)6);
     R a = (R)2 - q;
     return (A + B) * (a * a * a);
+}
+
+// ---- FP32 pre-test of the pair searches -----------------------------------------------
+// Positions are kept as float offsets from the origin of their own cell, so
+// a candidate in the neighbouring cell (ax, ay) sits at its offset plus an
+// exact shift of 0 or +-cs.  With offsets below PRE_GUARD cells the float
+// estimate of r^2 is within ~1e-6 (relative) of the exact one, far inside
+// the 1e-5 margin: the pre-test only rejects candidates that the exact FP64
+// test would reject too.  Particles farther from their binned cell skip it.
+constexpr float PRE_GUARD = 4.0f;
+constexpr double PRE_MARGIN = 1e-5;
+
+__device__ __forceinline__ bool pre_ok(float2 p, float csf) {
+    return fabsf(p.x) < PRE_GUARD * csf && fabsf(p.y) < PRE_GUARD * csf;
 }
 
 }  // namespace bsc

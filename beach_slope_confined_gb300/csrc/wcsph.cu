@@ -36,6 +36,7 @@
 #include <vector>
 
 #include "bsc_internal.cuh"
+#include "sph_kernel.cuh"
 
 struct bsc_ctx : bsc::Ctx {};  // the same definition as in api.cu
 
@@ -201,12 +202,23 @@ struct PorKeep {
     double* pgv;   // sum over that cell's solids of V_s W(r_is)
 };
 
-// porosity n_i from the solids in the 3x3 cells (fluid; 1 elsewhere)
+// Porosity n_i from the solids in the 3x3 cells (fluid; 1 elsewhere).  Bound:
+// the FP64 pipe, which an instruction holds for the whole warp however few
+// lanes run it.  Testing every candidate in FP64 inside the divergent cell
+// loop ran ~60 candidates' offsets a particle and their kernels at half the
+// lanes; the FP32 pre-test (sph_kernel.cuh) now compacts the survivors, in
+// cell order, into this thread's column of shared memory, and the FP64 terms
+// run over those.  Same terms, same order.  A particle with more survivors
+// than the column holds, or far from its binned cell, takes one pass.
+// 101573 particles, no adjoint record: 236 us before, 60 us.
+constexpr int WP_CAP = 32;
 __global__ void __launch_bounds__(WB) k_wc_por(int64_t n, State S, KParams KP, WcK K, const int32_t* __restrict__ pcell,
-                                               const int32_t* __restrict__ scs, const int32_t* __restrict__ scc,
+                                               const float2* __restrict__ posf, const int32_t* __restrict__ scs,
+                                               const int32_t* __restrict__ scc, const float2* __restrict__ sposf,
                                                const double* __restrict__ sx, const double* __restrict__ sy,
                                                const double* __restrict__ sw, const double* __restrict__ svol,
                                                const int32_t* __restrict__ sg, double* __restrict__ nout, PorKeep kp) {
+    __shared__ int32_t cand[WP_CAP * WB];
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     int cg[GCMAX];
@@ -220,34 +232,61 @@ __global__ void __launch_bounds__(WB) k_wc_por(int64_t n, State S, KParams KP, W
     if (is_fluid(S, i)) {
         const double xi = S.x[i], yi = S.y[i];
         const int c = pcell[i], cx = c / KP.ny, cy = c - cx * KP.ny;
-        for (int ax = cx - 1; ax <= cx + 1; ++ax) {
-            if (ax < 0 || ax >= KP.nx) continue;
-            for (int ay = cy - 1; ay <= cy + 1; ++ay) {
-                if (ay < 0 || ay >= KP.ny) continue;
-                const int cc = ax * KP.ny + ay;
-                for (int s = scs[cc], e = scs[cc] + scc[cc]; s < e; ++s) {
-                    const double dx = xi - sx[s], dy = yi - sy[s], d2 = dx * dx + dy * dy;
-                    if (!(d2 < K.H2)) continue;
-                    const double r = sqrt(d2), W = wW(K, r);
-                    frac += sw[s] * W;
-                    if (kp.dn) {
-                        const double F = wF(K, r);
-                        gx -= sw[s] * F * dx;  // grad n = -sum sw grad W
-                        gy -= sw[s] * F * dy;
-                        const int g = sg[s];
-                        if (g < 0) continue;
-                        const double v = svol[s] * W;
-                        bool kept = false;
+        const float H2f = (float)(KP.H2 * (1.0 + PRE_MARGIN)), csf = (float)KP.cs;
+        const float2 pi = posf[i];
+        const bool pre_i = pre_ok(pi, csf);
+        auto term = [&](int s) {
+            const double dx = xi - sx[s], dy = yi - sy[s], d2 = dx * dx + dy * dy;
+            if (!(d2 < K.H2)) return;
+            const double r = sqrt(d2), W = wW(K, r);
+            frac += sw[s] * W;
+            if (kp.dn) {
+                const double F = wF(K, r);
+                gx -= sw[s] * F * dx;  // grad n = -sum sw grad W
+                gy -= sw[s] * F * dy;
+                const int g = sg[s];
+                if (g < 0) return;
+                const double v = svol[s] * W;
+                bool kept = false;
 #pragma unroll
-                        for (int u = 0; u < GCMAX; ++u) {
-                            if (!kept && u < K.gc && (cg[u] == g || cg[u] < 0)) {
-                                cg[u] = g;
-                                cv[u] += v;
-                                kept = true;
-                            }
-                        }
+                for (int u = 0; u < GCMAX; ++u) {
+                    if (!kept && u < K.gc && (cg[u] == g || cg[u] < 0)) {
+                        cg[u] = g;
+                        cv[u] += v;
+                        kept = true;
                     }
                 }
+            }
+        };
+        int nc = 0;
+        // pass 0 compacts the survivors; pass 1 (only if they do not fit, or
+        // without the pre-test) sums over the cells directly
+        for (int pass = pre_i ? 0 : 1; pass < 2; ++pass) {
+            for (int ax = cx - 1; ax <= cx + 1; ++ax) {
+                if (ax < 0 || ax >= KP.nx) continue;
+                const float shx = (float)(ax - cx) * csf;
+                for (int ay = cy - 1; ay <= cy + 1; ++ay) {
+                    if (ay < 0 || ay >= KP.ny) continue;
+                    const float shy = (float)(ay - cy) * csf;
+                    const int cc = ax * KP.ny + ay;
+                    for (int s = scs[cc], e = scs[cc] + scc[cc]; s < e; ++s) {
+                        if (pass == 1) {
+                            term(s);
+                            continue;
+                        }
+                        const float2 ps = sposf[s];
+                        if (pre_ok(ps, csf)) {
+                            const float fdx = pi.x - (ps.x + shx), fdy = pi.y - (ps.y + shy);
+                            if (fdx * fdx + fdy * fdy > H2f) continue;
+                        }
+                        if (nc < WP_CAP) cand[nc * WB + threadIdx.x] = s;
+                        ++nc;
+                    }
+                }
+            }
+            if (pass == 0 && nc <= WP_CAP) {
+                for (int k = 0; k < nc; ++k) term(cand[k * WB + threadIdx.x]);
+                break;
             }
         }
     }
@@ -330,22 +369,32 @@ __global__ void __launch_bounds__(WB) k_wc_step(int64_t n, State S, WcK K, const
     Pbuf[n + i] = Py;
 }
 
-// probe elevations of a state: per-block partials of sum_i V_i w1(x_i - x_p)
+// Probe elevations of a state: per-block partials of sum_i V_i w1(x_i - x_p),
+// one thread per particle.  Almost every block is out of every probe's reach:
+// an FP32 test of the distance (widened past its rounding) keeps the divisions
+// and the block sums to the blocks that have a particle in reach, the others
+// write their exact zero.  101573 particles, four probes: 27 us before, 7 us.
 __global__ void __launch_bounds__(WB) k_wc_eta(int64_t n, const int8_t* __restrict__ tid, const double* __restrict__ mass,
                                                St s, WcK K, const double* __restrict__ xp, double* __restrict__ part) {
     __shared__ double sh[WB];
-    double acc[BSC_WCSPH_MAX_PROBES];
-    for (int p = 0; p < K.np; ++p) acc[p] = 0.0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        if (tid[i] != BSC_TID_FLUID) continue;
-        const double V = mass[i] / s.rho[i];
-        for (int p = 0; p < K.np; ++p) {
-            const double q = fabs(s.x[i] - xp[p]) / K.R1;
-            if (q < 1.0) acc[p] += V * w1(q, K.R1);
-        }
-    }
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const bool fluid = i < n && tid[i] == BSC_TID_FLUID;
+    const double xi = fluid ? s.x[i] : 0.0;
+    const float xf = (float)xi, reach = (float)K.R1 * 1.001f;
     for (int p = 0; p < K.np; ++p) {
-        sh[threadIdx.x] = acc[p];
+        const double xpp = xp[p];
+        const float xpf = (float)xpp;
+        const bool near = fluid && !(fabsf(xf - xpf) > reach + 4e-7f * (fabsf(xf) + fabsf(xpf)));
+        if (!__syncthreads_or(near)) {
+            if (threadIdx.x == 0) part[blockIdx.x * K.np + p] = 0.0;
+            continue;
+        }
+        double a = 0.0;
+        if (near) {
+            const double V = mass[i] / s.rho[i], q = fabs(xi - xpp) / K.R1;
+            if (q < 1.0) a = V * w1(q, K.R1);
+        }
+        sh[threadIdx.x] = a;
         __syncthreads();
         for (int o = WB / 2; o > 0; o >>= 1) {
             if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
@@ -710,8 +759,10 @@ Keep seg_keep(WcState* w, int q, int64_t n, int64_t slots) {
 // With `keep`, the step's lists, counts and cells are built straight into the
 // kept buffers (the context's own are pointed there for the step), and the
 // per-particle quotients, per-pair kernel values and porosity derivatives
-// are kept too.
-int wc_step(Ctx* c, WcState* w, double* nbuf, double* Pbuf, const Keep* keep = nullptr) {
+// are kept too.  The step reads the lists only; `last` (the last step that a
+// call runs) takes the full search, which leaves the context's grad W, L and
+// flags as those of the state it ends on.
+int wc_step(Ctx* c, WcState* w, double* nbuf, double* Pbuf, const Keep* keep, bool last) {
     const int64_t n = c->n;
     c->t += w->K.dt;
     int32_t *own_nbr = c->nbr, *own_cnt = c->cnt, *own_cell = c->pcell;
@@ -723,15 +774,15 @@ int wc_step(Ctx* c, WcState* w, double* nbuf, double* Pbuf, const Keep* keep = n
     const Pre pre = keep ? keep->pre : wc_pre(w);
     int rc = op_piston(c);
     if (!rc) rc = cells_build(c, false);
-    if (!rc) rc = op_neighbour(c);
+    if (!rc) rc = last ? op_neighbour(c) : op_neighbour_lists(c);
     if (!rc) {
         const unsigned g = blocks_for(n, WB);
         const State S = wc_view(c, w);
         k_wc_pre<<<g, WB, 0, c->stream>>>(n, S.tid, S.mass, S.y, S.rho, w->K, pre);
         rc = launch_check(c);
         if (!rc) {
-            k_wc_por<<<g, WB, 0, c->stream>>>(n, S, c->K, w->K, c->pcell, c->scell_start, c->scell_count, c->sx,
-                                              c->sy, w->sw, c->svol, w->sg, nbuf,
+            k_wc_por<<<g, WB, 0, c->stream>>>(n, S, c->K, w->K, c->pcell, c->posf, c->scell_start, c->scell_count,
+                                              c->sposf, c->sx, c->sy, w->sw, c->svol, w->sg, nbuf,
                                               keep ? keep->por : PorKeep{nullptr, nullptr, nullptr});
             rc = launch_check(c);
         }
@@ -888,10 +939,10 @@ int bsc_wcsph_forward(bsc_ctx* c, int32_t nsteps, int32_t every, double* eta) {
             const int q = s - last0;
             const Keep kq = seg_keep(w, q, n, slots);
             if ((rc = wc_save(c, w->seg + (int64_t)q * 5 * n)) ||
-                (rc = wc_step(c, w, w->segn + (int64_t)q * n, w->segP + (int64_t)q * 2 * n, &kq)))
+                (rc = wc_step(c, w, w->segn + (int64_t)q * n, w->segP + (int64_t)q * 2 * n, &kq, s == nsteps - 1)))
                 return rc;
             if (s == nsteps - 1 && (rc = wc_save(c, w->seg + (int64_t)(q + 1) * 5 * n))) return rc;
-        } else if ((rc = wc_step(c, w, w->segn, w->segP))) {
+        } else if ((rc = wc_step(c, w, w->segn, w->segP, nullptr, false))) {
             return rc;
         }
         k_wc_eta<<<nb, WB, 0, c->stream>>>(n, c->S.tid, w->mass, st_of(w->nxt, n), w->K, w->xp, w->part);
@@ -936,7 +987,8 @@ int bsc_wcsph_adjoint(bsc_ctx* c, const double* dJ_deta, double* grad) {
             const int q = s - s0;
             if ((rc = wc_save(c, w->seg + (int64_t)q * 5 * n))) return rc;
             const Keep kq = seg_keep(w, q, n, slots);
-            if ((rc = wc_step(c, w, w->segn + (int64_t)q * n, w->segP + (int64_t)q * 2 * n, &kq))) return rc;
+            if ((rc = wc_step(c, w, w->segn + (int64_t)q * n, w->segP + (int64_t)q * 2 * n, &kq, s == s1 - 1 && sgi == 0)))
+                return rc;
         }
         if (!kept && (rc = wc_save(c, w->seg + (int64_t)(s1 - s0) * 5 * n))) return rc;
         // reverse through the segment
