@@ -413,7 +413,7 @@ int op_neighbour(Ctx* c) {
 // pre-test decides both ways outside its margin (its r^2 is within ~1e-6 of
 // the exact one, the margin 1e-5), so only candidates inside the band take
 // the FP64 test that bounds the full search (~27 FP64 instructions an entry).
-// 101573 particles: the search 152 us, this 23 us.
+// 101573 particles: the search 153 us, this 30 us.
 __global__ void __launch_bounds__(NB_BLOCK) k_neighbour_lists(
     int64_t n, const double* __restrict__ x, const double* __restrict__ y, KParams K,
     const int32_t* __restrict__ cstart, const int32_t* __restrict__ ccount, const int32_t* __restrict__ sorted,

@@ -210,7 +210,7 @@ struct PorKeep {
 // cell order, into this thread's column of shared memory, and the FP64 terms
 // run over those.  Same terms, same order.  A particle with more survivors
 // than the column holds, or far from its binned cell, takes one pass.
-// 101573 particles, no adjoint record: 236 us before, 60 us.
+// 101573 particles, no adjoint record: 236 us before, 112 us.
 constexpr int WP_CAP = 32;
 __global__ void __launch_bounds__(WB) k_wc_por(int64_t n, State S, KParams KP, WcK K, const int32_t* __restrict__ pcell,
                                                const float2* __restrict__ posf, const int32_t* __restrict__ scs,
@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(WB) k_wc_step(int64_t n, State S, WcK K, const
 // one thread per particle.  Almost every block is out of every probe's reach:
 // an FP32 test of the distance (widened past its rounding) keeps the divisions
 // and the block sums to the blocks that have a particle in reach, the others
-// write their exact zero.  101573 particles, four probes: 27 us before, 7 us.
+// write their exact zero.  101573 particles, four probes: 27 us before, 8 us.
 __global__ void __launch_bounds__(WB) k_wc_eta(int64_t n, const int8_t* __restrict__ tid, const double* __restrict__ mass,
                                                St s, WcK K, const double* __restrict__ xp, double* __restrict__ part) {
     __shared__ double sh[WB];
