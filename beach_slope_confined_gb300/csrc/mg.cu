@@ -123,99 +123,133 @@ __global__ void k_mg_galerkin(int nxf, int nyf, const double* __restrict__ Af, i
 }
 
 // Dense inverse of the coarsest level by Gauss-Jordan elimination with
-// partial (row) pivoting, in place in shared memory, one CTA.  Empty cells
-// (all-zero rows) become identity rows.  A zero pivot is replaced by a tiny
-// one: the preconditioner then loses that direction but stays finite.
-// Computed in FP32 (R below) on both paths and written as O: one SM runs
-// it, where FP64 is ~60x slower, and the coarsest solve is part of a
-// preconditioner, whose rounding costs iterations, never accuracy.
+// partial (row) pivoting, one CTA.  Empty cells (all-zero rows) become
+// identity rows.  A zero pivot is replaced by a tiny one: the preconditioner
+// then loses that direction but stays finite.  Computed in FP32 on both paths
+// and written as O: one SM runs it, where FP64 is ~60x slower, and the
+// coarsest solve is part of a preconditioner, whose rounding costs
+// iterations, never accuracy.
+//
+// Bound: the chain of up to 128 elimination steps, each waiting on the one
+// before, on one SM's issue slots.  The matrix stays in registers: warp w
+// holds columns w, w + 32, ..., lanes hold rows, so column k's pivot is found
+// inside one warp, which publishes the multipliers; the pivot row reaches the
+// other lanes by shuffles, and a step has one block barrier.  Rows are not
+// moved but carry the position that interchanges would have given them.  The
+// elimination performs the same FP32 operations as with the matrix in shared
+// memory and its rows interchanged (six barriers a step): 136 us there at 86
+// cells, 36 us here.
+constexpr int GJ_E = MG_COARSE_MAX / 32;  // columns per warp, rows per lane
 template <typename O>
 __global__ void __launch_bounds__(1024) k_mg_dense_inverse(int nx, int ny, const double* __restrict__ A,
                                                             O* __restrict__ cinv) {
-    using R = float;
-    extern __shared__ __align__(16) unsigned char dense_sm[];
-    R* M = reinterpret_cast<R*>(dense_sm);  // n x n, row-major
-    __shared__ int perm[MG_COARSE_MAX];
-    __shared__ R fcol[MG_COARSE_MAX];
-    __shared__ int piv_row;
-    __shared__ R piv_inv;
+    __shared__ float scol[2][MG_COARSE_MAX];  // column k, by step parity
+    __shared__ float sinv[2];                 // 1 / pivot
+    __shared__ int sp[2];                     // pivot row
+    __shared__ int spos[MG_COARSE_MAX];       // position of an unused row; GJ_USED after its step
+    __shared__ int fpos[MG_COARSE_MAX], row_at[MG_COARSE_MAX];  // final position of a row, and its inverse
+    constexpr int GJ_USED = 0xffff;
+    const unsigned full = 0xffffffffu;
     const int n = nx * ny;
-    const int t = threadIdx.x, T = blockDim.x;
-    const int lane = t & 31, warp = t >> 5, nwarps = T >> 5;
-    for (int q = t; q < n * n; q += T) M[q] = (R)0;
-    __syncthreads();
-    for (int c = t; c < n; c += T) {
-        const int cx = c / ny, cy = c % ny;
-        bool any = false;
-        for (int s = 0; s < 9; ++s) {
-            const double v = A[(int64_t)s * n + c];
-            const int gx = cx + s / 3 - 1, gy = cy + s % 3 - 1;
-            if (v == 0.0 || gx < 0 || gx >= nx || gy < 0 || gy >= ny) continue;
-            M[c * n + gx * ny + gy] += (R)v;
-            any = true;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float M[GJ_E][GJ_E];  // row lane + 32 r, column w + 32 e
+#pragma unroll
+    for (int r = 0; r < GJ_E; ++r) {
+        const int c = lane + 32 * r, cx = c / ny, cy = c - cx * ny;
+#pragma unroll
+        for (int e = 0; e < GJ_E; ++e) {
+            const int g = w + 32 * e, dx = g / ny - cx, dy = g % ny - cy;
+            M[r][e] = 0.f;
+            if (c < n && g < n && dx >= -1 && dx <= 1 && dy >= -1 && dy <= 1)
+                M[r][e] = (float)A[(int64_t)stencil_slot(dx, dy) * n + c];
+            if (c == g && c < n) {  // an empty cell becomes an identity row
+                bool any = false;
+                for (int s = 0; s < 9; ++s) {
+                    const int gx = cx + s / 3 - 1, gy = cy + s % 3 - 1;
+                    if (gx >= 0 && gx < nx && gy >= 0 && gy < ny) any |= A[(int64_t)s * n + c] != 0.0;
+                }
+                if (!any) M[r][e] = 1.f;
+            }
         }
-        if (!any) M[c * n + c] = (R)1;
+        if (w == 0) spos[c] = c < n ? c : GJ_USED;
     }
     __syncthreads();
-    for (int k = 0; k < n; ++k) {
-        // pivot: the largest |M[i][k]| over i >= k (warp 0)
-        if (t < 32) {
-            R best = (R)-1;
-            int bi = k;
-            for (int i = k + t; i < n; i += 32) {
-                const R a = fabs(M[i * n + k]);
-                if (a > best) { best = a; bi = i; }
+#pragma unroll
+    for (int ke = 0; ke < GJ_E; ++ke) {
+        for (int kl = 0; kl < 32; ++kl) {
+            const int k = 32 * ke + kl, buf = kl & 1;
+            if (k >= n) break;
+            if (w == kl) {
+                // the largest |M[i][k]| over unused rows, the lowest position on ties; a NaN is never preferred
+                unsigned best = 0u, bkey = 0xffffffffu;
+                int ps[GJ_E];
+#pragma unroll
+                for (int r = 0; r < GJ_E; ++r) {
+                    ps[r] = spos[lane + 32 * r];
+                    const float a = fabsf(M[r][ke]);
+                    const unsigned ab = a == a ? __float_as_uint(a) : 0u;
+                    const unsigned key = (unsigned)ps[r] << 16 | (unsigned)(lane + 32 * r);
+                    if (ps[r] != GJ_USED && (ab > best || (ab == best && key < bkey))) {
+                        best = ab;
+                        bkey = key;
+                    }
+                    scol[buf][lane + 32 * r] = M[r][ke];
+                }
+                const unsigned top = __reduce_max_sync(full, best);
+                const unsigned key = __reduce_min_sync(full, best == top ? bkey : 0xffffffffu);
+                const int p = (int)(key & 0xffffu), ppos = (int)(key >> 16);
+#pragma unroll
+                for (int r = 0; r < GJ_E; ++r) {
+                    if (lane + 32 * r == p) {
+                        const float pv = M[r][ke] == 0.f ? 1e-30f : M[r][ke];
+                        sinv[buf] = 1.f / pv;
+                        sp[buf] = p;
+                        spos[p] = GJ_USED;
+                        fpos[p] = k;
+                    } else if (ps[r] == k) {
+                        spos[lane + 32 * r] = ppos;
+                    }
+                }
             }
-            for (int o = 16; o > 0; o >>= 1) {
-                const R ob = __shfl_down_sync(0xffffffffu, best, o);
-                const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-                if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
+            __syncthreads();
+            const float inv = sinv[buf];
+            const int p = sp[buf], pl = p & 31, pr = p >> 5;
+            float f[GJ_E], q[GJ_E];
+#pragma unroll
+            for (int r = 0; r < GJ_E; ++r) f[r] = scol[buf][lane + 32 * r];
+#pragma unroll
+            for (int r = 0; r < GJ_E; ++r)
+                if (r == pr)
+#pragma unroll
+                    for (int e = 0; e < GJ_E; ++e) q[e] = __shfl_sync(full, M[r][e], pl) * inv;
+            if (w == kl) {  // column k becomes column k of the inverse in place
+                q[ke] = inv;
+#pragma unroll
+                for (int r = 0; r < GJ_E; ++r) M[r][ke] = 0.f;
             }
-            if (t == 0) { piv_row = bi; perm[k] = bi; }
+#pragma unroll
+            for (int r = 0; r < GJ_E; ++r)
+#pragma unroll
+                for (int e = 0; e < GJ_E; ++e) M[r][e] = fmaf(-f[r], q[e], M[r][e]);
+#pragma unroll
+            for (int r = 0; r < GJ_E; ++r)
+                if (r == pr && lane == pl)
+#pragma unroll
+                    for (int e = 0; e < GJ_E; ++e) M[r][e] = q[e];
         }
-        __syncthreads();
-        const int p = piv_row;
-        if (p != k)
-            for (int j = t; j < n; j += T) {
-                const R a = M[k * n + j];
-                M[k * n + j] = M[p * n + j];
-                M[p * n + j] = a;
-            }
-        __syncthreads();
-        if (t == 0) {
-            R pv = M[k * n + k];
-            if (pv == (R)0) pv = (R)1e-30f;
-            piv_inv = (R)1 / pv;
-            M[k * n + k] = (R)1;
-        }
-        __syncthreads();
-        for (int j = t; j < n; j += T) M[k * n + j] *= piv_inv;
-        for (int i = t; i < n; i += T) fcol[i] = (i == k) ? (R)0 : M[i * n + k];
-        __syncthreads();
-        for (int i = t; i < n; i += T)
-            if (i != k) M[i * n + k] = (R)0;
-        __syncthreads();
-        // eliminate column k from every other row: a warp per row, lanes
-        // along it
-        for (int i = warp; i < n; i += nwarps) {
-            if (i == k) continue;
-            const R f = fcol[i];
-            for (int j = lane; j < n; j += 32) M[i * n + j] -= f * M[k * n + j];
-        }
-        __syncthreads();
     }
-    // undo the row interchanges as column interchanges, last first
-    for (int k = n - 1; k >= 0; --k) {
-        const int p = perm[k];
-        if (p != k)
-            for (int i = t; i < n; i += T) {
-                const R a = M[i * n + k];
-                M[i * n + k] = M[i * n + p];
-                M[i * n + p] = a;
-            }
-        __syncthreads();
-    }
-    for (int q = t; q < n * n; q += T) cinv[q] = (O)M[q];
+    // row i of the elimination is row fpos[i] of (P A)^-1, whose column j is
+    // column row_at[j] of A^-1
+    __syncthreads();
+    if (threadIdx.x < n) row_at[fpos[threadIdx.x]] = threadIdx.x;
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < GJ_E; ++r)
+#pragma unroll
+        for (int e = 0; e < GJ_E; ++e) {
+            const int i = lane + 32 * r, j = w + 32 * e;
+            if (i < n && j < n) cinv[fpos[i] * n + row_at[j]] = (O)M[r][e];
+        }
 }
 
 // ---- V-cycle, structured levels (l >= 1) -------------------------------------------
@@ -1141,14 +1175,10 @@ int mg_setup(Ctx* c) {
     }
     // the coarsest inverse (FP32 Gauss-Jordan), in the V-cycle's precision
     const MgLevel& Lc = mg.L[mg.nlev];
-    const int smem = (int)(Lc.nc * Lc.nc * sizeof(float));
-    const int smem_max = MG_COARSE_MAX * MG_COARSE_MAX * (int)sizeof(float);
-    BSC_CUDA(c, cudaFuncSetAttribute(k_mg_dense_inverse<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
-    BSC_CUDA(c, cudaFuncSetAttribute(k_mg_dense_inverse<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
     if (f32)
-        k_mg_dense_inverse<float><<<1, 1024, smem, c->stream>>>(Lc.nx, Lc.ny, Lc.A, mg.cinvf);
+        k_mg_dense_inverse<float><<<1, 1024, 0, c->stream>>>(Lc.nx, Lc.ny, Lc.A, mg.cinvf);
     else
-        k_mg_dense_inverse<double><<<1, 1024, smem, c->stream>>>(Lc.nx, Lc.ny, Lc.A, mg.cinv);
+        k_mg_dense_inverse<double><<<1, 1024, 0, c->stream>>>(Lc.nx, Lc.ny, Lc.A, mg.cinv);
     BSC_LAUNCH(c);
     // the restriction operators of the levels swept by per-level kernels
     if (c->P.mg_sweeps == 2 && !c->mg_cell4)
