@@ -30,17 +30,69 @@ int cuda_err(Ctx* c, cudaError_t e, const char* where) {
     return set_err(c, e == cudaErrorMemoryAllocation ? BSC_E_NOMEM : BSC_E_CUDA, buf);
 }
 
-void timing_flush(Ctx* c) {
-    if (c->ev_used == 0) return;
-    cudaEventSynchronize(c->evs[2 * (c->ev_used - 1) + 1]);
-    for (int k = 0; k < c->ev_used; ++k) {
+static cudaEvent_t span_event(Ctx* c, int64_t e) { return c->evs[e % Ctx::EVPOOL]; }
+
+// the event at this point of the stream: the last one, unless something was
+// launched after it (or `fresh`: the host may have been away since)
+static int64_t event_now(Ctx* c, bool fresh) {
+    if (!fresh && c->ev_next > 0 && c->ev_launches == c->launches) return c->ev_next - 1;
+    cudaEventRecord(span_event(c, c->ev_next), c->stream);
+    c->ev_launches = c->launches;
+    return c->ev_next++;
+}
+
+void timing_poll(Ctx* c) {
+    size_t keep = 0;
+    for (size_t k = 0; k < c->spans.size(); ++k) {
+        const Ctx::Span sp = c->spans[k];
         float f = 0.f;
-        if (cudaEventElapsedTime(&f, c->evs[2 * k], c->evs[2 * k + 1]) == cudaSuccess) {
-            c->ms[c->ev_slot[k]] += f;
-            c->calls[c->ev_slot[k]]++;
+        if (sp.e1 >= 0) {
+            const cudaError_t e = cudaEventElapsedTime(&f, span_event(c, sp.e0), span_event(c, sp.e1));
+            if (e == cudaSuccess) {
+                c->ms[sp.slot] += f;
+                c->calls[sp.slot]++;
+            } else {
+                (void)cudaGetLastError();  // a failed query must not fail what follows
+            }
+            if (e != cudaErrorNotReady) continue;
+        }
+        c->spans[keep++] = sp;
+    }
+    c->spans.resize(keep);
+}
+
+void timing_flush(Ctx* c) {
+    if (c->spans.empty()) return;
+    cudaEventSynchronize(span_event(c, c->ev_next - 1));
+    timing_poll(c);
+}
+
+void span_open(Ctx* c, int slot) {
+    // keep the ring ahead of the oldest unresolved span: its events may not be
+    // recorded again.  A span still open after so many events is taken up to
+    // the last one and carries on from there.
+    if (!c->spans.empty() && c->ev_next - c->spans.front().e0 > Ctx::EVPOOL - 64) {
+        timing_flush(c);
+        for (auto& sp : c->spans) {
+            float f = 0.f;
+            if (cudaEventElapsedTime(&f, span_event(c, sp.e0), span_event(c, c->ev_next - 1)) == cudaSuccess)
+                c->ms[sp.slot] += f;
+            else
+                (void)cudaGetLastError();
+            sp.e0 = c->ev_next - 1;
         }
     }
-    c->ev_used = 0;
+    c->spans.push_back({slot, event_now(c, c->ev_depth == 0), -1});
+    ++c->ev_depth;
+}
+
+void span_close(Ctx* c) {
+    for (size_t k = c->spans.size(); k-- > 0;)
+        if (c->spans[k].e1 < 0) {  // the innermost open one
+            c->spans[k].e1 = event_now(c, false);
+            break;
+        }
+    --c->ev_depth;
 }
 
 static void derive_kparams(Ctx* c) {
@@ -287,6 +339,7 @@ __global__ void k_to_id_order_u8(int64_t n, const uint8_t* __restrict__ src, uin
 static int check_flags(Ctx* c) {
     BSC_CUDA(c, cudaMemcpyAsync(c->h_flag, c->d_flag, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
     BSC_CUDA(c, cudaStreamSynchronize(c->stream));
+    c->ev_launches = -1;  // a stage ending here ends after this copy
     const int f = c->h_flag[0];
     if (f) {
         BSC_CUDA(c, cudaMemsetAsync(c->d_flag, 0, 4 * sizeof(int32_t), c->stream));
@@ -433,8 +486,8 @@ int bsc_create(const bsc_params* p, bsc_ctx** out) {
         delete c;
         return BSC_E_CUDA;
     }
-    for (int k = 0; k < 2 * Ctx::EVPOOL; ++k) cudaEventCreate(&c->evs[k]);
-    for (int k = 0; k < 6; ++k) cudaEventCreate(&c->ev_spmv[k]);
+    for (int k = 0; k < Ctx::EVPOOL; ++k) cudaEventCreate(&c->evs[k]);
+    for (int k = 0; k < 4; ++k) cudaEventCreate(&c->ev_spmv[k]);
     if (const char* e = std::getenv("BSC_GRAPHS")) c->use_graphs = e[0] != '0';
     if (const char* e = std::getenv("BSC_DEBUG")) c->debug = e[0] == '1';
     if (const char* e = std::getenv("BSC_SPMV_UNROLL")) c->spmv_unroll = e[0] == '1';
@@ -471,9 +524,9 @@ int bsc_destroy(bsc_ctx* c) {
     for (void* p : c->pallocs)
         if (p) cudaFree(p);
     c->pallocs.clear();
-    for (int k = 0; k < 2 * Ctx::EVPOOL; ++k)
+    for (int k = 0; k < Ctx::EVPOOL; ++k)
         if (c->evs[k]) cudaEventDestroy(c->evs[k]);
-    for (int k = 0; k < 6; ++k)
+    for (int k = 0; k < 4; ++k)
         if (c->ev_spmv[k]) cudaEventDestroy(c->ev_spmv[k]);
     for (int k = 0; k < 2; ++k)
         if (c->ev_lag[k]) cudaEventDestroy(c->ev_lag[k]);
@@ -827,9 +880,7 @@ int bsc_step(bsc_ctx* c, int32_t nsteps, bsc_solve_info* last) {
         if (c->P.salinity) RUN(BSC_T_EDDYVIS, op_eddyvis(c));
 #undef RUN
     }
-    int rc = check_flags(c);
-    if (c->timing) timing_flush(c);
-    return rc;
+    return check_flags(c);
 }
 
 int bsc_get_neighbors(bsc_ctx* c, int64_t* offsets, int32_t* ids) {

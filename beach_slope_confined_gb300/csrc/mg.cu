@@ -137,8 +137,8 @@ __global__ void k_mg_galerkin(int nxf, int nyf, const double* __restrict__ Af, i
 // other lanes by shuffles, and a step has one block barrier.  Rows are not
 // moved but carry the position that interchanges would have given them.  The
 // elimination performs the same FP32 operations as with the matrix in shared
-// memory and its rows interchanged (six barriers a step): 136 us there at 86
-// cells, 36 us here.
+// memory and its rows interchanged (six barriers a step): 136 us there at 105
+// cells, 83 us here (cold caches).
 constexpr int GJ_E = MG_COARSE_MAX / 32;  // columns per warp, rows per lane
 template <typename O>
 __global__ void __launch_bounds__(1024) k_mg_dense_inverse(int nx, int ny, const double* __restrict__ A,

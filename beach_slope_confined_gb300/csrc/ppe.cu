@@ -1068,6 +1068,7 @@ int run_bicgstab(Ctx* c, int64_t n, const Op& A, Work<T> w, double tol, int rel_
             for (int q = 0; q < nb; ++q) one();
         }
         c->launches += 5 * nb;
+        if (launched == 0 && c->timing) timing_poll(c);  // while the first batch runs
         launched += nb;
         BSC_CUDA(c, cudaGetLastError());
     }
@@ -1324,13 +1325,16 @@ int fg_cycle(Ctx* c, int m, int budget, Scalars* h, int* iters, Q queue) {
             if (int rc = queue(j, c->h_it + (j & 1))) return rc;
             BSC_CUDA(c, cudaEventRecord(c->ev_lag[j & 1], c->stream));
         }
+        // the host is about to wait for an iteration: the time to resolve the
+        // spans of the stages before the solve
+        if (j == 0 && c->timing) timing_poll(c);
         const int chk = lag ? last : (more ? j : -1);
         if (chk >= 0) {
             BSC_CUDA(c, cudaEventSynchronize(c->ev_lag[chk & 1]));
             *h = c->h_it[chk & 1];
             ++*iters;
             mg_iter_profile(c);
-            spmv_time(c, 1 + (chk & 1));
+            if (chk == 0) spmv_time(c, 1);
             if (h->tmp[2] != 0.0) return BSC_OK;  // iteration j, if queued, skips
         }
         if (!more) return BSC_OK;
@@ -1374,11 +1378,11 @@ int run_fgmres_mg(Ctx* c, int64_t n, bsc_solve_info* si) {
             // reorder swaps
             return graph_run(c, c->pcell, vj, zj, n, [&]() -> int {
                 if (int r = mg_vcycle_f64(c, vj, zj)) return r;
-                // the SpMV w = A z_j is bracketed by events: the dominant
-                // HBM-bound kernel, timed in place
-                if (c->timing) record_event(c, c->ev_spmv[2 + 2 * (j & 1)]);
+                // the first column's SpMV w = A z_j is bracketed by events: the
+                // dominant HBM-bound kernel, timed in place
+                if (c->timing && j == 0) record_event(c, c->ev_spmv[2]);
                 k_spmv_z<double><<<blocks_for(n, B), B, 0, c->stream>>>(n, A, zj, w, c->sc2);
-                if (c->timing) record_event(c, c->ev_spmv[3 + 2 * (j & 1)]);
+                if (c->timing && j == 0) record_event(c, c->ev_spmv[3]);
                 if (c->prof_iter) record_event(c, c->ev_it[4]);
                 // separate single-block kernels for the column of H and the
                 // Givens step: in FP64 the fused last-block forms (as on the
@@ -1614,11 +1618,11 @@ int run_fgmres_ir_mg(Ctx* c, int64_t n, bsc_solve_info* si) {
             // one inner iteration as a cached graph per column j (and cell map)
             return graph_run(c, c->pcell, vj, zj, n, [&]() -> int {
                 if (int r = mg_vcycle_f32(c, vj, zj)) return r;
-                // the FP32 SpMV w = A z_j is bracketed by events (the
-                // dominant HBM-bound kernel, timed in place)
-                if (c->timing) record_event(c, c->ev_spmv[2 + 2 * (j & 1)]);
+                // the first column's FP32 SpMV w = A z_j is bracketed by events
+                // (the dominant HBM-bound kernel, timed in place)
+                if (c->timing && j == 0) record_event(c, c->ev_spmv[2]);
                 k_spmv_f<<<blocks_for(n, B), B, 0, c->stream>>>(n, Af, zj, w, c->sc);
-                if (c->timing) record_event(c, c->ev_spmv[3 + 2 * (j & 1)]);
+                if (c->timing && j == 0) record_event(c, c->ev_spmv[3]);
                 if (c->prof_iter) record_event(c, c->ev_it[4]);
                 // the column of H and the Givens step finish in the last
                 // block of the dot and update kernels (no single-block launches)
