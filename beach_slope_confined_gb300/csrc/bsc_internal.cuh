@@ -211,10 +211,14 @@ struct MgLevel {
     // cell of level l+1, 36 weights over the 6x6 patch of this level's cells
     // around its 2x2 children (36 x nc of level l+1, in the V-cycle's type)
     void* R = nullptr;
+    void* T = nullptr;             // dense V-cycle operator from this level down (nc rows of ldT)
+    int ldT = 0;
 };
 struct Mg {
     int nlev = 0;                  // levels 1..nlev are structured; nlev is solved densely
-    int tail_l0 = 0;               // levels tail_l0..nlev run in one single-CTA kernel
+    int tail_l0 = 0;               // levels tail_l0..nlev run as one launch: a dense product, or one CTA
+    bool dense = false;            // the dense product (L[tail_l0].T)
+    void *dx = nullptr, *dz = nullptr;  // its work arrays while it is built
     MgLevel L[MG_MAX_LEVELS + 1];
     double* cinv = nullptr;        // inverse of the coarsest level, FP64, row-major
     float* cinvf = nullptr;        // its FP32 copy (mixed path)

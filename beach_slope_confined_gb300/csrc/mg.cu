@@ -524,45 +524,38 @@ __global__ void __launch_bounds__(MG_BLOCK) k_mg_restrict(int nx, int ny, const 
 constexpr int MG_RPATCH = 6;
 constexpr int MG_RW = MG_RPATCH * MG_RPATCH;
 
+// One thread per weight (a coarse cell's 36 weights as 36 threads): with a
+// thread per coarse cell the 4 x 9 x 9 products were one serial chain, which
+// on the small levels took 43 us in FP64 whatever their size.
 template <typename T>
 __global__ void k_mg_build_R(int nx, int ny, const T* __restrict__ A, const T* __restrict__ dinv, int nxc, int nyc,
                              T w0, T w1, T* __restrict__ R) {
-    const int C = blockIdx.x * blockDim.x + threadIdx.x;
-    if (C >= nxc * nyc) return;
-    const int CX = C / nyc, CY = C - CX * nyc, nc = nx * ny, ncc = nxc * nyc;
-    const int x0 = 2 * CX - 2, y0 = 2 * CY - 2;  // patch origin
-    T acc[MG_RW];
-#pragma unroll
-    for (int k = 0; k < MG_RW; ++k) acc[k] = 0;
-    const T wsum = w0 + w1, wprod = w0 * w1;
-    // fully unrolled: every accumulator index is a compile-time constant, so
-    // acc stays in registers
-#pragma unroll
+    const int nc = nx * ny, ncc = nxc * nyc;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= ncc * MG_RW) return;
+    const int k = q / ncc, C = q - k * ncc, CX = C / nyc, CY = C - CX * nyc;
+    const int gx = 2 * CX - 2 + k / MG_RPATCH, gy = 2 * CY - 2 + k % MG_RPATCH;  // the patch cell
+    if (gx < 0 || gx >= nx || gy < 0 || gy >= ny) {
+        R[q] = (T)0;
+        return;
+    }
+    const int g = gx * ny + gy;
+    T own = 0, one = 0, two = 0;  // sums of delta_fg, A_fg and (A D^-1 A)_fg over the children f
     for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const int fx = 2 * CX + a, fy = 2 * CY + q;
-            if (fx >= nx || fy >= ny) continue;
+        for (int b = 0; b < 2; ++b) {
+            const int fx = 2 * CX + a, fy = 2 * CY + b;
+            if (fx >= nx || fy >= ny || abs(fx - gx) > 2 || abs(fy - gy) > 2) continue;
             const int f = fx * ny + fy;
-            acc[(a + 2) * MG_RPATCH + (q + 2)] += (T)1;
-#pragma unroll
-            for (int s = 0; s < 9; ++s) {
-                const int hx = fx + s / 3 - 1, hy = fy + s % 3 - 1;
-                if (hx < 0 || hx >= nx || hy < 0 || hy >= ny) continue;
-                const int h = hx * ny + hy;
-                const T bfh = A[s * nc + f] * dinv[h];
-                acc[(a + 1 + s / 3) * MG_RPATCH + (q + 1 + s % 3)] -= wsum * bfh;
-#pragma unroll
-                for (int s2 = 0; s2 < 9; ++s2) {
-                    const int gx = hx + s2 / 3 - 1, gy = hy + s2 % 3 - 1;
-                    if (gx < 0 || gx >= nx || gy < 0 || gy >= ny) continue;
-                    acc[(a + s / 3 + s2 / 3) * MG_RPATCH + (q + s % 3 + s2 % 3)] +=
-                        wprod * bfh * A[s2 * nc + h] * dinv[gx * ny + gy];
+            if (f == g) own += (T)1;
+            if (abs(fx - gx) <= 1 && abs(fy - gy) <= 1) one += A[stencil_slot(gx - fx, gy - fy) * nc + f];
+            for (int hx = max(max(fx, gx) - 1, 0); hx <= min(min(fx, gx) + 1, nx - 1); ++hx)
+                for (int hy = max(max(fy, gy) - 1, 0); hy <= min(min(fy, gy) + 1, ny - 1); ++hy) {
+                    const int h = hx * ny + hy;
+                    two += A[stencil_slot(hx - fx, hy - fy) * nc + f] * dinv[h] *
+                           A[stencil_slot(gx - hx, gy - hy) * nc + h];
                 }
-            }
         }
-#pragma unroll
-    for (int k = 0; k < MG_RW; ++k) R[k * ncc + C] = acc[k];
+    R[q] = own + (w0 * w1 * two - (w0 + w1) * one) * dinv[g];
 }
 
 // pre-smoothing of level l (blocks [0, nbs): two sweeps from zero, as
@@ -593,6 +586,170 @@ __global__ void __launch_bounds__(MG_BLOCK) k_mg_pre_restrict(int nx, int ny, co
         sum += R[k * ncc + C] * b[gx * ny + gy];
     }
     if (!mg_skip(sk)) bc[C] = sum;
+}
+
+// ---- the small levels as one dense operator ------------------------------------------
+// With two sweeps each way the V-cycle from level l down is linear in b_l:
+//   T_l = (I - w1 D^-1 A)(Z + wp D^-1 (I - A Z)) + w1 D^-1,   Z = S + s P T_{l+1} R,
+// S the two pre-sweeps from zero, R the restriction operator above, P the
+// injection, s the correction's scale, T at the coarsest level its inverse.
+// T is built once per matrix, level by level, one thread per entry, and the
+// V-cycle then takes all these levels as one product x = T b: its entries
+// come from L2 with every SM reading, where the levels' sweeps are a chain of
+// dependent phases on a grid too small to fill the GPU.  Per V-cycle on the
+// 13.6k-particle tank (1411 cells and below): 16 us for the level and the
+// single-CTA tail under it, 4 us for the product.
+// The line lies where a product costs what the level's own two launches and
+// the levels below cost: T grows with the square of the cells (1500 FP32
+// cells: 9 MB), and a level's launches hardly grow at all.
+constexpr int MG_DENSE_CELLS = 2048;
+constexpr int MG_DENSE_CELLS_F64 = 1536;
+constexpr int MG_DENSE_BLOCK = 256;
+
+// X = T_{l+1} R: column j (fine cell) takes the 3x3 coarse cells whose patch
+// holds it; XROWS rows per thread share its nine weights
+constexpr int XROWS = 8;
+template <typename T>
+__global__ void __launch_bounds__(MG_DENSE_BLOCK) k_mg_dense_x(int nx, int ny, int nxc, int nyc,
+                                                                const T* __restrict__ R, const T* __restrict__ Tc,
+                                                                int ldc, T* __restrict__ X, int ld) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x, ncc = nxc * nyc;
+    if (j >= nx * ny) return;
+    const int jx = j / ny, jy = j - jx * ny;
+    T wgt[9];
+    int at[9];
+#pragma unroll
+    for (int s = 0; s < 9; ++s) {
+        const int CX = (jx >> 1) + s / 3 - 1, CY = (jy >> 1) + s % 3 - 1;
+        const int px = jx - 2 * CX + 2, py = jy - 2 * CY + 2;
+        const bool in = CX >= 0 && CX < nxc && CY >= 0 && CY < nyc && px >= 0 && px < MG_RPATCH && py >= 0 &&
+                        py < MG_RPATCH;
+        at[s] = in ? CX * nyc + CY : 0;
+        wgt[s] = in ? R[(px * MG_RPATCH + py) * ncc + at[s]] : (T)0;
+    }
+    const int I1 = min((int)(blockIdx.y + 1) * XROWS, ncc);
+    for (int I = blockIdx.y * XROWS; I < I1; ++I) {
+        T sum = 0;
+#pragma unroll
+        for (int s = 0; s < 9; ++s) sum += wgt[s] * Tc[(int64_t)I * ldc + at[s]];
+        X[(int64_t)I * ld + j] = sum;
+    }
+}
+
+// entry (a, j) of the two pre-sweeps from zero: w0 D^-1 + w1 D^-1 (I - w0 A D^-1)
+template <typename T>
+__device__ __forceinline__ T dense_s(int nx, int ny, const T* A, const T* dinv, T w0, T w1, int ax, int ay, int jx,
+                                     int jy) {
+    const int dx = jx - ax, dy = jy - ay, a = ax * ny + ay, j = jx * ny + jy;
+    if (dx < -1 || dx > 1 || dy < -1 || dy > 1) return (T)0;
+    const T aij = A[stencil_slot(dx, dy) * (nx * ny) + a] * dinv[j];
+    return dinv[a] * ((a == j ? w0 + w1 : (T)0) - w0 * w1 * aij);
+}
+
+// row i of Z1 = Z + wp D^-1 (I - A Z), a block per row: the dense part
+// s P X through the (at most four) parents of the 3x3 cells around i, then
+// the entries within two cells of i
+template <typename T>
+__global__ void __launch_bounds__(MG_DENSE_BLOCK) k_mg_dense_z(int nx, int ny, int nyc, const T* __restrict__ A,
+                                                                const T* __restrict__ dinv, const T* __restrict__ X,
+                                                                int ld, T scale, T w0, T w1, T wp,
+                                                                T* __restrict__ Z) {
+    __shared__ T cf[4];     // weight of parent (base + (q / 2, q % 2)) in row i of P - wp D^-1 A P
+    __shared__ int row[4];  // its row of X
+    const int i = blockIdx.x, nc = nx * ny, ix = i / ny, iy = i - ix * ny;
+    const int bx = (ix - 1) >> 1, by = (iy - 1) >> 1;  // the lowest parent (may lie outside)
+    if (threadIdx.x < 4) {
+        const int q = threadIdx.x, X0 = bx + q / 2, Y0 = by + q % 2;
+        T c = 0;
+        bool used = false;
+        for (int s = 0; s < 9; ++s) {
+            const int gx = ix + s / 3 - 1, gy = iy + s % 3 - 1;
+            if (gx < 0 || gx >= nx || gy < 0 || gy >= ny || (gx >> 1) != X0 || (gy >> 1) != Y0) continue;
+            c -= wp * dinv[i] * A[s * nc + i];
+            if (s == 4) c += (T)1;
+            used = true;
+        }
+        cf[q] = scale * c;
+        row[q] = used ? X0 * nyc + Y0 : -1;
+    }
+    __syncthreads();
+    for (int j = threadIdx.x; j < nc; j += blockDim.x) {
+        T z = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (row[q] >= 0) z += cf[q] * X[(int64_t)row[q] * ld + j];
+        Z[(int64_t)i * ld + j] = z;
+    }
+    __syncthreads();
+    if (threadIdx.x < 25) {
+        const int jx = ix + threadIdx.x / 5 - 2, jy = iy + threadIdx.x % 5 - 2;
+        if (jx >= 0 && jx < nx && jy >= 0 && jy < ny) {
+            T az = 0;
+            for (int s = 0; s < 9; ++s) {
+                const int gx = ix + s / 3 - 1, gy = iy + s % 3 - 1;
+                if (gx < 0 || gx >= nx || gy < 0 || gy >= ny) continue;
+                az += A[s * nc + i] * dense_s<T>(nx, ny, A, dinv, w0, w1, gx, gy, jx, jy);
+            }
+            const int j = jx * ny + jy;
+            Z[(int64_t)i * ld + j] += dense_s<T>(nx, ny, A, dinv, w0, w1, ix, iy, jx, jy) +
+                                      wp * dinv[i] * ((i == j ? (T)1 : (T)0) - az);
+        }
+    }
+}
+
+// row i of T = Z1 + w1 D^-1 (I - A Z1), a block per row
+template <typename T>
+__global__ void __launch_bounds__(MG_DENSE_BLOCK) k_mg_dense_t(int nx, int ny, const T* __restrict__ A,
+                                                                const T* __restrict__ dinv, const T* __restrict__ Z,
+                                                                int ld, T w1, T* __restrict__ out) {
+    const int i = blockIdx.x, nc = nx * ny, ix = i / ny, iy = i - ix * ny;
+    const T wd = w1 * dinv[i];
+    T a[9];
+    int64_t at[9];
+#pragma unroll
+    for (int s = 0; s < 9; ++s) {
+        const int gx = ix + s / 3 - 1, gy = iy + s % 3 - 1;
+        const bool in = gx >= 0 && gx < nx && gy >= 0 && gy < ny;
+        a[s] = (in ? -wd * A[s * nc + i] : (T)0) + (s == 4 ? (T)1 : (T)0);
+        at[s] = (int64_t)(in ? gx * ny + gy : i) * ld;
+    }
+    for (int j = threadIdx.x; j < nc; j += blockDim.x) {
+        T t = j == i ? wd : (T)0;
+#pragma unroll
+        for (int s = 0; s < 9; ++s) t += a[s] * Z[at[s] + j];
+        out[(int64_t)i * ld + j] = t;
+    }
+}
+
+// x = T b, a warp per row
+template <typename T>
+__global__ void __launch_bounds__(MG_DENSE_BLOCK) k_mg_dense_apply(int nc, const T* __restrict__ M, int ld,
+                                                                    const T* __restrict__ b, T* __restrict__ x,
+                                                                    const Scalars* __restrict__ sk) {
+    constexpr int V = 16 / sizeof(T);  // entries per load
+    struct alignas(16) Vec { T v[V]; };
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= nc) return;
+    const T* row = M + (int64_t)i * ld;
+    T s[V] = {};
+    int j = 0;
+    if (ld % V == 0) {  // rows on 16-byte boundaries
+        const int full = nc / V;
+#pragma unroll 4
+        for (int q = lane; q < full; q += 32) {
+            const Vec m = reinterpret_cast<const Vec*>(row)[q], v = reinterpret_cast<const Vec*>(b)[q];
+#pragma unroll
+            for (int u = 0; u < V; ++u) s[u] += m.v[u] * v.v[u];
+        }
+        j = full * V;
+    }
+    for (j += lane; j < nc; j += 32) s[0] += row[j] * b[j];
+    T t = s[0];
+#pragma unroll
+    for (int u = 1; u < V; ++u) t += s[u];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0 && !mg_skip(sk)) x[i] = t;
 }
 
 // The small levels l0..nlev in one CTA: the same sweeps, restrictions, dense
@@ -884,6 +1041,21 @@ int cycle_level(Ctx* c, int l) {
     const T w = (T)c->mg_w[0], w1 = (T)c->mg_w[1], sc = (T)c->P.mg_scale;
     const T wp = c->mg_wpost > 0 ? (T)c->mg_wpost : w;
     const int nu = c->P.mg_sweeps, nup = c->mg_post[0] > 0 ? c->mg_post[0] : nu;
+    if (l >= mg.tail_l0 && mg.dense) {  // this level and all coarser ones as one product
+        const bool coarsest = l == mg.nlev;
+        const T* M = (const T*)L.T;
+        if (coarsest) {
+            if constexpr (sizeof(T) == 4)
+                M = mg.cinvf;
+            else
+                M = mg.cinv;
+        }
+        const unsigned gd = blocks_for(L.nc * 32, MG_DENSE_BLOCK);
+        k_mg_dense_apply<T><<<gd, MG_DENSE_BLOCK, 0, c->stream>>>((int)L.nc, M, coarsest ? (int)L.nc : L.ldT, v.b,
+                                                                   v.x, mg.skip);
+        BSC_LAUNCH(c);
+        return BSC_OK;
+    }
     if (l >= mg.tail_l0) {  // this level and all coarser ones in one CTA
         TailArgs<T> P{};
         P.l0 = l;
@@ -1049,6 +1221,41 @@ int mg_dalloc(Ctx* c, T** p, int64_t count) {
     return BSC_OK;
 }
 
+// the V-cycle is the one the dense operator stands for
+bool dense_cycle(const Ctx* c) {
+    return c->P.mg_sweeps == 2 && (c->mg_post[0] == 0 || c->mg_post[0] == 2) && !c->mg_cell4 && c->mg_tail_cells < 0;
+}
+
+// T of the levels tail_l0..nlev - 1, from the coarsest inverse up
+template <typename T>
+int dense_build(Ctx* c) {
+    Mg& mg = c->mg;
+    const T w = (T)c->mg_w[0], w1 = (T)c->mg_w[1], sc = (T)c->P.mg_scale;
+    const T wp = c->mg_wpost > 0 ? (T)c->mg_wpost : w;
+    T *X = (T*)mg.dx, *Z = (T*)mg.dz;
+    for (int l = mg.nlev - 1; l >= mg.tail_l0; --l) {
+        const MgLevel &F = mg.L[l], &C = mg.L[l + 1];
+        const Lv<T> v = level_view<T>(F);
+        const T* Tc = (const T*)C.T;
+        if (l + 1 == mg.nlev) {
+            if constexpr (sizeof(T) == 4)
+                Tc = mg.cinvf;
+            else
+                Tc = mg.cinv;
+        }
+        const int ld = F.ldT, B = MG_DENSE_BLOCK;
+        const dim3 gx(blocks_for(F.nc, B), blocks_for(C.nc, XROWS));
+        k_mg_dense_x<T><<<gx, B, 0, c->stream>>>(F.nx, F.ny, C.nx, C.ny, (const T*)F.R, Tc,
+                                                 l + 1 == mg.nlev ? (int)C.nc : C.ldT, X, ld);
+        BSC_LAUNCH(c);
+        k_mg_dense_z<T><<<(unsigned)F.nc, B, 0, c->stream>>>(F.nx, F.ny, C.ny, v.A, v.dinv, X, ld, sc, w, w1, wp, Z);
+        BSC_LAUNCH(c);
+        k_mg_dense_t<T><<<(unsigned)F.nc, B, 0, c->stream>>>(F.nx, F.ny, v.A, v.dinv, Z, ld, w1, (T*)F.T);
+        BSC_LAUNCH(c);
+    }
+    return BSC_OK;
+}
+
 // buffers for the grid, the row count, the restart length and the precision
 int mg_alloc(Ctx* c) {
     Mg& mg = c->mg;
@@ -1071,9 +1278,13 @@ int mg_alloc(Ctx* c) {
         ++nlev;
     }
     mg.nlev = nlev;
-    // one SM runs the tail: FP32 levels up to MG_TAIL_CELLS cells, FP64 ones
-    // up to MG_TAIL_CELLS_F64
-    int64_t tail_cells = f32 ? MG_TAIL_CELLS : MG_TAIL_CELLS_F64;
+    // the small levels as one dense product where the cycle has two sweeps
+    // each way on every level; other cycles (and BSC_MG_TAIL) take the
+    // single-CTA tail, FP32 levels up to MG_TAIL_CELLS cells, FP64 ones up to
+    // MG_TAIL_CELLS_F64
+    mg.dense = dense_cycle(c);
+    int64_t tail_cells = mg.dense ? (f32 ? MG_DENSE_CELLS : MG_DENSE_CELLS_F64)
+                                  : (f32 ? MG_TAIL_CELLS : MG_TAIL_CELLS_F64);
     if (c->mg_tail_cells >= 0) tail_cells = c->mg_tail_cells;
     mg.tail_l0 = nlev;
     while (mg.tail_l0 > 1 && (int64_t)mg.L[mg.tail_l0 - 1].nx * mg.L[mg.tail_l0 - 1].ny <= tail_cells)
@@ -1094,15 +1305,26 @@ int mg_alloc(Ctx* c) {
         L.y = vec + 2 * stride;
         L.t = vec + 3 * stride;
     }
-    for (int l = 1; l < mg.tail_l0; ++l)  // the restriction operators of the per-level kernels
+    // the restriction operators: of the per-level kernels, and of the dense levels
+    for (int l = 1; l < (mg.dense ? nlev : mg.tail_l0); ++l)
         if ((rc = mg_dalloc(c, (unsigned char**)&mg.L[l].R, (int64_t)MG_RW * mg.L[l + 1].nc * (int64_t)vs))) return rc;
     if ((rc = mg_dalloc(c, &mg.rowslots, 9 * n))) return rc;  // the level-1 Galerkin pass
     if (f32 && (rc = mg_dalloc(c, &mg.rowslotsf, 9 * n))) return rc;
     const int64_t nco = mg.L[nlev].nc;
     if ((rc = mg_dalloc(c, &mg.cinv, nco * nco))) return rc;
     if (f32 && (rc = mg_dalloc(c, &mg.cinvf, nco * nco))) return rc;
+    if (mg.dense && mg.tail_l0 < nlev) {
+        for (int l = mg.tail_l0; l < nlev; ++l) {
+            mg.L[l].ldT = (int)((mg.L[l].nc + 31) / 32 * 32);
+            if ((rc = mg_dalloc(c, (unsigned char**)&mg.L[l].T, mg.L[l].nc * mg.L[l].ldT * (int64_t)vs))) return rc;
+        }
+        const MgLevel& D = mg.L[mg.tail_l0];
+        if ((rc = mg_dalloc(c, (unsigned char**)&mg.dz, D.nc * D.ldT * (int64_t)vs)) ||
+            (rc = mg_dalloc(c, (unsigned char**)&mg.dx, mg.L[mg.tail_l0 + 1].nc * D.ldT * (int64_t)vs)))
+            return rc;
+    }
     // stage the tail in shared memory when it fits
-    {
+    if (!mg.dense) {
         int64_t nc[MG_MAX_LEVELS + 1] = {};
         for (int l = 1; l <= nlev; ++l) nc[l] = mg.L[l].nc;
         const int64_t bytes = f32 ? tail_words<float>(nc, mg.tail_l0, nlev, nullptr) * (int64_t)sizeof(float)
@@ -1180,19 +1402,21 @@ int mg_setup(Ctx* c) {
     else
         k_mg_dense_inverse<double><<<1, 1024, 0, c->stream>>>(Lc.nx, Lc.ny, Lc.A, mg.cinv);
     BSC_LAUNCH(c);
-    // the restriction operators of the levels swept by per-level kernels
+    // the restriction operators of the levels swept by per-level kernels, and
+    // of the dense ones, whose operator is built from them
     if (c->P.mg_sweeps == 2 && !c->mg_cell4)
-        for (int l = 1; l < mg.tail_l0; ++l) {
+        for (int l = 1; l < (mg.dense ? mg.nlev : mg.tail_l0); ++l) {
             const MgLevel &F = mg.L[l], &C = mg.L[l + 1];
-            const unsigned gb = blocks_for(C.nc, 128);
+            const unsigned gb = blocks_for(C.nc * MG_RW, 256);
             if (f32)
-                k_mg_build_R<float><<<gb, 128, 0, c->stream>>>(F.nx, F.ny, F.Af, F.dinvf, C.nx, C.ny,
+                k_mg_build_R<float><<<gb, 256, 0, c->stream>>>(F.nx, F.ny, F.Af, F.dinvf, C.nx, C.ny,
                                                                (float)c->mg_w[0], (float)c->mg_w[1], (float*)F.R);
             else
-                k_mg_build_R<double><<<gb, 128, 0, c->stream>>>(F.nx, F.ny, F.A, F.dinv, C.nx, C.ny, c->mg_w[0],
+                k_mg_build_R<double><<<gb, 256, 0, c->stream>>>(F.nx, F.ny, F.A, F.dinv, C.nx, C.ny, c->mg_w[0],
                                                                 c->mg_w[1], (double*)F.R);
             BSC_LAUNCH(c);
         }
+    if (mg.dense) return f32 ? dense_build<float>(c) : dense_build<double>(c);
     return BSC_OK;
 }
 
