@@ -41,6 +41,7 @@ struct State {
     int32_t* id;
 };
 constexpr int N_DBL_FIELDS = 28;
+constexpr int TICKET_WORDS = 128;  // Ctx::ticket
 
 // ---- neighbour list (ELL, 32-slot slices) ----------------------------------
 __host__ __device__ inline int64_t ell(int64_t i, int k, int kmax) {
@@ -321,7 +322,8 @@ struct Ctx {
     float* xbf = nullptr;         // best inner iterate (mixed)
     float* Zf = nullptr;          // FGMRES-IR preconditioned vectors, ir_m x cap (mixed)
     Scalars* sc2 = nullptr;       // FGMRES-IR outer scalars (h_sc[1] mirrors them)
-    unsigned* ticket = nullptr;   // last-block counter of the Krylov reductions (kept at 0 between launches)
+    unsigned* ticket = nullptr;   // TICKET_WORDS: [0] last-block counter of the Krylov reductions (kept at 0
+                                  // between launches), [64] the cooperative BiCGSTAB's barrier
     int ir_m = 0;
     // instantiated CUDA graphs of one batch of Krylov iterations, keyed by
     // the operator and vectors they were captured with

@@ -22,6 +22,9 @@
 // the start of each call; two calls whose work overlaps on the GPU (two
 // streams, or two host threads) race on the array, and on the one host-side
 // copy of the solver scalars, which is process-wide.
+#include <algorithm>
+
+#include "bicg_coop.cuh"
 #include "bsc_internal.cuh"
 
 namespace bsc {
@@ -31,17 +34,17 @@ constexpr size_t kVecBytes = (size_t)BSC_NOALLOC_MAX_ROWS * sizeof(double);
 constexpr size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
 // layout of the scratch array, every region on a 256-byte boundary
 constexpr size_t kOffWork = 0;                                        // r rh p v s t (6 vectors)
-constexpr size_t kOffPart = kOffWork + 6 * kVecBytes;                // partials, 8 x RED_GRID
-constexpr size_t kOffHd = kOffPart + round256(8 * RED_GRID * sizeof(double));  // residual norms
+constexpr size_t kOffPart = kOffWork + 6 * kVecBytes;                // partials of either BiCGSTAB
+constexpr size_t kOffHd = kOffPart + round256(std::max(8 * RED_GRID, COOP_SETS * (BSC_NOALLOC_MAX_ROWS / 32)) * sizeof(double));  // residual norms
 constexpr size_t kOffSc = kOffHd + round256(64 * sizeof(double));    // device scalars
-constexpr size_t kOffTicket = kOffSc + round256(sizeof(Scalars));    // last-block ticket
-constexpr size_t kScratchBytes = kOffTicket + 256;
+constexpr size_t kOffTicket = kOffSc + round256(sizeof(Scalars));    // last-block ticket, barrier word
+constexpr size_t kScratchBytes = kOffTicket + round256(TICKET_WORDS * sizeof(unsigned));
 
 Scalars g_host_scalars;  // host copy read between iteration batches (process-wide)
 
 }  // namespace
 
-// the scratch itself: about 6.3 MB of device memory on every device that
+// the scratch itself: about 6.5 MB of device memory on every device that
 // loads this module, held until the process exits
 static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
@@ -108,7 +111,7 @@ int bsc_csr_solve_noalloc(const bsc_params* p, int32_t n, const int32_t* rowptr,
     c.sc = reinterpret_cast<Scalars*>(base + kOffSc);
     c.ticket = reinterpret_cast<unsigned*>(base + kOffTicket);
     c.h_sc = &g_host_scalars;
-    // the array keeps the previous call's ticket and scalars: start from zero
+    // the array keeps the previous call's scalars, ticket and barrier word: start from zero
     if (cudaMemsetAsync(base + kOffSc, 0, kScratchBytes - kOffSc, c.stream) != cudaSuccess) {
         (void)cudaGetLastError();
         return BSC_E_CUDA;

@@ -28,6 +28,7 @@
 #include "bsc_internal.cuh"
 #include "dfloat.cuh"
 #include "ellop.cuh"
+#include "warpsum.cuh"
 
 namespace bsc {
 
@@ -365,6 +366,11 @@ struct CsrOp {
     const int32_t* col;
     const double* val;
     const void* key() const { return val; }
+    static constexpr bool UNIT_DIAG = false;
+    __device__ __forceinline__ int len(int64_t i) const { return rp[i + 1] - rp[i]; }
+    __device__ __forceinline__ int64_t at(int64_t i, int k) const { return rp[i] + k; }
+    __device__ __forceinline__ int32_t col_at(int64_t e) const { return col[e]; }
+    __device__ __forceinline__ double val_at(int64_t e) const { return val[e]; }
     template <typename X, typename A>
     __device__ __forceinline__ A row(int64_t i, const X* __restrict__ x) const {
         A s = 0;
@@ -400,39 +406,6 @@ __device__ __forceinline__ float warp_sum_to_lane0(float x) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
     return x;
-}
-
-// The warp sums of D values (D a power of two up to 32) at once.  While more
-// than one value is left, the two halves of the warp split the values
-// between them: at each step a lane keeps half of its values and adds what
-// its partner at distance o holds of them, so D values take
-// D - 1 + 5 - log2(D) adds instead of 5 D.  An FP64 instruction holds this
-// GPU's FP64 pipe for the whole warp however few lanes want its result, and
-// the shuffle adds bounded the multi-dot kernels (eight dots: 9 adds, 40
-// before).  Every value is summed over the same tree as warp_sum_to_lane0's
-// (each addition's operands at most exchanged): the same bits.  Returns value
-// `which` in the lanes that hold it (all lanes of a group of 32 / D; the
-// group's first lane is 32 / D * which).
-template <int D, typename V>
-__device__ __forceinline__ V warp_sums(V (&v)[D], int& which) {
-    const int lane = threadIdx.x & 31;
-    which = 0;
-#pragma unroll
-    for (int o = 16, m = D; o > 0; o >>= 1) {
-        if (m > 1) {
-            const bool up = lane & o;
-            m >>= 1;
-#pragma unroll
-            for (int q = 0; q < m; ++q) {
-                const V send = up ? v[q] : v[q + m], keep = up ? v[q + m] : v[q];
-                v[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-            }
-            which = 2 * which + (up ? 1 : 0);
-        } else {
-            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-        }
-    }
-    return v[0];
 }
 
 // per-block partial sums of D values into part[d * RED_GRID + block]; the
@@ -517,6 +490,7 @@ __global__ void k_bicg_setup(const double* __restrict__ part, int nb, Scalars* s
         sc->done = (sc->r0norm <= sc->target) ? 1 : 0;
         sc->breakdown = 0;
         sc->it = 0;
+        sc->tmp[7] = 0.0;
         sc->alpha = sc->omega = 1.0;
     }
 }
@@ -665,6 +639,10 @@ __global__ void __launch_bounds__(RED_BLOCK) k_bicg_5(int64_t n, T* __restrict__
         }
     }
 }
+
+}  // namespace bsc
+#include "bicg_coop.cuh"
+namespace bsc {
 
 // ============================================================================
 // FGMRES(m) with CGS2, value type T, basis V[(m+1) x n], Hessenberg on device
@@ -981,6 +959,61 @@ int graph_run(Ctx* c, const void* k0, const void* k1, const void* k2, int64_t n,
     return BSC_OK;
 }
 
+// The cooperative BiCGSTAB for n rows: its kernel, blocks (one per SM at
+// most; none where it cannot run: more than three rows per thread, or no
+// resident grid) and shared memory.  Up to there it is the faster at every
+// size; the five kernels keep the larger systems, the FP32 sweeps and the
+// per-kernel profiling.
+struct CoopPlan {
+    const void* kernel = nullptr;
+    int blocks = 0, threads = 0, smem = 0;
+};
+template <typename Op>
+CoopPlan coop_plan(int64_t n) {
+    CoopPlan P;
+    int sms = 0, optin = 0, coop = 0, dev = 0, per_sm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop) {
+        (void)cudaGetLastError();
+        return P;
+    }
+    // K rows per thread; and beyond RED_GRID blocks of rows the sums of the
+    // kernels it stands for take another order
+    const int64_t per = (int64_t)sms * COOP_BLOCK;
+    if (n > std::min<int64_t>(3 * per, (int64_t)RED_GRID * RED_BLOCK)) return P;
+    const int K = (int)((n + per - 1) / per);
+    const void* f = K == 1 ? (n <= MERGE_ROWS ? (const void*)k_bicg_coop<Op, true, 1>
+                                              : (const void*)k_bicg_coop<Op, false, 1>)
+                    : K == 2 ? (const void*)k_bicg_coop<Op, false, 2>
+                             : (const void*)k_bicg_coop<Op, false, 3>;
+    const int64_t warps = (n + 31) / 32;
+    const int blocks = (int)std::min<int64_t>(sms, warps);
+    const int threads = 32 * (int)((warps + (int64_t)blocks * K - 1) / ((int64_t)blocks * K));
+    cudaFuncAttributes fa{};
+    if (cudaFuncGetAttributes(&fa, f) != cudaSuccess) return (void)cudaGetLastError(), P;
+    const int smem = (optin - (int)fa.sharedSizeBytes) / COOP_ENTRY * COOP_ENTRY;
+    // the attribute is per function, process-wide: the device's maximum, whatever this call needs
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads, smem) != cudaSuccess || per_sm < 1)
+        return (void)cudaGetLastError(), P;
+    P = {f, blocks, threads, smem};
+    return P;
+}
+
+template <typename Op>
+cudaError_t bicg_coop_launch(Ctx* c, int64_t n, Op A, Work<double> w, int iters, const CoopPlan& P) {
+    unsigned* count = c->ticket + COOP_BAR;
+    if (cudaError_t e = cudaMemsetAsync(count, 0, sizeof(unsigned), c->stream)) return e;
+    int cap = P.smem / COOP_ENTRY;
+    const double* rh = w.rh;
+    // MERGE: p and v double-buffered, their second halves in s and t
+    void* args[] = {&n, &A, &w.x, &w.r, &rh, &w.p, &w.v, &w.s, &w.s, &w.t, &c->part, &c->sc, &count, &iters, &cap};
+    c->launches++;
+    return cudaLaunchCooperativeKernel(P.kernel, dim3(P.blocks), dim3(P.threads), args, (size_t)P.smem, c->stream);
+}
+
 // `xbest` (optional): keep the minimum-residual iterate there and stop a
 // diverging solve; *rr_out is then the squared best residual
 template <typename Op, typename T>
@@ -1019,6 +1052,9 @@ int run_bicgstab(Ctx* c, int64_t n, const Op& A, Work<T> w, double tol, int rel_
         if (pr) rec(c->ev_it[5]);
     };
     const int batch = batch_for(n);
+    CoopPlan coop;
+    if constexpr (sizeof(T) == 8)
+        if (!xbest && !c->prof_iter) coop = coop_plan<Op>(n);
     constexpr int kMaxRestarts = 8;
     int launched = 0, restarts = 0;
     for (;;) {
@@ -1034,6 +1070,21 @@ int run_bicgstab(Ctx* c, int64_t n, const Op& A, Work<T> w, double tol, int rel_
             BSC_LAUNCH(c);
             c->launches += 2;
             continue;
+        }
+        if (coop.blocks > 0) {  // the scalars carry on from launch to launch
+            if (h.tmp[7] != 0.0) return set_err(c, BSC_E_CUDA, "BiCGSTAB: a grid barrier's wait ran out");
+            if (h.done || h.breakdown || h.it >= maxit) break;
+            cudaError_t e = cudaSuccess;
+            if constexpr (sizeof(T) == 8)
+                e = bicg_coop_launch<Op>(c, n, A, w, std::min(COOP_ITERS, maxit - h.it), coop);
+            if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs than the device has: the kernels below
+                (void)cudaGetLastError();
+                coop.blocks = 0;
+            } else {
+                BSC_CUDA(c, e);
+                if (c->timing) timing_poll(c);  // while it runs
+                continue;
+            }
         }
         if (h.done || h.breakdown || h.it >= maxit || launched >= maxit) break;
         const int nb = std::min(batch, maxit - h.it);

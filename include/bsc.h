@@ -324,7 +324,7 @@ int bsc_csr_solve(const bsc_params* p, int32_t n, const int32_t* rowptr,
  *    entry and the solution on return.  Work is queued on `stream` (NULL: the
  *    legacy default stream) and the call returns once it has finished.
  *  - Nothing is allocated: the work vectors live in a fixed device array of
- *    the library sized for n <= BSC_NOALLOC_MAX_ROWS rows (about 6.3 MB).
+ *    the library sized for n <= BSC_NOALLOC_MAX_ROWS rows (about 6.5 MB).
  *    Larger n returns BSC_E_CAPACITY; host pointers, pointers into another
  *    device's memory, a solver other than BSC_SOLVER_BICGSTAB, or n <= 0
  *    return BSC_E_INVALID.
