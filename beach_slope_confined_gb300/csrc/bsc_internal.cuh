@@ -458,13 +458,14 @@ int op_probe_eta(Ctx* c, int np, const double* xp, double depth, double* eta);
 // ppe.cu
 int op_ppe_assemble(Ctx* c);
 int op_ppe_solve(Ctx* c, bsc_solve_info* info);
-// multigrid: build the hierarchy for the assembled PPE; apply one V-cycle
-// z = M v to an FP64 vector (FP64 or FP32 arithmetic); release the buffers
+// multigrid: build the hierarchy for the assembled PPE; normalise a Krylov
+// vector, v = src * mg.skip->tmp[4], and apply one V-cycle z = M v; release the
+// buffers
 int mg_setup(Ctx* c);
 void wc_free(Ctx* c);
 void snap_free(Ctx* c);
-int mg_vcycle_f64(Ctx* c, const double* v, double* z);
-int mg_vcycle_f32(Ctx* c, const float* v, float* z);
+int mg_vcycle_f64(Ctx* c, const double* src, double* v, double* z);
+int mg_vcycle_f32(Ctx* c, const float* src, float* v, float* z);
 void mg_free(Ctx* c);
 int fg_layout_size(int m);
 int csr_solve_device(Ctx* c, int32_t n, const int32_t* rp, const int32_t* col, const double* val,

@@ -27,8 +27,12 @@ struct EllOp {
     // the column stride of the ELL layout is 32 slots
     template <typename X, typename A>
     __device__ __forceinline__ A row(int64_t i, const X* __restrict__ x) const {
+        return row<X, A>(i, x, cnt[i]);
+    }
+    // with the row's entry count, loaded ahead of the caller's other loads
+    template <typename X, typename A>
+    __device__ __forceinline__ A row(int64_t i, const X* __restrict__ x, int m) const {
         A s = (A)x[i];
-        const int m = cnt[i];
         const int64_t e0 = ell(i, 0, kmax);
         int k = 0;
         for (; unroll && k + 8 <= m; k += 8) {
@@ -79,8 +83,12 @@ struct EllPack16 {
     const void* key() const { return ent; }
     template <typename X, typename A>
     __device__ __forceinline__ A row(int64_t i, const X* __restrict__ x) const {
+        return row<X, A>(i, x, cnt[i]);
+    }
+    // with the row's entry count, loaded ahead of the caller's other loads
+    template <typename X, typename A>
+    __device__ __forceinline__ A row(int64_t i, const X* __restrict__ x, int m) const {
         A s = (A)x[i];
-        const int m = cnt[i];
         const int64_t e0 = ell(i, 0, kmax);
         if (ok[i >> 5]) {
             const int64_t b = i & ~(int64_t)31;
@@ -119,8 +127,12 @@ struct EllPackF {
     const void* key() const { return ent; }
     template <typename X, typename A>
     __device__ __forceinline__ A row(int64_t i, const X* __restrict__ x) const {
+        return row<X, A>(i, x, cnt[i]);
+    }
+    // with the row's entry count, loaded ahead of the caller's other loads
+    template <typename X, typename A>
+    __device__ __forceinline__ A row(int64_t i, const X* __restrict__ x, int m) const {
         A s = (A)x[i];
-        const int m = cnt[i];
         const int64_t e0 = ell(i, 0, kmax);
         int k = 0;
         for (; k + 8 <= m; k += 8) {

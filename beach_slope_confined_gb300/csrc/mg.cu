@@ -910,42 +910,60 @@ __global__ void __launch_bounds__(MG_TAIL_THREADS) k_mg_tail(TailArgs<T> P) {
 }
 
 // ---- V-cycle, level 0 (the PPE, unit diagonal) ---------------------------------------
-// VI: type of the right-hand side v; O: type of the result z (the last sweep)
-// two sweeps from a zero guess: x1 = w v; x2 = x1 + w (v - A x1)
-template <typename T, typename VI, typename Op>
-__global__ void __launch_bounds__(MG_BLOCK) k_mg0_pre2(int64_t n, Op A, const VI* __restrict__ v, T w,
-                                                        T w1, T* __restrict__ x, const Scalars* __restrict__ sk) {
+// The entry counts load before the skip test's own loads return.
+// v = scale * src (the Krylov vector, normalised here rather than in a pass of
+// its own; scale is sc->tmp[4], the reciprocal of its norm), and two sweeps
+// from a zero guess: x1 = w v; x2 = x1 + w1 (v - A x1)
+template <typename T, typename Op>
+__global__ void __launch_bounds__(MG_BLOCK) k_mg0_pre2(int64_t n, Op A, const T* __restrict__ src, T* __restrict__ v,
+                                                        T w, T w1, T* __restrict__ x,
+                                                        const Scalars* __restrict__ sk) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int m = A.cnt[i];
+    const T si = src[i], scale = to_r<T>(sk->tmp[4]);
     if (mg_skip(sk)) return;
-    GRID_LOOP(i, n) {
-        const T Av = A.template row<VI, T>(i, v);
-        const T vi = (T)v[i];
-        x[i] = w * vi + w1 * (vi - w * Av);  // x1 = w v; x2 = x1 + w1 (v - A x1)
-    }
+    const T Av = scale * A.template row<T, T>(i, src, m);
+    const T vi = scale * si;
+    v[i] = vi;
+    x[i] = w * vi + w1 * (vi - w * Av);  // x1 = w v; x2 = x1 + w1 (v - A x1)
 }
 
-template <typename T, typename VI>
-__global__ void k_mg0_scale(int64_t n, const VI* __restrict__ v, T w, T* __restrict__ x,
+// the same with one sweep: x = w v
+template <typename T>
+__global__ void k_mg0_scale(int64_t n, const T* __restrict__ src, T* __restrict__ v, T w, T* __restrict__ x,
                             const Scalars* __restrict__ sk) {
-    if (mg_skip(sk)) return;
-    GRID_LOOP(i, n) x[i] = w * (T)v[i];
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n || mg_skip(sk)) return;
+    const T vi = to_r<T>(sk->tmp[4]) * src[i];
+    v[i] = vi;
+    x[i] = w * vi;
 }
 
 // x_out = x + w (v - A x)
-template <typename T, typename VI, typename O, typename Op>
-__global__ void __launch_bounds__(MG_BLOCK) k_mg0_sweep(int64_t n, Op A, const VI* __restrict__ v,
-                                                         const T* __restrict__ x, T w, O* __restrict__ xout,
+template <typename T, typename Op>
+__global__ void __launch_bounds__(MG_BLOCK) k_mg0_sweep(int64_t n, Op A, const T* __restrict__ v,
+                                                         const T* __restrict__ x, T w, T* __restrict__ xout,
                                                          const Scalars* __restrict__ sk) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int m = A.cnt[i];
+    const T vi = v[i], xi = x[i];
     if (mg_skip(sk)) return;
-    GRID_LOOP(i, n) xout[i] = (O)(x[i] + w * ((T)v[i] - A.template row<T, T>(i, x)));
+    xout[i] = xi + w * (vi - A.template row<T, T>(i, x, m));
 }
 
 // r = v - A x
-template <typename T, typename VI, typename Op>
-__global__ void __launch_bounds__(MG_BLOCK) k_mg0_resid(int64_t n, Op A, const VI* __restrict__ v,
+template <typename T, typename Op>
+__global__ void __launch_bounds__(MG_BLOCK) k_mg0_resid(int64_t n, Op A, const T* __restrict__ v,
                                                          const T* __restrict__ x, T* __restrict__ r,
                                                          const Scalars* __restrict__ sk) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int m = A.cnt[i];
+    const T vi = v[i];
     if (mg_skip(sk)) return;
-    GRID_LOOP(i, n) r[i] = (T)v[i] - A.template row<T, T>(i, x);
+    r[i] = vi - A.template row<T, T>(i, x, m);
 }
 
 // level-1 right-hand side: the residual summed over each cell's particles
@@ -953,13 +971,13 @@ template <typename T>
 __global__ void k_mg0_restrict(int64_t nc, const int32_t* __restrict__ cell_start, const int32_t* __restrict__ cell_count,
                                const int32_t* __restrict__ sorted, const T* __restrict__ r, T* __restrict__ b1,
                                const Scalars* __restrict__ sk) {
+    const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (c >= nc) return;
+    const int q0 = cell_start[c], qn = cell_count[c];
     if (mg_skip(sk)) return;
-    GRID_LOOP(c, nc) {
-        const int q0 = cell_start[c], qn = cell_count[c];
-        T s = 0;
-        for (int q = q0; q < q0 + qn; ++q) s += r[sorted[q]];
-        b1[c] = s;
-    }
+    T s = 0;
+    for (int q = q0; q < q0 + qn; ++q) s += r[sorted[q]];
+    b1[c] = s;
 }
 
 // First post-sweep, with the prolonged level-1 correction folded in and no
@@ -969,25 +987,25 @@ __global__ void k_mg0_restrict(int64_t nc, const int32_t* __restrict__ cell_star
 // rs_k(i) being row i's sums over its 3x3 neighbour cells (with the unit
 // diagonal), the same sums the level-1 Galerkin product is built from.
 // Reads 9 sums and 9 cell values per row instead of the row's entries.
-template <typename T, typename O>
+template <typename T>
 __global__ void __launch_bounds__(MG_BLOCK) k_mg0_post(int64_t n, int nx, int ny, const T* __restrict__ x,
                                                         const T* __restrict__ r, const T* __restrict__ x1,
                                                         const int32_t* __restrict__ pcell, const T* __restrict__ rs,
-                                                        T scale, T w, O* __restrict__ xout,
+                                                        T scale, T w, T* __restrict__ xout,
                                                         const Scalars* __restrict__ sk) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int c = pcell[i], cx = c / ny, cy = c - cx * ny;
+    const T xi = x[i], ri = r[i];
     if (mg_skip(sk)) return;
-    GRID_LOOP(i, n) {
-        const int c = pcell[i], cx = c / ny, cy = c - cx * ny;
-        T apx = 0;
+    T apx = 0;
 #pragma unroll
-        for (int s = 0; s < 9; ++s) {
-            const int gx = cx + s / 3 - 1, gy = cy + s % 3 - 1;
-            if (gx < 0 || gx >= nx || gy < 0 || gy >= ny) continue;
-            apx += rs[s * n + i] * x1[(int64_t)gx * ny + gy];
-        }
-        const T yi = x[i] + scale * x1[c];
-        xout[i] = (O)(yi + w * (r[i] - scale * apx));
+    for (int s = 0; s < 9; ++s) {
+        const int gx = cx + s / 3 - 1, gy = cy + s % 3 - 1;
+        if (gx < 0 || gx >= nx || gy < 0 || gy >= ny) continue;
+        apx += rs[s * n + i] * x1[(int64_t)gx * ny + gy];
     }
+    xout[i] = xi + scale * x1[c] + w * (ri - scale * apx);
 }
 
 template <typename T>
@@ -1147,9 +1165,9 @@ int cycle_level(Ctx* c, int l) {
     return BSC_OK;
 }
 
-// z = M v: V-cycle arithmetic in T, right-hand side in VI, result in O
-template <typename T, typename VI, typename O>
-int vcycle(Ctx* c, const VI* vin, O* z) {
+// v = src / ||src|| (by mg.skip->tmp[4]) and z = M v, all in T
+template <typename T>
+int vcycle(Ctx* c, const T* src, T* vin, T* z) {
     Mg& mg = c->mg;
     const int64_t n = c->n;
     using AV = typename FineOp<T>::type;  // the fine operator's type
@@ -1166,17 +1184,17 @@ int vcycle(Ctx* c, const VI* vin, O* z) {
     T* cur = P0;
     const int nupre = c->mg_pre_fine > 0 ? c->mg_pre_fine : nu;
     if (nupre == 1)
-        k_mg0_scale<T, VI><<<G, MG_BLOCK, 0, c->stream>>>(n, vin, w, cur, c->mg.skip);
+        k_mg0_scale<T><<<G, MG_BLOCK, 0, c->stream>>>(n, src, vin, w, cur, c->mg.skip);
     else
-        k_mg0_pre2<T, VI, AV><<<G, MG_BLOCK, 0, c->stream>>>(n, A, vin, w, w1, cur, c->mg.skip);
+        k_mg0_pre2<T, AV><<<G, MG_BLOCK, 0, c->stream>>>(n, A, src, vin, w, w1, cur, c->mg.skip);
     BSC_LAUNCH(c);
     for (int k = 2; k < nupre; ++k) {
         T* out = cur == P0 ? Q0 : P0;
-        k_mg0_sweep<T, VI, T, AV><<<G, MG_BLOCK, 0, c->stream>>>(n, A, vin, cur, w1, out, c->mg.skip);
+        k_mg0_sweep<T, AV><<<G, MG_BLOCK, 0, c->stream>>>(n, A, vin, cur, w1, out, c->mg.skip);
         BSC_LAUNCH(c);
         cur = out;
     }
-    k_mg0_resid<T, VI, AV><<<G, MG_BLOCK, 0, c->stream>>>(n, A, vin, cur, R0, c->mg.skip);
+    k_mg0_resid<T, AV><<<G, MG_BLOCK, 0, c->stream>>>(n, A, vin, cur, R0, c->mg.skip);
     BSC_LAUNCH(c);
     const MgLevel& L1 = mg.L[1];
     Lv<T> v1 = level_view<T>(L1);
@@ -1192,18 +1210,12 @@ int vcycle(Ctx* c, const VI* vin, O* z) {
     else
         rs = mg.rowslots;
     for (int k = 0; k < nup; ++k) {
-        const bool last = k == nup - 1;
-        T* out = cur == P0 ? Q0 : P0;
-        if (k == 0 && last)
-            k_mg0_post<T, O><<<G, MG_BLOCK, 0, c->stream>>>(n, L1.nx, L1.ny, cur, R0, v1.x, c->pcell, rs, sc, wp, z,
-                                                            c->mg.skip);
-        else if (k == 0)
-            k_mg0_post<T, T><<<G, MG_BLOCK, 0, c->stream>>>(n, L1.nx, L1.ny, cur, R0, v1.x, c->pcell, rs, sc, wp,
-                                                            out, c->mg.skip);
-        else if (last)
-            k_mg0_sweep<T, VI, O, AV><<<G, MG_BLOCK, 0, c->stream>>>(n, A, vin, cur, w1, z, c->mg.skip);
+        T* out = k == nup - 1 ? z : cur == P0 ? Q0 : P0;
+        if (k == 0)
+            k_mg0_post<T><<<G, MG_BLOCK, 0, c->stream>>>(n, L1.nx, L1.ny, cur, R0, v1.x, c->pcell, rs, sc, wp, out,
+                                                         c->mg.skip);
         else
-            k_mg0_sweep<T, VI, T, AV><<<G, MG_BLOCK, 0, c->stream>>>(n, A, vin, cur, w1, out, c->mg.skip);
+            k_mg0_sweep<T, AV><<<G, MG_BLOCK, 0, c->stream>>>(n, A, vin, cur, w1, out, c->mg.skip);
         BSC_LAUNCH(c);
         cur = out;
     }
@@ -1420,7 +1432,7 @@ int mg_setup(Ctx* c) {
     return BSC_OK;
 }
 
-int mg_vcycle_f64(Ctx* c, const double* v, double* z) { return vcycle<double, double, double>(c, v, z); }
-int mg_vcycle_f32(Ctx* c, const float* v, float* z) { return vcycle<float, float, float>(c, v, z); }
+int mg_vcycle_f64(Ctx* c, const double* src, double* v, double* z) { return vcycle<double>(c, src, v, z); }
+int mg_vcycle_f32(Ctx* c, const float* src, float* v, float* z) { return vcycle<float>(c, src, v, z); }
 
 }  // namespace bsc

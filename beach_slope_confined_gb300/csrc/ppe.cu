@@ -692,6 +692,7 @@ __global__ void k_fg_start(const double* __restrict__ part, int nb, Scalars* sc,
         sc->rr = v[0];
         sc->done = (beta <= sc->target) ? 1 : 0;
         sc->tmp[0] = beta;  // scale for v0
+        sc->tmp[4] = 1.0 / beta;  // (its reciprocal, for the multigrid cycles)
         sc->tmp[1] = 0.0;   // j (columns completed in this cycle)
         sc->tmp[2] = 0.0;   // cycle finished flag
         for (int k = 0; k <= F.m; ++k) Hd[F.g(k)] = 0.0;
@@ -1202,14 +1203,6 @@ __global__ void k_ir_norms(const double* __restrict__ part, int nb, double* out)
     }
 }
 
-__global__ void k_ir_add(int64_t n, double* __restrict__ x, const float* __restrict__ d) {
-    GRID_LOOP(i, n) x[i] += (double)d[i];
-}
-
-__global__ void k_copy_f64(int64_t n, const double* __restrict__ a, double* __restrict__ b) {
-    GRID_LOOP(i, n) b[i] = a[i];
-}
-
 // ---- FGMRES-IR pieces (mixed path) ----------------------------------------------
 __global__ void k_d2f(int64_t n, const double* __restrict__ a, float* __restrict__ b) {
     GRID_LOOP(i, n) b[i] = (float)a[i];
@@ -1393,6 +1386,210 @@ int fg_cycle(Ctx* c, int m, int budget, Scalars* h, int* iters, Q queue) {
     }
 }
 
+// ============================================================================
+// Gram-Schmidt of the multigrid-preconditioned FGMRES, either precision T
+// ============================================================================
+// One classical pass in two kernels: the dots h_i = V_i . w (with the SpMV
+// w = A z that they follow in the same kernel while every row has a thread of
+// the reduction grid), and the update w -= sum h_i V_i with its norm and the
+// Givens step.  The next basis vector is not written here: the V-cycle's
+// first pass scales w by the reciprocal of the norm (sc->tmp[4]).
+// What bounds them on systems below ~10^5 rows is the chain of dependent
+// steps, FP64 ones above all (~140 clocks each here): hence the finishing
+// block's four partial sums per lane, the earlier rotations of the column in
+// a block of their own beside the update, and one division for the reciprocal
+// of the norm (k_fg_next divided once per thread: 5 us at any size).
+// Measured per iteration, the SpMV and the timing events around it included:
+// 3816 rows FP64 33 us before, 24 now; 13.6k rows mixed 30 and 24; 198k FP64
+// 62 and 52; 846k mixed 71 and 65, FP64 119 and 117.
+
+// column j of the dots from the blocks' partials, one warp per dot; by the
+// last block to finish
+__device__ __forceinline__ void gs_finish_dots(const double* part, int nb, int j, double* Hd, FgLayout F) {
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int i = wp; i <= j; i += nw) {
+        const double* q = part + (int64_t)i * RED_GRID;
+        double x[4] = {0.0, 0.0, 0.0, 0.0};
+        int k = lane;
+        for (; k + 96 < nb; k += 128) {
+            double y[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) y[u] = __ldcg(q + k + 32 * u);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) x[u] += y[u];
+        }
+        for (; k < nb; k += 32) x[0] += __ldcg(q + k);
+        const double y = warp_sum_to_lane0((x[0] + x[1]) + (x[2] + x[3]));
+        if (lane == 0) Hd[F.hc(i)] = y;
+    }
+}
+
+// true in every thread of the block that arrives last (all blocks call it once)
+__device__ __forceinline__ bool gs_last_block(unsigned* ticket) {
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (last) {
+        __threadfence();
+        if (threadIdx.x == 0) *ticket = 0u;
+    }
+    return last;
+}
+
+// the dots of w, 8 columns per pass, summed per thread in T; SPMV: w = A z
+// first (one row per thread: n <= gridDim.x * RED_BLOCK)
+template <bool SPMV, typename T, typename Op>
+__global__ void __launch_bounds__(RED_BLOCK) k_gs_dots(int64_t n, Op A, const T* __restrict__ z,
+                                                        const T* __restrict__ V, T* __restrict__ w, int j,
+                                                        double* __restrict__ part, const Scalars* __restrict__ sc,
+                                                        unsigned* __restrict__ ticket, double* Hd, FgLayout F) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int m = SPMV && i < n ? A.cnt[i] : 0;  // loads before the skip test's own return
+    if (fg_skip(sc)) return;
+    T wi = 0;
+    if (SPMV && i < n) {
+        wi = A.template row<T, T>(i, z, m);
+        w[i] = wi;
+    }
+    for (int i0 = 0; i0 <= j; i0 += 8) {
+        T acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        const int cntv = min(8, j + 1 - i0);
+        if (SPMV) {
+            if (i < n)
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    if (q < cntv) acc[q] = V[(int64_t)(i0 + q) * n + i] * wi;
+        } else {
+            GRID_LOOP(k, n) {
+                const T wk = w[k];
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    if (q < cntv) acc[q] += V[(int64_t)(i0 + q) * n + k] * wk;
+            }
+        }
+        block_partials<8>(acc, part + (int64_t)i0 * RED_GRID);
+        __syncthreads();
+    }
+    if (gs_last_block(ticket)) gs_finish_dots(part, (int)gridDim.x, j, Hd, F);
+}
+
+// w -= sum_i h_i V_i and its norm.  The last block of the grid has no rows: it
+// applies the earlier rotations to the column meanwhile.  The block that
+// finishes last takes the column's own rotation, the residual estimate and
+// the cycle's control (h(j+1,j) = ||w||) and copies the scalars to the host
+// mirror.
+template <typename T>
+__global__ void __launch_bounds__(RED_BLOCK) k_gs_update(int64_t n, const T* __restrict__ V, T* __restrict__ w, int j,
+                                                          double* Hd, FgLayout F, double* __restrict__ part,
+                                                          Scalars* sc, unsigned* __restrict__ ticket,
+                                                          Scalars* mirror) {
+    const int rows = (int)gridDim.x - 1;  // blocks with rows
+    if (fg_skip(sc)) {  // the cycle has stopped: publish the scalars all the same
+        if (mirror && blockIdx.x == 0 && threadIdx.x == 0) *mirror = *sc;
+        return;
+    }
+    const int t = threadIdx.x;
+    if ((int)blockIdx.x == rows) {
+        __shared__ double hs[FG_MAXM], csv[FG_MAXM], snv[FG_MAXM];
+        for (int i = t; i <= j; i += blockDim.x) hs[i] = Hd[F.hc(i)];
+        for (int i = t; i < j; i += blockDim.x) {
+            csv[i] = Hd[F.cs(i)];
+            snv[i] = Hd[F.sn(i)];
+        }
+        __syncthreads();
+        if (t == 0)
+            for (int i = 0; i < j; ++i) {
+                const double a = hs[i], c = hs[i + 1];
+                hs[i] = csv[i] * a + snv[i] * c;
+                hs[i + 1] = -snv[i] * a + csv[i] * c;
+            }
+        __syncthreads();
+        for (int i = t; i <= j; i += blockDim.x) Hd[F.H(i, j)] = hs[i];
+    } else {
+        __shared__ T h[FG_MAXM];
+        for (int i = t; i <= j; i += blockDim.x) h[i] = (T)Hd[F.hc(i)];
+        __syncthreads();
+        T acc = 0;
+        for (int64_t k = blockIdx.x * (int64_t)blockDim.x + t; k < n; k += (int64_t)rows * blockDim.x) {
+            T s = w[k], s1 = 0;  // two chains
+            int i = 0;
+            for (; i + 4 <= j + 1; i += 4) {
+                T y[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) y[u] = V[(int64_t)(i + u) * n + k];
+                s -= h[i] * y[0];
+                s1 -= h[i + 1] * y[1];
+                s -= h[i + 2] * y[2];
+                s1 -= h[i + 3] * y[3];
+            }
+            for (; i <= j; ++i) s -= h[i] * V[(int64_t)i * n + k];
+            s += s1;
+            w[k] = s;
+            acc += s * s;
+        }
+        T a[1] = {acc};
+        block_partials<1>(a, part);
+    }
+    if (!gs_last_block(ticket)) return;
+    double v[1];
+    reduce_partials<1>(part, rows, v);
+    if (t == 0) {
+        const double a = __ldcg(Hd + F.H(j, j));
+        const double hn = sqrt(v[0]), den = sqrt(a * a + v[0]);
+        sc->it += 1;
+        sc->tmp[1] = (double)(j + 1);
+        if (den == 0.0) {
+            sc->breakdown = 1;
+            sc->tmp[1] = (double)j;
+            sc->tmp[2] = 1.0;
+        } else {
+            const double cs = a / den, sn = hn / den;
+            const double gj = Hd[F.g(j)], gn = -sn * gj;
+            Hd[F.cs(j)] = cs;
+            Hd[F.sn(j)] = sn;
+            Hd[F.H(j, j)] = den;
+            Hd[F.H(j + 1, j)] = 0.0;
+            Hd[F.g(j + 1)] = gn;
+            Hd[F.g(j)] = cs * gj;
+            sc->tmp[3] = hn;
+            sc->tmp[4] = 1.0 / hn;
+            if (fabs(gn) <= sc->target || hn == 0.0 || j + 1 == F.m) sc->tmp[2] = 1.0;
+        }
+        if (mirror) *mirror = *sc;
+    }
+}
+
+// one iteration's Krylov work after the V-cycle
+template <typename T, typename Op>
+int gs_iteration(Ctx* c, int64_t n, const Op& A, const T* z, T* V, T* w, int j, FgLayout F, Scalars* sc,
+                 Scalars* mirror) {
+    const int G = red_blocks(n), B = RED_BLOCK;
+    const bool fused = n <= (int64_t)RED_GRID * RED_BLOCK;
+    // the first column's SpMV is bracketed by events, the dominant HBM-bound
+    // kernel timed in place (a kernel of its own there)
+    const bool timed = c->timing && j == 0;
+    if (timed || !fused) {
+        if (timed) record_event(c, c->ev_spmv[2]);
+        k_spmv<T, Op><<<blocks_for(n, B), B, 0, c->stream>>>(n, A, z, w, sc);
+        if (timed) record_event(c, c->ev_spmv[3]);
+        c->launches++;
+    }
+    if (c->prof_iter) record_event(c, c->ev_it[4]);
+    if (timed || !fused)
+        k_gs_dots<false, T, Op><<<G, B, 0, c->stream>>>(n, A, z, V, w, j, c->part, sc, c->ticket, c->Hd, F);
+    else
+        k_gs_dots<true, T, Op><<<G, B, 0, c->stream>>>(n, A, z, V, w, j, c->part, sc, c->ticket, c->Hd, F);
+    k_gs_update<T><<<G + 1, B, 0, c->stream>>>(n, V, w, j, c->Hd, F, c->part, sc, c->ticket, mirror);
+    if (c->prof_iter) record_event(c, c->ev_it[5]);
+    c->launches += 2;
+    BSC_CUDA(c, cudaGetLastError());
+    return BSC_OK;
+}
+
 // Flexible GMRES(m) in FP64 on the FP64 operator, right-preconditioned by
 // one FP64 multigrid V-cycle per iteration (mg.cu).  Each iteration runs as a
 // cached CUDA graph, one per Krylov column.  Stops on the Arnoldi residual
@@ -1410,6 +1607,7 @@ int run_fgmres_mg(Ctx* c, int64_t n, bsc_solve_info* si) {
     double* V = mg.V;
     double* Z = mg.Z;
     int first = 1, iters = 0, rc;
+    double rnorm = 0.0;
     for (;;) {
         k_resid<EllOp<double>, double><<<G, B, 0, c->stream>>>(n, A, x, c->b, c->r, c->part);
         BSC_LAUNCH(c);
@@ -1417,38 +1615,18 @@ int run_fgmres_mg(Ctx* c, int64_t n, bsc_solve_info* si) {
         BSC_LAUNCH(c);
         first = 0;
         if ((rc = fetch_outer(c))) return rc;
+        rnorm = c->h_sc[1].tmp[0];  // ||b - A x||
         if (c->h_sc[1].done || iters >= P.maxit) break;
-        k_fg_v0<double><<<G, B, 0, c->stream>>>(n, c->r, V, c->sc2);
-        BSC_LAUNCH(c);
         mg.skip = c->sc2;
         rc = fg_cycle(c, m, P.maxit, c->h_sc + 1, &iters, [&](int j, Scalars* mirror) -> int {
             double* zj = Z + (int64_t)j * n;
-            const double* vj = V + (int64_t)j * n;
+            double* vj = V + (int64_t)j * n;
             // one iteration (V-cycle, SpMV, Gram-Schmidt, Givens) as a cached graph per
             // column j, keyed by the cell map too, whose buffer a Morton
             // reorder swaps
             return graph_run(c, c->pcell, vj, zj, n, [&]() -> int {
-                if (int r = mg_vcycle_f64(c, vj, zj)) return r;
-                // the first column's SpMV w = A z_j is bracketed by events: the
-                // dominant HBM-bound kernel, timed in place
-                if (c->timing && j == 0) record_event(c, c->ev_spmv[2]);
-                k_spmv_z<double><<<blocks_for(n, B), B, 0, c->stream>>>(n, A, zj, w, c->sc2);
-                if (c->timing && j == 0) record_event(c, c->ev_spmv[3]);
-                if (c->prof_iter) record_event(c, c->ev_it[4]);
-                // separate single-block kernels for the column of H and the
-                // Givens step: in FP64 the fused last-block forms (as on the
-                // mixed path) measured slower, 122 against 107 us per
-                // iteration at 846k rows (their last block has a quarter of
-                // k_fg_hcol's warps)
-                k_fg_mdot<double><<<G, B, 0, c->stream>>>(n, V, w, j, c->part, c->sc2);
-                k_fg_hcol<<<1, 1024, 0, c->stream>>>(c->part, G, c->Hd, F, j, 0, c->sc2);
-                k_fg_maxpy<double><<<G, B, 0, c->stream>>>(n, V, w, j, c->Hd, F, 1, c->part, c->sc2);
-                k_fg_givens<<<1, B, 0, c->stream>>>(c->part, G, c->sc2, c->Hd, F, j, mirror);
-                k_fg_next<double><<<G, B, 0, c->stream>>>(n, w, V, j, c->sc2);
-                if (c->prof_iter) record_event(c, c->ev_it[5]);
-                c->launches += 6;
-                BSC_CUDA(c, cudaGetLastError());
-                return BSC_OK;
+                if (int r = mg_vcycle_f64(c, j == 0 ? c->r : w, vj, zj)) return r;
+                return gs_iteration<double>(c, n, A, zj, V, w, j, F, c->sc2, mirror);
             });
         });
         mg.skip = nullptr;
@@ -1459,14 +1637,8 @@ int run_fgmres_mg(Ctx* c, int64_t n, bsc_solve_info* si) {
         BSC_CUDA(c, cudaGetLastError());
         if (c->h_sc[1].breakdown && c->h_sc[1].tmp[1] == 0.0) break;
     }
-    double* norms = c->Hd + F.size();
-    k_resid<EllOp<double>, double><<<G, B, 0, c->stream>>>(n, A, x, c->b, c->r, c->part);
-    BSC_LAUNCH(c);
-    k_ir_norms<<<1, B, 0, c->stream>>>(c->part, G, norms);
-    BSC_LAUNCH(c);
-    double nrm[2];
-    BSC_CUDA(c, cudaMemcpyAsync(nrm, norms, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    BSC_CUDA(c, cudaStreamSynchronize(c->stream));
+    // x has not moved since the loop's last residual
+    const double nrm[2] = {rnorm, c->h_sc[1].bnorm};
     si->iterations = iters;
     si->outer = 1;
     si->b_norm = c->h_sc[1].bnorm;
@@ -1489,129 +1661,6 @@ __global__ void __launch_bounds__(RED_BLOCK) k_norm2f(int64_t n, const float* __
     GRID_LOOP(i, n) acc += r[i] * r[i];
     float a[2] = {acc, acc};
     block_partials<2>(a, part);
-}
-
-__global__ void k_fgf_v0(int64_t n, const float* __restrict__ r, float* __restrict__ V0,
-                         const Scalars* __restrict__ sc) {
-    if (sc->done) return;
-    const float inv = (float)(1.0 / sc->tmp[0]);
-    GRID_LOOP(i, n) V0[i] = r[i] * inv;
-}
-
-__global__ void k_fgf_next(int64_t n, const float* __restrict__ w, float* __restrict__ V, int j,
-                           const Scalars* __restrict__ sc) {
-    if (fg_skip(sc)) return;
-    const float inv = (float)(1.0 / sc->tmp[3]);
-    float* vn = V + (int64_t)(j + 1) * n;
-    GRID_LOOP(i, n) vn[i] = w[i] * inv;
-}
-
-__global__ void __launch_bounds__(RED_BLOCK) k_spmv_f(int64_t n, EllPackF A, const float* __restrict__ z,
-                                                       float* __restrict__ w, const Scalars* __restrict__ sc) {
-    if (fg_skip(sc)) return;
-    GRID_LOOP(i, n) w[i] = A.template row<float, float>(i, z);
-}
-
-// h_i = V_i . w for i <= j, 8 columns per pass, summed per thread in T; the
-// block that finishes last (ticket taken after a fence) sums the partials
-// into column j of H, one warp per dot in lane order as k_fg_hcol does
-template <typename T>
-__global__ void __launch_bounds__(RED_BLOCK) k_fgf_mdot(int64_t n, const T* __restrict__ V,
-                                                         const T* __restrict__ w, int j,
-                                                         double* __restrict__ part, const Scalars* __restrict__ sc,
-                                                         unsigned* __restrict__ ticket, double* Hd, FgLayout F) {
-    if (fg_skip(sc)) return;
-    for (int i0 = 0; i0 <= j; i0 += 8) {
-        T acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        const int cntv = min(8, j + 1 - i0);
-        GRID_LOOP(k, n) {
-            const T wk = w[k];
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-                if (q < cntv) acc[q] += V[(int64_t)(i0 + q) * n + k] * wk;
-        }
-        block_partials<8>(acc, part + (int64_t)i0 * RED_GRID);
-        __syncthreads();
-    }
-    __shared__ bool last;
-    if (threadIdx.x == 0) {
-        __threadfence();
-        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int i = wp; i <= j; i += nw) {
-        double x = 0.0;
-        for (int k = lane; k < (int)gridDim.x; k += 32) x += __ldcg(part + (int64_t)i * RED_GRID + k);
-        x = warp_sum_to_lane0(x);
-        if (lane == 0) {
-            Hd[F.hc(i)] = x;
-            Hd[F.H(i, j)] = x;
-        }
-    }
-    if (threadIdx.x == 0) *ticket = 0u;
-}
-
-// w -= sum_i h_i V_i and the partials of w.w; the block that finishes last
-// runs the Givens step of k_fg_givens (h(j+1,j) = ||w||, rotations,
-// residual estimate) and copies the scalars to the host mirror
-template <typename T>
-__global__ void __launch_bounds__(RED_BLOCK) k_fgf_maxpy_givens(int64_t n, const T* __restrict__ V,
-                                                                 T* __restrict__ w, int j, double* Hd, FgLayout F,
-                                                                 double* __restrict__ part, Scalars* sc,
-                                                                 unsigned* __restrict__ ticket, Scalars* mirror) {
-    if (fg_skip(sc)) {  // the cycle has stopped: publish the scalars as k_fg_givens does
-        if (mirror && blockIdx.x == 0 && threadIdx.x == 0) *mirror = *sc;
-        return;
-    }
-    __shared__ T h[FG_MAXM];
-    for (int i = threadIdx.x; i <= j; i += blockDim.x) h[i] = (T)Hd[F.hc(i)];
-    __syncthreads();
-    T acc = 0;
-    GRID_LOOP(k, n) {
-        T s = w[k];
-        for (int i = 0; i <= j; ++i) s -= h[i] * V[(int64_t)i * n + k];
-        w[k] = s;
-        acc += s * s;
-    }
-    T a[1] = {acc};
-    block_partials<1>(a, part);
-    __shared__ bool last;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    fg_givens(part, (int)gridDim.x, sc, Hd, F, j);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        *ticket = 0u;
-        if (mirror) *mirror = *sc;
-    }
-}
-
-// w -= sum_i h_i V_i; partial (w.w) when `norm`
-__global__ void __launch_bounds__(RED_BLOCK) k_fgf_maxpy(int64_t n, const float* __restrict__ V, float* __restrict__ w,
-                                                          int j, const double* __restrict__ Hd, FgLayout F, int norm,
-                                                          double* __restrict__ part, const Scalars* __restrict__ sc) {
-    if (fg_skip(sc)) return;
-    __shared__ float h[FG_MAXM];
-    for (int i = threadIdx.x; i <= j; i += blockDim.x) h[i] = (float)Hd[F.hc(i)];
-    __syncthreads();
-    float acc = 0.f;
-    GRID_LOOP(k, n) {
-        float s = w[k];
-        for (int i = 0; i <= j; ++i) s -= h[i] * V[(int64_t)i * n + k];
-        w[k] = s;
-        acc += s * s;
-    }
-    float a[1] = {acc};
-    if (norm) block_partials<1>(a, part);
 }
 
 // x += sum_i y_i z_i (FP64 pressure, FP32 preconditioned vectors)
@@ -1645,6 +1694,7 @@ int run_fgmres_ir_mg(Ctx* c, int64_t n, bsc_solve_info* si) {
     // to deliver; the FP64 outer loop compounds the reductions
     const double floor_tol = std::min(std::max(P.inner_tol, 1e-7), 0.5);
     int first = 1, outer = 0, inner = 0, rc;
+    double rnorm = 0.0;
     for (;;) {
         k_resid<EllOp<double>, double><<<G, B, 0, c->stream>>>(n, A, x, c->b, c->r, c->part);
         BSC_LAUNCH(c);
@@ -1652,6 +1702,7 @@ int run_fgmres_ir_mg(Ctx* c, int64_t n, bsc_solve_info* si) {
         BSC_LAUNCH(c);
         first = 0;
         if ((rc = fetch_outer(c))) return rc;
+        rnorm = c->h_sc[1].tmp[0];  // ||b - A x||
         if (c->h_sc[1].done || outer >= P.max_outer || inner >= P.maxit) break;
         ++outer;
         const double beta = c->h_sc[1].tmp[0], need = c->h_sc[1].target / beta;
@@ -1660,31 +1711,15 @@ int run_fgmres_ir_mg(Ctx* c, int64_t n, bsc_solve_info* si) {
         k_d2f<<<G, B, 0, c->stream>>>(n, c->r, rf);
         k_norm2f<<<G, B, 0, c->stream>>>(n, rf, c->part);
         k_fg_start<<<1, B, 0, c->stream>>>(c->part, G, c->sc, c->Hd, F, 1, inner_tol, 1);
-        k_fgf_v0<<<G, B, 0, c->stream>>>(n, rf, V, c->sc);
-        c->launches += 4;
+        c->launches += 3;
         mg.skip = c->sc;
         rc = fg_cycle(c, m, P.maxit, c->h_sc, &inner, [&](int j, Scalars* mirror) -> int {
             float* zj = Z + (int64_t)j * n;
-            const float* vj = V + (int64_t)j * n;
+            float* vj = V + (int64_t)j * n;
             // one inner iteration as a cached graph per column j (and cell map)
             return graph_run(c, c->pcell, vj, zj, n, [&]() -> int {
-                if (int r = mg_vcycle_f32(c, vj, zj)) return r;
-                // the first column's FP32 SpMV w = A z_j is bracketed by events
-                // (the dominant HBM-bound kernel, timed in place)
-                if (c->timing && j == 0) record_event(c, c->ev_spmv[2]);
-                k_spmv_f<<<blocks_for(n, B), B, 0, c->stream>>>(n, Af, zj, w, c->sc);
-                if (c->timing && j == 0) record_event(c, c->ev_spmv[3]);
-                if (c->prof_iter) record_event(c, c->ev_it[4]);
-                // the column of H and the Givens step finish in the last
-                // block of the dot and update kernels (no single-block launches)
-                k_fgf_mdot<float><<<G, B, 0, c->stream>>>(n, V, w, j, c->part, c->sc, c->ticket, c->Hd, F);
-                k_fgf_maxpy_givens<float><<<G, B, 0, c->stream>>>(n, V, w, j, c->Hd, F, c->part, c->sc, c->ticket,
-                                                                  mirror);
-                k_fgf_next<<<G, B, 0, c->stream>>>(n, w, V, j, c->sc);
-                if (c->prof_iter) record_event(c, c->ev_it[5]);
-                c->launches += 4;
-                BSC_CUDA(c, cudaGetLastError());
-                return BSC_OK;
+                if (int r = mg_vcycle_f32(c, j == 0 ? rf : w, vj, zj)) return r;
+                return gs_iteration<float>(c, n, Af, zj, V, w, j, F, c->sc, mirror);
             });
         });
         mg.skip = nullptr;
@@ -1697,14 +1732,8 @@ int run_fgmres_ir_mg(Ctx* c, int64_t n, bsc_solve_info* si) {
             std::fprintf(stderr, "[bsc] FGMRES-IR outer %d: |r|/target %.3e, inner tol %.1e, %d inner iterations\n",
                          outer, beta / c->h_sc[1].target, inner_tol, inner);
     }
-    double* norms = c->Hd + F.size();
-    k_resid<EllOp<double>, double><<<G, B, 0, c->stream>>>(n, A, x, c->b, c->r, c->part);
-    BSC_LAUNCH(c);
-    k_ir_norms<<<1, B, 0, c->stream>>>(c->part, G, norms);
-    BSC_LAUNCH(c);
-    double nrm[2];
-    BSC_CUDA(c, cudaMemcpyAsync(nrm, norms, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    BSC_CUDA(c, cudaStreamSynchronize(c->stream));
+    // x has not moved since the loop's last residual
+    const double nrm[2] = {rnorm, c->h_sc[1].bnorm};
     si->iterations = inner;
     si->outer = outer;
     si->b_norm = c->h_sc[1].bnorm;
