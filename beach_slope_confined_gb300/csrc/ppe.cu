@@ -1403,6 +1403,17 @@ int fg_cycle(Ctx* c, int m, int budget, Scalars* h, int* iters, Q queue) {
 // 3816 rows FP64 33 us before, 24 now; 13.6k rows mixed 30 and 24; 198k FP64
 // 62 and 52; 846k mixed 71 and 65, FP64 119 and 117.
 
+// w = A z, one row per thread
+template <typename T, typename Op>
+__global__ void __launch_bounds__(RED_BLOCK) k_spmv(int64_t n, Op A, const T* __restrict__ z, T* __restrict__ w,
+                                                     const Scalars* __restrict__ sc) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int m = A.cnt[i];
+    if (fg_skip(sc)) return;
+    w[i] = A.template row<T, T>(i, z, m);
+}
+
 // column j of the dots from the blocks' partials, one warp per dot; by the
 // last block to finish
 __device__ __forceinline__ void gs_finish_dots(const double* part, int nb, int j, double* Hd, FgLayout F) {
