@@ -44,6 +44,8 @@ namespace bsc {
 
 struct WcK {
     double rho0, B, gam, inv_gam, grav_c, ys;  // EOS; rhoH(y) = rho0 (1 + grav_c (ys - y))^(1/gamma)
+    int igam;                                  // gamma where it is a whole number of 1..EOS_MAX, else 0
+    double binom[8];                           // then binom(gamma, k + 1): (1 + t)^gamma - 1 = t (binom[0] + t (...))
     double c2;                                 // delta 2h c0
     double nu, lam, g, dt, d50, H2;
     double alpha, beta;
@@ -62,7 +64,7 @@ struct WcState {
     double* mass = nullptr;                    // particle masses rho_init dl^2
     double *theta = nullptr, *sw = nullptr;    // grid porosities; (1 - phi_s) V_s
     int32_t* sg = nullptr;                     // solid -> grid cell or -1
-    double *rt = nullptr, *pp = nullptr, *rh = nullptr, *drh = nullptr;  // per step
+    double *rt = nullptr, *pp = nullptr, *ex = nullptr, *drh = nullptr;  // per step
     double *vol = nullptr, *pr = nullptr;      // m/rt, p/rt^2 (per step)
     double* dpdr = nullptr;                    // dp/drt (per step)
     double* nxt = nullptr;                     // next state (5n)
@@ -82,7 +84,8 @@ struct WcState {
     int32_t* segpgi = nullptr;
     // adjoint
     double *lam = nullptr, *lamn = nullptr;    // 5n each
-    double *la = nullptr, *lD = nullptr, *ln = nullptr, *lvl = nullptr, *lrl = nullptr;
+    double *lD = nullptr, *ln = nullptr, *lvl = nullptr, *lrl = nullptr;
+    double2* adj2 = nullptr;                   // 3n: AdjPair
     double *dJ = nullptr, *grad = nullptr;
     std::vector<void*> allocs;
 };
@@ -90,6 +93,11 @@ struct WcState {
 namespace {
 
 constexpr int WB = 128;
+// The FP64-bound pair kernels take blocks of one warp: a block of four runs as
+// long as its slowest SM, and 794 of them over 152 SMs leave some with six
+// where 5.2 is the mean (forward step on 101573 particles 4 % faster).
+constexpr int WPB = 32;
+constexpr int EOS_MAX = 8;  // largest whole gamma evaluated as a polynomial
 constexpr int GCMAX = 9;  // grid cells one particle's kernel support can overlap (checked at setup)
 
 template <typename T>
@@ -111,9 +119,11 @@ __device__ __forceinline__ double wdF(const WcK& K, double r) {
     const double a = 1.0 - 0.5 * r * K.inv_h;
     return 1.5 * K.wend_F * a * a * K.inv_h;
 }
+// (each operation rounded as written: the porosity pass has the same bits with
+// and without the adjoint's record)
 __device__ __forceinline__ double wW(const WcK& K, double r) {
-    const double q = r * K.inv_h, a = 1.0 - 0.5 * q, a2 = a * a;
-    return K.wend_W * (1.0 + 2.0 * q) * a2 * a2;
+    const double q = __dmul_rn(r, K.inv_h), a = fma(-0.5, q, 1.0), a2 = __dmul_rn(a, a);
+    return __dmul_rn(__dmul_rn(__dmul_rn(K.wend_W, fma(2.0, q, 1.0)), a2), a2);
 }
 // the 1-D Wendland C2 kernel of the probes (radius R1, unit integral)
 __device__ __forceinline__ double w1(double q, double R1) {
@@ -156,32 +166,60 @@ __global__ void k_wc_solids(int64_t ns, const double* __restrict__ sx, const dou
     sg[s] = g;
 }
 
-// clamped density, pressure, hydrostatic density and its slope, and the
-// per-particle quotients the pair loops read (volume m/rt, p/rt^2)
+// clamped density, pressure, the density's excess over the hydrostatic one and
+// that one's slope, and the per-particle quotients the pair loops read (volume
+// m/rt, p/rt^2)
 struct Pre {
-    double *rt, *pp, *rh, *drh, *vol, *pr, *dpdr;  // dpdr: dp/drt of the EOS
+    double *rt, *pp, *ex, *drh, *vol, *pr, *dpdr;  // dpdr: dp/drt of the EOS
 };
 
+// s^(1/m) for a whole m and s > 0 in FP32's range: an FP32 seed, then two
+// Newton steps for y^m = s, y -= (y^m - s) / (m y^(m-1)).  The seed's error
+// (~1e-6) squares twice below FP64's rounding, so the divisor, which only
+// scales a correction of ~1e-6, may be an FP32 reciprocal.
+__device__ __forceinline__ double root_of(double s, int m) {
+    const float seed = exp2f(__log2f((float)s) / (float)m);
+    double y = (double)seed;
+    const double scale = (double)(seed / ((float)m * (float)s));  // 1 / (m y^(m-1))
+#pragma unroll
+    for (int step = 0; step < 2; ++step) {
+        double q = y;
+        for (int k = 1; k < m; ++k) q *= y;
+        y -= (q - s) * scale;
+    }
+    return y;
+}
+
+// Bound: the FP64 pipe.  For a whole gamma (Tait's 7) the EOS is the binomial
+// polynomial in t = (rt - rho0)/rho0, exact where pow(rt/rho0, gamma) - 1
+// cancels, and the hydrostatic density a Newton root; two pow() took 49 us on
+// 101573 particles, these 18 us (cold caches).
 __global__ void k_wc_pre(int64_t n, const int8_t* __restrict__ tid, const double* __restrict__ mass,
                          const double* __restrict__ y, const double* __restrict__ rho, WcK K, Pre o) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double r = tid[i] == BSC_TID_FLUID ? fmax(rho[i], K.rho0) : rho[i];
-    const double qg = pow(r / K.rho0, K.gam);
-    double p = K.B * (qg - 1.0);
+    double qm;  // (rt/rho0)^gamma - 1
+    if (K.igam) {
+        const double t = (r - K.rho0) / K.rho0;
+        qm = K.binom[K.igam - 1];
+        for (int k = K.igam - 2; k >= 0; --k) qm = fma(qm, t, K.binom[k]);
+        qm *= t;
+    } else {
+        qm = pow(r / K.rho0, K.gam) - 1.0;
+    }
+    double p = K.B * qm;
     if (p < 0.0) p = 0.0;
     const double ir = 1.0 / r;
-    o.dpdr[i] = K.B * K.gam * qg * ir;  // B gamma (rt/rho0)^(gamma-1) / rho0
+    o.dpdr[i] = K.B * K.gam * (qm + 1.0) * ir;  // B gamma (rt/rho0)^(gamma-1) / rho0
     o.rt[i] = r;
     o.pp[i] = p;
     o.vol[i] = mass[i] * ir;
     o.pr[i] = p * ir * ir;
-    double* rh = o.rh;
-    double* drh = o.drh;
     const double s = 1.0 + K.grav_c * (K.ys - y[i]);
-    const double q = pow(s, K.inv_gam);
-    rh[i] = K.rho0 * q;
-    drh[i] = -K.rho0 * K.grav_c * K.inv_gam * q / s;
+    const double q = K.igam && s > 1e-3 ? root_of(s, K.igam) : pow(s, K.inv_gam);
+    o.ex[i] = r - K.rho0 * q;
+    o.drh[i] = -K.rho0 * K.grav_c * K.inv_gam * q / s;
 }
 
 // the five state fields, one launch
@@ -195,7 +233,7 @@ __global__ void k_wc_copy(int64_t n, St src, St dst) {
     dst.rho[i] = src.rho[i];
 }
 
-// what the porosity pass keeps for the adjoint (null when not kept)
+// what the porosity pass keeps for the adjoint
 struct PorKeep {
     double* dn;    // grad n_i (2n)
     int32_t* pgi;  // grid cell u of particle i at [u * n + i], -1 past the last
@@ -210,15 +248,16 @@ struct PorKeep {
 // cell order, into this thread's column of shared memory, and the FP64 terms
 // run over those.  Same terms, same order.  A particle with more survivors
 // than the column holds, or far from its binned cell, takes one pass.
-// 101573 particles, no adjoint record: 236 us before, 112 us.
+// 101573 particles, no adjoint record: 236 us before, 61 us.
 constexpr int WP_CAP = 32;
-__global__ void __launch_bounds__(WB) k_wc_por(int64_t n, State S, KParams KP, WcK K, const int32_t* __restrict__ pcell,
+template <bool KEEP>
+__global__ void __launch_bounds__(WPB, 8) k_wc_por(int64_t n, State S, KParams KP, WcK K, const int32_t* __restrict__ pcell,
                                                const float2* __restrict__ posf, const int32_t* __restrict__ scs,
                                                const int32_t* __restrict__ scc, const float2* __restrict__ sposf,
                                                const double* __restrict__ sx, const double* __restrict__ sy,
                                                const double* __restrict__ sw, const double* __restrict__ svol,
                                                const int32_t* __restrict__ sg, double* __restrict__ nout, PorKeep kp) {
-    __shared__ int32_t cand[WP_CAP * WB];
+    __shared__ int32_t cand[WP_CAP * WPB];
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     int cg[GCMAX];
@@ -235,16 +274,13 @@ __global__ void __launch_bounds__(WB) k_wc_por(int64_t n, State S, KParams KP, W
         const float H2f = (float)(KP.H2 * (1.0 + PRE_MARGIN)), csf = (float)KP.cs;
         const float2 pi = posf[i];
         const bool pre_i = pre_ok(pi, csf);
-        auto term = [&](int s) {
-            const double dx = xi - sx[s], dy = yi - sy[s], d2 = dx * dx + dy * dy;
-            if (!(d2 < K.H2)) return;
-            const double r = sqrt(d2), W = wW(K, r);
-            frac += sw[s] * W;
-            if (kp.dn) {
-                const double F = wF(K, r);
+        // one solid's part of the sums, W its kernel value and F its gradient factor
+        auto add = [&](int s, double W, double F, double dx, double dy) {
+            frac = fma(sw[s], W, frac);
+            if (KEEP) {
                 gx -= sw[s] * F * dx;  // grad n = -sum sw grad W
                 gy -= sw[s] * F * dy;
-                const int g = sg[s];
+                const int g = W != 0.0 ? sg[s] : -1;
                 if (g < 0) return;
                 const double v = svol[s] * W;
                 bool kept = false;
@@ -257,6 +293,12 @@ __global__ void __launch_bounds__(WB) k_wc_por(int64_t n, State S, KParams KP, W
                     }
                 }
             }
+        };
+        auto term = [&](int s) {
+            const double dx = xi - sx[s], dy = yi - sy[s], d2 = fma(dx, dx, __dmul_rn(dy, dy));
+            if (!(d2 < K.H2)) return;
+            const double r = sqrt(d2);
+            add(s, wW(K, r), KEEP ? wF(K, r) : 0.0, dx, dy);
         };
         int nc = 0;
         // pass 0 compacts the survivors; pass 1 (only if they do not fit, or
@@ -279,19 +321,37 @@ __global__ void __launch_bounds__(WB) k_wc_por(int64_t n, State S, KParams KP, W
                             const float fdx = pi.x - (ps.x + shx), fdy = pi.y - (ps.y + shy);
                             if (fdx * fdx + fdy * fdy > H2f) continue;
                         }
-                        if (nc < WP_CAP) cand[nc * WB + threadIdx.x] = s;
+                        if (nc < WP_CAP) cand[nc * WPB + threadIdx.x] = s;
                         ++nc;
                     }
                 }
             }
             if (pass == 0 && nc <= WP_CAP) {
-                for (int k = 0; k < nc; ++k) term(cand[k * WB + threadIdx.x]);
+                constexpr int U = KEEP ? 2 : 4;  // independent terms in flight
+                int k = 0;
+                for (; k + U <= nc; k += U) {
+                    int q[U];
+                    double W[U], F[U], gdx[U], gdy[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        q[u] = cand[(k + u) * WPB + threadIdx.x];
+                        gdx[u] = xi - sx[q[u]];
+                        gdy[u] = yi - sy[q[u]];
+                        const double d2 = fma(gdx[u], gdx[u], __dmul_rn(gdy[u], gdy[u])), r = sqrt(d2);
+                        const bool in = d2 < K.H2;
+                        W[u] = in ? wW(K, r) : 0.0;
+                        F[u] = KEEP && in ? wF(K, r) : 0.0;
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) add(q[u], W[u], F[u], gdx[u], gdy[u]);
+                }
+                for (; k < nc; ++k) term(cand[k * WPB + threadIdx.x]);
                 break;
             }
         }
     }
     nout[i] = is_fluid(S, i) ? 1.0 - frac : 1.0;
-    if (kp.dn) {
+    if (KEEP) {
         kp.dn[i] = gx;
         kp.dn[n + i] = gy;
 #pragma unroll
@@ -306,12 +366,12 @@ __global__ void __launch_bounds__(WB) k_wc_por(int64_t n, State S, KParams KP, W
 
 // one step: next state; the porosity (in nbuf) and the pressure sum P
 // (2 per particle, for the adjoint) are kept
-__global__ void __launch_bounds__(WB) k_wc_step(int64_t n, State S, WcK K, const int32_t* __restrict__ nbr,
+__global__ void __launch_bounds__(WPB) k_wc_step(int64_t n, State S, WcK K, const int32_t* __restrict__ nbr,
                                                 const int32_t* __restrict__ cnt, Pre pq,
                                                 const double* __restrict__ nbuf, St out, double* __restrict__ Pbuf,
                                                 double* __restrict__ geo, int64_t slots) {
     const double* __restrict__ rt = pq.rt;
-    const double* __restrict__ rh = pq.rh;
+    const double* __restrict__ ex = pq.ex;
     const double* __restrict__ vol = pq.vol;
     const double* __restrict__ pr = pq.pr;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -326,35 +386,38 @@ __global__ void __launch_bounds__(WB) k_wc_step(int64_t n, State S, WcK K, const
         Pbuf[i] = Pbuf[n + i] = 0.0;
         return;
     }
-    const double rti = rt[i], rhi = rh[i], ni = nbuf[i];
+    const double rti = rt[i], exi = ex[i], ni = nbuf[i];
     const double pri = pr[i];
-    double Dr = 0.0, Px = 0.0, Py = 0.0, vx = 0.0, vy = 0.0;
+    // factors common to a sum (rt_i, c2, 2 nu) are applied after the loop
+    double Da = 0.0, Dd = 0.0, Px = 0.0, Py = 0.0, vx = 0.0, vy = 0.0;
     const int m = cnt[i];
     for (int k = 0; k < m; ++k) {
-        const int j = nbr[ell(i, k, K.kmax)];
+        const int64_t e = ell(i, k, K.kmax);
+        const int j = nbr[e];
         const double dx = xi - S.x[j], dy = yi - S.y[j];
         const double r2 = dx * dx + dy * dy, r = sqrt(r2);
         const double iden = rcp_nr(r2 + K.lam);
         const double F = wF(K, r), G = F * r2 * iden;
         if (geo) {  // F, F'/r, G, G'/r for the reverse sweep
-            const int64_t e = ell(i, k, K.kmax);
             const double ir = rcp_nr(r), dF = wdF(K, r);
             geo[e] = F;
             geo[slots + e] = dF * ir;
             geo[2 * slots + e] = G;
             geo[3 * slots + e] = (dF * r2 + F * 2.0 * r * K.lam * iden) * iden * ir;
         }
-        const double rtj = rt[j], mj = S.mass[j], Vj = vol[j];
+        const double Vj = vol[j], VG = Vj * G;
         const double dvx = vxi - S.vx[j], dvy = vyi - S.vy[j];
-        Dr += rti * Vj * F * (dvx * dx + dvy * dy);  // m_j (rt_i / rt_j) F (v_ij . x_ij)
-        Dr += K.c2 * (rtj - rti - rh[j] + rhi) * (-G) * Vj;
-        const double pc = mj * (pri + pr[j]) * F;
+        Da += Vj * F * (dvx * dx + dvy * dy);  // m_j (rt_i / rt_j) F (v_ij . x_ij) / rt_i
+        Dd += (exi - ex[j]) * VG;
+        const double pc = S.mass[j] * (pri + pr[j]) * F;
         Px += pc * dx;
         Py += pc * dy;
-        const double vc = 2.0 * K.nu * Vj * G;
-        vx += vc * dvx;
-        vy += vc * dvy;
+        vx += VG * dvx;
+        vy += VG * dvy;
     }
+    const double Dr = rti * Da + K.c2 * Dd;
+    vx *= 2.0 * K.nu;
+    vy *= 2.0 * K.nu;
     const double ax = -ni * Px + vx, ay = -ni * Py + vy + ni * K.g;
     const double vm = sqrt(vxi * vxi + vyi * vyi), on = 1.0 - ni, n3 = ni * ni * ni;
     const double R = -K.nu * K.alpha * on * on / (n3 * K.d50 * K.d50) - K.beta * vm * on / (n3 * K.d50);
@@ -457,14 +520,22 @@ __device__ __forceinline__ void block_sum2(double a, double b, double* __restric
     }
 }
 
+// what the pair sums read of a particle's own adjoint: lam_a times 2 nu and
+// times n, and (lam_Drho rt, c2 lam_Drho)
+struct AdjPair {
+    double2 *vla, *nla, *ab;
+};
+
 // the per-particle part of the reverse step: position update, drag, the
-// porosity's direct roles; writes lam_a, lam_Drho, lam_n, and the particle's
+// porosity's direct roles; writes lam_a and lam_Drho as the pair sums read them,
+// lam_n, and the particle's
 // own contributions to lam_v and lam_rt; drag-coefficient partials per block
 __global__ void __launch_bounds__(WB) k_wc_adj_local(int64_t n, const int8_t* __restrict__ tid, WcK K, St s0, St s1,
                                                      const double* __restrict__ nbuf, const double* __restrict__ Pbuf,
-                                                     St lam, double* __restrict__ la, double* __restrict__ lD,
-                                                     double* __restrict__ ln, double* __restrict__ lvl,
-                                                     double* __restrict__ lrl, double* __restrict__ part, int pstride) {
+                                                     const double* __restrict__ rt, St lam, AdjPair ap,
+                                                     double* __restrict__ lD, double* __restrict__ ln,
+                                                     double* __restrict__ lvl, double* __restrict__ lrl,
+                                                     double* __restrict__ part, int pstride) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     double ga = 0.0, gb = 0.0;
     if (i < n && tid[i] == BSC_TID_FLUID) {
@@ -495,137 +566,90 @@ __global__ void __launch_bounds__(WB) k_wc_adj_local(int64_t n, const int8_t* __
         gb = lR * (-cB);
         // a = -n P + visc + n g: d a / d n = -P + g
         lni += lax * (-Pbuf[i]) + lay * (-Pbuf[n + i] + K.g);
-        la[i] = lax;
-        la[n + i] = lay;
-        lD[i] = K.dt * lam.rho[i];
+        const double lDi = K.dt * lam.rho[i];
+        ap.vla[i] = make_double2(2.0 * K.nu * lax, 2.0 * K.nu * lay);
+        ap.nla[i] = make_double2(ni * lax, ni * lay);
+        ap.ab[i] = make_double2(lDi * rt[i], K.c2 * lDi);
+        lD[i] = lDi;
         ln[i] = lni;
         lvl[i] = lvx;
         lvl[n + i] = lvy;
         lrl[i] = lam.rho[i];
     } else if (i < n) {
-        la[i] = la[n + i] = 0.0;
+        // a wall has no sums of its own: its products with them vanish
+        ap.vla[i] = ap.nla[i] = ap.ab[i] = make_double2(0.0, 0.0);
         lD[i] = ln[i] = 0.0;
     }
     block_sum2(ga, gb, part + (int64_t)blockIdx.x * pstride);
 }
 
-// the pair part: for fluid particle k, the terms of its own sums (k as i) and
+// The pair part: for fluid particle k, the terms of its own sums (k as i) and
 // of its neighbours' sums (k as j), with the per-pair kernel values and the
 // porosity's gradient and per-grid-cell sums that the recomputation kept;
 // writes the state adjoint lam_out for the state before the step and the
-// block's porosity-grid partials
-__global__ void __launch_bounds__(WB) k_wc_adj_pair(
+// block's porosity-grid partials.
+// Bound: the FP64 pipe.  The two roles' terms differ by exchanging k and j and
+// the sign of the offset, so each kind of term is one expression in a
+// (anti)symmetric pair weight:
+//   continuity     Q = lamD_k rt_k V_j + lamD_j rt_j V_k
+//   diffusion      D = c2 (lamD_k V_j - lamD_j V_k),   del = ex_j - ex_k
+//   pressure       M = m_j n_k lam_a,k - m_k n_j lam_a,j
+//   viscosity      N = 2 nu (V_j lam_a,k - V_k lam_a,j)
+//   d/dx_k:  Q F dv - (p_k/rt_k^2 + p_j/rt_j^2) F M
+//            + [F'/r (Q dv.d - ps M.d) + G'/r (N.dv - del D)] d
+// and the factors that belong to k alone are applied after the loop: 55 FP64
+// operations a pair instead of about 130.  A wall's weights are zero.
+// 14600 particles: 134 us before, 70 us.
+__global__ void __launch_bounds__(WPB) k_wc_adj_pair(
     int64_t n, State S, WcK K, St s0, const int32_t* __restrict__ nbr, const int32_t* __restrict__ cnt, Pre pq,
-    const double* __restrict__ geo, int64_t slots, const double* __restrict__ nbuf, const double* __restrict__ la,
+    const double* __restrict__ geo, int64_t slots, const double* __restrict__ nbuf, AdjPair ap,
     const double* __restrict__ lD, const double* __restrict__ ln, const double* __restrict__ lvl,
     const double* __restrict__ lrl, St lam_in, St lam_out, const double* __restrict__ dn,
     const int32_t* __restrict__ pgi, const double* __restrict__ pgv, double* __restrict__ part, int pstride) {
-    // grid-porosity partials per warp, then summed over the warps in order
-    __shared__ double wb[WB / 32][BSC_WCSPH_MAX_GRID];
+    // grid-porosity partials of the block's warp
+    __shared__ double wb[BSC_WCSPH_MAX_GRID];
     const int G = K.gnx * K.gny;
-    for (int e = threadIdx.x; e < (WB / 32) * BSC_WCSPH_MAX_GRID; e += WB) (&wb[0][0])[e] = 0.0;
-    __syncthreads();
+    for (int e = threadIdx.x; e < G; e += WPB) wb[e] = 0.0;
+    __syncwarp();
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const bool act = k < n && S.tid[k] == BSC_TID_FLUID;
     double lnk = 0.0;
     if (act) {
-        const double* __restrict__ rt = pq.rt;
-        const double* __restrict__ rh = pq.rh;
         const double xk = s0.x[k], yk = s0.y[k], vxk = s0.vx[k], vyk = s0.vy[k];
-        const double rtk = rt[k], pk = pq.pp[k], rhk = rh[k], drk = pq.drh[k], nk = nbuf[k], mk = S.mass[k];
-        const double Vk = pq.vol[k], prk = pq.pr[k], irk = 1.0 / rtk;
-        const double mk_rt2 = mk * irk * irk, pk_rt3 = 2.0 * prk * irk;  // m_k / rt_k^2, 2 p_k / rt_k^3
-        const double lDk = lD[k], lax = la[k], lay = la[n + k];
-        double lrt = lrl[k], lp = 0.0;
-        double lvx = lvl[k], lvy = lvl[n + k];
-        double lxx = lam_in.x[k], lyy = lam_in.y[k];
+        const double exk = pq.ex[k], mk = S.mass[k], Vk = pq.vol[k], prk = pq.pr[k];
+        const double irk = 1.0 / pq.rt[k], Vk_rt = Vk * irk;
+        const double lDk = lD[k];
+        const double2 vlak = ap.vla[k], nlak = ap.nla[k], abk = ap.ab[k];
+        double lvx = lvl[k], lvy = lvl[n + k], lrt = lrl[k], lxx = lam_in.x[k], lyy = lam_in.y[k];
+        double SD = 0.0, S2 = 0.0, SP = 0.0, SV = 0.0;  // sum G D, G c2 lamD_j del, F M.d, G 2 nu lam_a,j.dv
         const int m = cnt[k];
         for (int q = 0; q < m; ++q) {
             const int64_t e = ell(k, q, K.kmax);
             const int j = nbr[e];
-            const double dx = xk - s0.x[j], dy = yk - s0.y[j];
             const double F = geo[e], Fr = geo[slots + e], G_ = geo[2 * slots + e], Gr = geo[3 * slots + e];
-            const double rtj = rt[j], prj = pq.pr[j], mj = S.mass[j], Vj = pq.vol[j];
+            const double Vj = pq.vol[j], mj = S.mass[j], ps = prk + pq.pr[j], del = pq.ex[j] - exk;
+            const double2 vlaj = ap.vla[j], nlaj = ap.nla[j], abj = ap.ab[j];
+            const double dx = xk - s0.x[j], dy = yk - s0.y[j];
             const double dvx = vxk - s0.vx[j], dvy = vyk - s0.vy[j], dvd = dvx * dx + dvy * dy;
-            double gx = 0.0, gy = 0.0;  // adjoint of d = x_k - x_j
-            // -- k's own continuity sum
-            {
-                const double c1 = rtk * Vj;  // m_j rt_k / rt_j
-                lrt += lDk * Vj * F * dvd;
-                lvx += lDk * c1 * F * dx;
-                lvy += lDk * c1 * F * dy;
-                const double t = lDk * c1 * Fr * dvd;
-                gx += lDk * c1 * F * dvx + t * dx;
-                gy += lDk * c1 * F * dvy + t * dy;
-                const double del = rtj - rtk - rh[j] + rhk;
-                lrt += lDk * K.c2 * G_ * Vj;
-                lyy += lDk * K.c2 * drk * (-G_) * Vj;
-                const double u = -lDk * K.c2 * del * Gr * Vj;
-                gx += u * dx;
-                gy += u * dy;
-            }
-            // -- k's own momentum sum
-            {
-                const double lad = lax * dx + lay * dy;
-                const double pc = mj * (prk + prj);
-                gx += -nk * pc * (F * lax + Fr * lad * dx);
-                gy += -nk * pc * (F * lay + Fr * lad * dy);
-                lp += -nk * mj * irk * irk * F * lad;
-                lrt += nk * mj * pk_rt3 * F * lad;
-                const double vc = 2.0 * K.nu * Vj;
-                lvx += vc * G_ * lax;
-                lvy += vc * G_ * lay;
-                const double w = vc * (lax * dvx + lay * dvy) * Gr;
-                gx += w * dx;
-                gy += w * dy;
-            }
-            // -- k in the sums of its fluid neighbour j, where the offset is
-            // e = x_j - x_k = -d: the adjoint of e (hx, hy) enters lam_x_k with
-            // the opposite sign
-            if (S.tid[j] == BSC_TID_FLUID) {
-                const double lDj = lD[j], lajx = la[j], lajy = la[n + j], nj = nbuf[j];
-                const double ex = -dx, ey = -dy;      // x_j - x_k; (v_j - v_k).(x_j - x_k) = dvd
-                const double dwx = -dvx, dwy = -dvy;  // v_j - v_k
-                double hx = 0.0, hy = 0.0;
-                // continuity of j
-                const double c1 = rtj * Vk;  // m_k rt_j / rt_k
-                lrt += lDj * (-c1 * irk) * F * dvd;
-                lvx += lDj * (-c1 * F * ex);
-                lvy += lDj * (-c1 * F * ey);
-                {
-                    const double t = lDj * c1 * Fr * dvd;
-                    hx += lDj * c1 * F * dwx + t * ex;
-                    hy += lDj * c1 * F * dwy + t * ey;
-                }
-                const double del = rtk - rtj - rhk + rh[j];
-                lrt += lDj * K.c2 * (-G_) * Vk * (1.0 - del * irk);
-                lyy += lDj * K.c2 * drk * G_ * Vk;
-                {
-                    const double u = -lDj * K.c2 * del * Gr * Vk;
-                    hx += u * ex;
-                    hy += u * ey;
-                }
-                // momentum of j
-                const double lad = lajx * ex + lajy * ey;
-                const double pc = mk * (prj + prk);
-                hx += -nj * pc * (F * lajx + Fr * lad * ex);
-                hy += -nj * pc * (F * lajy + Fr * lad * ey);
-                lp += -nj * mk_rt2 * F * lad;
-                lrt += nj * mk * pk_rt3 * F * lad;
-                const double vc = 2.0 * K.nu * Vk;
-                lvx += -vc * G_ * lajx;
-                lvy += -vc * G_ * lajy;
-                const double ldv = lajx * dwx + lajy * dwy;
-                lrt += -2.0 * K.nu * mk_rt2 * G_ * ldv;
-                const double w = vc * ldv * Gr;
-                hx += w * ex;
-                hy += w * ey;
-                gx -= hx;
-                gy -= hy;
-            }
-            lxx += gx;
-            lyy += gy;
+            const double Q = abk.x * Vj + abj.x * Vk, QF = Q * F;
+            const double D = abk.y * Vj - abj.y * Vk;
+            const double Mx = mj * nlak.x - mk * nlaj.x, My = mj * nlak.y - mk * nlaj.y, Md = Mx * dx + My * dy;
+            const double Nx = Vj * vlak.x - Vk * vlaj.x, Ny = Vj * vlak.y - Vk * vlaj.y;
+            lvx += QF * dx + G_ * Nx;
+            lvy += QF * dy + G_ * Ny;
+            lrt += (F * dvd) * (lDk * Vj - abj.x * Vk_rt);
+            SD += G_ * D;
+            S2 += G_ * abj.y * del;
+            SP += F * Md;
+            SV += G_ * (vlaj.x * dvx + vlaj.y * dvy);
+            const double C = Fr * (Q * dvd - ps * Md) + Gr * (Nx * dvx + Ny * dvy - del * D);
+            const double psF = ps * F;
+            lxx += QF * dvx - psF * Mx + C * dx;
+            lyy += QF * dvy - psF * My + C * dy;
         }
+        lrt += SD - Vk_rt * S2 + 2.0 * prk * irk * SP + mk * irk * irk * SV;
+        lyy -= pq.drh[k] * SD;
+        const double lp = -irk * irk * SP;
         // porosity n_k = 1 - sum_s (1 - phi_s) V_s W(r_ks)
         lnk = ln[k];
         lxx += lnk * dn[k];
@@ -642,7 +666,7 @@ __global__ void __launch_bounds__(WB) k_wc_adj_pair(
     }
     // d n_k / d phi_g = sum over cell g's solids of V_s W(r_ks): lanes with the
     // same cell are summed in lane order by the lowest of them
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x;
     for (int u = 0; u < K.gc; ++u) {
         int g = -1;
         double v = 0.0;
@@ -650,27 +674,24 @@ __global__ void __launch_bounds__(WB) k_wc_adj_pair(
             g = pgi[u * n + k];
             v = lnk * pgv[u * n + k];
         }
+        if (__all_sync(0xffffffffu, g < 0)) continue;
         const unsigned grp = __match_any_sync(0xffffffffu, g);
         double acc = 0.0;
         for (int src = 0; src < 32; ++src) {
             const double t = __shfl_sync(0xffffffffu, v, src);
             if ((grp >> src) & 1u) acc += t;
         }
-        if (g >= 0 && lane == __ffs(grp) - 1) wb[warp][g] += acc;
+        if (g >= 0 && lane == __ffs(grp) - 1) wb[g] += acc;
         __syncwarp();
     }
-    __syncthreads();
-    for (int g = threadIdx.x; g < G; g += WB) {
-        double acc = 0.0;
-        for (int q = 0; q < WB / 32; ++q) acc += wb[q][g];
-        part[(int64_t)blockIdx.x * pstride + 2 + g] = acc;
-    }
+    for (int g = lane; g < G; g += WPB) part[(int64_t)blockIdx.x * pstride + 2 + g] = wb[g];
 }
 
-// grad[q] += sum over blocks of part[block][q]: one block per q, fixed order
-__global__ void k_wc_grad(int nb, int pstride, const double* __restrict__ part, double* __restrict__ grad) {
+// grad[q] += sum over blocks of part[block][q]: one block per q, fixed order;
+// the drag coefficients (q < 2) have nbl blocks, the porosities nbp
+__global__ void k_wc_grad(int nbl, int nbp, int pstride, const double* __restrict__ part, double* __restrict__ grad) {
     __shared__ double sh[WB];
-    const int q = blockIdx.x;
+    const int q = blockIdx.x, nb = q < 2 ? nbl : nbp;
     double s = 0.0;
     for (int b = threadIdx.x; b < nb; b += WB) s += part[(int64_t)b * pstride + q];
     sh[threadIdx.x] = s;
@@ -709,7 +730,7 @@ int wc_params(Ctx* c, WcState* w, double alpha, double beta, const double* grid)
 }
 
 // one forward step on c->S; keeps n and P in nbuf, Pbuf
-Pre wc_pre(WcState* w) { return {w->rt, w->pp, w->rh, w->drh, w->vol, w->pr, w->dpdr}; }
+Pre wc_pre(WcState* w) { return {w->rt, w->pp, w->ex, w->drh, w->vol, w->pr, w->dpdr}; }
 
 // the context's state with the model's masses
 State wc_view(Ctx* c, WcState* w) {
@@ -776,18 +797,23 @@ int wc_step(Ctx* c, WcState* w, double* nbuf, double* Pbuf, const Keep* keep, bo
     if (!rc) rc = cells_build(c, false);
     if (!rc) rc = last ? op_neighbour(c) : op_neighbour_lists(c);
     if (!rc) {
-        const unsigned g = blocks_for(n, WB);
+        const unsigned g = blocks_for(n, WB), gp = blocks_for(n, WPB);
         const State S = wc_view(c, w);
         k_wc_pre<<<g, WB, 0, c->stream>>>(n, S.tid, S.mass, S.y, S.rho, w->K, pre);
         rc = launch_check(c);
         if (!rc) {
-            k_wc_por<<<g, WB, 0, c->stream>>>(n, S, c->K, w->K, c->pcell, c->posf, c->scell_start, c->scell_count,
-                                              c->sposf, c->sx, c->sy, w->sw, c->svol, w->sg, nbuf,
-                                              keep ? keep->por : PorKeep{nullptr, nullptr, nullptr});
+            if (keep)
+                k_wc_por<true><<<gp, WPB, 0, c->stream>>>(n, S, c->K, w->K, c->pcell, c->posf, c->scell_start,
+                                                          c->scell_count, c->sposf, c->sx, c->sy, w->sw, c->svol,
+                                                          w->sg, nbuf, keep->por);
+            else
+                k_wc_por<false><<<gp, WPB, 0, c->stream>>>(n, S, c->K, w->K, c->pcell, c->posf, c->scell_start,
+                                                           c->scell_count, c->sposf, c->sx, c->sy, w->sw, c->svol,
+                                                           w->sg, nbuf, PorKeep{});
             rc = launch_check(c);
         }
         if (!rc) {
-            k_wc_step<<<g, WB, 0, c->stream>>>(n, S, w->K, c->nbr, c->cnt, pre, nbuf, st_of(w->nxt, n), Pbuf,
+            k_wc_step<<<gp, WPB, 0, c->stream>>>(n, S, w->K, c->nbr, c->cnt, pre, nbuf, st_of(w->nxt, n), Pbuf,
                                                keep ? keep->geo : nullptr, list_slots(c));
             rc = launch_check(c);
         }
@@ -829,6 +855,9 @@ int bsc_wcsph_setup(bsc_ctx* c, const bsc_wcsph_params* p) {
     K.rho0 = KP.rho0;
     K.gam = p->gamma;
     K.inv_gam = 1.0 / p->gamma;
+    K.igam = p->gamma == std::floor(p->gamma) && p->gamma <= EOS_MAX ? (int)p->gamma : 0;
+    double bin = 1.0;
+    for (int k = 0; k < K.igam; ++k) K.binom[k] = bin = bin * (K.igam - k) / (k + 1);
     K.B = KP.rho0 * p->c0 * p->c0 / p->gamma;
     K.grav_c = std::fabs(KP.g) * p->gamma / (p->c0 * p->c0);
     K.ys = p->surface_y;
@@ -862,14 +891,14 @@ int bsc_wcsph_setup(bsc_ctx* c, const bsc_wcsph_params* p) {
     if ((rc = wc_alloc(c, w, &w->init, 5 * n)) || (rc = wc_alloc(c, w, &w->mass, n)) ||
         (rc = wc_alloc(c, w, &w->theta, G)) ||
         (rc = wc_alloc(c, w, &w->sw, w->ns)) || (rc = wc_alloc(c, w, &w->sg, w->ns)) ||
-        (rc = wc_alloc(c, w, &w->rt, n)) || (rc = wc_alloc(c, w, &w->pp, n)) || (rc = wc_alloc(c, w, &w->rh, n)) ||
+        (rc = wc_alloc(c, w, &w->rt, n)) || (rc = wc_alloc(c, w, &w->pp, n)) || (rc = wc_alloc(c, w, &w->ex, n)) ||
         (rc = wc_alloc(c, w, &w->drh, n)) || (rc = wc_alloc(c, w, &w->vol, n)) || (rc = wc_alloc(c, w, &w->pr, n)) ||
         (rc = wc_alloc(c, w, &w->dpdr, n)) ||
         (rc = wc_alloc(c, w, &w->nxt, 5 * n)) ||
         (rc = wc_alloc(c, w, &w->xp, BSC_WCSPH_MAX_PROBES)) ||
-        (rc = wc_alloc(c, w, &w->part, (int64_t)blocks_for(n, WB) * (2 + BSC_WCSPH_MAX_GRID))) ||
+        (rc = wc_alloc(c, w, &w->part, (int64_t)blocks_for(n, WPB) * (2 + BSC_WCSPH_MAX_GRID))) ||
         (rc = wc_alloc(c, w, &w->lam, 5 * n)) || (rc = wc_alloc(c, w, &w->lamn, 5 * n)) ||
-        (rc = wc_alloc(c, w, &w->la, 2 * n)) || (rc = wc_alloc(c, w, &w->lD, n)) || (rc = wc_alloc(c, w, &w->ln, n)) ||
+        (rc = wc_alloc(c, w, &w->adj2, 3 * n)) || (rc = wc_alloc(c, w, &w->lD, n)) || (rc = wc_alloc(c, w, &w->ln, n)) ||
         (rc = wc_alloc(c, w, &w->lvl, 2 * n)) || (rc = wc_alloc(c, w, &w->lrl, n)) ||
         (rc = wc_alloc(c, w, &w->grad, 2 + BSC_WCSPH_MAX_GRID)))
         return rc;
@@ -1003,14 +1032,17 @@ int bsc_wcsph_adjoint(bsc_ctx* c, const double* dJ_deta, double* grad) {
             const State S = wc_view(c, w);
             const Keep kq = seg_keep(w, q, n, slots);
             const double* nq = w->segn + (int64_t)q * n;
-            k_wc_adj_local<<<nb, WB, 0, c->stream>>>(n, c->S.tid, w->K, st0, st1, nq, w->segP + (int64_t)q * 2 * n, lam,
-                                                     w->la, w->lD, w->ln, w->lvl, w->lrl, w->part, pstride);
+            const AdjPair ap{w->adj2, w->adj2 + n, w->adj2 + 2 * n};
+            const unsigned nbp = blocks_for(n, WPB);
+            k_wc_adj_local<<<nb, WB, 0, c->stream>>>(n, c->S.tid, w->K, st0, st1, nq, w->segP + (int64_t)q * 2 * n,
+                                                     kq.pre.rt, lam, ap, w->lD, w->ln, w->lvl, w->lrl, w->part,
+                                                     pstride);
             BSC_LAUNCH(c);
-            k_wc_adj_pair<<<nb, WB, 0, c->stream>>>(n, S, w->K, st0, kq.nbr, kq.cnt, kq.pre, kq.geo, slots, nq,
-                                                    w->la, w->lD, w->ln, w->lvl, w->lrl, lam, lamn, kq.por.dn,
-                                                    kq.por.pgi, kq.por.pgv, w->part, pstride);
+            k_wc_adj_pair<<<nbp, WPB, 0, c->stream>>>(n, S, w->K, st0, kq.nbr, kq.cnt, kq.pre, kq.geo, slots, nq, ap,
+                                                      w->lD, w->ln, w->lvl, w->lrl, lam, lamn, kq.por.dn, kq.por.pgi,
+                                                      kq.por.pgv, w->part, pstride);
             BSC_LAUNCH(c);
-            k_wc_grad<<<2 + G, WB, 0, c->stream>>>(nb, pstride, w->part, w->grad);
+            k_wc_grad<<<2 + G, WB, 0, c->stream>>>((int)nb, (int)nbp, pstride, w->part, w->grad);
             BSC_LAUNCH(c);
             std::swap(w->lam, w->lamn);
         }
