@@ -1,0 +1,67 @@
+// lanes.cuh -- several lanes per particle for the FP64 pair sums.
+//
+// A warp has one FP64 instruction in flight per ~100 clocks on this GPU
+// (dependent or not), and the FP64 pipe takes one per 16: below about eight
+// warps an SM a pair sum's time is the length of a thread's own loop, whatever
+// the particle count.  L lanes of a warp then share a particle: each takes
+// every L-th neighbour, and the sums are added up across them.
+#pragma once
+
+#include <type_traits>
+
+#include "bsc_internal.cuh"
+
+namespace bsc {
+
+// Lanes per particle for n particles.  Measured, 20 WCSPH steps with 1, 2, 4
+// and 8 lanes: 3.59, 3.56, 2.67, 2.42 ms at 3816 particles; 3.99, 4.10, 3.48,
+// 3.82 at 15797; 4.35, 4.84, 4.70, 5.39 at 30732: by then the particles alone
+// give the SMs their warps, and the sums across lanes cost more than the
+// shorter loops save.
+inline int lanes_for(int64_t n) { return n <= 10000 ? 8 : n <= 20000 ? 4 : 1; }
+
+template <int L>
+struct Lanes {
+    int sub;         // this lane's share of its particle
+    unsigned mask;   // the lanes of the particle
+    unsigned below;  // those before this one
+    __device__ __forceinline__ Lanes() {
+        const int lane = threadIdx.x & 31;
+        sub = lane & (L - 1);
+        mask = (L == 32 ? 0xffffffffu : ((1u << L) - 1u)) << (lane - sub);
+        below = mask & ((1u << lane) - 1u);
+    }
+    static __device__ __forceinline__ int64_t particle() {
+        return (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / L;
+    }
+    // the sum over the particle's lanes, in each of them
+    __device__ __forceinline__ double sum(double x) const {
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) x += __shfl_xor_sync(mask, x, o);
+        return x;
+    }
+    // the place of this lane's kept item among the particle's, after `count`
+    // of them; count moves past them
+    __device__ __forceinline__ int place(bool keep, int& count) const {
+        if (L == 1) return keep ? count++ : count;
+        const unsigned b = __ballot_sync(mask, keep) & mask;
+        const int at = count + __popc(b & below);
+        count += __popc(b);
+        return at;
+    }
+    __device__ __forceinline__ void sync() const {
+        if (L > 1) __syncwarp(mask);
+    }
+};
+
+// f with the number of lanes as a compile-time constant
+template <typename F>
+void with_lanes(int lanes, F f) {
+    switch (lanes) {
+        case 8: f(std::integral_constant<int, 8>{}); break;
+        case 4: f(std::integral_constant<int, 4>{}); break;
+        default: f(std::integral_constant<int, 1>{}); break;
+    }
+}
+
+}  // namespace bsc

@@ -17,6 +17,7 @@
 
 #include "bsc_internal.cuh"
 #include "dfloat.cuh"
+#include "lanes.cuh"
 #include "sph_kernel.cuh"
 
 namespace bsc {
@@ -414,12 +415,14 @@ int op_neighbour(Ctx* c) {
 // the exact one, the margin 1e-5), so only candidates inside the band take
 // the FP64 test that bounds the full search (~27 FP64 instructions an entry).
 // 101573 particles: the search 153 us, this 30 us.
+template <int L>
 __global__ void __launch_bounds__(NB_BLOCK) k_neighbour_lists(
     int64_t n, const double* __restrict__ x, const double* __restrict__ y, KParams K,
     const int32_t* __restrict__ cstart, const int32_t* __restrict__ ccount, const int32_t* __restrict__ sorted,
     const int32_t* __restrict__ pcell, const float2* __restrict__ posf, int32_t* __restrict__ nbr,
     int32_t* __restrict__ cnt, int32_t* __restrict__ flag) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const Lanes<L> ln;
+    const int64_t i = ln.particle();
     if (i >= n) return;
     const int c = pcell[i], cx = c / K.ny, cy = c - cx * K.ny;
     const float H2hi = (float)(K.H2 * (1.0 + PRE_MARGIN)), H2lo = (float)(K.H2 * (1.0 - PRE_MARGIN));
@@ -435,26 +438,28 @@ __global__ void __launch_bounds__(NB_BLOCK) k_neighbour_lists(
             const float shy = (float)(ay - cy) * csf;
             const int cc = ax * K.ny + ay;
             const int s0 = cstart[cc], s1 = s0 + ccount[cc];
-            for (int s = s0; s < s1; ++s) {
-                const int j = sorted[s];
-                if (j == (int)i) continue;
-                const float2 pj = posf[j];
-                bool sure = false;
-                if (pre_i && pre_ok(pj, csf)) {
-                    const float fdx = pi.x - (pj.x + shx), fdy = pi.y - (pj.y + shy);
-                    const float r2 = fdx * fdx + fdy * fdy;
-                    if (r2 > H2hi) continue;
-                    sure = r2 < H2lo;
+            for (int s = s0; s < s1; s += L) {
+                const int j = s + ln.sub < s1 ? sorted[s + ln.sub] : (int)i;
+                bool keep = j != (int)i, sure = false;
+                if (keep) {
+                    const float2 pj = posf[j];
+                    if (pre_i && pre_ok(pj, csf)) {
+                        const float fdx = pi.x - (pj.x + shx), fdy = pi.y - (pj.y + shy);
+                        const float r2 = fdx * fdx + fdy * fdy;
+                        keep = !(r2 > H2hi);
+                        sure = r2 < H2lo;
+                    }
                 }
-                if (!sure) {
+                if (keep && !sure) {
                     const double dx = x[i] - x[j], dy = y[i] - y[j];
-                    if (!nonneg_below(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), K.H2x)) continue;
+                    keep = nonneg_below(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), K.H2x);
                 }
-                if (count < K.kmax) nbr[ell(i, count, K.kmax)] = j;
-                ++count;
+                const int at = ln.place(keep, count);
+                if (keep && at < K.kmax) nbr[ell(i, at, K.kmax)] = j;
             }
         }
     }
+    if (ln.sub != 0) return;
     if (count > K.kmax) {
         atomicOr(flag, 1);
         count = K.kmax;
@@ -466,9 +471,11 @@ int op_neighbour_lists(Ctx* c) {
     k_posf<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->S.x, c->S.y, c->pcell, c->K, c->posf, c->S.vol,
                                                          nullptr, nullptr, nullptr);
     BSC_LAUNCH(c);
-    k_neighbour_lists<<<blocks_for(c->n, NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
-        c->n, c->S.x, c->S.y, c->K, c->cell_start, c->cell_count, c->sorted, c->pcell, c->posf, c->nbr, c->cnt,
-        c->d_flag);
+    with_lanes(lanes_for(c->n), [&](auto L) {
+        k_neighbour_lists<L.value><<<blocks_for(c->n * L.value, NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
+            c->n, c->S.x, c->S.y, c->K, c->cell_start, c->cell_count, c->sorted, c->pcell, c->posf, c->nbr, c->cnt,
+            c->d_flag);
+    });
     BSC_LAUNCH(c);
     return BSC_OK;
 }

@@ -36,6 +36,7 @@
 #include <vector>
 
 #include "bsc_internal.cuh"
+#include "lanes.cuh"
 #include "sph_kernel.cuh"
 
 struct bsc_ctx : bsc::Ctx {};  // the same definition as in api.cu
@@ -248,25 +249,28 @@ struct PorKeep {
 // cell order, into this thread's column of shared memory, and the FP64 terms
 // run over those.  Same terms, same order.  A particle with more survivors
 // than the column holds, or far from its binned cell, takes one pass.
-// 101573 particles, no adjoint record: 236 us before, 61 us.
+// The particles with solids are few and sit together, so several lanes share
+// one at any size.  101573 particles: 236 us before, 61 us, with the adjoint's
+// record 106 us.
 constexpr int WP_CAP = 32;
-template <bool KEEP>
+template <bool KEEP, int L>
 __global__ void __launch_bounds__(WPB, 8) k_wc_por(int64_t n, State S, KParams KP, WcK K, const int32_t* __restrict__ pcell,
                                                const float2* __restrict__ posf, const int32_t* __restrict__ scs,
                                                const int32_t* __restrict__ scc, const float2* __restrict__ sposf,
                                                const double* __restrict__ sx, const double* __restrict__ sy,
                                                const double* __restrict__ sw, const double* __restrict__ svol,
                                                const int32_t* __restrict__ sg, double* __restrict__ nout, PorKeep kp) {
-    __shared__ int32_t cand[WP_CAP * WPB];
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    constexpr int NP = WPB / L;  // particles of the block
+    __shared__ int32_t cand[WP_CAP * NP];
+    __shared__ double wval[KEEP && L > 1 ? WP_CAP * NP : 1];  // V W of the survivors, for the per-cell sums
+    const Lanes<L> ln;
+    const int64_t i = ln.particle();
     if (i >= n) return;
-    int cg[GCMAX];
-    double cv[GCMAX];
-#pragma unroll
-    for (int u = 0; u < GCMAX; ++u) {
-        cg[u] = -1;
-        cv[u] = 0.0;
-    }
+    const int p = threadIdx.x / L;
+    // the grid cells met so far and their sums (in shared memory: indexed)
+    __shared__ int cg[KEEP ? GCMAX * NP : 1];
+    __shared__ double cv[KEEP ? GCMAX * NP : 1];
+    int ncell = 0;
     double frac = 0.0, gx = 0.0, gy = 0.0;
     if (is_fluid(S, i)) {
         const double xi = S.x[i], yi = S.y[i];
@@ -274,35 +278,51 @@ __global__ void __launch_bounds__(WPB, 8) k_wc_por(int64_t n, State S, KParams K
         const float H2f = (float)(KP.H2 * (1.0 + PRE_MARGIN)), csf = (float)KP.cs;
         const float2 pi = posf[i];
         const bool pre_i = pre_ok(pi, csf);
+        // one solid's part of the per-cell sums
+        auto cell = [&](int g, double v) {
+            if (g < 0) return;
+            int u = 0;
+            while (u < ncell && cg[u * NP + p] != g) ++u;
+            if (u >= K.gc) return;
+            cv[u * NP + p] = u < ncell ? cv[u * NP + p] + v : v;
+            if (u == ncell) {
+                cg[u * NP + p] = g;
+                ++ncell;
+            }
+        };
+        auto cell_of = [&](int s, double W) { return W != 0.0 ? sg[s] : -1; };
         // one solid's part of the sums, W its kernel value and F its gradient factor
         auto add = [&](int s, double W, double F, double dx, double dy) {
             frac = fma(sw[s], W, frac);
             if (KEEP) {
                 gx -= sw[s] * F * dx;  // grad n = -sum sw grad W
                 gy -= sw[s] * F * dy;
-                const int g = W != 0.0 ? sg[s] : -1;
-                if (g < 0) return;
-                const double v = svol[s] * W;
-                bool kept = false;
-#pragma unroll
-                for (int u = 0; u < GCMAX; ++u) {
-                    if (!kept && u < K.gc && (cg[u] == g || cg[u] < 0)) {
-                        cg[u] = g;
-                        cv[u] += v;
-                        kept = true;
-                    }
-                }
             }
         };
-        auto term = [&](int s) {
-            const double dx = xi - sx[s], dy = yi - sy[s], d2 = fma(dx, dx, __dmul_rn(dy, dy));
-            if (!(d2 < K.H2)) return;
-            const double r = sqrt(d2);
-            add(s, wW(K, r), KEEP ? wF(K, r) : 0.0, dx, dy);
+        // U solids at once: independent terms in flight
+        auto terms = [&](auto U_, const int* q) {
+            constexpr int U = decltype(U_)::value;
+            double W[U], F[U], dx[U], dy[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                dx[u] = xi - sx[q[u]];
+                dy[u] = yi - sy[q[u]];
+                const double d2 = fma(dx[u], dx[u], __dmul_rn(dy[u], dy[u])), r = sqrt(d2);
+                const bool in = d2 < K.H2;
+                W[u] = in ? wW(K, r) : 0.0;
+                F[u] = KEEP && in ? wF(K, r) : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                add(q[u], W[u], F[u], dx[u], dy[u]);
+                if (KEEP && L == 1) cell(cell_of(q[u], W[u]), svol[q[u]] * W[u]);
+            }
+            return W[0];
         };
+        using One = std::integral_constant<int, 1>;
         int nc = 0;
         // pass 0 compacts the survivors; pass 1 (only if they do not fit, or
-        // without the pre-test) sums over the cells directly
+        // without the pre-test) sums over the cells directly, by one lane
         for (int pass = pre_i ? 0 : 1; pass < 2; ++pass) {
             for (int ax = cx - 1; ax <= cx + 1; ++ax) {
                 if (ax < 0 || ax >= KP.nx) continue;
@@ -311,61 +331,78 @@ __global__ void __launch_bounds__(WPB, 8) k_wc_por(int64_t n, State S, KParams K
                     if (ay < 0 || ay >= KP.ny) continue;
                     const float shy = (float)(ay - cy) * csf;
                     const int cc = ax * KP.ny + ay;
-                    for (int s = scs[cc], e = scs[cc] + scc[cc]; s < e; ++s) {
-                        if (pass == 1) {
-                            term(s);
-                            continue;
+                    const int s0 = scs[cc], s1 = s0 + scc[cc];
+                    if (pass == 1) {
+                        for (int s = s0; s < s1 && ln.sub == 0; ++s) {
+                            const double W = terms(One{}, &s);
+                            if (KEEP && L > 1) cell(cell_of(s, W), svol[s] * W);
                         }
-                        const float2 ps = sposf[s];
-                        if (pre_ok(ps, csf)) {
-                            const float fdx = pi.x - (ps.x + shx), fdy = pi.y - (ps.y + shy);
-                            if (fdx * fdx + fdy * fdy > H2f) continue;
+                        continue;
+                    }
+                    for (int s = s0; s < s1; s += L) {
+                        const int q = s + ln.sub;
+                        bool keep = q < s1;
+                        if (keep) {
+                            const float2 ps = sposf[q];
+                            if (pre_ok(ps, csf)) {
+                                const float fdx = pi.x - (ps.x + shx), fdy = pi.y - (ps.y + shy);
+                                keep = !(fdx * fdx + fdy * fdy > H2f);
+                            }
                         }
-                        if (nc < WP_CAP) cand[nc * WPB + threadIdx.x] = s;
-                        ++nc;
+                        const int at = ln.place(keep, nc);
+                        if (keep && at < WP_CAP) cand[at * NP + p] = q;
                     }
                 }
             }
             if (pass == 0 && nc <= WP_CAP) {
-                constexpr int U = KEEP ? 2 : 4;  // independent terms in flight
-                int k = 0;
-                for (; k + U <= nc; k += U) {
-                    int q[U];
-                    double W[U], F[U], gdx[U], gdy[U];
+                ln.sync();
+                if (L == 1) {
+                    constexpr int U = KEEP ? 2 : 4;
+                    int k = 0;
+                    for (; k + U <= nc; k += U) {
+                        int q[U];
 #pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        q[u] = cand[(k + u) * WPB + threadIdx.x];
-                        gdx[u] = xi - sx[q[u]];
-                        gdy[u] = yi - sy[q[u]];
-                        const double d2 = fma(gdx[u], gdx[u], __dmul_rn(gdy[u], gdy[u])), r = sqrt(d2);
-                        const bool in = d2 < K.H2;
-                        W[u] = in ? wW(K, r) : 0.0;
-                        F[u] = KEEP && in ? wF(K, r) : 0.0;
+                        for (int u = 0; u < U; ++u) q[u] = cand[(k + u) * NP + p];
+                        terms(std::integral_constant<int, U>{}, q);
                     }
-#pragma unroll
-                    for (int u = 0; u < U; ++u) add(q[u], W[u], F[u], gdx[u], gdy[u]);
+                    for (; k < nc; ++k) terms(One{}, &cand[k * NP + p]);
+                } else {
+                    for (int k = ln.sub; k < nc; k += L) {
+                        const double W = terms(One{}, &cand[k * NP + p]);
+                        if (KEEP) {
+                            const int s = cand[k * NP + p];
+                            wval[k * NP + p] = svol[s] * W;
+                            cand[k * NP + p] = cell_of(s, W);  // read by this lane only
+                        }
+                    }
+                    ln.sync();
+                    if (KEEP && ln.sub == 0)
+                        for (int k = 0; k < nc; ++k) cell(cand[k * NP + p], wval[k * NP + p]);
                 }
-                for (; k < nc; ++k) term(cand[k * WPB + threadIdx.x]);
                 break;
             }
         }
     }
+    frac = ln.sum(frac);
+    if (KEEP) {
+        gx = ln.sum(gx);
+        gy = ln.sum(gy);
+    }
+    if (ln.sub != 0) return;
     nout[i] = is_fluid(S, i) ? 1.0 - frac : 1.0;
     if (KEEP) {
         kp.dn[i] = gx;
         kp.dn[n + i] = gy;
-#pragma unroll
-        for (int u = 0; u < GCMAX; ++u) {
-            if (u < K.gc) {
-                kp.pgi[u * n + i] = cg[u];
-                kp.pgv[u * n + i] = cv[u];
-            }
+        for (int u = 0; u < K.gc; ++u) {
+            kp.pgi[u * n + i] = u < ncell ? cg[u * NP + p] : -1;
+            kp.pgv[u * n + i] = u < ncell ? cv[u * NP + p] : 0.0;
         }
     }
 }
 
 // one step: next state; the porosity (in nbuf) and the pressure sum P
 // (2 per particle, for the adjoint) are kept
+template <int L>
 __global__ void __launch_bounds__(WPB) k_wc_step(int64_t n, State S, WcK K, const int32_t* __restrict__ nbr,
                                                 const int32_t* __restrict__ cnt, Pre pq,
                                                 const double* __restrict__ nbuf, St out, double* __restrict__ Pbuf,
@@ -374,10 +411,12 @@ __global__ void __launch_bounds__(WPB) k_wc_step(int64_t n, State S, WcK K, cons
     const double* __restrict__ ex = pq.ex;
     const double* __restrict__ vol = pq.vol;
     const double* __restrict__ pr = pq.pr;
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const Lanes<L> ln;
+    const int64_t i = ln.particle();
     if (i >= n) return;
     const double xi = S.x[i], yi = S.y[i], vxi = S.vx[i], vyi = S.vy[i];
     if (!is_fluid(S, i)) {
+        if (ln.sub != 0) return;
         out.x[i] = xi;
         out.y[i] = yi;
         out.vx[i] = vxi;
@@ -391,7 +430,7 @@ __global__ void __launch_bounds__(WPB) k_wc_step(int64_t n, State S, WcK K, cons
     // factors common to a sum (rt_i, c2, 2 nu) are applied after the loop
     double Da = 0.0, Dd = 0.0, Px = 0.0, Py = 0.0, vx = 0.0, vy = 0.0;
     const int m = cnt[i];
-    for (int k = 0; k < m; ++k) {
+    for (int k = ln.sub; k < m; k += L) {
         const int64_t e = ell(i, k, K.kmax);
         const int j = nbr[e];
         const double dx = xi - S.x[j], dy = yi - S.y[j];
@@ -415,18 +454,37 @@ __global__ void __launch_bounds__(WPB) k_wc_step(int64_t n, State S, WcK K, cons
         vx += VG * dvx;
         vy += VG * dvy;
     }
+    Da = ln.sum(Da);
+    Dd = ln.sum(Dd);
+    Px = ln.sum(Px);
+    Py = ln.sum(Py);
+    vx = ln.sum(vx);
+    vy = ln.sum(vy);
+    if (ln.sub != 0) return;
     const double Dr = rti * Da + K.c2 * Dd;
     vx *= 2.0 * K.nu;
     vy *= 2.0 * K.nu;
     const double ax = -ni * Px + vx, ay = -ni * Py + vy + ni * K.g;
-    const double vm = sqrt(vxi * vxi + vyi * vyi), on = 1.0 - ni, n3 = ni * ni * ni;
-    const double R = -K.nu * K.alpha * on * on / (n3 * K.d50 * K.d50) - K.beta * vm * on / (n3 * K.d50);
-    const double D = 1.0 - K.dt * R * ni;
-    const double vxn = (vxi + K.dt * ax) / D, vyn = (vyi + K.dt * ay) / D;
+    // outside the porous layer (whole warps of it) the drag's quotients and
+    // roots, a tenth of this kernel's FP64 work, leave the values as they are
+    const bool clear = ni == 1.0 && isfinite(vxi) && isfinite(vyi);
+    double vxn = vxi + K.dt * ax, vyn = vyi + K.dt * ay, sxn, syn;
+    if (clear) {  // n = 1: no drag, and quotients by 1
+        sxn = K.dt * vxn;
+        syn = K.dt * vyn;
+    } else {
+        const double vm = sqrt(vxi * vxi + vyi * vyi), on = 1.0 - ni, n3 = ni * ni * ni;
+        const double R = -K.nu * K.alpha * on * on / (n3 * K.d50 * K.d50) - K.beta * vm * on / (n3 * K.d50);
+        const double D = 1.0 - K.dt * R * ni;
+        vxn /= D;
+        vyn /= D;
+        sxn = K.dt * vxn / ni;
+        syn = K.dt * vyn / ni;
+    }
     out.vx[i] = vxn;
     out.vy[i] = vyn;
-    out.x[i] = xi + K.dt * vxn / ni;
-    out.y[i] = yi + K.dt * vyn / ni;
+    out.x[i] = xi + sxn;
+    out.y[i] = yi + syn;
     out.rho[i] = rti + K.dt * Dr;
     Pbuf[i] = Px;
     Pbuf[n + i] = Py;
@@ -600,6 +658,7 @@ __global__ void __launch_bounds__(WB) k_wc_adj_local(int64_t n, const int8_t* __
 // and the factors that belong to k alone are applied after the loop: 55 FP64
 // operations a pair instead of about 130.  A wall's weights are zero.
 // 14600 particles: 134 us before, 70 us.
+template <int L>
 __global__ void __launch_bounds__(WPB) k_wc_adj_pair(
     int64_t n, State S, WcK K, St s0, const int32_t* __restrict__ nbr, const int32_t* __restrict__ cnt, Pre pq,
     const double* __restrict__ geo, int64_t slots, const double* __restrict__ nbuf, AdjPair ap,
@@ -611,8 +670,9 @@ __global__ void __launch_bounds__(WPB) k_wc_adj_pair(
     const int G = K.gnx * K.gny;
     for (int e = threadIdx.x; e < G; e += WPB) wb[e] = 0.0;
     __syncwarp();
-    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const bool act = k < n && S.tid[k] == BSC_TID_FLUID;
+    const Lanes<L> ls;
+    const int64_t k = ls.particle();
+    const bool act = k < n && S.tid[k] == BSC_TID_FLUID, first = ls.sub == 0;
     double lnk = 0.0;
     if (act) {
         const double xk = s0.x[k], yk = s0.y[k], vxk = s0.vx[k], vyk = s0.vy[k];
@@ -620,10 +680,17 @@ __global__ void __launch_bounds__(WPB) k_wc_adj_pair(
         const double irk = 1.0 / pq.rt[k], Vk_rt = Vk * irk;
         const double lDk = lD[k];
         const double2 vlak = ap.vla[k], nlak = ap.nla[k], abk = ap.ab[k];
-        double lvx = lvl[k], lvy = lvl[n + k], lrt = lrl[k], lxx = lam_in.x[k], lyy = lam_in.y[k];
+        double lvx = 0.0, lvy = 0.0, lrt = 0.0, lxx = 0.0, lyy = 0.0;
+        if (first) {
+            lvx = lvl[k];
+            lvy = lvl[n + k];
+            lrt = lrl[k];
+            lxx = lam_in.x[k];
+            lyy = lam_in.y[k];
+        }
         double SD = 0.0, S2 = 0.0, SP = 0.0, SV = 0.0;  // sum G D, G c2 lamD_j del, F M.d, G 2 nu lam_a,j.dv
         const int m = cnt[k];
-        for (int q = 0; q < m; ++q) {
+        for (int q = ls.sub; q < m; q += L) {
             const int64_t e = ell(k, q, K.kmax);
             const int j = nbr[e];
             const double F = geo[e], Fr = geo[slots + e], G_ = geo[2 * slots + e], Gr = geo[3 * slots + e];
@@ -647,30 +714,42 @@ __global__ void __launch_bounds__(WPB) k_wc_adj_pair(
             lxx += QF * dvx - psF * Mx + C * dx;
             lyy += QF * dvy - psF * My + C * dy;
         }
-        lrt += SD - Vk_rt * S2 + 2.0 * prk * irk * SP + mk * irk * irk * SV;
-        lyy -= pq.drh[k] * SD;
-        const double lp = -irk * irk * SP;
-        // porosity n_k = 1 - sum_s (1 - phi_s) V_s W(r_ks)
-        lnk = ln[k];
-        lxx += lnk * dn[k];
-        lyy += lnk * dn[n + k];
-        // pressure and the clamp
-        lrt += lp * pq.dpdr[k];
-        lam_out.x[k] = lxx;
-        lam_out.y[k] = lyy;
-        lam_out.vx[k] = lvx;
-        lam_out.vy[k] = lvy;
-        lam_out.rho[k] = s0.rho[k] >= K.rho0 ? lrt : 0.0;
-    } else if (k < n) {
+        lvx = ls.sum(lvx);
+        lvy = ls.sum(lvy);
+        lrt = ls.sum(lrt);
+        lxx = ls.sum(lxx);
+        lyy = ls.sum(lyy);
+        SD = ls.sum(SD);
+        S2 = ls.sum(S2);
+        SP = ls.sum(SP);
+        SV = ls.sum(SV);
+        if (first) {
+            lrt += SD - Vk_rt * S2 + 2.0 * prk * irk * SP + mk * irk * irk * SV;
+            lyy -= pq.drh[k] * SD;
+            const double lp = -irk * irk * SP;
+            // porosity n_k = 1 - sum_s (1 - phi_s) V_s W(r_ks)
+            lnk = ln[k];
+            lxx += lnk * dn[k];
+            lyy += lnk * dn[n + k];
+            // pressure and the clamp
+            lrt += lp * pq.dpdr[k];
+            lam_out.x[k] = lxx;
+            lam_out.y[k] = lyy;
+            lam_out.vx[k] = lvx;
+            lam_out.vy[k] = lvy;
+            lam_out.rho[k] = s0.rho[k] >= K.rho0 ? lrt : 0.0;
+        }
+    } else if (k < n && first) {
         lam_out.x[k] = lam_out.y[k] = lam_out.vx[k] = lam_out.vy[k] = lam_out.rho[k] = 0.0;
     }
+    __syncwarp();
     // d n_k / d phi_g = sum over cell g's solids of V_s W(r_ks): lanes with the
     // same cell are summed in lane order by the lowest of them
     const int lane = threadIdx.x;
     for (int u = 0; u < K.gc; ++u) {
         int g = -1;
         double v = 0.0;
-        if (act) {
+        if (act && first) {
             g = pgi[u * n + k];
             v = lnk * pgv[u * n + k];
         }
@@ -797,24 +876,33 @@ int wc_step(Ctx* c, WcState* w, double* nbuf, double* Pbuf, const Keep* keep, bo
     if (!rc) rc = cells_build(c, false);
     if (!rc) rc = last ? op_neighbour(c) : op_neighbour_lists(c);
     if (!rc) {
-        const unsigned g = blocks_for(n, WB), gp = blocks_for(n, WPB);
+        const unsigned g = blocks_for(n, WB);
+        const int lanes = lanes_for(n);
         const State S = wc_view(c, w);
         k_wc_pre<<<g, WB, 0, c->stream>>>(n, S.tid, S.mass, S.y, S.rho, w->K, pre);
         rc = launch_check(c);
         if (!rc) {
-            if (keep)
-                k_wc_por<true><<<gp, WPB, 0, c->stream>>>(n, S, c->K, w->K, c->pcell, c->posf, c->scell_start,
-                                                          c->scell_count, c->sposf, c->sx, c->sy, w->sw, c->svol,
-                                                          w->sg, nbuf, keep->por);
-            else
-                k_wc_por<false><<<gp, WPB, 0, c->stream>>>(n, S, c->K, w->K, c->pcell, c->posf, c->scell_start,
-                                                           c->scell_count, c->sposf, c->sx, c->sy, w->sw, c->svol,
-                                                           w->sg, nbuf, PorKeep{});
+            with_lanes(std::max(lanes, 4), [&](auto L) {
+                constexpr int l = decltype(L)::value;
+                const unsigned gp = blocks_for(n * l, WPB);
+                if (keep)
+                    k_wc_por<true, l><<<gp, WPB, 0, c->stream>>>(n, S, c->K, w->K, c->pcell, c->posf, c->scell_start,
+                                                                 c->scell_count, c->sposf, c->sx, c->sy, w->sw,
+                                                                 c->svol, w->sg, nbuf, keep->por);
+                else
+                    k_wc_por<false, l><<<gp, WPB, 0, c->stream>>>(n, S, c->K, w->K, c->pcell, c->posf,
+                                                                  c->scell_start, c->scell_count, c->sposf, c->sx,
+                                                                  c->sy, w->sw, c->svol, w->sg, nbuf, PorKeep{});
+            });
             rc = launch_check(c);
         }
         if (!rc) {
-            k_wc_step<<<gp, WPB, 0, c->stream>>>(n, S, w->K, c->nbr, c->cnt, pre, nbuf, st_of(w->nxt, n), Pbuf,
-                                               keep ? keep->geo : nullptr, list_slots(c));
+            with_lanes(lanes, [&](auto L) {
+                constexpr int l = decltype(L)::value;
+                k_wc_step<l><<<blocks_for(n * l, WPB), WPB, 0, c->stream>>>(
+                    n, S, w->K, c->nbr, c->cnt, pre, nbuf, st_of(w->nxt, n), Pbuf, keep ? keep->geo : nullptr,
+                    list_slots(c));
+            });
             rc = launch_check(c);
         }
     }
@@ -896,7 +984,7 @@ int bsc_wcsph_setup(bsc_ctx* c, const bsc_wcsph_params* p) {
         (rc = wc_alloc(c, w, &w->dpdr, n)) ||
         (rc = wc_alloc(c, w, &w->nxt, 5 * n)) ||
         (rc = wc_alloc(c, w, &w->xp, BSC_WCSPH_MAX_PROBES)) ||
-        (rc = wc_alloc(c, w, &w->part, (int64_t)blocks_for(n, WPB) * (2 + BSC_WCSPH_MAX_GRID))) ||
+        (rc = wc_alloc(c, w, &w->part, (int64_t)std::max(blocks_for(n * lanes_for(n), WPB), blocks_for(n, WB)) * (2 + BSC_WCSPH_MAX_GRID))) ||
         (rc = wc_alloc(c, w, &w->lam, 5 * n)) || (rc = wc_alloc(c, w, &w->lamn, 5 * n)) ||
         (rc = wc_alloc(c, w, &w->adj2, 3 * n)) || (rc = wc_alloc(c, w, &w->lD, n)) || (rc = wc_alloc(c, w, &w->ln, n)) ||
         (rc = wc_alloc(c, w, &w->lvl, 2 * n)) || (rc = wc_alloc(c, w, &w->lrl, n)) ||
@@ -1033,14 +1121,17 @@ int bsc_wcsph_adjoint(bsc_ctx* c, const double* dJ_deta, double* grad) {
             const Keep kq = seg_keep(w, q, n, slots);
             const double* nq = w->segn + (int64_t)q * n;
             const AdjPair ap{w->adj2, w->adj2 + n, w->adj2 + 2 * n};
-            const unsigned nbp = blocks_for(n, WPB);
+            const int lanes = lanes_for(n);
+            const unsigned nbp = blocks_for(n * lanes, WPB);
             k_wc_adj_local<<<nb, WB, 0, c->stream>>>(n, c->S.tid, w->K, st0, st1, nq, w->segP + (int64_t)q * 2 * n,
                                                      kq.pre.rt, lam, ap, w->lD, w->ln, w->lvl, w->lrl, w->part,
                                                      pstride);
             BSC_LAUNCH(c);
-            k_wc_adj_pair<<<nbp, WPB, 0, c->stream>>>(n, S, w->K, st0, kq.nbr, kq.cnt, kq.pre, kq.geo, slots, nq, ap,
-                                                      w->lD, w->ln, w->lvl, w->lrl, lam, lamn, kq.por.dn, kq.por.pgi,
-                                                      kq.por.pgv, w->part, pstride);
+            with_lanes(lanes, [&](auto L) {
+                k_wc_adj_pair<decltype(L)::value><<<nbp, WPB, 0, c->stream>>>(
+                    n, S, w->K, st0, kq.nbr, kq.cnt, kq.pre, kq.geo, slots, nq, ap, w->lD, w->ln, w->lvl, w->lrl, lam,
+                    lamn, kq.por.dn, kq.por.pgi, kq.por.pgv, w->part, pstride);
+            });
             BSC_LAUNCH(c);
             k_wc_grad<<<2 + G, WB, 0, c->stream>>>((int)nb, (int)nbp, pstride, w->part, w->grad);
             BSC_LAUNCH(c);
