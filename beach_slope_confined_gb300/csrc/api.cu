@@ -114,11 +114,13 @@ static void derive_kparams(Ctx* c) {
     K.dl = P.dl;
     K.rho0 = P.rho0;
     K.rel_den = P.rel_den;
+    K.inv_rho_sea = 1.0 / (K.rho0 * K.rel_den);
     K.g = P.g;
     K.csh = P.csh;
     K.maxshift = P.maxshift;
     K.free_thr = P.free_threshold;
     K.por = P.por;
+    K.por_le1 = P.por <= 1.0;
     K.alpha = P.darcy_alpha;
     K.beta = P.forch_beta;
     K.d50 = P.d50;
@@ -646,6 +648,7 @@ int bsc_upload_porosity(bsc_ctx* c, int32_t nx, int32_t ny, double x0, double y0
     c->hpgrid.assign(v, v + (int64_t)nx * ny);
     c->K.pnx = nx; c->K.pny = ny; c->K.px0 = x0; c->K.py0 = y0; c->K.pdx = dx; c->K.pdy = dy;
     c->K.pgrid = c->pgrid;
+    c->K.por_le1 = c->K.por <= 1.0 && std::all_of(v, v + (int64_t)nx * ny, [](double q) { return q <= 1.0; });
     return BSC_OK;
 }
 

@@ -120,6 +120,11 @@ __device__ __forceinline__ double sqrt_nr(double x) {
     return fma(r0, e, r0);
 }
 
+// a / n for a porosity n that is 1 outside the porous layer: a quotient
+// by 1 is its numerator, and whole warps lie there.  An FP64 division is about
+// ten instructions on the pipe that bounds the kernels that take it.
+__device__ __forceinline__ double over_por(double a, double n) { return n == 1.0 ? a : a / n; }
+
 // a < b for non-negative doubles a and b (b finite), on the integer pipe:
 // the bit patterns of non-negative IEEE doubles order like their values, and
 // any a with the sign bit set (only a NaN can have it here) compares as not
@@ -139,6 +144,7 @@ struct KParams {
     int kernel;
     double h, H, H2, lam, dl, rho0, rel_den, g, csh, maxshift, free_thr;
     double H2x;  // sqrt_rn(d2) < H exactly when d2 < H2x (the reference's neighbour test)
+    double inv_rho_sea;  // 1 / (rho0 rel_den)
     double por, alpha, beta, d50;
     double eddy_cs, eddy_cv, eddy_ce, varts_ps;
     double bxmin, bxmax;
@@ -153,6 +159,7 @@ struct KParams {
     int pnx, pny;
     double px0, py0, pdx, pdy;
     const double* pgrid;
+    bool por_le1;  // no porosity of the field (or outside it) above 1: the solid fraction's cap is never below 0
 };
 
 struct Ctx;

@@ -55,12 +55,21 @@ __global__ void __launch_bounds__(NB_BLOCK) k_assemble(int64_t n, State S, KPara
     const R L0 = (R)S.L0[i], L1 = (R)S.L1[i], L2 = (R)S.L2[i], L3 = (R)S.L3[i];
     const double usxi = usx[i], usyi = usy[i];
     auto quot = [](double a, double d) -> double { return FAST ? a * rcp_nr(d) : a / d; };
-    const R mi_over_rhoi = (R)quot(S.mass[i], S.rho[i]);
-    const R lamp_f = (R)(1.0 / (K.rho0 * K.rel_den));
+    const R lamp_f = (R)K.inv_rho_sea;
     // per-row quotients hoisted out of the pair loop (FP64 divisions are
-    // expensive on this GPU): 1/n_i, and v*_i/n_i for the fixed-wall rows
-    const R inv_ni = (R)quot(1.0, ni);
-    const double vxi_n = quot(S.vxs[i], (double)ni), vyi_n = quot(S.vys[i], (double)ni);
+    // expensive on this GPU), each for the rows that read it: 1/n_i (fluid
+    // rows), m_i/rho_i and v*_i/n_i (fixed-wall rows), and 2 q_i q_j / (q_i +
+    // q_j) with a neighbour of the same q
+    R mi_over_rhoi = 0, inv_ni = 0, rho_ii = 0;
+    double vxi_n = 0.0, vyi_n = 0.0;
+    if (tid_i == BSC_TID_FLUID) {
+        inv_ni = ni == (R)1 ? (R)1 : (R)quot(1.0, ni);
+        rho_ii = (R)quot((R)2 * qi * qi, qi + qi);
+    } else if (tid_i == BSC_TID_WALL) {
+        mi_over_rhoi = (R)quot(S.mass[i], S.rho[i]);
+        vxi_n = quot(S.vxs[i], (double)ni);
+        vyi_n = quot(S.vys[i], (double)ni);
+    }
     const int m = cnt[i];
     R dia = 0, fv = 0;
     for (int k = 0; k < m; ++k) {
@@ -83,7 +92,7 @@ __global__ void __launch_bounds__(NB_BLOCK) k_assemble(int64_t n, State S, KPara
             if (tid_j == BSC_TID_FLUID) {
                 // 2 rho_i rho_j / (n_i n_j (rho_i/n_i + rho_j/n_j)) = 2 q_i q_j / (q_i + q_j)
                 const R qj = (R)q[j];
-                const R rho_ij = (R)quot((R)2 * qi * qj, qi + qj);
+                const R rho_ij = qj == qi ? rho_ii : (R)quot((R)2 * qi * qj, qi + qj);
                 ddx = rho_ij * (R)(usx[j] - usxi);
                 ddy = rho_ij * (R)(usy[j] - usyi);
             } else {
@@ -164,7 +173,7 @@ __global__ void k_asm_df_pre(int64_t n, State S, KParams K, const int32_t* __res
     pre[n + i] = df_pack(df_of(S.y[i] - (K.gy0 + cy * K.cs)));
     pre[2 * n + i] = df_pack(df_of(S.vol[i]));
     pre[3 * n + i] = df_pack(df_of(q[i]));
-    pre[4 * n + i] = df_pack(df_of(1.0 + S.oden[i] * (1.0 / (K.rho0 * K.rel_den))));
+    pre[4 * n + i] = df_pack(df_of(1.0 + S.oden[i] * K.inv_rho_sea));
 }
 
 __global__ void __launch_bounds__(NB_BLOCK) k_assemble_df(int64_t n, State S, KParams K,
@@ -199,7 +208,7 @@ __global__ void __launch_bounds__(NB_BLOCK) k_assemble_df(int64_t n, State S, KP
     const df2 mi_over_rhoi = df_mul(df_of(S.mass[i]), df_rcp(df_of(S.rho[i])));
     const df2 inv_ni = df_rcp(df_of(ni64));
     const double vxsi = S.vxs[i], vysi = S.vys[i];
-    const double vxi_n = vxsi / ni64, vyi_n = vysi / ni64;
+    const double vxi_n = tid_i == BSC_TID_WALL ? vxsi / ni64 : 0.0, vyi_n = tid_i == BSC_TID_WALL ? vysi / ni64 : 0.0;
     const int m = cnt[i];
     df2 dia{0.0f, 0.0f}, fv{0.0f, 0.0f};
     for (int k = 0; k < m; ++k) {
@@ -292,9 +301,9 @@ __global__ void k_vs_over_por(int64_t n, State S, double* __restrict__ q, double
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double nn = S.por[i];
-    q[i] = S.rho[i] / nn;
-    ux[i] = S.vxs[i] / nn;
-    uy[i] = S.vys[i] / nn;
+    q[i] = over_por(S.rho[i], nn);
+    ux[i] = over_por(S.vxs[i], nn);
+    uy[i] = over_por(S.vys[i], nn);
 }
 
 // the V-cycle's packed FP16 entries (EllPack16) of the assembled rows: one
