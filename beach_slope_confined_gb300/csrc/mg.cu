@@ -275,14 +275,14 @@ __device__ __forceinline__ T smooth_at(int nx, int ny, int c, const T* A, const 
         if (MODE == 2) return xin[g] + scale * xc[(gx >> 1) * nyc + (gy >> 1)];
         return xin[g];
     };
-    T ax = 0;
+    T ax[3] = {0, 0, 0};  // a chain per stencil row
 #pragma unroll
     for (int s = 0; s < 9; ++s) {
         const int gx = cx + s / 3 - 1, gy = cy + s % 3 - 1;
         if (gx < 0 || gx >= nx || gy < 0 || gy >= ny) continue;
-        ax += A[s * nc + c] * xv(gx, gy);  // no test on the loaded value: loads stay independent
+        ax[s / 3] += A[s * nc + c] * xv(gx, gy);  // no test on the loaded value: loads stay independent
     }
-    return xv(cx, cy) + w * dinv[c] * (b[c] - ax);
+    return xv(cx, cy) + w * dinv[c] * (b[c] - ((ax[0] + ax[1]) + ax[2]));
 }
 
 // the residual b - A x summed over the 2x2 children of coarse cell C
@@ -327,45 +327,70 @@ __global__ void __launch_bounds__(MG_BLOCK) k_mg_smooth(int nx, int ny, const T*
     if (!mg_skip(sk)) xout[c] = v;
 }
 
-// Both post-sweeps of a cell level in one launch: a block owns a tile of
-// PT_X x PT_Y cells (PT_Y along the grid's contiguous y index) and computes
-// the first sweep (prolonged correction folded in, weight w) on the tile and
-// its one-cell ring into shared memory, then the second sweep (weight w1) on
-// the tile from there.  The ring's first sweep is recomputed by the
-// neighbouring blocks (a third more first-sweep work) and one launch of the
-// latency-bound chain is saved per level.
+// Both post-sweeps of a cell level in one launch.  A block owns a tile of
+// PT_X x PT_Y cells (PT_Y along the grid's contiguous y index): the prolonged
+// correction on the tile and two cells around it, the first sweep (weight w)
+// on the tile and one cell around it, the second (w1) on the tile, from shared
+// memory each.  The rings are recomputed by the neighbouring blocks, and one
+// launch of the latency-bound chain is saved per level.  A thread has one cell
+// of the first sweep, threads of the tile the same cell in both, so the
+// stencil, diagonal and right-hand side load once, ahead of the first barrier
+// (with 256 threads looping over the 340 cells, and the neighbours' values
+// formed by every reader, a level took 10-12 us, FP64's finest 29).  With the
+// sums below in several chains (an FP64 result takes ~140 clocks to its next
+// use), the cell levels of a V-cycle went from 72 to 63 us at 846k rows mixed,
+// 129 to 111 in FP64, 74 to 61 at 198k FP64.
 constexpr int PT_X = 8, PT_Y = 32;
 constexpr int PT_HX = PT_X + 2, PT_HY = PT_Y + 2;
+constexpr int PT_VX = PT_X + 4, PT_VY = PT_Y + 4;
+constexpr int PT_THREADS = (PT_HX * PT_HY + 31) / 32 * 32;
 template <typename T>
-__global__ void __launch_bounds__(PT_X * PT_Y) k_mg_post2(int nx, int ny, const T* __restrict__ A,
-                                                           const T* __restrict__ dinv, const T* __restrict__ b,
-                                                           const T* __restrict__ xin, const T* __restrict__ xc,
-                                                           int nyc, T scale, T w, T w1, T* __restrict__ xout,
-                                                           const Scalars* __restrict__ sk) {
-    __shared__ T y1[PT_HX * PT_HY];
-    const int nc = nx * ny;
-    const int x0 = blockIdx.x * PT_X - 1, y0 = blockIdx.y * PT_Y - 1;  // ring origin
-    for (int h = threadIdx.x; h < PT_HX * PT_HY; h += blockDim.x) {
-        const int gx = x0 + h / PT_HY, gy = y0 + h % PT_HY;
-        T v = 0;
-        if (gx >= 0 && gx < nx && gy >= 0 && gy < ny)
-            v = smooth_at<T, 2>(nx, ny, gx * ny + gy, A, dinv, b, xin, xc, nyc, scale, w);
-        y1[h] = v;
+__global__ void __launch_bounds__(PT_THREADS) k_mg_post2(int nx, int ny, const T* __restrict__ A,
+                                                          const T* __restrict__ dinv, const T* __restrict__ b,
+                                                          const T* __restrict__ xin, const T* __restrict__ xc,
+                                                          int nyc, T scale, T w, T w1, T* __restrict__ xout,
+                                                          const Scalars* __restrict__ sk) {
+    __shared__ T v[PT_VX * PT_VY], y1[PT_HX * PT_HY];
+    const int nc = nx * ny, t = threadIdx.x;
+    const int x0 = blockIdx.x * PT_X, y0 = blockIdx.y * PT_Y;  // tile origin
+    // this thread's cell, relative to the tile: the tile's first, then its ring
+    int rx, ry;
+    if (t < PT_X * PT_Y) {
+        rx = t / PT_Y;
+        ry = t % PT_Y;
+    } else {
+        const int q = t - PT_X * PT_Y;  // rows above and below (PT_HY each), then the two columns
+        rx = q < PT_HY ? -1 : q < 2 * PT_HY ? PT_X : (q - 2 * PT_HY) >> 1;
+        ry = q < 2 * PT_HY ? q % PT_HY - 1 : ((q - 2 * PT_HY) & 1 ? PT_Y : -1);
     }
-    __syncthreads();
-    const int tx = threadIdx.x / PT_Y, ty = threadIdx.x % PT_Y;
-    const int cx = x0 + 1 + tx, cy = y0 + 1 + ty;
-    if (cx >= nx || cy >= ny) return;
-    const int c = cx * ny + cy;
-    T ax = 0;
+    const int cx = x0 + rx, cy = y0 + ry, c = cx * ny + cy;
+    const bool ring = t < PT_HX * PT_HY, in = ring && cx >= 0 && cx < nx && cy >= 0 && cy < ny;
+    T a[9], d = 0, bc = 0;
 #pragma unroll
-    for (int q = 0; q < 9; ++q) {
-        const int gx = cx + q / 3 - 1, gy = cy + q % 3 - 1;
-        if (gx < 0 || gx >= nx || gy < 0 || gy >= ny) continue;
-        ax += A[q * nc + c] * y1[(tx + q / 3) * PT_HY + (ty + q % 3)];
+    for (int q = 0; q < 9; ++q) a[q] = in ? A[q * nc + c] : (T)0;
+    if (in) {
+        d = dinv[c];
+        bc = b[c];
     }
-    const T v = y1[(tx + 1) * PT_HY + (ty + 1)] + w1 * dinv[c] * (b[c] - ax);
-    if (!mg_skip(sk)) xout[c] = v;
+    for (int h = t; h < PT_VX * PT_VY; h += PT_THREADS) {
+        const int gx = x0 - 2 + h / PT_VY, gy = y0 - 2 + h % PT_VY;
+        // zero outside the grid, where the stencil's coefficients may be anything
+        v[h] = gx >= 0 && gx < nx && gy >= 0 && gy < ny ? xin[gx * ny + gy] + scale * xc[(gx >> 1) * nyc + (gy >> 1)]
+                                                        : (T)0;
+    }
+    const bool skip = mg_skip(sk);
+    __syncthreads();
+    // a damped-Jacobi update from the 3x3 values around p, W to a row: a chain per stencil row
+    auto sweep = [&](const T* p, int W, T weight) -> T {
+        T s[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+            s[q] = (a[3 * q] * p[(q - 1) * W - 1] + a[3 * q + 1] * p[(q - 1) * W]) + a[3 * q + 2] * p[(q - 1) * W + 1];
+        return p[0] + weight * d * (bc - ((s[0] + s[1]) + s[2]));
+    };
+    if (ring) y1[(rx + 1) * PT_HY + ry + 1] = in ? sweep(v + (rx + 2) * PT_VY + ry + 2, PT_VY, w) : (T)0;
+    __syncthreads();
+    if (t < PT_X * PT_Y && in && !skip) xout[c] = sweep(y1 + (rx + 1) * PT_HY + ry + 1, PT_HY, w1);
 }
 
 // Four sweeps per cell level (BSC_MG_CELL_SWEEPS=4), each direction in one
@@ -579,13 +604,13 @@ __global__ void __launch_bounds__(MG_BLOCK) k_mg_pre_restrict(int nx, int ny, co
     const int CX = C / nyc, CY = C - CX * nyc, x0 = 2 * CX - 2, y0 = 2 * CY - 2;
     // the weights of patch cells outside the grid are exactly zero: clamped,
     // unconditional loads keep all 72 in flight
-    T sum = 0;
+    T sum[MG_RPATCH] = {};  // a chain per patch row
 #pragma unroll
     for (int k = 0; k < MG_RW; ++k) {
         const int gx = min(max(x0 + k / MG_RPATCH, 0), nx - 1), gy = min(max(y0 + k % MG_RPATCH, 0), ny - 1);
-        sum += R[k * ncc + C] * b[gx * ny + gy];
+        sum[k / MG_RPATCH] += R[k * ncc + C] * b[gx * ny + gy];
     }
-    if (!mg_skip(sk)) bc[C] = sum;
+    if (!mg_skip(sk)) bc[C] = ((sum[0] + sum[1]) + (sum[2] + sum[3])) + (sum[4] + sum[5]);
 }
 
 // ---- the small levels as one dense operator ------------------------------------------
@@ -731,22 +756,35 @@ __global__ void __launch_bounds__(MG_DENSE_BLOCK) k_mg_dense_apply(int nc, const
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (i >= nc) return;
     const T* row = M + (int64_t)i * ld;
-    T s[V] = {};
+    constexpr int C = 8 / V;  // loads in flight, each its own chains
+    T s[8] = {};
     int j = 0;
     if (ld % V == 0) {  // rows on 16-byte boundaries
+        const Vec* m = reinterpret_cast<const Vec*>(row);
+        const Vec* v = reinterpret_cast<const Vec*>(b);
         const int full = nc / V;
-#pragma unroll 4
-        for (int q = lane; q < full; q += 32) {
-            const Vec m = reinterpret_cast<const Vec*>(row)[q], v = reinterpret_cast<const Vec*>(b)[q];
+        int q = lane;
+        for (; q + 32 * (C - 1) < full; q += 32 * C) {
+            Vec mv[C], bv[C];
 #pragma unroll
-            for (int u = 0; u < V; ++u) s[u] += m.v[u] * v.v[u];
+            for (int c = 0; c < C; ++c) {
+                mv[c] = m[q + 32 * c];
+                bv[c] = v[q + 32 * c];
+            }
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+#pragma unroll
+                for (int u = 0; u < V; ++u) s[c * V + u] += mv[c].v[u] * bv[c].v[u];
+        }
+        for (; q < full; q += 32) {
+            const Vec mv = m[q], bv = v[q];
+#pragma unroll
+            for (int u = 0; u < V; ++u) s[u] += mv.v[u] * bv.v[u];
         }
         j = full * V;
     }
     for (j += lane; j < nc; j += 32) s[0] += row[j] * b[j];
-    T t = s[0];
-#pragma unroll
-    for (int u = 1; u < V; ++u) t += s[u];
+    T t = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     if (lane == 0 && !mg_skip(sk)) x[i] = t;
@@ -1146,7 +1184,7 @@ int cycle_level(Ctx* c, int l) {
     // sweep writes x_l
     if (nup == 2 && c->mg_post_fused) {  // both sweeps in one launch
         const dim3 gt((unsigned)((L.nx + PT_X - 1) / PT_X), (unsigned)((L.ny + PT_Y - 1) / PT_Y));
-        k_mg_post2<T><<<gt, PT_X * PT_Y, 0, c->stream>>>(L.nx, L.ny, v.A, v.dinv, v.b, cur, vc.x, Lc.ny, sc, wp, w1,
+        k_mg_post2<T><<<gt, PT_THREADS, 0, c->stream>>>(L.nx, L.ny, v.A, v.dinv, v.b, cur, vc.x, Lc.ny, sc, wp, w1,
                                                           v.x, c->mg.skip);
         BSC_LAUNCH(c);
         return BSC_OK;
