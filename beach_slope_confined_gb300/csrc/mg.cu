@@ -271,7 +271,7 @@ __device__ __forceinline__ T smooth_at(int nx, int ny, int c, const T* A, const 
     const int cx = c / ny, cy = c - cx * ny;
     auto xv = [&](int gx, int gy) -> T {
         const int g = gx * ny + gy;
-        if (MODE == 1) return w0 * dinv[g] * b[g];
+        if (MODE == 1) return dinv[g] * b[g];  // times w0, taken out of the sum
         if (MODE == 2) return xin[g] + scale * xc[(gx >> 1) * nyc + (gy >> 1)];
         return xin[g];
     };
@@ -279,10 +279,14 @@ __device__ __forceinline__ T smooth_at(int nx, int ny, int c, const T* A, const 
 #pragma unroll
     for (int s = 0; s < 9; ++s) {
         const int gx = cx + s / 3 - 1, gy = cy + s % 3 - 1;
-        if (gx < 0 || gx >= nx || gy < 0 || gy >= ny) continue;
-        ax[s / 3] += A[s * nc + c] * xv(gx, gy);  // no test on the loaded value: loads stay independent
+        const bool in = gx >= 0 && gx < nx && gy >= 0 && gy < ny;
+        // clamped, unconditional loads: all of them in flight
+        const T a = A[s * nc + c], y = xv(min(max(gx, 0), nx - 1), min(max(gy, 0), ny - 1));
+        ax[s / 3] += (in ? a : (T)0) * y;
     }
-    return xv(cx, cy) + w * dinv[c] * (b[c] - ((ax[0] + ax[1]) + ax[2]));
+    const T sum = (ax[0] + ax[1]) + ax[2], own = xv(cx, cy);
+    if (MODE == 1) return w0 * own + w * dinv[c] * (b[c] - w0 * sum);
+    return own + w * dinv[c] * (b[c] - sum);
 }
 
 // the residual b - A x summed over the 2x2 children of coarse cell C
@@ -585,32 +589,44 @@ __global__ void k_mg_build_R(int nx, int ny, const T* __restrict__ A, const T* _
 
 // pre-smoothing of level l (blocks [0, nbs): two sweeps from zero, as
 // k_mg_smooth<1>) and the restriction to level l+1 through R (the other
-// blocks), in one launch
+// blocks), in one launch.  Bound: latency.  A restricting block takes 32
+// coarse cells, a warp per row of their patches, so that a thread has 12 loads
+// where one thread per coarse cell had 72 (of which the compiler kept a few in
+// flight: 9.5 us a launch however small the level, 4.4 now; the 260k cells of
+// 850k particles 13.5 us in FP32 and 28 in FP64, 8.2 and 21.5 now).
+constexpr int PR_BLOCK = 32 * MG_RPATCH;
 template <typename T>
-__global__ void __launch_bounds__(MG_BLOCK) k_mg_pre_restrict(int nx, int ny, const T* __restrict__ A,
+__global__ void __launch_bounds__(PR_BLOCK) k_mg_pre_restrict(int nx, int ny, const T* __restrict__ A,
                                                                const T* __restrict__ dinv, const T* __restrict__ b,
                                                                T scale, T w, T w0, T* __restrict__ xout, int nbs,
                                                                int nxc, int nyc, const T* __restrict__ R,
                                                                T* __restrict__ bc, const Scalars* __restrict__ sk) {
     if ((int)blockIdx.x < nbs) {
-        const int c = blockIdx.x * blockDim.x + threadIdx.x;
+        const int c = blockIdx.x * PR_BLOCK + threadIdx.x;
         if (c >= nx * ny) return;
         const T v = smooth_at<T, 1>(nx, ny, c, A, dinv, b, nullptr, nullptr, 0, scale, w, w0);
         if (!mg_skip(sk)) xout[c] = v;
         return;
     }
-    const int C = (blockIdx.x - nbs) * blockDim.x + threadIdx.x, ncc = nxc * nyc;
-    if (C >= ncc) return;
-    const int CX = C / nyc, CY = C - CX * nyc, x0 = 2 * CX - 2, y0 = 2 * CY - 2;
+    __shared__ T part[MG_RPATCH][32];
+    const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+    const int C = (blockIdx.x - nbs) * 32 + lane, ncc = nxc * nyc;
+    const int Cl = min(C, ncc - 1), CX = Cl / nyc, CY = Cl - CX * nyc;
     // the weights of patch cells outside the grid are exactly zero: clamped,
-    // unconditional loads keep all 72 in flight
-    T sum[MG_RPATCH] = {};  // a chain per patch row
+    // unconditional loads keep all of them in flight
+    const T* bx = b + (int64_t)min(max(2 * CX - 2 + row, 0), nx - 1) * ny;
+    T wt[MG_RPATCH], v[MG_RPATCH], sum = 0;
 #pragma unroll
-    for (int k = 0; k < MG_RW; ++k) {
-        const int gx = min(max(x0 + k / MG_RPATCH, 0), nx - 1), gy = min(max(y0 + k % MG_RPATCH, 0), ny - 1);
-        sum[k / MG_RPATCH] += R[k * ncc + C] * b[gx * ny + gy];
+    for (int k = 0; k < MG_RPATCH; ++k) {
+        wt[k] = R[(row * MG_RPATCH + k) * ncc + Cl];
+        v[k] = bx[min(max(2 * CY - 2 + k, 0), ny - 1)];
     }
-    if (!mg_skip(sk)) bc[C] = ((sum[0] + sum[1]) + (sum[2] + sum[3])) + (sum[4] + sum[5]);
+#pragma unroll
+    for (int k = 0; k < MG_RPATCH; ++k) sum += wt[k] * v[k];
+    part[row][lane] = sum;
+    __syncthreads();
+    if (row == 0 && C < ncc && !mg_skip(sk))
+        bc[C] = ((sum + part[1][lane]) + (part[2][lane] + part[3][lane])) + (part[4][lane] + part[5][lane]);
 }
 
 // ---- the small levels as one dense operator ------------------------------------------
@@ -1159,8 +1175,9 @@ int cycle_level(Ctx* c, int l) {
     }
     if (nu == 2 && L.R) {
         // both sweeps and the restriction in one launch
-        k_mg_pre_restrict<T><<<g + blocks_for(Lc.nc, MG_BLOCK), MG_BLOCK, 0, c->stream>>>(
-            L.nx, L.ny, v.A, v.dinv, v.b, sc, w1, w, cur, (int)g, Lc.nx, Lc.ny, (const T*)L.R, vc.b, c->mg.skip);
+        const unsigned gs = blocks_for(L.nc, PR_BLOCK);
+        k_mg_pre_restrict<T><<<gs + blocks_for(Lc.nc, 32), PR_BLOCK, 0, c->stream>>>(
+            L.nx, L.ny, v.A, v.dinv, v.b, sc, w1, w, cur, (int)gs, Lc.nx, Lc.ny, (const T*)L.R, vc.b, c->mg.skip);
         BSC_LAUNCH(c);
     } else {
     if (nu == 1)
