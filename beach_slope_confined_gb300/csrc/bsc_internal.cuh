@@ -198,6 +198,35 @@ template <typename T> struct Vec2;
 template <> struct Vec2<double> { using type = double2; };
 template <> struct Vec2<float> { using type = float2; };
 
+// ---- dependent launches ----------------------------------------------------------
+// The kernels of an FGMRES iteration are a chain, each a few microseconds long
+// on tanks that do not fill the GPU, and a plain launch costs its share of
+// that: the next kernel's blocks start only after the last one's have drained.
+// launch_dep lets a kernel's blocks start once every block of its predecessor
+// has (dep_start, the predecessor's first statement).  Until dep_wait they may
+// read only what no kernel since the chain's last plain launch writes: the
+// matrix and the cells' operators.  dep_wait returns when the predecessor has
+// completed and its writes are visible; every thread calls it, so that a
+// kernel's completion implies its predecessors'.  What is read after it must
+// not be a __restrict__ parameter (whose reads the compiler may move ahead).  After a plain launch both statements do nothing.
+__device__ __forceinline__ void dep_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// dep: false makes it a plain launch (the first of a chain, or after an event record)
+template <typename... P, typename... A>
+void launch_dep(cudaStream_t stream, bool dep, void (*f)(P...), dim3 grid, unsigned block, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.stream = stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = dep ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, f, static_cast<P>(args)...);  // BSC_LAUNCH reads the error
+}
+
 inline unsigned blocks_for(int64_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
 // ---- the context ---------------------------------------------------------------

@@ -350,10 +350,10 @@ constexpr int PT_VX = PT_X + 4, PT_VY = PT_Y + 4;
 constexpr int PT_THREADS = (PT_HX * PT_HY + 31) / 32 * 32;
 template <typename T>
 __global__ void __launch_bounds__(PT_THREADS) k_mg_post2(int nx, int ny, const T* __restrict__ A,
-                                                          const T* __restrict__ dinv, const T* __restrict__ b,
-                                                          const T* __restrict__ xin, const T* __restrict__ xc,
-                                                          int nyc, T scale, T w, T w1, T* __restrict__ xout,
-                                                          const Scalars* __restrict__ sk) {
+                                                          const T* __restrict__ dinv, const T* b, const T* xin,
+                                                          const T* xc, int nyc, T scale, T w, T w1,
+                                                          T* __restrict__ xout, const Scalars* sk) {
+    dep_start();
     __shared__ T v[PT_VX * PT_VY], y1[PT_HX * PT_HY];
     const int nc = nx * ny, t = threadIdx.x;
     const int x0 = blockIdx.x * PT_X, y0 = blockIdx.y * PT_Y;  // tile origin
@@ -372,10 +372,9 @@ __global__ void __launch_bounds__(PT_THREADS) k_mg_post2(int nx, int ny, const T
     T a[9], d = 0, bc = 0;
 #pragma unroll
     for (int q = 0; q < 9; ++q) a[q] = in ? A[q * nc + c] : (T)0;
-    if (in) {
-        d = dinv[c];
-        bc = b[c];
-    }
+    if (in) d = dinv[c];
+    dep_wait();
+    if (in) bc = b[c];
     for (int h = t; h < PT_VX * PT_VY; h += PT_THREADS) {
         const int gx = x0 - 2 + h / PT_VY, gy = y0 - 2 + h % PT_VY;
         // zero outside the grid, where the stencil's coefficients may be anything
@@ -597,15 +596,37 @@ __global__ void k_mg_build_R(int nx, int ny, const T* __restrict__ A, const T* _
 constexpr int PR_BLOCK = 32 * MG_RPATCH;
 template <typename T>
 __global__ void __launch_bounds__(PR_BLOCK) k_mg_pre_restrict(int nx, int ny, const T* __restrict__ A,
-                                                               const T* __restrict__ dinv, const T* __restrict__ b,
-                                                               T scale, T w, T w0, T* __restrict__ xout, int nbs,
-                                                               int nxc, int nyc, const T* __restrict__ R,
-                                                               T* __restrict__ bc, const Scalars* __restrict__ sk) {
+                                                               const T* __restrict__ dinv, const T* b, T w, T w0,
+                                                               T* __restrict__ xout, int nbs, int nxc, int nyc,
+                                                               const T* __restrict__ R, T* __restrict__ bc,
+                                                               const Scalars* sk) {
+    dep_start();
     if ((int)blockIdx.x < nbs) {
-        const int c = blockIdx.x * PR_BLOCK + threadIdx.x;
-        if (c >= nx * ny) return;
-        const T v = smooth_at<T, 1>(nx, ny, c, A, dinv, b, nullptr, nullptr, 0, scale, w, w0);
-        if (!mg_skip(sk)) xout[c] = v;
+        const int c = blockIdx.x * PR_BLOCK + threadIdx.x, nc = nx * ny, cl = min(c, nc - 1);
+        const int cx = cl / ny, cy = cl - cx * ny;
+        T a[9], d[9];
+        int g[9];
+#pragma unroll
+        for (int s = 0; s < 9; ++s) {  // clamped, unconditional loads: all of them in flight
+            const int gx = cx + s / 3 - 1, gy = cy + s % 3 - 1;
+            g[s] = min(max(gx, 0), nx - 1) * ny + min(max(gy, 0), ny - 1);
+            a[s] = A[s * nc + cl];
+            if (gx < 0 || gx >= nx || gy < 0 || gy >= ny) a[s] = 0;
+            d[s] = dinv[g[s]];
+        }
+        dep_wait();
+        T y[9], ax[3] = {0, 0, 0};  // a chain per stencil row
+#pragma unroll
+        for (int s = 0; s < 9; ++s) y[s] = b[g[s]];
+        const bool skip = mg_skip(sk);
+        const T bc4 = y[4];
+#pragma unroll
+        for (int s = 0; s < 9; ++s) {
+            y[s] *= d[s];
+            ax[s / 3] += a[s] * y[s];
+        }
+        // the first sweep, x = w0 D^-1 b, its weight taken out of the sum
+        if (c < nc && !skip) xout[c] = w0 * y[4] + w * d[4] * (bc4 - w0 * ((ax[0] + ax[1]) + ax[2]));
         return;
     }
     __shared__ T part[MG_RPATCH][32];
@@ -617,10 +638,10 @@ __global__ void __launch_bounds__(PR_BLOCK) k_mg_pre_restrict(int nx, int ny, co
     const T* bx = b + (int64_t)min(max(2 * CX - 2 + row, 0), nx - 1) * ny;
     T wt[MG_RPATCH], v[MG_RPATCH], sum = 0;
 #pragma unroll
-    for (int k = 0; k < MG_RPATCH; ++k) {
-        wt[k] = R[(row * MG_RPATCH + k) * ncc + Cl];
-        v[k] = bx[min(max(2 * CY - 2 + k, 0), ny - 1)];
-    }
+    for (int k = 0; k < MG_RPATCH; ++k) wt[k] = R[(row * MG_RPATCH + k) * ncc + Cl];
+    dep_wait();
+#pragma unroll
+    for (int k = 0; k < MG_RPATCH; ++k) v[k] = bx[min(max(2 * CY - 2 + k, 0), ny - 1)];
 #pragma unroll
     for (int k = 0; k < MG_RPATCH; ++k) sum += wt[k] * v[k];
     part[row][lane] = sum;
@@ -765,11 +786,13 @@ __global__ void __launch_bounds__(MG_DENSE_BLOCK) k_mg_dense_t(int nx, int ny, c
 // x = T b, a warp per row
 template <typename T>
 __global__ void __launch_bounds__(MG_DENSE_BLOCK) k_mg_dense_apply(int nc, const T* __restrict__ M, int ld,
-                                                                    const T* __restrict__ b, T* __restrict__ x,
-                                                                    const Scalars* __restrict__ sk) {
+                                                                    const T* b, T* __restrict__ x,
+                                                                    const Scalars* sk) {
+    dep_start();
     constexpr int V = 16 / sizeof(T);  // entries per load
     struct alignas(16) Vec { T v[V]; };
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    dep_wait();
     if (i >= nc) return;
     const T* row = M + (int64_t)i * ld;
     constexpr int C = 8 / V;  // loads in flight, each its own chains
@@ -972,6 +995,7 @@ template <typename T, typename Op>
 __global__ void __launch_bounds__(MG_BLOCK) k_mg0_pre2(int64_t n, Op A, const T* __restrict__ src, T* __restrict__ v,
                                                         T w, T w1, T* __restrict__ x,
                                                         const Scalars* __restrict__ sk) {
+    dep_start();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int m = A.cnt[i];
@@ -996,12 +1020,13 @@ __global__ void k_mg0_scale(int64_t n, const T* __restrict__ src, T* __restrict_
 
 // x_out = x + w (v - A x)
 template <typename T, typename Op>
-__global__ void __launch_bounds__(MG_BLOCK) k_mg0_sweep(int64_t n, Op A, const T* __restrict__ v,
-                                                         const T* __restrict__ x, T w, T* __restrict__ xout,
-                                                         const Scalars* __restrict__ sk) {
+__global__ void __launch_bounds__(MG_BLOCK) k_mg0_sweep(int64_t n, Op A, const T* v, const T* x, T w,
+                                                         T* __restrict__ xout, const Scalars* sk) {
+    dep_start();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int m = i < n ? A.cnt[i] : 0;
+    dep_wait();
     if (i >= n) return;
-    const int m = A.cnt[i];
     const T vi = v[i], xi = x[i];
     if (mg_skip(sk)) return;
     xout[i] = xi + w * (vi - A.template row<T, T>(i, x, m));
@@ -1009,12 +1034,13 @@ __global__ void __launch_bounds__(MG_BLOCK) k_mg0_sweep(int64_t n, Op A, const T
 
 // r = v - A x
 template <typename T, typename Op>
-__global__ void __launch_bounds__(MG_BLOCK) k_mg0_resid(int64_t n, Op A, const T* __restrict__ v,
-                                                         const T* __restrict__ x, T* __restrict__ r,
-                                                         const Scalars* __restrict__ sk) {
+__global__ void __launch_bounds__(MG_BLOCK) k_mg0_resid(int64_t n, Op A, const T* v, const T* x,
+                                                         T* __restrict__ r, const Scalars* sk) {
+    dep_start();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int m = i < n ? A.cnt[i] : 0;
+    dep_wait();
     if (i >= n) return;
-    const int m = A.cnt[i];
     const T vi = v[i];
     if (mg_skip(sk)) return;
     r[i] = vi - A.template row<T, T>(i, x, m);
@@ -1023,11 +1049,13 @@ __global__ void __launch_bounds__(MG_BLOCK) k_mg0_resid(int64_t n, Op A, const T
 // level-1 right-hand side: the residual summed over each cell's particles
 template <typename T>
 __global__ void k_mg0_restrict(int64_t nc, const int32_t* __restrict__ cell_start, const int32_t* __restrict__ cell_count,
-                               const int32_t* __restrict__ sorted, const T* __restrict__ r, T* __restrict__ b1,
-                               const Scalars* __restrict__ sk) {
+                               const int32_t* __restrict__ sorted, const T* r, T* __restrict__ b1,
+                               const Scalars* sk) {
+    dep_start();
     const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int q0 = c < nc ? cell_start[c] : 0, qn = c < nc ? cell_count[c] : 0;
+    dep_wait();
     if (c >= nc) return;
-    const int q0 = cell_start[c], qn = cell_count[c];
     if (mg_skip(sk)) return;
     T s = 0;
     for (int q = q0; q < q0 + qn; ++q) s += r[sorted[q]];
@@ -1042,14 +1070,16 @@ __global__ void k_mg0_restrict(int64_t nc, const int32_t* __restrict__ cell_star
 // diagonal), the same sums the level-1 Galerkin product is built from.
 // Reads 9 sums and 9 cell values per row instead of the row's entries.
 template <typename T>
-__global__ void __launch_bounds__(MG_BLOCK) k_mg0_post(int64_t n, int nx, int ny, const T* __restrict__ x,
-                                                        const T* __restrict__ r, const T* __restrict__ x1,
-                                                        const int32_t* __restrict__ pcell, const T* __restrict__ rs,
-                                                        T scale, T w, T* __restrict__ xout,
-                                                        const Scalars* __restrict__ sk) {
+__global__ void __launch_bounds__(MG_BLOCK) k_mg0_post(int64_t n, int nx, int ny, const T* x, const T* r,
+                                                        const T* x1, const int32_t* __restrict__ pcell,
+                                                        const T* __restrict__ rs, T scale, T w,
+                                                        T* __restrict__ xout, const Scalars* sk) {
+    dep_start();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int c = i < n ? pcell[i] : 0;
+    dep_wait();
     if (i >= n) return;
-    const int c = pcell[i], cx = c / ny, cy = c - cx * ny;
+    const int cx = c / ny, cy = c - cx * ny;
     const T xi = x[i], ri = r[i];
     if (mg_skip(sk)) return;
     T apx = 0;
@@ -1113,6 +1143,7 @@ int cycle_level(Ctx* c, int l) {
     const T w = (T)c->mg_w[0], w1 = (T)c->mg_w[1], sc = (T)c->P.mg_scale;
     const T wp = c->mg_wpost > 0 ? (T)c->mg_wpost : w;
     const int nu = c->P.mg_sweeps, nup = c->mg_post[0] > 0 ? c->mg_post[0] : nu;
+    const bool dep = !c->prof_iter;  // an event record precedes some of the launches then
     if (l >= mg.tail_l0 && mg.dense) {  // this level and all coarser ones as one product
         const bool coarsest = l == mg.nlev;
         const T* M = (const T*)L.T;
@@ -1123,8 +1154,8 @@ int cycle_level(Ctx* c, int l) {
                 M = mg.cinv;
         }
         const unsigned gd = blocks_for(L.nc * 32, MG_DENSE_BLOCK);
-        k_mg_dense_apply<T><<<gd, MG_DENSE_BLOCK, 0, c->stream>>>((int)L.nc, M, coarsest ? (int)L.nc : L.ldT, v.b,
-                                                                   v.x, mg.skip);
+        launch_dep(c->stream, dep, k_mg_dense_apply<T>, gd, MG_DENSE_BLOCK, (int)L.nc, M,
+                   coarsest ? (int)L.nc : L.ldT, v.b, v.x, mg.skip);
         BSC_LAUNCH(c);
         return BSC_OK;
     }
@@ -1176,8 +1207,8 @@ int cycle_level(Ctx* c, int l) {
     if (nu == 2 && L.R) {
         // both sweeps and the restriction in one launch
         const unsigned gs = blocks_for(L.nc, PR_BLOCK);
-        k_mg_pre_restrict<T><<<gs + blocks_for(Lc.nc, 32), PR_BLOCK, 0, c->stream>>>(
-            L.nx, L.ny, v.A, v.dinv, v.b, sc, w1, w, cur, (int)gs, Lc.nx, Lc.ny, (const T*)L.R, vc.b, c->mg.skip);
+        launch_dep(c->stream, dep, k_mg_pre_restrict<T>, gs + blocks_for(Lc.nc, 32), PR_BLOCK, L.nx, L.ny, v.A, v.dinv,
+                   v.b, w1, w, cur, (int)gs, Lc.nx, Lc.ny, (const T*)L.R, vc.b, c->mg.skip);
         BSC_LAUNCH(c);
     } else {
     if (nu == 1)
@@ -1201,8 +1232,8 @@ int cycle_level(Ctx* c, int l) {
     // sweep writes x_l
     if (nup == 2 && c->mg_post_fused) {  // both sweeps in one launch
         const dim3 gt((unsigned)((L.nx + PT_X - 1) / PT_X), (unsigned)((L.ny + PT_Y - 1) / PT_Y));
-        k_mg_post2<T><<<gt, PT_THREADS, 0, c->stream>>>(L.nx, L.ny, v.A, v.dinv, v.b, cur, vc.x, Lc.ny, sc, wp, w1,
-                                                          v.x, c->mg.skip);
+        launch_dep(c->stream, dep, k_mg_post2<T>, gt, PT_THREADS, L.nx, L.ny, v.A, v.dinv, v.b, cur, vc.x, Lc.ny, sc,
+                   wp, w1, v.x, c->mg.skip);
         BSC_LAUNCH(c);
         return BSC_OK;
     }
@@ -1234,7 +1265,8 @@ int vcycle(Ctx* c, const T* src, T* vin, T* z) {
     // one row per thread: the fine-level passes have no reduction, and a full
     // grid keeps more rows' loads in flight than a grid-stride loop over a
     // fixed grid (measured: 10% faster fine passes at 846k rows)
-    const int G = (int)blocks_for(n, MG_BLOCK);
+    const unsigned G = blocks_for(n, MG_BLOCK);
+    const bool dep = !c->prof_iter;  // an event record precedes some of the launches then
     if (c->prof_iter) record_event(c, c->ev_it[0]);
     T* cur = P0;
     const int nupre = c->mg_pre_fine > 0 ? c->mg_pre_fine : nu;
@@ -1245,15 +1277,16 @@ int vcycle(Ctx* c, const T* src, T* vin, T* z) {
     BSC_LAUNCH(c);
     for (int k = 2; k < nupre; ++k) {
         T* out = cur == P0 ? Q0 : P0;
-        k_mg0_sweep<T, AV><<<G, MG_BLOCK, 0, c->stream>>>(n, A, vin, cur, w1, out, c->mg.skip);
+        launch_dep(c->stream, dep, k_mg0_sweep<T, AV>, G, MG_BLOCK, n, A, vin, cur, w1, out, c->mg.skip);
         BSC_LAUNCH(c);
         cur = out;
     }
-    k_mg0_resid<T, AV><<<G, MG_BLOCK, 0, c->stream>>>(n, A, vin, cur, R0, c->mg.skip);
+    launch_dep(c->stream, dep, k_mg0_resid<T, AV>, G, MG_BLOCK, n, A, vin, cur, R0, c->mg.skip);
     BSC_LAUNCH(c);
     const MgLevel& L1 = mg.L[1];
     Lv<T> v1 = level_view<T>(L1);
-    k_mg0_restrict<T><<<blocks_for(L1.nc, MG_BLOCK), MG_BLOCK, 0, c->stream>>>(L1.nc, c->cell_start, c->cell_count, c->sorted, R0, v1.b, c->mg.skip);
+    launch_dep(c->stream, dep, k_mg0_restrict<T>, blocks_for(L1.nc, MG_BLOCK), MG_BLOCK, L1.nc, c->cell_start,
+               c->cell_count, c->sorted, R0, v1.b, c->mg.skip);
     BSC_LAUNCH(c);
     if (c->prof_iter) record_event(c, c->ev_it[1]);
     if (int rc = cycle_level<T>(c, 1)) return rc;
@@ -1267,10 +1300,10 @@ int vcycle(Ctx* c, const T* src, T* vin, T* z) {
     for (int k = 0; k < nup; ++k) {
         T* out = k == nup - 1 ? z : cur == P0 ? Q0 : P0;
         if (k == 0)
-            k_mg0_post<T><<<G, MG_BLOCK, 0, c->stream>>>(n, L1.nx, L1.ny, cur, R0, v1.x, c->pcell, rs, sc, wp, out,
-                                                         c->mg.skip);
+            launch_dep(c->stream, dep, k_mg0_post<T>, G, MG_BLOCK, n, L1.nx, L1.ny, cur, R0, v1.x, c->pcell, rs, sc,
+                       wp, out, c->mg.skip);
         else
-            k_mg0_sweep<T, AV><<<G, MG_BLOCK, 0, c->stream>>>(n, A, vin, cur, w1, out, c->mg.skip);
+            launch_dep(c->stream, dep, k_mg0_sweep<T, AV>, G, MG_BLOCK, n, A, vin, cur, w1, out, c->mg.skip);
         BSC_LAUNCH(c);
         cur = out;
     }

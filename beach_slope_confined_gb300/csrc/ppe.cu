@@ -1414,11 +1414,13 @@ int fg_cycle(Ctx* c, int m, int budget, Scalars* h, int* iters, Q queue) {
 
 // w = A z, one row per thread
 template <typename T, typename Op>
-__global__ void __launch_bounds__(RED_BLOCK) k_spmv(int64_t n, Op A, const T* __restrict__ z, T* __restrict__ w,
-                                                     const Scalars* __restrict__ sc) {
+__global__ void __launch_bounds__(RED_BLOCK) k_spmv(int64_t n, Op A, const T* z, T* __restrict__ w,
+                                                     const Scalars* sc) {
+    dep_start();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int m = i < n ? A.cnt[i] : 0;
+    dep_wait();
     if (i >= n) return;
-    const int m = A.cnt[i];
     if (fg_skip(sc)) return;
     w[i] = A.template row<T, T>(i, z, m);
 }
@@ -1463,12 +1465,14 @@ __device__ __forceinline__ bool gs_last_block(unsigned* ticket) {
 // the dots of w, 8 columns per pass, summed per thread in T; SPMV: w = A z
 // first (one row per thread: n <= gridDim.x * RED_BLOCK)
 template <bool SPMV, typename T, typename Op>
-__global__ void __launch_bounds__(RED_BLOCK) k_gs_dots(int64_t n, Op A, const T* __restrict__ z,
-                                                        const T* __restrict__ V, T* __restrict__ w, int j,
-                                                        double* __restrict__ part, const Scalars* __restrict__ sc,
-                                                        unsigned* __restrict__ ticket, double* Hd, FgLayout F) {
+__global__ void __launch_bounds__(RED_BLOCK) k_gs_dots(int64_t n, Op A, const T* z, const T* V,
+                                                        T* w, int j, double* __restrict__ part,
+                                                        const Scalars* sc, unsigned* ticket, double* Hd,
+                                                        FgLayout F) {
+    dep_start();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int m = SPMV && i < n ? A.cnt[i] : 0;  // loads before the skip test's own return
+    const int m = SPMV && i < n ? A.cnt[i] : 0;
+    dep_wait();
     if (fg_skip(sc)) return;
     T wi = 0;
     if (SPMV && i < n) {
@@ -1503,10 +1507,10 @@ __global__ void __launch_bounds__(RED_BLOCK) k_gs_dots(int64_t n, Op A, const T*
 // the cycle's control (h(j+1,j) = ||w||) and copies the scalars to the host
 // mirror.
 template <typename T>
-__global__ void __launch_bounds__(RED_BLOCK) k_gs_update(int64_t n, const T* __restrict__ V, T* __restrict__ w, int j,
+__global__ void __launch_bounds__(RED_BLOCK) k_gs_update(int64_t n, const T* V, T* w, int j,
                                                           double* Hd, FgLayout F, double* __restrict__ part,
-                                                          Scalars* sc, unsigned* __restrict__ ticket,
-                                                          Scalars* mirror) {
+                                                          Scalars* sc, unsigned* ticket, Scalars* mirror) {
+    dep_wait();
     const int rows = (int)gridDim.x - 1;  // blocks with rows
     if (fg_skip(sc)) {  // the cycle has stopped: publish the scalars all the same
         if (mirror && blockIdx.x == 0 && threadIdx.x == 0) *mirror = *sc;
@@ -1592,18 +1596,17 @@ int gs_iteration(Ctx* c, int64_t n, const Op& A, const T* z, T* V, T* w, int j, 
     // the first column's SpMV is bracketed by events, the dominant HBM-bound
     // kernel timed in place (a kernel of its own there)
     const bool timed = c->timing && j == 0;
+    const bool dep = !c->prof_iter;
     if (timed || !fused) {
         if (timed) record_event(c, c->ev_spmv[2]);
-        k_spmv<T, Op><<<blocks_for(n, B), B, 0, c->stream>>>(n, A, z, w, sc);
+        launch_dep(c->stream, dep && !timed, k_spmv<T, Op>, blocks_for(n, B), B, n, A, z, w, sc);
         if (timed) record_event(c, c->ev_spmv[3]);
         c->launches++;
     }
     if (c->prof_iter) record_event(c, c->ev_it[4]);
-    if (timed || !fused)
-        k_gs_dots<false, T, Op><<<G, B, 0, c->stream>>>(n, A, z, V, w, j, c->part, sc, c->ticket, c->Hd, F);
-    else
-        k_gs_dots<true, T, Op><<<G, B, 0, c->stream>>>(n, A, z, V, w, j, c->part, sc, c->ticket, c->Hd, F);
-    k_gs_update<T><<<G + 1, B, 0, c->stream>>>(n, V, w, j, c->Hd, F, c->part, sc, c->ticket, mirror);
+    launch_dep(c->stream, dep && !timed, timed || !fused ? k_gs_dots<false, T, Op> : k_gs_dots<true, T, Op>, G, B, n,
+               A, z, V, w, j, c->part, sc, c->ticket, c->Hd, F);
+    launch_dep(c->stream, dep, k_gs_update<T>, G + 1, B, n, V, w, j, c->Hd, F, c->part, sc, c->ticket, mirror);
     if (c->prof_iter) record_event(c, c->ev_it[5]);
     c->launches += 2;
     BSC_CUDA(c, cudaGetLastError());
