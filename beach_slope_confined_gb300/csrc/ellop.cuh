@@ -24,6 +24,11 @@ struct EllOp {
     __device__ __forceinline__ int64_t at(int64_t i, int k) const { return ell(i, k, kmax); }
     __device__ __forceinline__ int32_t col_at(int64_t e) const { return nbr[e]; }
     __device__ __forceinline__ T val_at(int64_t e) const { return aval[e]; }
+    __device__ __forceinline__ void entry(int64_t i, int k, int32_t& j, T& a) const {
+        const int64_t e = at(i, k);
+        j = nbr[e];
+        a = aval[e];
+    }
     // the column stride of the ELL layout is 32 slots
     template <typename X, typename A>
     __device__ __forceinline__ A row(int64_t i, const X* __restrict__ x) const {
@@ -81,6 +86,18 @@ struct EllPack16 {
     const int32_t* cnt;
     int kmax;
     const void* key() const { return ent; }
+    // entry k of row i
+    __device__ __forceinline__ void entry(int64_t i, int k, int32_t& j, float& a) const {
+        const int64_t e = ell(i, k, kmax);
+        if (ok[i >> 5]) {
+            const uint32_t p = ent[e];
+            j = (int32_t)(i & ~(int64_t)31) + (int16_t)(p & 0xffffu);
+            a = __half2float(__ushort_as_half((unsigned short)(p >> 16)));
+        } else {
+            j = nbr[e];
+            a = __half2float(aval[e]);
+        }
+    }
     template <typename X, typename A>
     __device__ __forceinline__ A row(int64_t i, const X* __restrict__ x) const {
         return row<X, A>(i, x, cnt[i]);
@@ -125,6 +142,11 @@ struct EllPackF {
     const int32_t* cnt;
     int kmax;
     const void* key() const { return ent; }
+    __device__ __forceinline__ void entry(int64_t i, int k, int32_t& j, float& a) const {
+        const int2 p = ent[ell(i, k, kmax)];
+        j = p.x;
+        a = __int_as_float(p.y);
+    }
     template <typename X, typename A>
     __device__ __forceinline__ A row(int64_t i, const X* __restrict__ x) const {
         return row<X, A>(i, x, cnt[i]);
@@ -160,6 +182,60 @@ struct EllPackF {
             s += (A)__int_as_float(p.y) * (A)x[p.x];
         }
         return s;
+    }
+};
+
+// One row of such an operator by L lanes of a warp (L a power of two): lane
+// `sub` of them takes entries sub, sub + L, ...  The constructor loads the
+// first 32 / L of each lane, all in flight and ahead of the vector; dot() is
+// the row times x in every lane of the row.  With L = 1 the constructor loads
+// the entry count alone and dot() is the operator's own loop.
+// Small systems' passes are the length of one row's chain of rounds (entries,
+// then the gathers they index) and sums, FP64 ones above all (one in flight
+// per warp and ~100 clocks); L lanes shorten it.
+template <typename T, typename Op, int L>
+struct RowLanes {
+    static constexpr int E = L == 1 ? 1 : 32 / L;
+    int64_t i;
+    int sub, m;
+    bool in;
+    int32_t j[E];
+    T a[E];
+    __device__ __forceinline__ RowLanes(int64_t n, const Op& A) {
+        const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+        sub = (int)(t & (L - 1));
+        i = t / L;
+        in = i < n;
+        m = in ? A.cnt[i] : 0;
+        if constexpr (L > 1)
+#pragma unroll
+            for (int u = 0; u < E; ++u) {
+                j[u] = in ? (int32_t)i : 0;
+                a[u] = (T)0;
+                if (sub + L * u < m) A.entry(i, sub + L * u, j[u], a[u]);
+            }
+    }
+    // every lane of the warp calls it (the rows past the end are empty)
+    __device__ __forceinline__ T dot(const Op& A, const T* x) const {
+        if constexpr (L == 1) {
+            return in ? A.template row<T, T>(i, x, m) : (T)0;
+        } else {
+            T y[E], s = 0;
+#pragma unroll
+            for (int u = 0; u < E; ++u) y[u] = x[j[u]];
+            if (in && sub == 0) s = x[i];
+#pragma unroll
+            for (int u = 0; u < E; ++u) s += a[u] * y[u];
+            for (int k = sub + 32; k < m; k += L) {
+                int32_t c;
+                T v;
+                A.entry(i, k, c, v);
+                s += v * x[c];
+            }
+#pragma unroll
+            for (int o = L / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            return s;
+        }
     }
 };
 

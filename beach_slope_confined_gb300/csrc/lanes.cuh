@@ -20,6 +20,14 @@ namespace bsc {
 // shorter loops save.
 inline int lanes_for(int64_t n) { return n <= 10000 ? 8 : n <= 20000 ? 4 : 1; }
 
+// Lanes per row in the fine-level passes and products of an FGMRES iteration.
+// Measured, four steps with 1 and 4 lanes: FP64 5.53 and 5.22 ms at 3816 rows,
+// 5.83 and 5.66 at 10414, 6.91 and 6.90 at 18322, 6.85 and 7.15 at 25881;
+// mixed 5.24 and 5.07, 5.31 and 5.14, 6.40 and 6.16, 5.86 and 5.76, and 8.90
+// and 9.47 at 78948.  (Two lanes gain
+// less at the smallest, eight less everywhere.)
+inline int row_lanes(int64_t n) { return n <= 20000 ? 4 : 1; }
+
 template <int L>
 struct Lanes {
     int sub;         // this lane's share of its particle

@@ -27,6 +27,7 @@
 
 #include "bsc_internal.cuh"
 #include "ellop.cuh"
+#include "lanes.cuh"
 
 namespace bsc {
 
@@ -991,18 +992,18 @@ __global__ void __launch_bounds__(MG_TAIL_THREADS) k_mg_tail(TailArgs<T> P) {
 // v = scale * src (the Krylov vector, normalised here rather than in a pass of
 // its own; scale is sc->tmp[4], the reciprocal of its norm), and two sweeps
 // from a zero guess: x1 = w v; x2 = x1 + w1 (v - A x1)
-template <typename T, typename Op>
+template <int L, typename T, typename Op>
 __global__ void __launch_bounds__(MG_BLOCK) k_mg0_pre2(int64_t n, Op A, const T* __restrict__ src, T* __restrict__ v,
                                                         T w, T w1, T* __restrict__ x,
                                                         const Scalars* __restrict__ sk) {
     dep_start();
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int m = A.cnt[i];
-    const T si = src[i], scale = to_r<T>(sk->tmp[4]);
+    const RowLanes<T, Op, L> row(n, A);
+    const int64_t i = row.i;
+    const T scale = to_r<T>(sk->tmp[4]);
     if (mg_skip(sk)) return;
-    const T Av = scale * A.template row<T, T>(i, src, m);
-    const T vi = scale * si;
+    const T Av = scale * row.dot(A, src);
+    if (!row.in || row.sub) return;
+    const T vi = scale * src[i];
     v[i] = vi;
     x[i] = w * vi + w1 * (vi - w * Av);  // x1 = w v; x2 = x1 + w1 (v - A x1)
 }
@@ -1019,31 +1020,31 @@ __global__ void k_mg0_scale(int64_t n, const T* __restrict__ src, T* __restrict_
 }
 
 // x_out = x + w (v - A x)
-template <typename T, typename Op>
+template <int L, typename T, typename Op>
 __global__ void __launch_bounds__(MG_BLOCK) k_mg0_sweep(int64_t n, Op A, const T* v, const T* x, T w,
                                                          T* __restrict__ xout, const Scalars* sk) {
     dep_start();
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int m = i < n ? A.cnt[i] : 0;
+    const RowLanes<T, Op, L> row(n, A);
+    const int64_t i = row.i;
     dep_wait();
-    if (i >= n) return;
-    const T vi = v[i], xi = x[i];
+    const T vi = row.in ? v[i] : (T)0, xi = row.in ? x[i] : (T)0;
     if (mg_skip(sk)) return;
-    xout[i] = xi + w * (vi - A.template row<T, T>(i, x, m));
+    const T Ax = row.dot(A, x);
+    if (row.in && row.sub == 0) xout[i] = xi + w * (vi - Ax);
 }
 
 // r = v - A x
-template <typename T, typename Op>
+template <int L, typename T, typename Op>
 __global__ void __launch_bounds__(MG_BLOCK) k_mg0_resid(int64_t n, Op A, const T* v, const T* x,
                                                          T* __restrict__ r, const Scalars* sk) {
     dep_start();
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int m = i < n ? A.cnt[i] : 0;
+    const RowLanes<T, Op, L> row(n, A);
+    const int64_t i = row.i;
     dep_wait();
-    if (i >= n) return;
-    const T vi = v[i];
+    const T vi = row.in ? v[i] : (T)0;
     if (mg_skip(sk)) return;
-    r[i] = vi - A.template row<T, T>(i, x, m);
+    const T Ax = row.dot(A, x);
+    if (row.in && row.sub == 0) r[i] = vi - Ax;
 }
 
 // level-1 right-hand side: the residual summed over each cell's particles
@@ -1267,21 +1268,32 @@ int vcycle(Ctx* c, const T* src, T* vin, T* z) {
     // fixed grid (measured: 10% faster fine passes at 846k rows)
     const unsigned G = blocks_for(n, MG_BLOCK);
     const bool dep = !c->prof_iter;  // an event record precedes some of the launches then
+    const int lanes = row_lanes(n);
+    const unsigned GL = blocks_for(n * lanes, MG_BLOCK);
+    auto sweep = [&](const T* in, T* out) {
+        with_lanes(lanes, [&](auto L) {
+            launch_dep(c->stream, dep, k_mg0_sweep<L(), T, AV>, GL, MG_BLOCK, n, A, vin, in, w1, out, c->mg.skip);
+        });
+    };
     if (c->prof_iter) record_event(c, c->ev_it[0]);
     T* cur = P0;
     const int nupre = c->mg_pre_fine > 0 ? c->mg_pre_fine : nu;
     if (nupre == 1)
         k_mg0_scale<T><<<G, MG_BLOCK, 0, c->stream>>>(n, src, vin, w, cur, c->mg.skip);
     else
-        k_mg0_pre2<T, AV><<<G, MG_BLOCK, 0, c->stream>>>(n, A, src, vin, w, w1, cur, c->mg.skip);
+        with_lanes(lanes, [&](auto L) {
+            k_mg0_pre2<L(), T, AV><<<GL, MG_BLOCK, 0, c->stream>>>(n, A, src, vin, w, w1, cur, c->mg.skip);
+        });
     BSC_LAUNCH(c);
     for (int k = 2; k < nupre; ++k) {
         T* out = cur == P0 ? Q0 : P0;
-        launch_dep(c->stream, dep, k_mg0_sweep<T, AV>, G, MG_BLOCK, n, A, vin, cur, w1, out, c->mg.skip);
+        sweep(cur, out);
         BSC_LAUNCH(c);
         cur = out;
     }
-    launch_dep(c->stream, dep, k_mg0_resid<T, AV>, G, MG_BLOCK, n, A, vin, cur, R0, c->mg.skip);
+    with_lanes(lanes, [&](auto L) {
+        launch_dep(c->stream, dep, k_mg0_resid<L(), T, AV>, GL, MG_BLOCK, n, A, vin, cur, R0, c->mg.skip);
+    });
     BSC_LAUNCH(c);
     const MgLevel& L1 = mg.L[1];
     Lv<T> v1 = level_view<T>(L1);
@@ -1303,7 +1315,7 @@ int vcycle(Ctx* c, const T* src, T* vin, T* z) {
             launch_dep(c->stream, dep, k_mg0_post<T>, G, MG_BLOCK, n, L1.nx, L1.ny, cur, R0, v1.x, c->pcell, rs, sc,
                        wp, out, c->mg.skip);
         else
-            launch_dep(c->stream, dep, k_mg0_sweep<T, AV>, G, MG_BLOCK, n, A, vin, cur, w1, out, c->mg.skip);
+            sweep(cur, out);
         BSC_LAUNCH(c);
         cur = out;
     }

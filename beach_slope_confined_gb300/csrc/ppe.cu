@@ -28,6 +28,7 @@
 #include "bsc_internal.cuh"
 #include "dfloat.cuh"
 #include "ellop.cuh"
+#include "lanes.cuh"
 #include "warpsum.cuh"
 
 namespace bsc {
@@ -1413,16 +1414,15 @@ int fg_cycle(Ctx* c, int m, int budget, Scalars* h, int* iters, Q queue) {
 // 62 and 52; 846k mixed 71 and 65, FP64 119 and 117.
 
 // w = A z, one row per thread
-template <typename T, typename Op>
+template <int L, typename T, typename Op>
 __global__ void __launch_bounds__(RED_BLOCK) k_spmv(int64_t n, Op A, const T* z, T* __restrict__ w,
                                                      const Scalars* sc) {
     dep_start();
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int m = i < n ? A.cnt[i] : 0;
+    const RowLanes<T, Op, L> row(n, A);
     dep_wait();
-    if (i >= n) return;
     if (fg_skip(sc)) return;
-    w[i] = A.template row<T, T>(i, z, m);
+    const T s = row.dot(A, z);
+    if (row.in && row.sub == 0) w[row.i] = s;
 }
 
 // column j of the dots from the blocks' partials, one warp per dot; by the
@@ -1463,30 +1463,29 @@ __device__ __forceinline__ bool gs_last_block(unsigned* ticket) {
 }
 
 // the dots of w, 8 columns per pass, summed per thread in T; SPMV: w = A z
-// first (one row per thread: n <= gridDim.x * RED_BLOCK)
-template <bool SPMV, typename T, typename Op>
+// first, L lanes per row, which then share the columns (n L <= gridDim.x RED_BLOCK)
+template <bool SPMV, int L, typename T, typename Op>
 __global__ void __launch_bounds__(RED_BLOCK) k_gs_dots(int64_t n, Op A, const T* z, const T* V,
                                                         T* w, int j, double* __restrict__ part,
                                                         const Scalars* sc, unsigned* ticket, double* Hd,
                                                         FgLayout F) {
     dep_start();
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int m = SPMV && i < n ? A.cnt[i] : 0;
+    const RowLanes<T, Op, L> row(SPMV ? n : 0, A);
     dep_wait();
     if (fg_skip(sc)) return;
     T wi = 0;
-    if (SPMV && i < n) {
-        wi = A.template row<T, T>(i, z, m);
-        w[i] = wi;
+    if (SPMV) {
+        wi = row.dot(A, z);
+        if (row.in && row.sub == 0) w[row.i] = wi;
     }
     for (int i0 = 0; i0 <= j; i0 += 8) {
         T acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         const int cntv = min(8, j + 1 - i0);
         if (SPMV) {
-            if (i < n)
+            if (row.in)
 #pragma unroll
                 for (int q = 0; q < 8; ++q)
-                    if (q < cntv) acc[q] = V[(int64_t)(i0 + q) * n + i] * wi;
+                    if (q < cntv && q % L == row.sub) acc[q] = V[(int64_t)(i0 + q) * n + row.i] * wi;
         } else {
             GRID_LOOP(k, n) {
                 const T wk = w[k];
@@ -1592,20 +1591,30 @@ template <typename T, typename Op>
 int gs_iteration(Ctx* c, int64_t n, const Op& A, const T* z, T* V, T* w, int j, FgLayout F, Scalars* sc,
                  Scalars* mirror) {
     const int G = red_blocks(n), B = RED_BLOCK;
-    const bool fused = n <= (int64_t)RED_GRID * RED_BLOCK;
+    const int lanes = row_lanes(n);
+    const int64_t GL = blocks_for(n * lanes, B);
+    const bool fused = GL <= RED_GRID;
     // the first column's SpMV is bracketed by events, the dominant HBM-bound
     // kernel timed in place (a kernel of its own there)
     const bool timed = c->timing && j == 0;
     const bool dep = !c->prof_iter;
     if (timed || !fused) {
         if (timed) record_event(c, c->ev_spmv[2]);
-        launch_dep(c->stream, dep && !timed, k_spmv<T, Op>, blocks_for(n, B), B, n, A, z, w, sc);
+        with_lanes(lanes, [&](auto L) {
+            launch_dep(c->stream, dep && !timed, k_spmv<L(), T, Op>, (unsigned)GL, B, n, A, z, w, sc);
+        });
         if (timed) record_event(c, c->ev_spmv[3]);
         c->launches++;
     }
     if (c->prof_iter) record_event(c, c->ev_it[4]);
-    launch_dep(c->stream, dep && !timed, timed || !fused ? k_gs_dots<false, T, Op> : k_gs_dots<true, T, Op>, G, B, n,
-               A, z, V, w, j, c->part, sc, c->ticket, c->Hd, F);
+    if (timed || !fused)
+        launch_dep(c->stream, dep && !timed, k_gs_dots<false, 1, T, Op>, G, B, n, A, z, V, w, j, c->part, sc, c->ticket,
+                   c->Hd, F);
+    else
+        with_lanes(lanes, [&](auto L) {
+            launch_dep(c->stream, dep, k_gs_dots<true, L(), T, Op>, (unsigned)GL, B, n, A, z, V, w, j, c->part, sc,
+                       c->ticket, c->Hd, F);
+        });
     launch_dep(c->stream, dep, k_gs_update<T>, G + 1, B, n, V, w, j, c->Hd, F, c->part, sc, c->ticket, mirror);
     if (c->prof_iter) record_event(c, c->ev_it[5]);
     c->launches += 2;
