@@ -203,13 +203,33 @@ template <> struct Vec2<float> { using type = float2; };
 // on tanks that do not fill the GPU, and a plain launch costs its share of
 // that: the next kernel's blocks start only after the last one's have drained.
 // launch_dep lets a kernel's blocks start once every block of its predecessor
-// has (dep_start, the predecessor's first statement).  Until dep_wait they may
-// read only what no kernel since the chain's last plain launch writes: the
-// matrix and the cells' operators.  dep_wait returns when the predecessor has
+// has said so (dep_start or dep_start_late).  Until dep_wait they may read
+// only what no kernel since the chain's last plain launch writes: the matrix
+// and the cells' operators.  dep_wait returns when the predecessor has
 // completed and its writes are visible; every thread calls it, so that a
 // kernel's completion implies its predecessors'.  What is read after it must
-// not be a __restrict__ parameter (whose reads the compiler may move ahead).  After a plain launch both statements do nothing.
-__device__ __forceinline__ void dep_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+// not be a __restrict__ parameter (whose reads the compiler may move ahead).
+// After a plain launch all of them do nothing.
+// A kernel says so in its first statement, or, in FP64 on more than
+// DEP_EARLY_BLOCKS blocks, when its sums are done: the SMs with fewer of its
+// blocks would otherwise take more of the successor's, and the FP64 pipe, one
+// per SM, bounds those.  Plain, early and late, four steps: FP64 5.25, 5.08,
+// 5.08 ms at 3816 rows, 18.4, 19.0, 18.2 at 198k, 55.8, 56.4, 55.2 at 846k;
+// mixed 5.60, 5.32, 5.38 at 13.6k, 28.0, 27.3, 27.7 at 846k.
+constexpr unsigned DEP_EARLY_BLOCKS = 128;
+__device__ __forceinline__ void dep_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
+template <typename T>
+__device__ __forceinline__ bool dep_early() {
+    return sizeof(T) == 4 || gridDim.x * gridDim.y <= DEP_EARLY_BLOCKS;
+}
+template <typename T>
+__device__ __forceinline__ void dep_start() {
+    if (dep_early<T>()) dep_trigger();
+}
+template <typename T>
+__device__ __forceinline__ void dep_start_late() {
+    if (!dep_early<T>()) dep_trigger();
+}
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // dep: false makes it a plain launch (the first of a chain, or after an event record)

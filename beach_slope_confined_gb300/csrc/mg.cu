@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(PT_THREADS) k_mg_post2(int nx, int ny, const T
                                                           const T* __restrict__ dinv, const T* b, const T* xin,
                                                           const T* xc, int nyc, T scale, T w, T w1,
                                                           T* __restrict__ xout, const Scalars* sk) {
-    dep_start();
+    dep_start<T>();
     __shared__ T v[PT_VX * PT_VY], y1[PT_HX * PT_HY];
     const int nc = nx * ny, t = threadIdx.x;
     const int x0 = blockIdx.x * PT_X, y0 = blockIdx.y * PT_Y;  // tile origin
@@ -394,6 +394,7 @@ __global__ void __launch_bounds__(PT_THREADS) k_mg_post2(int nx, int ny, const T
     };
     if (ring) y1[(rx + 1) * PT_HY + ry + 1] = in ? sweep(v + (rx + 2) * PT_VY + ry + 2, PT_VY, w) : (T)0;
     __syncthreads();
+    dep_start_late<T>();
     if (t < PT_X * PT_Y && in && !skip) xout[c] = sweep(y1 + (rx + 1) * PT_HY + ry + 1, PT_HY, w1);
 }
 
@@ -601,7 +602,7 @@ __global__ void __launch_bounds__(PR_BLOCK) k_mg_pre_restrict(int nx, int ny, co
                                                                T* __restrict__ xout, int nbs, int nxc, int nyc,
                                                                const T* __restrict__ R, T* __restrict__ bc,
                                                                const Scalars* sk) {
-    dep_start();
+    dep_start<T>();
     if ((int)blockIdx.x < nbs) {
         const int c = blockIdx.x * PR_BLOCK + threadIdx.x, nc = nx * ny, cl = min(c, nc - 1);
         const int cx = cl / ny, cy = cl - cx * ny;
@@ -626,6 +627,7 @@ __global__ void __launch_bounds__(PR_BLOCK) k_mg_pre_restrict(int nx, int ny, co
             y[s] *= d[s];
             ax[s / 3] += a[s] * y[s];
         }
+        dep_start_late<T>();
         // the first sweep, x = w0 D^-1 b, its weight taken out of the sum
         if (c < nc && !skip) xout[c] = w0 * y[4] + w * d[4] * (bc4 - w0 * ((ax[0] + ax[1]) + ax[2]));
         return;
@@ -647,6 +649,7 @@ __global__ void __launch_bounds__(PR_BLOCK) k_mg_pre_restrict(int nx, int ny, co
     for (int k = 0; k < MG_RPATCH; ++k) sum += wt[k] * v[k];
     part[row][lane] = sum;
     __syncthreads();
+    dep_start_late<T>();
     if (row == 0 && C < ncc && !mg_skip(sk))
         bc[C] = ((sum + part[1][lane]) + (part[2][lane] + part[3][lane])) + (part[4][lane] + part[5][lane]);
 }
@@ -789,7 +792,7 @@ template <typename T>
 __global__ void __launch_bounds__(MG_DENSE_BLOCK) k_mg_dense_apply(int nc, const T* __restrict__ M, int ld,
                                                                     const T* b, T* __restrict__ x,
                                                                     const Scalars* sk) {
-    dep_start();
+    dep_start<T>();
     constexpr int V = 16 / sizeof(T);  // entries per load
     struct alignas(16) Vec { T v[V]; };
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -827,6 +830,7 @@ __global__ void __launch_bounds__(MG_DENSE_BLOCK) k_mg_dense_apply(int nc, const
     T t = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    dep_start_late<T>();
     if (lane == 0 && !mg_skip(sk)) x[i] = t;
 }
 
@@ -996,12 +1000,13 @@ template <int L, typename T, typename Op>
 __global__ void __launch_bounds__(MG_BLOCK) k_mg0_pre2(int64_t n, Op A, const T* __restrict__ src, T* __restrict__ v,
                                                         T w, T w1, T* __restrict__ x,
                                                         const Scalars* __restrict__ sk) {
-    dep_start();
+    dep_start<T>();
     const RowLanes<T, Op, L> row(n, A);
     const int64_t i = row.i;
     const T scale = to_r<T>(sk->tmp[4]);
     if (mg_skip(sk)) return;
     const T Av = scale * row.dot(A, src);
+    dep_start_late<T>();
     if (!row.in || row.sub) return;
     const T vi = scale * src[i];
     v[i] = vi;
@@ -1023,13 +1028,14 @@ __global__ void k_mg0_scale(int64_t n, const T* __restrict__ src, T* __restrict_
 template <int L, typename T, typename Op>
 __global__ void __launch_bounds__(MG_BLOCK) k_mg0_sweep(int64_t n, Op A, const T* v, const T* x, T w,
                                                          T* __restrict__ xout, const Scalars* sk) {
-    dep_start();
+    dep_start<T>();
     const RowLanes<T, Op, L> row(n, A);
     const int64_t i = row.i;
     dep_wait();
     const T vi = row.in ? v[i] : (T)0, xi = row.in ? x[i] : (T)0;
     if (mg_skip(sk)) return;
     const T Ax = row.dot(A, x);
+    dep_start_late<T>();
     if (row.in && row.sub == 0) xout[i] = xi + w * (vi - Ax);
 }
 
@@ -1037,13 +1043,14 @@ __global__ void __launch_bounds__(MG_BLOCK) k_mg0_sweep(int64_t n, Op A, const T
 template <int L, typename T, typename Op>
 __global__ void __launch_bounds__(MG_BLOCK) k_mg0_resid(int64_t n, Op A, const T* v, const T* x,
                                                          T* __restrict__ r, const Scalars* sk) {
-    dep_start();
+    dep_start<T>();
     const RowLanes<T, Op, L> row(n, A);
     const int64_t i = row.i;
     dep_wait();
     const T vi = row.in ? v[i] : (T)0;
     if (mg_skip(sk)) return;
     const T Ax = row.dot(A, x);
+    dep_start_late<T>();
     if (row.in && row.sub == 0) r[i] = vi - Ax;
 }
 
@@ -1052,7 +1059,7 @@ template <typename T>
 __global__ void k_mg0_restrict(int64_t nc, const int32_t* __restrict__ cell_start, const int32_t* __restrict__ cell_count,
                                const int32_t* __restrict__ sorted, const T* r, T* __restrict__ b1,
                                const Scalars* sk) {
-    dep_start();
+    dep_start<T>();
     const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int q0 = c < nc ? cell_start[c] : 0, qn = c < nc ? cell_count[c] : 0;
     dep_wait();
@@ -1060,6 +1067,7 @@ __global__ void k_mg0_restrict(int64_t nc, const int32_t* __restrict__ cell_star
     if (mg_skip(sk)) return;
     T s = 0;
     for (int q = q0; q < q0 + qn; ++q) s += r[sorted[q]];
+    dep_start_late<T>();
     b1[c] = s;
 }
 
@@ -1075,7 +1083,7 @@ __global__ void __launch_bounds__(MG_BLOCK) k_mg0_post(int64_t n, int nx, int ny
                                                         const T* x1, const int32_t* __restrict__ pcell,
                                                         const T* __restrict__ rs, T scale, T w,
                                                         T* __restrict__ xout, const Scalars* sk) {
-    dep_start();
+    dep_start<T>();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int c = i < n ? pcell[i] : 0;
     dep_wait();
@@ -1090,6 +1098,7 @@ __global__ void __launch_bounds__(MG_BLOCK) k_mg0_post(int64_t n, int nx, int ny
         if (gx < 0 || gx >= nx || gy < 0 || gy >= ny) continue;
         apx += rs[s * n + i] * x1[(int64_t)gx * ny + gy];
     }
+    dep_start_late<T>();
     xout[i] = xi + scale * x1[c] + w * (ri - scale * apx);
 }
 

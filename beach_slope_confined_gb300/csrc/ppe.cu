@@ -1417,11 +1417,12 @@ int fg_cycle(Ctx* c, int m, int budget, Scalars* h, int* iters, Q queue) {
 template <int L, typename T, typename Op>
 __global__ void __launch_bounds__(RED_BLOCK) k_spmv(int64_t n, Op A, const T* z, T* __restrict__ w,
                                                      const Scalars* sc) {
-    dep_start();
+    dep_start<T>();
     const RowLanes<T, Op, L> row(n, A);
     dep_wait();
     if (fg_skip(sc)) return;
     const T s = row.dot(A, z);
+    dep_start_late<T>();
     if (row.in && row.sub == 0) w[row.i] = s;
 }
 
@@ -1469,7 +1470,7 @@ __global__ void __launch_bounds__(RED_BLOCK) k_gs_dots(int64_t n, Op A, const T*
                                                         T* w, int j, double* __restrict__ part,
                                                         const Scalars* sc, unsigned* ticket, double* Hd,
                                                         FgLayout F) {
-    dep_start();
+    dep_start<T>();
     const RowLanes<T, Op, L> row(SPMV ? n : 0, A);
     dep_wait();
     if (fg_skip(sc)) return;
@@ -1497,6 +1498,7 @@ __global__ void __launch_bounds__(RED_BLOCK) k_gs_dots(int64_t n, Op A, const T*
         block_partials<8>(acc, part + (int64_t)i0 * RED_GRID);
         __syncthreads();
     }
+    dep_start_late<T>();
     if (gs_last_block(ticket)) gs_finish_dots(part, (int)gridDim.x, j, Hd, F);
 }
 
