@@ -132,34 +132,109 @@ __global__ void k_mg_galerkin(int nxf, int nyf, const double* __restrict__ Af, i
 // iterations, never accuracy.
 //
 // Bound: the chain of up to 128 elimination steps, each waiting on the one
-// before, on one SM's issue slots.  The matrix stays in registers: warp w
-// holds columns w, w + 32, ..., lanes hold rows, so column k's pivot is found
-// inside one warp, which publishes the multipliers; the pivot row reaches the
-// other lanes by shuffles, and a step has one block barrier.  Rows are not
-// moved but carry the position that interchanges would have given them.  The
-// elimination performs the same FP32 operations as with the matrix in shared
-// memory and its rows interchanged (six barriers a step): 136 us there at 105
-// cells, 83 us here (cold caches).
+// before, and within a step the length of one warp's code.  The matrix stays
+// in registers: warp w holds GJ_E columns from GJ_E w on, lanes hold rows.  A
+// warp eliminates its own columns, a panel, without a barrier: it finds each
+// pivot, publishes the multipliers and brings its later columns up to date;
+// the other warps then apply the panel's steps, and the next panel's warp,
+// once it has, goes straight on to eliminate its own.  A pivot row reaches the
+// other lanes by shuffles, rows are not moved, and a panel has one block
+// barrier.  With a barrier per step and the rows' interchanges tracked 113 us
+// at the 3.8k-particle tank's coarsest level and 81 us at the 13.6k one's, 83
+// and 56 here (cold caches).
 constexpr int GJ_E = MG_COARSE_MAX / 32;  // columns per warp, rows per lane
+struct GjShared {
+    float col[2][GJ_E][MG_COARSE_MAX];  // the panel's columns at their steps, by panel parity
+    float inv[2][GJ_E];                 // 1 / pivot
+    int piv[2][GJ_E];                   // pivot row
+    int pos[MG_COARSE_MAX], row[MG_COARSE_MAX];  // the step that a row was the pivot of, and its inverse
+};
+// one step on this warp's columns: pivot row p, its reciprocal, the
+// multipliers f; own: the step's column among them, or -1.  `used` collects
+// the pivot rows, a bit per row of the lane.
+__device__ __forceinline__ void gj_step(float (&M)[GJ_E][GJ_E], unsigned& used, int lane, int p, float inv,
+                                        const float (&f)[GJ_E], int own) {
+    const int pl = p & 31, pr = p >> 5;
+    float q[GJ_E];
+#pragma unroll
+    for (int e = 0; e < GJ_E; ++e) {
+        float x = M[0][e];
+#pragma unroll
+        for (int r = 1; r < GJ_E; ++r) x = r == pr ? M[r][e] : x;
+        q[e] = __shfl_sync(0xffffffffu, x, pl) * inv;
+    }
+#pragma unroll
+    for (int e = 0; e < GJ_E; ++e)
+        if (e == own) {  // this column becomes the inverse's in place
+            q[e] = inv;
+#pragma unroll
+            for (int r = 0; r < GJ_E; ++r) M[r][e] = 0.f;
+        }
+#pragma unroll
+    for (int r = 0; r < GJ_E; ++r) {
+        const bool pivot = lane + 32 * r == p;
+        if (pivot) used |= 1u << r;
+#pragma unroll
+        for (int e = 0; e < GJ_E; ++e) {
+            const float m = fmaf(-f[r], q[e], M[r][e]);
+            M[r][e] = pivot ? q[e] : m;
+        }
+    }
+}
+// panel w, by its warp
+__device__ __forceinline__ void gj_panel(float (&M)[GJ_E][GJ_E], unsigned& used, GjShared& S, int w, int lane,
+                                         int n) {
+    const unsigned full = 0xffffffffu;
+    const int buf = w & 1;
+#pragma unroll
+    for (int ke = 0; ke < GJ_E; ++ke) {
+        const int k = GJ_E * w + ke;
+        if (k >= n) break;
+        // the largest |M[i][k]| over unused rows, the lowest on ties (a NaN as a zero): their bits plus one, used
+        // rows zero
+        unsigned a[GJ_E], best = 0u;
+        float f[GJ_E];
+#pragma unroll
+        for (int r = 0; r < GJ_E; ++r) {
+            f[r] = M[r][ke];
+            S.col[buf][ke][lane + 32 * r] = f[r];
+            const unsigned bits = __float_as_uint(f[r]) & 0x7fffffffu;
+            a[r] = used >> r & 1u ? 0u : bits <= 0x7f800000u ? bits + 1u : 1u;
+            best = max(best, a[r]);
+        }
+        const unsigned top = __reduce_max_sync(full, best);
+        unsigned at = 0xffffffffu;
+#pragma unroll
+        for (int r = GJ_E - 1; r >= 0; --r) at = a[r] == top ? (unsigned)(lane + 32 * r) : at;
+        const int p = (int)__reduce_min_sync(full, at);
+        float x = f[0];
+#pragma unroll
+        for (int r = 1; r < GJ_E; ++r) x = r == p >> 5 ? f[r] : x;
+        const float pv = __shfl_sync(full, x, p & 31);
+        const float inv = 1.f / (pv == 0.f ? 1e-30f : pv);
+        if (lane == 0) {
+            S.inv[buf][ke] = inv;
+            S.piv[buf][ke] = p;
+            S.pos[p] = k;
+            S.row[k] = p;
+        }
+        gj_step(M, used, lane, p, inv, f, ke);
+    }
+}
 template <typename O>
 __global__ void __launch_bounds__(1024) k_mg_dense_inverse(int nx, int ny, const double* __restrict__ A,
                                                             O* __restrict__ cinv) {
-    __shared__ float scol[2][MG_COARSE_MAX];  // column k, by step parity
-    __shared__ float sinv[2];                 // 1 / pivot
-    __shared__ int sp[2];                     // pivot row
-    __shared__ int spos[MG_COARSE_MAX];       // position of an unused row; GJ_USED after its step
-    __shared__ int fpos[MG_COARSE_MAX], row_at[MG_COARSE_MAX];  // final position of a row, and its inverse
-    constexpr int GJ_USED = 0xffff;
-    const unsigned full = 0xffffffffu;
+    __shared__ GjShared S;
     const int n = nx * ny;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    float M[GJ_E][GJ_E];  // row lane + 32 r, column w + 32 e
+    float M[GJ_E][GJ_E];  // row lane + 32 r, column GJ_E w + e
+    unsigned used = 0u;   // rows past the end and pivot rows
 #pragma unroll
     for (int r = 0; r < GJ_E; ++r) {
         const int c = lane + 32 * r, cx = c / ny, cy = c - cx * ny;
 #pragma unroll
         for (int e = 0; e < GJ_E; ++e) {
-            const int g = w + 32 * e, dx = g / ny - cx, dy = g % ny - cy;
+            const int g = GJ_E * w + e, dx = g / ny - cx, dy = g % ny - cy;
             M[r][e] = 0.f;
             if (c < n && g < n && dx >= -1 && dx <= 1 && dy >= -1 && dy <= 1)
                 M[r][e] = (float)A[(int64_t)stencil_slot(dx, dy) * n + c];
@@ -172,84 +247,32 @@ __global__ void __launch_bounds__(1024) k_mg_dense_inverse(int nx, int ny, const
                 if (!any) M[r][e] = 1.f;
             }
         }
-        if (w == 0) spos[c] = c < n ? c : GJ_USED;
+        if (c >= n) used |= 1u << r;
     }
+    if (w == 0) gj_panel(M, used, S, 0, lane, n);
     __syncthreads();
+    for (int P = 0; GJ_E * P < n; ++P) {
+        if (w != P && GJ_E * w < n) {
 #pragma unroll
-    for (int ke = 0; ke < GJ_E; ++ke) {
-        for (int kl = 0; kl < 32; ++kl) {
-            const int k = 32 * ke + kl, buf = kl & 1;
-            if (k >= n) break;
-            if (w == kl) {
-                // the largest |M[i][k]| over unused rows, the lowest position on ties; a NaN is never preferred
-                unsigned best = 0u, bkey = 0xffffffffu;
-                int ps[GJ_E];
+            for (int ke = 0; ke < GJ_E; ++ke) {
+                if (GJ_E * P + ke >= n) break;
+                float f[GJ_E];
 #pragma unroll
-                for (int r = 0; r < GJ_E; ++r) {
-                    ps[r] = spos[lane + 32 * r];
-                    const float a = fabsf(M[r][ke]);
-                    const unsigned ab = a == a ? __float_as_uint(a) : 0u;
-                    const unsigned key = (unsigned)ps[r] << 16 | (unsigned)(lane + 32 * r);
-                    if (ps[r] != GJ_USED && (ab > best || (ab == best && key < bkey))) {
-                        best = ab;
-                        bkey = key;
-                    }
-                    scol[buf][lane + 32 * r] = M[r][ke];
-                }
-                const unsigned top = __reduce_max_sync(full, best);
-                const unsigned key = __reduce_min_sync(full, best == top ? bkey : 0xffffffffu);
-                const int p = (int)(key & 0xffffu), ppos = (int)(key >> 16);
-#pragma unroll
-                for (int r = 0; r < GJ_E; ++r) {
-                    if (lane + 32 * r == p) {
-                        const float pv = M[r][ke] == 0.f ? 1e-30f : M[r][ke];
-                        sinv[buf] = 1.f / pv;
-                        sp[buf] = p;
-                        spos[p] = GJ_USED;
-                        fpos[p] = k;
-                    } else if (ps[r] == k) {
-                        spos[lane + 32 * r] = ppos;
-                    }
-                }
+                for (int r = 0; r < GJ_E; ++r) f[r] = S.col[P & 1][ke][lane + 32 * r];
+                gj_step(M, used, lane, S.piv[P & 1][ke], S.inv[P & 1][ke], f, -1);
             }
-            __syncthreads();
-            const float inv = sinv[buf];
-            const int p = sp[buf], pl = p & 31, pr = p >> 5;
-            float f[GJ_E], q[GJ_E];
-#pragma unroll
-            for (int r = 0; r < GJ_E; ++r) f[r] = scol[buf][lane + 32 * r];
-#pragma unroll
-            for (int r = 0; r < GJ_E; ++r)
-                if (r == pr)
-#pragma unroll
-                    for (int e = 0; e < GJ_E; ++e) q[e] = __shfl_sync(full, M[r][e], pl) * inv;
-            if (w == kl) {  // column k becomes column k of the inverse in place
-                q[ke] = inv;
-#pragma unroll
-                for (int r = 0; r < GJ_E; ++r) M[r][ke] = 0.f;
-            }
-#pragma unroll
-            for (int r = 0; r < GJ_E; ++r)
-#pragma unroll
-                for (int e = 0; e < GJ_E; ++e) M[r][e] = fmaf(-f[r], q[e], M[r][e]);
-#pragma unroll
-            for (int r = 0; r < GJ_E; ++r)
-                if (r == pr && lane == pl)
-#pragma unroll
-                    for (int e = 0; e < GJ_E; ++e) M[r][e] = q[e];
+            if (w == P + 1) gj_panel(M, used, S, w, lane, n);
         }
+        __syncthreads();
     }
-    // row i of the elimination is row fpos[i] of (P A)^-1, whose column j is
-    // column row_at[j] of A^-1
-    __syncthreads();
-    if (threadIdx.x < n) row_at[fpos[threadIdx.x]] = threadIdx.x;
-    __syncthreads();
+    // row i was the pivot of step pos[i] and is that row of the inverse; column
+    // j is its column row[j]
 #pragma unroll
     for (int r = 0; r < GJ_E; ++r)
 #pragma unroll
         for (int e = 0; e < GJ_E; ++e) {
-            const int i = lane + 32 * r, j = w + 32 * e;
-            if (i < n && j < n) cinv[fpos[i] * n + row_at[j]] = (O)M[r][e];
+            const int i = lane + 32 * r, j = GJ_E * w + e;
+            if (i < n && j < n) cinv[S.pos[i] * n + S.row[j]] = (O)M[r][e];
         }
 }
 
