@@ -810,7 +810,8 @@ __global__ void __launch_bounds__(MG_DENSE_BLOCK) k_mg_dense_t(int nx, int ny, c
     }
 }
 
-// x = T b, a warp per row
+// x = T b, a warp per row: the first PRE vectors of each lane ahead of the
+// wait for b (1024 FP32 or 512 FP64 entries of a row)
 template <typename T>
 __global__ void __launch_bounds__(MG_DENSE_BLOCK) k_mg_dense_apply(int nc, const T* __restrict__ M, int ld,
                                                                     const T* b, T* __restrict__ x,
@@ -818,38 +819,48 @@ __global__ void __launch_bounds__(MG_DENSE_BLOCK) k_mg_dense_apply(int nc, const
     dep_start<T>();
     constexpr int V = 16 / sizeof(T);  // entries per load
     struct alignas(16) Vec { T v[V]; };
+    constexpr int C = 8 / V;  // chains of vectors
+    constexpr int PRE = 8;
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    const T* row = M + (int64_t)min(i, nc - 1) * ld;
+    const Vec* m = reinterpret_cast<const Vec*>(row);
+    const int full = ld % V == 0 ? nc / V : 0;  // vectors of a row, where rows lie on 16-byte boundaries
+    Vec mv[PRE];
+#pragma unroll
+    for (int q = 0; q < PRE; ++q)
+        if (lane + 32 * q < full) mv[q] = m[lane + 32 * q];
     dep_wait();
     if (i >= nc) return;
-    const T* row = M + (int64_t)i * ld;
-    constexpr int C = 8 / V;  // loads in flight, each its own chains
+    const Vec* v = reinterpret_cast<const Vec*>(b);
+    Vec bv[PRE];
+#pragma unroll
+    for (int q = 0; q < PRE; ++q)
+        if (lane + 32 * q < full) bv[q] = v[lane + 32 * q];
     T s[8] = {};
-    int j = 0;
-    if (ld % V == 0) {  // rows on 16-byte boundaries
-        const Vec* m = reinterpret_cast<const Vec*>(row);
-        const Vec* v = reinterpret_cast<const Vec*>(b);
-        const int full = nc / V;
-        int q = lane;
-        for (; q + 32 * (C - 1) < full; q += 32 * C) {
-            Vec mv[C], bv[C];
 #pragma unroll
-            for (int c = 0; c < C; ++c) {
-                mv[c] = m[q + 32 * c];
-                bv[c] = v[q + 32 * c];
-            }
+    for (int q = 0; q < PRE; ++q)
+        if (lane + 32 * q < full)
 #pragma unroll
-            for (int c = 0; c < C; ++c)
+            for (int u = 0; u < V; ++u) s[q % C * V + u] += mv[q].v[u] * bv[q].v[u];
+    int q = lane + 32 * PRE;
+    for (; q + 32 * (C - 1) < full; q += 32 * C) {
+        Vec mr[C], br[C];
 #pragma unroll
-                for (int u = 0; u < V; ++u) s[c * V + u] += mv[c].v[u] * bv[c].v[u];
+        for (int c = 0; c < C; ++c) {
+            mr[c] = m[q + 32 * c];
+            br[c] = v[q + 32 * c];
         }
-        for (; q < full; q += 32) {
-            const Vec mv = m[q], bv = v[q];
 #pragma unroll
-            for (int u = 0; u < V; ++u) s[u] += mv.v[u] * bv.v[u];
-        }
-        j = full * V;
+        for (int c = 0; c < C; ++c)
+#pragma unroll
+            for (int u = 0; u < V; ++u) s[c * V + u] += mr[c].v[u] * br[c].v[u];
     }
-    for (j += lane; j < nc; j += 32) s[0] += row[j] * b[j];
+    for (; q < full; q += 32) {
+        const Vec mr = m[q], br = v[q];
+#pragma unroll
+        for (int u = 0; u < V; ++u) s[u] += mr.v[u] * br.v[u];
+    }
+    for (int j = full * V + lane; j < nc; j += 32) s[0] += row[j] * b[j];
     T t = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
@@ -1085,11 +1096,29 @@ __global__ void k_mg0_restrict(int64_t nc, const int32_t* __restrict__ cell_star
     dep_start<T>();
     const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int q0 = c < nc ? cell_start[c] : 0, qn = c < nc ? cell_count[c] : 0;
+    // four particles at a time, the first ones' indices ahead of the wait
+    // (one at a time, each index and residual in turn, a cell of four took
+    // eight dependent loads)
+    constexpr int U = 4;
+    int j[U];
+    auto load = [&](int k) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) j[u] = k + u < qn ? sorted[q0 + k + u] : 0;
+    };
+    load(0);
     dep_wait();
     if (c >= nc) return;
     if (mg_skip(sk)) return;
     T s = 0;
-    for (int q = q0; q < q0 + qn; ++q) s += r[sorted[q]];
+    for (int k = 0; k < qn; k += U) {
+        T y[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) y[u] = r[j[u]];
+        load(k + U);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (k + u < qn) s += y[u];
+    }
     dep_start_late<T>();
     b1[c] = s;
 }
@@ -1109,20 +1138,26 @@ __global__ void __launch_bounds__(MG_BLOCK) k_mg0_post(int64_t n, int nx, int ny
     dep_start<T>();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int c = i < n ? pcell[i] : 0;
+    const int cx = c / ny, cy = c - cx * ny;
+    T a[9];
+#pragma unroll
+    for (int s = 0; s < 9; ++s) a[s] = i < n ? rs[s * n + i] : (T)0;
     dep_wait();
     if (i >= n) return;
-    const int cx = c / ny, cy = c - cx * ny;
     const T xi = x[i], ri = r[i];
+    T y[9];  // clamped, unconditional loads: all of them in flight
+#pragma unroll
+    for (int s = 0; s < 9; ++s)
+        y[s] = x1[min(max(cx + s / 3 - 1, 0), nx - 1) * ny + min(max(cy + s % 3 - 1, 0), ny - 1)];
     if (mg_skip(sk)) return;
     T apx = 0;
 #pragma unroll
     for (int s = 0; s < 9; ++s) {
         const int gx = cx + s / 3 - 1, gy = cy + s % 3 - 1;
-        if (gx < 0 || gx >= nx || gy < 0 || gy >= ny) continue;
-        apx += rs[s * n + i] * x1[(int64_t)gx * ny + gy];
+        if (gx >= 0 && gx < nx && gy >= 0 && gy < ny) apx += a[s] * y[s];
     }
     dep_start_late<T>();
-    xout[i] = xi + scale * x1[c] + w * (ri - scale * apx);
+    xout[i] = xi + scale * y[4] + w * (ri - scale * apx);
 }
 
 template <typename T>
