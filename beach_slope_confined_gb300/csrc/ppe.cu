@@ -1560,31 +1560,42 @@ __global__ void __launch_bounds__(RED_BLOCK) k_gs_update(int64_t n, const T* V, 
         block_partials<1>(a, part);
     }
     if (!gs_last_block(ticket)) return;
+    const double a = __ldcg(Hd + F.H(j, j)), gj = Hd[F.g(j)];  // before another warp writes them
     double v[1];
     reduce_partials<1>(part, rows, v);
+    // a square root and a quotient each in three warps (five in a row by one
+    // thread took ~10 instructions of ~100 clocks each): the norm and its
+    // reciprocal, the rotation's cosine, its sine sqrt(v / (a^2 + v))
+    const double d2 = a * a + v[0];
     if (t == 0) {
-        const double a = __ldcg(Hd + F.H(j, j));
-        const double hn = sqrt(v[0]), den = sqrt(a * a + v[0]);
+        const double hn = sqrt(v[0]);
         sc->it += 1;
-        sc->tmp[1] = (double)(j + 1);
-        if (den == 0.0) {
-            sc->breakdown = 1;
-            sc->tmp[1] = (double)j;
-            sc->tmp[2] = 1.0;
-        } else {
-            const double cs = a / den, sn = hn / den;
-            const double gj = Hd[F.g(j)], gn = -sn * gj;
-            Hd[F.cs(j)] = cs;
-            Hd[F.sn(j)] = sn;
-            Hd[F.H(j, j)] = den;
-            Hd[F.H(j + 1, j)] = 0.0;
-            Hd[F.g(j + 1)] = gn;
-            Hd[F.g(j)] = cs * gj;
+        sc->tmp[1] = (double)(d2 == 0.0 ? j : j + 1);
+        if (d2 != 0.0) {
             sc->tmp[3] = hn;
             sc->tmp[4] = 1.0 / hn;
-            if (fabs(gn) <= sc->target || hn == 0.0 || j + 1 == F.m) sc->tmp[2] = 1.0;
+            Hd[F.H(j + 1, j)] = 0.0;
+        } else {
+            sc->breakdown = 1;
         }
-        if (mirror) *mirror = *sc;
+    } else if (t == 32 && d2 != 0.0) {
+        const double den = sqrt(d2), cs = a / den;
+        Hd[F.cs(j)] = cs;
+        Hd[F.H(j, j)] = den;
+        Hd[F.g(j)] = cs * gj;
+    } else if (t == 64) {
+        if (d2 != 0.0) {
+            const double sn = sqrt(v[0] / d2), gn = -sn * gj;
+            Hd[F.sn(j)] = sn;
+            Hd[F.g(j + 1)] = gn;
+            if (fabs(gn) <= sc->target || v[0] == 0.0 || j + 1 == F.m) sc->tmp[2] = 1.0;
+        } else {
+            sc->tmp[2] = 1.0;
+        }
+    }
+    if (mirror) {
+        __syncthreads();
+        if (t == 0) *mirror = *sc;
     }
 }
 
