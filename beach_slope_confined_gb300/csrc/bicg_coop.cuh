@@ -64,7 +64,8 @@ struct GridBarrier {
 constexpr int COOP_WARPS = 16;                     // warps per block at most
 constexpr int COOP_BLOCK = COOP_WARPS * 32;
 constexpr int64_t MERGE_ROWS = 12000;              // measured: the gathered p and s cost more than two barriers above
-constexpr int COOP_ENTRY = 32 * (int)(sizeof(double) + sizeof(int32_t));  // one entry of a warp's 32 rows
+// shared memory of one entry of a warp's 32 rows: value and column, and with MERGE the formed vector's value
+constexpr int coop_entry(bool merge) { return 32 * (int)(sizeof(double) + sizeof(int32_t) + (merge ? sizeof(double) : 0)); }
 constexpr int COOP_ITERS = 1024;                   // iterations per launch: tens of milliseconds at the largest sizes
 constexpr int COOP_BAR = 64;                       // the barrier's word in the ticket array
 constexpr int COOP_SETS = 5;                       // partials of an iteration's three reductions, a set per value
@@ -117,18 +118,21 @@ __device__ __forceinline__ double eight_sum(const double (&q)[8], int nwarps) {
 // update order and every sum are those of k_bicg_1..5: the same bits.  K: rows
 // per thread.  p2 and v2 are the second halves of the double-buffered p and v
 // (MERGE: gathered by other threads while this iteration's are written).
-template <typename Op, bool MERGE, int K>
-__global__ void __launch_bounds__(COOP_BLOCK, 1)
+template <typename Op, bool MERGE, int K, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1)
     k_bicg_coop(int64_t n, Op A, double* x, double* r, const double* rh, double* p, double* v, double* s, double* p2,
                 double* v2, double* part, Scalars* sc, unsigned* count, int iters, int cap) {
     extern __shared__ __align__(16) unsigned char coop_sm[];
     double* sval = reinterpret_cast<double*>(coop_sm);
-    int32_t* scol = reinterpret_cast<int32_t*>(coop_sm + (size_t)cap * 32 * sizeof(double));
+    double* sy = sval + (size_t)cap * 32;  // MERGE: the formed vector at the entries' columns
+    int32_t* scol = reinterpret_cast<int32_t*>(sval + (size_t)cap * 32 * (MERGE ? 2 : 1));
     __shared__ int used;
-    // scalars: warp 0 computes them once per block and hands them on
-    __shared__ double sh1[1][8], sh2[2][8], sh3[2][8], s_alpha, s_omega, s_beta;
-    __shared__ int s_state;  // 0: carry on, 1: converged, 2: breakdown
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // MERGE: the places, lengths and rows' lengths of the block's units, for the warps that form their entries
+    __shared__ int u_off[COOP_WARPS], u_len[COOP_WARPS], u_m[COOP_WARPS][32];
+    // scalars: one warp computes each once per block and hands it on
+    __shared__ double sh1[1][8], sh2[2][8], sh3[2][8], s_alpha, s_omega, s_q, s_ao, s_rr, s_rho;
+    __shared__ int s_brk, s_conv;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, W = blockDim.x >> 5;
     if (sc->done | sc->breakdown) return;  // the same for every block
     if (threadIdx.x == 0) used = 0;
     __syncthreads();
@@ -147,6 +151,13 @@ __global__ void __launch_bounds__(COOP_BLOCK, 1)
         if (lane == 0) o = atomicAdd(&used, mw);
         o = __shfl_sync(0xffffffffu, o, 0);
         off[q] = o + mw <= cap ? o : -1;
+        if (MERGE) {
+            u_m[w][lane] = m[q];
+            if (lane == 0) {
+                u_off[w] = off[q];
+                u_len[w] = mw;
+            }
+        }
         if (off[q] >= 0)
             for (int k = 0; k < m[q]; ++k) {
                 const int64_t e = A.at(i, k);
@@ -196,6 +207,38 @@ __global__ void __launch_bounds__(COOP_BLOCK, 1)
         }
         return acc;
     };
+    // MERGE: the vector `get` yields, at every entry of the block's rows, formed
+    // by all warps together
+    const int units = (nwarps + (int)gridDim.x - 1) / (int)gridDim.x;  // warps with rows, of any block
+    auto form = [&](auto get) {
+        int base = 0;  // deal the units' entries to the warps in one sequence
+        for (int u = 0; u < units; ++u) {
+            const int o = u_off[u], len = u_len[u], mu = u_m[u][lane];
+            if (o < 0) continue;
+            for (int k = (w - base % W + W) % W; k < len; k += W)
+                if (k < mu) sy[(o + k) * 32 + lane] = get(scol[(o + k) * 32 + lane]);
+            base += len;
+        }
+        __syncthreads();
+    };
+    // its product with this thread's row, the diagonal's term first
+    auto formed_product = [&](double diag) -> double {
+        const int o = off[0];
+        double acc = Op::UNIT_DIAG ? diag : 0.0;
+        int k = 0;
+        for (; k + 4 <= m[0]; k += 4) {
+            double a[4], y[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                a[u] = sval[(o + k + u) * 32 + lane];
+                y[u] = sy[(o + k + u) * 32 + lane];
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) acc += a[u] * y[u];
+        }
+        for (; k < m[0]; ++k) acc += sval[(o + k) * 32 + lane] * sy[(o + k) * 32 + lane];
+        return acc;
+    };
     // the warp sums of two values, a partial each
     auto partials2 = [&](int q, double a, double b, double* out) {
         double ab[2] = {a, b};
@@ -207,6 +250,7 @@ __global__ void __launch_bounds__(COOP_BLOCK, 1)
     const double target = sc->target;
     int it = sc->it, state = 0;
     bool first = true;
+    __syncthreads();  // the units' matrix entries
     GridBarrier grid{count, &sc->tmp[7]};
     double *pold = p, *pnew = p2, *vold = v, *vnew = MERGE ? v2 : v;
     double* part1 = part + nwarps;      // each reduction its own partials: a block may still
@@ -222,11 +266,18 @@ __global__ void __launch_bounds__(COOP_BLOCK, 1)
                 }
             if (!MERGE && !grid.sync()) return;
         }
+        if (MERGE && first) form([&](int32_t j) { return pold[j]; });
+        if (MERGE && !first) {
+            const double be = s_q * s_ao;
+            form([&](int32_t j) { return r[j] + be * (pold[j] - omega * vold[j]); });
+        }
 #pragma unroll
         for (int q = 0; q < K; ++q)
             if (busy(q)) {
                 if (act(q)) {
-                    if (MERGE && !first)
+                    if (MERGE && off[q] >= 0)
+                        vi[q] = formed_product(pi[q]);
+                    else if (MERGE && !first)
                         vi[q] = product(q, [&](int32_t j) { return r[j] + beta * (pold[j] - omega * vold[j]); });
                     else
                         vi[q] = product(q, [&](int32_t j) { return pold[j]; });
@@ -244,12 +295,14 @@ __global__ void __launch_bounds__(COOP_BLOCK, 1)
             if (!b) alpha = rho / d;
             if (lane == 0) {
                 s_alpha = alpha;
-                s_state = b ? 2 : 0;
+                s_brk = b;
             }
         }
         __syncthreads();
-        state = s_state;
-        if (state) break;
+        if (s_brk) {
+            state = 2;
+            break;
+        }
         alpha = s_alpha;
         // t = A s, s = r - alpha v
 #pragma unroll
@@ -259,11 +312,14 @@ __global__ void __launch_bounds__(COOP_BLOCK, 1)
                 if (!MERGE && act(q)) s[row(q)] = si[q];
             }
         if (!MERGE && !grid.sync()) return;
+        if (MERGE) form([&](int32_t j) { return r[j] - alpha * vnew[j]; });
 #pragma unroll
         for (int q = 0; q < K; ++q)
             if (busy(q)) {
                 if (act(q)) {
-                    if (MERGE)
+                    if (MERGE && off[q] >= 0)
+                        ti[q] = formed_product(si[q]);
+                    else if (MERGE)
                         ti[q] = product(q, [&](int32_t j) { return r[j] - alpha * vnew[j]; });
                     else
                         ti[q] = product(q, [&](int32_t j) { return s[j]; });
@@ -279,6 +335,10 @@ __global__ void __launch_bounds__(COOP_BLOCK, 1)
         }
         __syncthreads();
         omega = s_omega;
+        if (w == W - 1) {  // beta's second quotient, while the others update
+            const double ao = alpha / omega;
+            if (lane == 0) s_ao = ao;
+        }
         // x and r, the residual and rho
 #pragma unroll
         for (int q = 0; q < K; ++q)
@@ -291,21 +351,26 @@ __global__ void __launch_bounds__(COOP_BLOCK, 1)
         if (!grid.sync()) return;
         coop_sum<2>(part2, nwarps, sh3);
         ++it;
+        // beta = (rho' / rho) (alpha / omega) by one warp, the stop by another
         if (w == 0) {
-            const double d1 = eight_sum(sh3[1], nwarps);
-            rr = eight_sum(sh3[0], nwarps);
-            const bool conv = sqrt(rr) <= target;
-            const bool brk = !conv && (omega == 0.0 || d1 == 0.0);
-            if (!conv && !brk) beta = (d1 / rho) * (alpha / omega);
+            const double d1 = eight_sum(sh3[1], nwarps), q = d1 / rho;
             rho = d1;
             if (lane == 0) {
-                s_beta = beta;
-                s_state = conv ? 1 : brk ? 2 : 0;
+                s_q = q;
+                s_rho = d1;
+                s_brk = omega == 0.0 || d1 == 0.0;
+            }
+        }
+        if (w == W - 1) {
+            rr = eight_sum(sh3[0], nwarps);
+            if (lane == 0) {
+                s_rr = rr;
+                s_conv = sqrt(rr) <= target;
             }
         }
         __syncthreads();
-        state = s_state;
-        beta = s_beta;
+        state = s_conv ? 1 : s_brk ? 2 : 0;
+        if (!state && busy(0)) beta = s_q * s_ao;
         first = false;
         if (MERGE) {
             double* t = pold; pold = pnew; pnew = t;
@@ -320,8 +385,10 @@ __global__ void __launch_bounds__(COOP_BLOCK, 1)
             if (!state) p[row(q)] = ri[q] + beta * (pi[q] - omega * vi[q]);  // the next launch's p
         }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        sc->rr = rr;
-        sc->rho = rho;
+        if (!first) {  // an iteration came to its end
+            sc->rr = s_rr;
+            sc->rho = s_rho;
+        }
         sc->it = it;
         sc->done = state == 1 ? 1 : 0;
         sc->breakdown = state == 2 ? 1 : 0;

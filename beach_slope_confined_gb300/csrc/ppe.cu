@@ -977,7 +977,7 @@ int graph_run(Ctx* c, const void* k0, const void* k1, const void* k2, int64_t n,
 // per-kernel profiling.
 struct CoopPlan {
     const void* kernel = nullptr;
-    int blocks = 0, threads = 0, smem = 0;
+    int blocks = 0, threads = 0, smem = 0, cap = 0;  // cap: entries of 32 rows in shared memory
 };
 template <typename Op>
 CoopPlan coop_plan(int64_t n) {
@@ -995,21 +995,25 @@ CoopPlan coop_plan(int64_t n) {
     const int64_t per = (int64_t)sms * COOP_BLOCK;
     if (n > std::min<int64_t>(3 * per, (int64_t)RED_GRID * RED_BLOCK)) return P;
     const int K = (int)((n + per - 1) / per);
-    const void* f = K == 1 ? (n <= MERGE_ROWS ? (const void*)k_bicg_coop<Op, true, 1>
-                                              : (const void*)k_bicg_coop<Op, false, 1>)
-                    : K == 2 ? (const void*)k_bicg_coop<Op, false, 2>
-                             : (const void*)k_bicg_coop<Op, false, 3>;
+    const bool merge = K == 1 && n <= MERGE_ROWS;
+    const void* f = K == 1 ? (merge ? (const void*)k_bicg_coop<Op, true, 1, COOP_BLOCK>
+                                    : (const void*)k_bicg_coop<Op, false, 1, COOP_BLOCK>)
+                    : K == 2 ? (const void*)k_bicg_coop<Op, false, 1, 2 * COOP_BLOCK>
+                             : (const void*)k_bicg_coop<Op, false, 3, COOP_BLOCK>;
     const int64_t warps = (n + 31) / 32;
     const int blocks = (int)std::min<int64_t>(sms, warps);
-    const int threads = 32 * (int)((warps + (int64_t)blocks * K - 1) / ((int64_t)blocks * K));
+    const int per_thread = K == 3 ? 3 : 1;
+    // MERGE: all warps of the block form its rows' entries; else at least two, which share the scalars
+    const int threads = merge ? COOP_BLOCK : 32 * std::max(2, (int)((warps + (int64_t)blocks * per_thread - 1) / ((int64_t)blocks * per_thread)));
     cudaFuncAttributes fa{};
     if (cudaFuncGetAttributes(&fa, f) != cudaSuccess) return (void)cudaGetLastError(), P;
-    const int smem = (optin - (int)fa.sharedSizeBytes) / COOP_ENTRY * COOP_ENTRY;
+    const int entry = coop_entry(merge);
+    const int smem = (optin - (int)fa.sharedSizeBytes) / entry * entry;
     // the attribute is per function, process-wide: the device's maximum, whatever this call needs
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads, smem) != cudaSuccess || per_sm < 1)
         return (void)cudaGetLastError(), P;
-    P = {f, blocks, threads, smem};
+    P = {f, blocks, threads, smem, smem / entry};
     return P;
 }
 
@@ -1017,7 +1021,7 @@ template <typename Op>
 cudaError_t bicg_coop_launch(Ctx* c, int64_t n, Op A, Work<double> w, int iters, const CoopPlan& P) {
     unsigned* count = c->ticket + COOP_BAR;
     if (cudaError_t e = cudaMemsetAsync(count, 0, sizeof(unsigned), c->stream)) return e;
-    int cap = P.smem / COOP_ENTRY;
+    int cap = P.cap;
     const double* rh = w.rh;
     // MERGE: p and v double-buffered, their second halves in s and t
     void* args[] = {&n, &A, &w.x, &w.r, &rh, &w.p, &w.v, &w.s, &w.s, &w.t, &c->part, &c->sc, &count, &iters, &cap};
