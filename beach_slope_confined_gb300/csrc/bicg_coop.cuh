@@ -63,7 +63,9 @@ struct GridBarrier {
 
 constexpr int COOP_WARPS = 16;                     // warps per block at most
 constexpr int COOP_BLOCK = COOP_WARPS * 32;
-constexpr int64_t MERGE_ROWS = 12000;              // measured: the gathered p and s cost more than two barriers above
+// Measured, a step with and without MERGE: 31.5 and 36.9 ms at 13599 rows,
+// 41.7 and 43.9 at 18322, 51.6 and 52.3 at 25881, 81.3 and 68.9 at 42138.
+constexpr int64_t MERGE_ROWS = 20000;
 // shared memory of one entry of a warp's 32 rows: value and column, and with MERGE the formed vector's value
 constexpr int coop_entry(bool merge) { return 32 * (int)(sizeof(double) + sizeof(int32_t) + (merge ? sizeof(double) : 0)); }
 constexpr int COOP_ITERS = 1024;                   // iterations per launch: tens of milliseconds at the largest sizes
@@ -88,8 +90,11 @@ __device__ __forceinline__ double warp_sum_all(double x) {
 // FP64 pipe for its whole warp, and every idle warp's copy of the sums cost as
 // much as a working one's (38 us an iteration at 7600 rows with all 16 warps
 // computing all scalars).
-template <int D>
-__device__ __forceinline__ void coop_sum(const double* part, int nwarps, double (&sh)[D][8]) {
+// PAIRS: a partial per four warps, the even and the odd ones of a group, added
+// up by their block: 156 KB of partials a reduction step of 4096 warps made
+// every block read, and seven adds each, are a quarter and one.
+template <int D, bool PAIRS>
+__device__ __forceinline__ void coop_sum(const double* part, int stride, int nwarps, double (&sh)[D][8]) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, W = blockDim.x >> 5;
     const int groups = (nwarps + 7) / 8, parts = min((groups + 31) / 32, 8);
     if (threadIdx.x < 8 * D && (int)(threadIdx.x % 8) >= parts) sh[threadIdx.x / 8][threadIdx.x % 8] = 0.0;
@@ -97,11 +102,16 @@ __device__ __forceinline__ void coop_sum(const double* part, int nwarps, double 
         const int d = z / parts, vw = z - d * parts;
         double x = 0.0;
         for (int g = 32 * vw + lane; g < groups; g += 256) {
-            const double* q = part + d * nwarps + 8 * g;
-            double y[8];
+            if (PAIRS) {
+                const double2 y = __ldcg(reinterpret_cast<const double2*>(part + d * stride) + g);
+                x += y.x + y.y;
+            } else {
+                const double* q = part + d * stride + 8 * g;
+                double y[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) y[k] = 8 * g + k < nwarps ? __ldcg(q + k) : 0.0;
-            x += ((y[0] + y[4]) + (y[2] + y[6])) + ((y[1] + y[5]) + (y[3] + y[7]));
+                for (int k = 0; k < 8; ++k) y[k] = 8 * g + k < nwarps ? __ldcg(q + k) : 0.0;
+                x += ((y[0] + y[4]) + (y[2] + y[6])) + ((y[1] + y[5]) + (y[3] + y[7]));
+            }
         }
         x = warp_sum_all(x);
         if (lane == 0) sh[d][vw] = x;
@@ -122,6 +132,9 @@ template <typename Op, bool MERGE, int K, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1)
     k_bicg_coop(int64_t n, Op A, double* x, double* r, const double* rh, double* p, double* v, double* s, double* p2,
                 double* v2, double* part, Scalars* sc, unsigned* count, int iters, int cap) {
+    // beyond 512 threads a block's rows come in half groups of four warps, whose partials it adds up
+    constexpr bool PAIRS = THREADS > COOP_BLOCK;
+    static_assert(!PAIRS || (K == 1 && !MERGE), "half groups: one row per thread, no formed vectors");
     extern __shared__ __align__(16) unsigned char coop_sm[];
     double* sval = reinterpret_cast<double*>(coop_sm);
     double* sy = sval + (size_t)cap * 32;  // MERGE: the formed vector at the entries' columns
@@ -142,7 +155,12 @@ __global__ void __launch_bounds__(THREADS, 1)
     double xi[K], ri[K], pi[K], vi[K], rhi[K], si[K], ti[K];
 #pragma unroll
     for (int q = 0; q < K; ++q) {
-        unit[q] = (w + q * (int)(blockDim.x >> 5)) * (int)gridDim.x + (int)blockIdx.x;
+        if (PAIRS) {
+            const int half = (w >> 2) * (int)gridDim.x + (int)blockIdx.x;
+            unit[q] = 8 * (half >> 1) + (half & 1) + 2 * (w & 3);
+        } else {
+            unit[q] = (w + q * W) * (int)gridDim.x + (int)blockIdx.x;
+        }
         const int64_t i = (int64_t)unit[q] * 32 + lane;
         const bool act = i < n;
         m[q] = act ? A.len(i) : 0;
@@ -239,12 +257,35 @@ __global__ void __launch_bounds__(THREADS, 1)
         for (; k < m[0]; ++k) acc += sval[(o + k) * 32 + lane] * sy[(o + k) * 32 + lane];
         return acc;
     };
-    // the warp sums of two values, a partial each
+    // a reduction's partials: a warp's sums of one or two values, and the
+    // block's part once every warp has handed them over (before grid.sync)
+    const int stride = PAIRS ? 2 * ((nwarps + 7) / 8) : nwarps;
+    __shared__ double s_part[2][PAIRS ? THREADS / 32 : 1];
+    if (PAIRS && lane < 2) s_part[lane][w] = 0.0;  // warps without rows leave it so
+    auto partial1 = [&](int q, double a) {
+        a = warp_sum_all(a);
+        if (lane == 0) {
+            if (PAIRS) s_part[0][w] = a;
+            else part[unit[q]] = a;
+        }
+    };
     auto partials2 = [&](int q, double a, double b, double* out) {
         double ab[2] = {a, b};
         int which;
         const double y = warp_sums<2, double>(ab, which);
-        if ((lane & 15) == 0) out[which * nwarps + unit[q]] = y;
+        if ((lane & 15) == 0) {
+            if (PAIRS) s_part[which][w] = y;
+            else out[which * stride + unit[q]] = y;
+        }
+    };
+    auto hand_over = [&](int D, double* out) {
+        if (!PAIRS) return;
+        __syncthreads();
+        const int d = lane >> 3, h = lane & 7, half = h * (int)gridDim.x + (int)blockIdx.x;
+        if (w == 0 && d < D && 4 * h < W && half < stride) {
+            const double* y = &s_part[d][4 * h];
+            out[d * stride + half] = (y[0] + y[2]) + (y[1] + y[3]);
+        }
     };
     double rho = sc->rho, alpha = 0.0, omega = 0.0, beta = 0.0, rr = sc->rr;
     const double target = sc->target;
@@ -253,8 +294,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     __syncthreads();  // the units' matrix entries
     GridBarrier grid{count, &sc->tmp[7]};
     double *pold = p, *pnew = p2, *vold = v, *vnew = MERGE ? v2 : v;
-    double* part1 = part + nwarps;      // each reduction its own partials: a block may still
-    double* part2 = part + 3 * nwarps;  // read one while another writes the next
+    double* part1 = part + stride;      // each reduction its own partials: a block may still
+    double* part2 = part + 3 * stride;  // read one while another writes the next
     for (int iter = 0; iter < iters; ++iter) {
         // v = A p
         if (!first) {
@@ -284,11 +325,11 @@ __global__ void __launch_bounds__(THREADS, 1)
                     if (MERGE) pnew[row(q)] = pi[q];
                     vnew[row(q)] = vi[q];
                 }
-                const double a = warp_sum_all(rhi[q] * vi[q]);
-                if (lane == 0) part[unit[q]] = a;
+                partial1(q, rhi[q] * vi[q]);
             }
+        hand_over(1, part);
         if (!grid.sync()) return;
-        coop_sum<1>(part, nwarps, sh1);
+        coop_sum<1, PAIRS>(part, stride, nwarps, sh1);
         if (w == 0) {
             const double d = eight_sum(sh1[0], nwarps);
             const bool b = d == 0.0 || rho == 0.0;
@@ -326,8 +367,9 @@ __global__ void __launch_bounds__(THREADS, 1)
                 }
                 partials2(q, ti[q] * si[q], ti[q] * ti[q], part1);
             }
+        hand_over(2, part1);
         if (!grid.sync()) return;
-        coop_sum<2>(part1, nwarps, sh2);
+        coop_sum<2, PAIRS>(part1, stride, nwarps, sh2);
         if (w == 0) {
             const double d0 = eight_sum(sh2[0], nwarps), d1 = eight_sum(sh2[1], nwarps);
             omega = d1 == 0.0 ? 0.0 : d0 / d1;
@@ -348,8 +390,9 @@ __global__ void __launch_bounds__(THREADS, 1)
                 if (act(q)) r[row(q)] = ri[q];
                 partials2(q, ri[q] * ri[q], rhi[q] * ri[q], part2);
             }
+        hand_over(2, part2);
         if (!grid.sync()) return;
-        coop_sum<2>(part2, nwarps, sh3);
+        coop_sum<2, PAIRS>(part2, stride, nwarps, sh3);
         ++it;
         // beta = (rho' / rho) (alpha / omega) by one warp, the stop by another
         if (w == 0) {

@@ -1002,9 +1002,12 @@ CoopPlan coop_plan(int64_t n) {
                              : (const void*)k_bicg_coop<Op, false, 3, COOP_BLOCK>;
     const int64_t warps = (n + 31) / 32;
     const int blocks = (int)std::min<int64_t>(sms, warps);
-    const int per_thread = K == 3 ? 3 : 1;
-    // MERGE: all warps of the block form its rows' entries; else at least two, which share the scalars
-    const int threads = merge ? COOP_BLOCK : 32 * std::max(2, (int)((warps + (int64_t)blocks * per_thread - 1) / ((int64_t)blocks * per_thread)));
+    // warps per block: all there are with MERGE (they form the rows' entries); whole half groups with 1024
+    // threads; else the rows', at least two, which share the scalars
+    const int64_t halves = 2 * ((warps + 7) / 8), pt = (int64_t)blocks * (K == 3 ? 3 : 1);
+    const int threads = merge    ? COOP_BLOCK
+                        : K == 2 ? 128 * (int)((halves + blocks - 1) / blocks)
+                                 : 32 * std::max(2, (int)((warps + pt - 1) / pt));
     cudaFuncAttributes fa{};
     if (cudaFuncGetAttributes(&fa, f) != cudaSuccess) return (void)cudaGetLastError(), P;
     const int entry = coop_entry(merge);

@@ -2,7 +2,7 @@
 
 The reductions take one block per 256 rows up to 912 blocks, and a thread
 takes several rows beyond that; the cooperative BiCGSTAB forms p and s on the
-fly up to 12000 rows and holds one, two or three rows a thread up to 77824,
+fly up to 20000 rows and holds one, two or three rows a thread up to 77824,
 155648 and 233472 (on 152 SMs).  The counts here sit on both sides of a warp,
 a block, and each of those lines.  The system is tridiagonal (-1/4, 1, -1/4): its
 inverse's norm is at most 2 and ||A|| at most 1.5, so a stop at ||r|| <= 1e-12
@@ -35,7 +35,7 @@ def apply(n, x):
 
 
 @pytest.mark.parametrize("solver", ["bicgstab", "fgmres"])
-@pytest.mark.parametrize("n", [1, 31, 33, 255, 257, 1025, 12000, 12001, 77824, 77825, 131071, 155648, 155649, 912 * 256,
+@pytest.mark.parametrize("n", [1, 31, 33, 255, 257, 1025, 12000, 20000, 20001, 77824, 77825, 131071, 155648, 155649, 912 * 256,
                                912 * 256 + 257])
 def test_solve_over_row_counts(n, solver):
     x = np.random.default_rng(n).standard_normal(n)
@@ -65,10 +65,10 @@ def test_rows_too_long_for_shared_memory():
     assert np.linalg.norm(got - x) <= 5e-12 * np.linalg.norm(x)
 
 
-@pytest.mark.parametrize("dx", [0.02, 0.009])
+@pytest.mark.parametrize("dx", [0.02, 0.009, 0.0075, 0.0038])
 def test_cooperative_bicgstab_has_the_kernels_bits(dx, monkeypatch):
-    """The per-kernel profiling keeps the five-kernel iteration: same pressures, bit for bit (one tank on each side
-    of the 12000 rows)."""
+    """The per-kernel profiling keeps the five-kernel iteration: same pressures, bit for bit (tanks up to
+    20000 rows, up to 77824, and beyond)."""
     spec = sc.TankSpec(dx=dx)
     scen = sc.build(spec)
     P = sc.make_params(spec, scen.bounds, solver="bicgstab", tol=1e-10, maxit=20000)
