@@ -9,13 +9,18 @@
 //  - the matrix rows in shared memory (read once per launch);
 //  - a row's own vector entries in its thread's registers;
 //  - a grid barrier per phase, after which every block sums the partials
-//    itself, so that no block waits for a reducing one;
-//  - up to MERGE_ROWS rows, p and s formed where they are gathered (two and
-//    one fused multiply-adds per entry) instead of in phases of their own:
+//    itself, so that no block waits for a reducing one.  That sum is read and
+//    added up by every SM: its layout (a lane's eight values at a stride, so
+//    that a warp reads whole lines) and, in larger systems, partials that
+//    stand for four warps are what keep it short;
+//  - up to MERGE_ROWS rows, p and s formed where they are gathered instead of
+//    in phases of their own, by all warps of the block into shared memory:
 //    three barriers an iteration instead of five.
-// Measured per iteration at 7600 rows: 35 us as five kernels in a graph, 19 us
-// here: three barriers ~1.8 us each, two products 4 us each (28 dependent FP64
-// additions of ~140 clocks), three sums with their divisions ~2.5 us each.
+// Per iteration at 7600 rows: 35 us as five kernels in a graph, ~15 us here:
+// three barriers ~1.8 us each, two products ~2.5 us each (28 dependent FP64
+// additions of ~140 clocks), three sums with their quotients ~1.5 us each.
+// 125k rows of 21 entries: 48.8 us with a partial per warp and two rows per
+// thread, 33.5 us here.
 // The grid is launched cooperatively (all blocks resident), and every wait is
 // bounded.
 #pragma once
@@ -63,8 +68,8 @@ struct GridBarrier {
 
 constexpr int COOP_WARPS = 16;                     // warps per block at most
 constexpr int COOP_BLOCK = COOP_WARPS * 32;
-// Measured, a step with and without MERGE: 31.5 and 36.9 ms at 13599 rows,
-// 41.7 and 43.9 at 18322, 51.6 and 52.3 at 25881, 81.3 and 68.9 at 42138.
+// Measured, four steps with and without MERGE: 24.5 and 24.9 ms at 10414 rows,
+// 33.2 and 34.0 at 18322, 38.2 and 35.5 at 21490, 70.3 and 54.7 at 42138.
 constexpr int64_t MERGE_ROWS = 20000;
 // shared memory of one entry of a warp's 32 rows: value and column, and with MERGE the formed vector's value
 constexpr int coop_entry(bool merge) { return 32 * (int)(sizeof(double) + sizeof(int32_t) + (merge ? sizeof(double) : 0)); }
@@ -72,7 +77,7 @@ constexpr int COOP_ITERS = 1024;                   // iterations per launch: ten
 constexpr int COOP_BAR = 64;                       // the barrier's word in the ticket array
 constexpr int COOP_SETS = 5;                       // partials of an iteration's three reductions, a set per value
 // doubles a set takes: a partial per warp of rows
-__host__ __device__ inline int coop_part(int64_t n) { return (int)((n + 31) / 32); }
+__host__ __device__ inline int coop_part(int64_t n) { return (int)((n + 255) / 256 * 8); }
 
 // the warp sum over the tree of warp_sum_to_lane0, in every lane
 __device__ __forceinline__ double warp_sum_all(double x) {
@@ -90,10 +95,13 @@ __device__ __forceinline__ double warp_sum_all(double x) {
 // FP64 pipe for its whole warp, and every idle warp's copy of the sums cost as
 // much as a working one's (38 us an iteration at 7600 rows with all 16 warps
 // computing all scalars).
-// PAIRS: a partial per four warps, the even and the odd ones of a group, added
-// up by their block: 156 KB of partials a reduction step of 4096 warps made
-// every block read, and seven adds each, are a quarter and one.
-template <int D, bool PAIRS>
+// G = 4: a partial stands for four warps, the even or the odd ones of a group,
+// which one block holds and adds up first: a quarter of the loads and one
+// addition a group instead of seven.  Used without MERGE: the blocks' rows
+// come in fours of warps, which below some 20000 rows leaves SMs idle (18322
+// rows: 33.2 ms with MERGE and G = 1, 33.3 with G = 4; 7281: 18.7 and 21.8;
+// 25881 without MERGE: 43.3 and 40.2; 62118: 76.9 and 73.1).
+template <int D, int G>
 __device__ __forceinline__ void coop_sum(const double* part, int stride, int nwarps, double (&sh)[D][8]) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, W = blockDim.x >> 5;
     const int groups = (nwarps + 7) / 8, parts = min((groups + 31) / 32, 8);
@@ -102,14 +110,14 @@ __device__ __forceinline__ void coop_sum(const double* part, int stride, int nwa
         const int d = z / parts, vw = z - d * parts;
         double x = 0.0;
         for (int g = 32 * vw + lane; g < groups; g += 256) {
-            if (PAIRS) {
+            if (G == 4) {
                 const double2 y = __ldcg(reinterpret_cast<const double2*>(part + d * stride) + g);
                 x += y.x + y.y;
             } else {
-                const double* q = part + d * stride + 8 * g;
+                const double* q = part + d * stride + g;
                 double y[8];
 #pragma unroll
-                for (int k = 0; k < 8; ++k) y[k] = 8 * g + k < nwarps ? __ldcg(q + k) : 0.0;
+                for (int k = 0; k < 8; ++k) y[k] = 8 * g + k < nwarps ? __ldcg(q + k * groups) : 0.0;
                 x += ((y[0] + y[4]) + (y[2] + y[6])) + ((y[1] + y[5]) + (y[3] + y[7]));
             }
         }
@@ -128,13 +136,11 @@ __device__ __forceinline__ double eight_sum(const double (&q)[8], int nwarps) {
 // update order and every sum are those of k_bicg_1..5: the same bits.  K: rows
 // per thread.  p2 and v2 are the second halves of the double-buffered p and v
 // (MERGE: gathered by other threads while this iteration's are written).
-template <typename Op, bool MERGE, int K, int THREADS>
+template <typename Op, bool MERGE, int K, int THREADS, int G>
 __global__ void __launch_bounds__(THREADS, 1)
     k_bicg_coop(int64_t n, Op A, double* x, double* r, const double* rh, double* p, double* v, double* s, double* p2,
                 double* v2, double* part, Scalars* sc, unsigned* count, int iters, int cap) {
-    // beyond 512 threads a block's rows come in half groups of four warps, whose partials it adds up
-    constexpr bool PAIRS = THREADS > COOP_BLOCK;
-    static_assert(!PAIRS || (K == 1 && !MERGE), "half groups: one row per thread, no formed vectors");
+    static_assert(G == 1 || K == 1, "G > 1: one row per thread");
     extern __shared__ __align__(16) unsigned char coop_sm[];
     double* sval = reinterpret_cast<double*>(coop_sm);
     double* sy = sval + (size_t)cap * 32;  // MERGE: the formed vector at the entries' columns
@@ -155,9 +161,9 @@ __global__ void __launch_bounds__(THREADS, 1)
     double xi[K], ri[K], pi[K], vi[K], rhi[K], si[K], ti[K];
 #pragma unroll
     for (int q = 0; q < K; ++q) {
-        if (PAIRS) {
-            const int half = (w >> 2) * (int)gridDim.x + (int)blockIdx.x;
-            unit[q] = 8 * (half >> 1) + (half & 1) + 2 * (w & 3);
+        if (G > 1) {  // the units of a partial: every (8 / G)-th of a group of eight
+            const int z = (w / G) * (int)gridDim.x + (int)blockIdx.x;
+            unit[q] = 8 * (z / (8 / G)) + z % (8 / G) + (8 / G) * (w % G);
         } else {
             unit[q] = (w + q * W) * (int)gridDim.x + (int)blockIdx.x;
         }
@@ -227,7 +233,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     };
     // MERGE: the vector `get` yields, at every entry of the block's rows, formed
     // by all warps together
-    const int units = (nwarps + (int)gridDim.x - 1) / (int)gridDim.x;  // warps with rows, of any block
+    const int units = G * ((8 / G * ((nwarps + 7) / 8) + (int)gridDim.x - 1) / (int)gridDim.x);  // warps with rows, of any block
     auto form = [&](auto get) {
         int base = 0;  // deal the units' entries to the warps in one sequence
         for (int u = 0; u < units; ++u) {
@@ -259,14 +265,15 @@ __global__ void __launch_bounds__(THREADS, 1)
     };
     // a reduction's partials: a warp's sums of one or two values, and the
     // block's part once every warp has handed them over (before grid.sync)
-    const int stride = PAIRS ? 2 * ((nwarps + 7) / 8) : nwarps;
-    __shared__ double s_part[2][PAIRS ? THREADS / 32 : 1];
-    if (PAIRS && lane < 2) s_part[lane][w] = 0.0;  // warps without rows leave it so
+    const int groups = (nwarps + 7) / 8, stride = 8 / G * groups;
+    auto place = [&](int u) { return (u & 7) * groups + (u >> 3); };  // G = 1: a group's eight at a stride, read by a lane
+    __shared__ double s_part[2][G > 1 ? THREADS / 32 : 1];
+    if ((G > 1) && lane < 2) s_part[lane][w] = 0.0;  // warps without rows leave it so
     auto partial1 = [&](int q, double a) {
         a = warp_sum_all(a);
         if (lane == 0) {
-            if (PAIRS) s_part[0][w] = a;
-            else part[unit[q]] = a;
+            if (G > 1) s_part[0][w] = a;
+            else part[place(unit[q])] = a;
         }
     };
     auto partials2 = [&](int q, double a, double b, double* out) {
@@ -274,17 +281,17 @@ __global__ void __launch_bounds__(THREADS, 1)
         int which;
         const double y = warp_sums<2, double>(ab, which);
         if ((lane & 15) == 0) {
-            if (PAIRS) s_part[which][w] = y;
-            else out[which * stride + unit[q]] = y;
+            if (G > 1) s_part[which][w] = y;
+            else out[which * stride + place(unit[q])] = y;
         }
     };
     auto hand_over = [&](int D, double* out) {
-        if (!PAIRS) return;
+        if (G == 1) return;
         __syncthreads();
-        const int d = lane >> 3, h = lane & 7, half = h * (int)gridDim.x + (int)blockIdx.x;
-        if (w == 0 && d < D && 4 * h < W && half < stride) {
-            const double* y = &s_part[d][4 * h];
-            out[d * stride + half] = (y[0] + y[2]) + (y[1] + y[3]);
+        const int d = lane >> 3, h = lane & 7, z = h * (int)gridDim.x + (int)blockIdx.x;
+        if (w == 0 && d < D && G * h < W && z < stride) {
+            const double* y = &s_part[d][G * h];
+            out[d * stride + z] = (y[0] + y[2]) + (y[1] + y[3]);
         }
     };
     double rho = sc->rho, alpha = 0.0, omega = 0.0, beta = 0.0, rr = sc->rr;
@@ -329,7 +336,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
         hand_over(1, part);
         if (!grid.sync()) return;
-        coop_sum<1, PAIRS>(part, stride, nwarps, sh1);
+        coop_sum<1, G>(part, stride, nwarps, sh1);
         if (w == 0) {
             const double d = eight_sum(sh1[0], nwarps);
             const bool b = d == 0.0 || rho == 0.0;
@@ -369,7 +376,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
         hand_over(2, part1);
         if (!grid.sync()) return;
-        coop_sum<2, PAIRS>(part1, stride, nwarps, sh2);
+        coop_sum<2, G>(part1, stride, nwarps, sh2);
         if (w == 0) {
             const double d0 = eight_sum(sh2[0], nwarps), d1 = eight_sum(sh2[1], nwarps);
             omega = d1 == 0.0 ? 0.0 : d0 / d1;
@@ -392,7 +399,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
         hand_over(2, part2);
         if (!grid.sync()) return;
-        coop_sum<2, PAIRS>(part2, stride, nwarps, sh3);
+        coop_sum<2, G>(part2, stride, nwarps, sh3);
         ++it;
         // beta = (rho' / rho) (alpha / omega) by one warp, the stop by another
         if (w == 0) {

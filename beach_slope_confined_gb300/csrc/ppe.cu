@@ -996,18 +996,19 @@ CoopPlan coop_plan(int64_t n) {
     if (n > std::min<int64_t>(3 * per, (int64_t)RED_GRID * RED_BLOCK)) return P;
     const int K = (int)((n + per - 1) / per);
     const bool merge = K == 1 && n <= MERGE_ROWS;
-    const void* f = K == 1 ? (merge ? (const void*)k_bicg_coop<Op, true, 1, COOP_BLOCK>
-                                    : (const void*)k_bicg_coop<Op, false, 1, COOP_BLOCK>)
-                    : K == 2 ? (const void*)k_bicg_coop<Op, false, 1, 2 * COOP_BLOCK>
-                             : (const void*)k_bicg_coop<Op, false, 3, COOP_BLOCK>;
+    const int G = K <= 2 && !merge ? 4 : 1;
+    const void* f = merge    ? (const void*)k_bicg_coop<Op, true, 1, COOP_BLOCK, 1>
+                    : K == 1 ? (const void*)k_bicg_coop<Op, false, 1, COOP_BLOCK, 4>
+                    : K == 2 ? (const void*)k_bicg_coop<Op, false, 1, 2 * COOP_BLOCK, 4>
+                             : (const void*)k_bicg_coop<Op, false, 3, COOP_BLOCK, 1>;
     const int64_t warps = (n + 31) / 32;
     const int blocks = (int)std::min<int64_t>(sms, warps);
-    // warps per block: all there are with MERGE (they form the rows' entries); whole half groups with 1024
-    // threads; else the rows', at least two, which share the scalars
-    const int64_t halves = 2 * ((warps + 7) / 8), pt = (int64_t)blocks * (K == 3 ? 3 : 1);
-    const int threads = merge    ? COOP_BLOCK
-                        : K == 2 ? 128 * (int)((halves + blocks - 1) / blocks)
-                                 : 32 * std::max(2, (int)((warps + pt - 1) / pt));
+    // warps per block: all there are with MERGE (they form the rows' entries); whole partials' warps; else the
+    // rows', at least two, which share the scalars
+    const int64_t partials = 8 / G * ((warps + 7) / 8), pt = (int64_t)blocks * (K == 3 ? 3 : 1);
+    const int threads = merge   ? COOP_BLOCK
+                        : G > 1 ? 32 * G * (int)((partials + blocks - 1) / blocks)
+                                : 32 * std::max(2, (int)((warps + pt - 1) / pt));
     cudaFuncAttributes fa{};
     if (cudaFuncGetAttributes(&fa, f) != cudaSuccess) return (void)cudaGetLastError(), P;
     const int entry = coop_entry(merge);
