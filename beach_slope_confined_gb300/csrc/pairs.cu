@@ -372,43 +372,6 @@ __global__ void __launch_bounds__(WC_WARPS * 32) k_cand_warpcell(int ncell, KPar
     }
 }
 
-int op_neighbour(Ctx* c) {
-    k_posf<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->S.x, c->S.y, c->pcell, c->K, c->posf, c->S.vol,
-                                                         c->mixed ? c->f_vol : nullptr,
-                                                         c->mixed ? c->f_vol_lo : nullptr,
-                                                         c->mixed ? c->posd : nullptr);
-    BSC_LAUNCH(c);
-    const unsigned g = blocks_for(c->n, NB_BLOCK);
-    // mixed path: grad W as a double-float only, unless an FP64 assembly
-    // variant (BSC_ASSEMBLY=rcp, BSC_EXACT_DIV=1) reads the FP64 copy
-    double2* gw64 = (c->asm_rcp || c->exact_div) ? c->gw : nullptr;
-    StageTimer tk(c, BSC_T_K_NEIGHBOUR);
-    if (c->nb_warpcell) {
-        const unsigned gc = (unsigned)std::min<int64_t>((c->ncell + WC_WARPS - 1) / WC_WARPS, 152 * 32);
-        k_cand_warpcell<<<gc, WC_WARPS * 32, 0, c->stream>>>((int)c->ncell, c->K, c->cell_start, c->cell_count,
-                                                              c->sorted, c->posf, c->nbr, c->cand_nc);
-        BSC_LAUNCH(c);
-        if (c->mixed)
-            k_neighbour<float, true><<<g, NB_BLOCK, 0, c->stream>>>(
-                c->n, c->S, c->K, c->cell_start, c->cell_count, c->sorted, c->pcell, c->posf, c->posd, c->nbr, gw64,
-                c->gwf, c->gwl, c->f_vol, c->ndist, c->cnt, c->d_flag, c->cand_nc);
-        else
-            k_neighbour<double, true><<<g, NB_BLOCK, 0, c->stream>>>(
-                c->n, c->S, c->K, c->cell_start, c->cell_count, c->sorted, c->pcell, c->posf, nullptr, c->nbr, c->gw,
-                nullptr, nullptr, nullptr, c->ndist, c->cnt, c->d_flag, c->cand_nc);
-    } else if (c->mixed)
-        k_neighbour<float><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->cell_start, c->cell_count, c->sorted,
-                                                          c->pcell, c->posf, c->posd, c->nbr, gw64, c->gwf, c->gwl,
-                                                          c->f_vol, c->ndist, c->cnt, c->d_flag);
-    else
-        k_neighbour<double><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->cell_start, c->cell_count,
-                                                           c->sorted, c->pcell, c->posf, nullptr, c->nbr, c->gw,
-                                                           nullptr, nullptr, nullptr, c->ndist, c->cnt, c->d_flag);
-    BSC_LAUNCH(c);
-    c->have_lists = true;
-    return BSC_OK;
-}
-
 // The lists alone, for the WCSPH step (wcsph.cu), whose pair sums read neither
 // grad W nor L: the same sets in the same order as k_neighbour's.  The FP32
 // pre-test decides both ways outside its margin (its r^2 is within ~1e-6 of
@@ -467,16 +430,122 @@ __global__ void __launch_bounds__(NB_BLOCK) k_neighbour_lists(
     cnt[i] = count;
 }
 
-int op_neighbour_lists(Ctx* c) {
-    k_posf<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->S.x, c->S.y, c->pcell, c->K, c->posf, c->S.vol,
-                                                         nullptr, nullptr, nullptr);
-    BSC_LAUNCH(c);
+static void launch_lists(Ctx* c) {
     with_lanes(lanes_for(c->n), [&](auto L) {
         k_neighbour_lists<L.value><<<blocks_for(c->n * L.value, NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
             c->n, c->S.x, c->S.y, c->K, c->cell_start, c->cell_count, c->sorted, c->pcell, c->posf, c->nbr, c->cnt,
             c->d_flag);
     });
+}
+
+int op_neighbour_lists(Ctx* c) {
+    k_posf<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->S.x, c->S.y, c->pcell, c->K, c->posf, c->S.vol,
+                                                         nullptr, nullptr, nullptr);
     BSC_LAUNCH(c);
+    launch_lists(c);
+    BSC_LAUNCH(c);
+    return BSC_OK;
+}
+
+// The rest of the FP64 search on small tanks, over those lists: grad W, the
+// distances, the M sums and what follows from them (the end of k_neighbour),
+// four lanes to a particle.  A round takes four pairs, and lane a then adds
+// their terms of M_a in list order: the bits of the one-thread sums.
+__global__ void __launch_bounds__(NB_BLOCK) k_neighbour_rows(int64_t n, State S, KParams K,
+                                                              const int32_t* __restrict__ nbr,
+                                                              const int32_t* __restrict__ cnt,
+                                                              double2* __restrict__ gw, double* __restrict__ ndist) {
+    constexpr int L = 4;
+    const Lanes<L> ln;
+    const int64_t i = ln.particle();
+    if (i >= n) return;
+    __shared__ double2 sg[NB_BLOCK], sr[NB_BLOCK];
+    const double* g = reinterpret_cast<const double*>(sg + (threadIdx.x & ~(L - 1))) + (ln.sub & 1);
+    const double* d = reinterpret_cast<const double*>(sr + (threadIdx.x & ~(L - 1))) + (ln.sub >> 1);
+    const double xi = S.x[i], yi = S.y[i];
+    const int count = cnt[i];
+    double m = 0.0;  // M_sub: gx rx, gy rx, gx ry, gy ry
+    for (int k0 = 0; k0 < count; k0 += L) {
+        const int k = k0 + ln.sub;
+        double2 gxy = {0.0, 0.0}, rxy = {0.0, 0.0};
+        if (k < count) {
+            const int64_t e = ell(i, k, K.kmax);
+            const int j = nbr[e];
+            const double dx = xi - S.x[j], dy = yi - S.y[j];
+            const double r = __dsqrt_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
+            const double F = grad_factor<double>(K, r);
+            gxy = {F * dx, F * dy};
+            gw[e] = gxy;
+            if (ndist) ndist[e] = r;
+            const double vj = S.vol[j];
+            rxy = {-vj * dx, -vj * dy};  // m_j (x_j - x_i) / rho_j
+        }
+        ln.sync();
+        sg[threadIdx.x] = gxy;
+        sr[threadIdx.x] = rxy;
+        ln.sync();
+#pragma unroll
+        for (int u = 0; u < L; ++u) m = fma(g[2 * u], d[2 * u], m);
+    }
+    const double a0 = __shfl_sync(ln.mask, m, 0, L), a1 = __shfl_sync(ln.mask, m, 1, L);
+    const double a2 = __shfl_sync(ln.mask, m, 2, L), a3 = __shfl_sync(ln.mask, m, 3, L);
+    uint8_t f = S.flags[i] & (uint8_t)~BSC_FLAG_FREE;  // search.f90:41
+    double gv = 0.0;
+    if (S.tid[i] == BSC_TID_FLUID) {  // search.f90:268-306
+        f &= (uint8_t)~BSC_FLAG_VICINITY;
+        gv = a0 + a3;
+        const double det = __dsub_rn(__dmul_rn(a0, a3), __dmul_rn(a1, a2));
+        double l = ln.sub == 0 || ln.sub == 3 ? 1.0 : 0.0;
+        if (fabs(det) >= (double)1e-5f && isfinite(det))
+            l = (ln.sub == 0 ? a3 : ln.sub == 1 ? -a1 : ln.sub == 2 ? -a2 : a0) / det;
+        (ln.sub == 0 ? S.L0 : ln.sub == 1 ? S.L1 : ln.sub == 2 ? S.L2 : S.L3)[i] = l;
+        if (gv <= K.free_thr && !(f & BSC_FLAG_BUFFER)) f |= BSC_FLAG_FREE;
+    }
+    ln.sync();  // every lane has read the flags
+    if (ln.sub != 0) return;
+    S.gradvx[i] = gv;
+    S.flags[i] = f;
+}
+
+int op_neighbour(Ctx* c) {
+    k_posf<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->S.x, c->S.y, c->pcell, c->K, c->posf, c->S.vol,
+                                                         c->mixed ? c->f_vol : nullptr,
+                                                         c->mixed ? c->f_vol_lo : nullptr,
+                                                         c->mixed ? c->posd : nullptr);
+    BSC_LAUNCH(c);
+    const unsigned g = blocks_for(c->n, NB_BLOCK);
+    // mixed path: grad W as a double-float only, unless an FP64 assembly
+    // variant (BSC_ASSEMBLY=rcp, BSC_EXACT_DIV=1) reads the FP64 copy
+    double2* gw64 = (c->asm_rcp || c->exact_div) ? c->gw : nullptr;
+    StageTimer tk(c, BSC_T_K_NEIGHBOUR);
+    if (c->nb_warpcell) {
+        const unsigned gc = (unsigned)std::min<int64_t>((c->ncell + WC_WARPS - 1) / WC_WARPS, 152 * 32);
+        k_cand_warpcell<<<gc, WC_WARPS * 32, 0, c->stream>>>((int)c->ncell, c->K, c->cell_start, c->cell_count,
+                                                              c->sorted, c->posf, c->nbr, c->cand_nc);
+        BSC_LAUNCH(c);
+        if (c->mixed)
+            k_neighbour<float, true><<<g, NB_BLOCK, 0, c->stream>>>(
+                c->n, c->S, c->K, c->cell_start, c->cell_count, c->sorted, c->pcell, c->posf, c->posd, c->nbr, gw64,
+                c->gwf, c->gwl, c->f_vol, c->ndist, c->cnt, c->d_flag, c->cand_nc);
+        else
+            k_neighbour<double, true><<<g, NB_BLOCK, 0, c->stream>>>(
+                c->n, c->S, c->K, c->cell_start, c->cell_count, c->sorted, c->pcell, c->posf, nullptr, c->nbr, c->gw,
+                nullptr, nullptr, nullptr, c->ndist, c->cnt, c->d_flag, c->cand_nc);
+    } else if (c->mixed)
+        k_neighbour<float><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->cell_start, c->cell_count, c->sorted,
+                                                          c->pcell, c->posf, c->posd, c->nbr, gw64, c->gwf, c->gwl,
+                                                          c->f_vol, c->ndist, c->cnt, c->d_flag);
+    else if (lanes_for(c->n) > 1) {
+        launch_lists(c);
+        BSC_LAUNCH(c);
+        k_neighbour_rows<<<blocks_for(c->n * 4, NB_BLOCK), NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->cnt,
+                                                                                  c->gw, c->ndist);
+    } else
+        k_neighbour<double><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->cell_start, c->cell_count,
+                                                           c->sorted, c->pcell, c->posf, nullptr, c->nbr, c->gw,
+                                                           nullptr, nullptr, nullptr, c->ndist, c->cnt, c->d_flag);
+    BSC_LAUNCH(c);
+    c->have_lists = true;
     return BSC_OK;
 }
 
@@ -504,7 +573,7 @@ int op_freesurf(Ctx* c) {
 }
 
 // ---- porous.f90:107-224 effpor ---------------------------------------------------
-template <typename R>
+template <typename R, int L>
 __global__ void __launch_bounds__(NB_BLOCK) k_effpor(int64_t n, State S, KParams K, const int32_t* __restrict__ pcell,
                                                       const int32_t* __restrict__ scs, const int32_t* __restrict__ scc,
                                                       const double* __restrict__ sx, const double* __restrict__ sy,
@@ -514,9 +583,11 @@ __global__ void __launch_bounds__(NB_BLOCK) k_effpor(int64_t n, State S, KParams
                                                       const double* __restrict__ spor,
                                                       float* __restrict__ f_vol = nullptr,
                                                       float* __restrict__ f_vol_lo = nullptr) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    static_assert(L == 1 || sizeof(R) == 8, "several lanes: the FP64 path's two phases");
+    const Lanes<L> ln;
+    const int64_t i = ln.particle();
     if (i >= n) return;
-    S.resist[i] = 0.0;
+    if (ln.sub == 0) S.resist[i] = 0.0;
     if (S.tid[i] != BSC_TID_FLUID) return;
     const double xi = S.x[i], yi = S.y[i];
     const int c = pcell[i], cx = c / K.ny, cy = c - cx * K.ny;
@@ -529,14 +600,19 @@ __global__ void __launch_bounds__(NB_BLOCK) k_effpor(int64_t n, State S, KParams
     // pipe; ~48 bits, more than the FP64 sum of FP32 terms needed, with no
     // FP64 work inside the divergent candidate loop)
     df2 fsum{0.0f, 0.0f};
-    // the FP64 work of one solid: the exact test and its weighted W
-    auto solid_term = [&](int s) {
+    // the FP64 work of one solid: the exact test and its weighted W (false: outside)
+    auto solid_weight = [&](int s, R& wt) {
         const double dx = xi - sx[s], dy = yi - sy[s];
         const double d2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
-        if (!nonneg_below(d2, K.H2x)) return;  // exactly sqrt(d2) < 2h
+        if (!nonneg_below(d2, K.H2x)) return false;  // exactly sqrt(d2) < 2h
         // W(r) in R: an FP32 root for the FP32 sum, the exact one for FP64
         const R r = sizeof(R) == 4 ? (R)sqrtf((float)d2) : (R)__dsqrt_rn(d2);
-        frac += ((R)1 - (R)spor[s]) * kern_w<R>(K, r) * (R)svol[s];
+        wt = ((R)1 - (R)spor[s]) * kern_w<R>(K, r);
+        return true;
+    };
+    auto solid_term = [&](int s) {
+        R wt;
+        if (solid_weight(s, wt)) frac = fma(wt, (R)svol[s], frac);
     };
     // FP64 path, two phases as in the neighbour search: the FP32 pre-test
     // first compacts the surviving solids (in cell order) into this thread's
@@ -545,8 +621,10 @@ __global__ void __launch_bounds__(NB_BLOCK) k_effpor(int64_t n, State S, KParams
     // loop, at about half the lanes of each FP64 instruction.  The sum keeps
     // its order, so the result is the same.  A particle with more survivors
     // than the column holds, or far from its binned cell, takes the one pass.
-    constexpr int EP_CAP = 32;
-    __shared__ int32_t cand[sizeof(R) == 8 ? EP_CAP * NB_BLOCK : 1];
+    // L lanes share both phases, and the sum takes their terms in order.
+    constexpr int EP_CAP = 32, EP_COLS = NB_BLOCK / L;
+    __shared__ int32_t cand[sizeof(R) == 8 ? EP_CAP * EP_COLS : 1];
+    const int col = threadIdx.x / L;
     bool one_pass = true;
     if constexpr (sizeof(R) == 8) {
         if (pre_i) {
@@ -559,20 +637,38 @@ __global__ void __launch_bounds__(NB_BLOCK) k_effpor(int64_t n, State S, KParams
                     const float shy = (float)(ay - cy) * csf;
                     const int cc = ax * K.ny + ay;
                     const int s0 = scs[cc], s1 = s0 + scc[cc];
-                    for (int s = s0; s < s1; ++s) {
-                        const float2 ps = sposf[s];
-                        if (pre_ok(ps, csf)) {
-                            const float fdx = pi.x - (ps.x + shx), fdy = pi.y - (ps.y + shy);
-                            if (fdx * fdx + fdy * fdy > H2f) continue;
+                    for (int sl = s0; sl < s1; sl += L) {
+                        const int s = sl + ln.sub;
+                        bool keep = s < s1;
+                        if (keep) {
+                            const float2 ps = sposf[s];
+                            if (pre_ok(ps, csf)) {
+                                const float fdx = pi.x - (ps.x + shx), fdy = pi.y - (ps.y + shy);
+                                keep = !(fdx * fdx + fdy * fdy > H2f);
+                            }
                         }
-                        if (nc < EP_CAP) cand[nc * NB_BLOCK + threadIdx.x] = s;
-                        ++nc;
+                        const int at = ln.place(keep, nc);
+                        if (keep && at < EP_CAP) cand[at * EP_COLS + col] = s;
                     }
                 }
             }
             if (nc <= EP_CAP) {
                 one_pass = false;
-                for (int k = 0; k < nc; ++k) solid_term(cand[k * NB_BLOCK + threadIdx.x]);
+                ln.sync();
+                if constexpr (L == 1) {
+                    for (int k = 0; k < nc; ++k) solid_term(cand[k * EP_COLS + col]);
+                } else {
+                    for (int k = 0; k < nc; k += L) {
+                        R wt = 0, v = 0;
+                        if (k + ln.sub < nc) {
+                            const int s = cand[(k + ln.sub) * EP_COLS + col];
+                            if (solid_weight(s, wt)) v = svol[s];
+                        }
+#pragma unroll
+                        for (int u = 0; u < L; ++u)
+                            frac = fma(__shfl_sync(ln.mask, wt, u, L), __shfl_sync(ln.mask, v, u, L), frac);
+                    }
+                }
             }
         }
     }
@@ -609,6 +705,7 @@ __global__ void __launch_bounds__(NB_BLOCK) k_effpor(int64_t n, State S, KParams
             }
         }
     }
+    if (ln.sub != 0) return;
     double sf = (double)frac + df_to_double(fsum);
     // away from the solids (whole warps) there is nothing to cap and no drag:
     // the field's lookup and the Ergun coefficient, some hundred FP64
@@ -659,12 +756,15 @@ int op_effpor(Ctx* c) {
     const unsigned g = blocks_for(c->n, NB_BLOCK);
     StageTimer tk(c, BSC_T_K_EFFPOR);
     if (c->mixed)
-        k_effpor<float><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->pcell, c->scell_start, c->scell_count,
+        k_effpor<float, 1><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->pcell, c->scell_start, c->scell_count,
                                                        c->sx, c->sy, c->sposf, c->swf, c->svol, c->spor, c->f_vol,
                                                        c->f_vol_lo);
     else
-        k_effpor<double><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->pcell, c->scell_start, c->scell_count,
-                                                        c->sx, c->sy, c->sposf, c->swf, c->svol, c->spor);
+        with_lanes(std::min(lanes_for(c->n), 4), [&](auto L) {
+            k_effpor<double, (L() < 4 ? L() : 4)><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
+                c->n, c->S, c->K, c->pcell, c->scell_start, c->scell_count, c->sx, c->sy, c->sposf, c->swf, c->svol,
+                c->spor);
+        });
     BSC_LAUNCH(c);
     return BSC_OK;
 }
