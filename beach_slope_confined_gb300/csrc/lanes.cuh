@@ -48,6 +48,17 @@ struct Lanes {
         for (int o = L / 2; o > 0; o >>= 1) x += __shfl_xor_sync(mask, x, o);
         return x;
     }
+    // acc[q] += a[q] b[q] over the particle's lanes in turn, in each of them: the
+    // bits of one thread's fused sums over the same terms (a lane past the end
+    // of the list hands in zeros)
+    template <typename R, int N>
+    __device__ __forceinline__ void ordered(R (&acc)[N], const R (&a)[N], const R (&b)[N]) const {
+#pragma unroll
+        for (int u = 0; u < L; ++u)
+#pragma unroll
+            for (int q = 0; q < N; ++q)
+                acc[q] = fma(L == 1 ? a[q] : __shfl_sync(mask, a[q], u, L), L == 1 ? b[q] : __shfl_sync(mask, b[q], u, L), acc[q]);
+    }
     // the place of this lane's kept item among the particle's, after `count`
     // of them; count moves past them
     __device__ __forceinline__ int place(bool keep, int& count) const {
@@ -70,6 +81,13 @@ void with_lanes(int lanes, F f) {
         case 4: f(std::integral_constant<int, 4>{}); break;
         default: f(std::integral_constant<int, 1>{}); break;
     }
+}
+
+// the FP64 step's pair sums, whose rounds cost more than WCSPH's: one lane or four
+template <typename F>
+void with_pair_lanes(int64_t n, F f) {
+    if (lanes_for(n) > 1) f(std::integral_constant<int, 4>{});
+    else f(std::integral_constant<int, 1>{});
 }
 
 }  // namespace bsc

@@ -760,8 +760,8 @@ int op_effpor(Ctx* c) {
                                                        c->sx, c->sy, c->sposf, c->swf, c->svol, c->spor, c->f_vol,
                                                        c->f_vol_lo);
     else
-        with_lanes(std::min(lanes_for(c->n), 4), [&](auto L) {
-            k_effpor<double, (L() < 4 ? L() : 4)><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
+        with_pair_lanes(c->n, [&](auto L) {
+            k_effpor<double, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
                 c->n, c->S, c->K, c->pcell, c->scell_start, c->scell_count, c->sx, c->sy, c->sposf, c->swf, c->svol,
                 c->spor);
         });
@@ -904,7 +904,7 @@ __global__ void __launch_bounds__(NB_BLOCK) k_varts(int64_t n, State S, KParams 
 
 // pass 2: viscous (Morris, harmonic mu/oden), eddy viscosity, SPS k gradient,
 // implicit porous drag and gravity (:509-711)
-template <typename R>
+template <typename R, int L>
 __global__ void __launch_bounds__(NB_BLOCK) k_int_vel(int64_t n, State S, KParams K, const int32_t* __restrict__ nbr,
                                                        const typename Vec2<R>::type* __restrict__ gw,
                                                        const int32_t* __restrict__ cnt,
@@ -912,7 +912,8 @@ __global__ void __launch_bounds__(NB_BLOCK) k_int_vel(int64_t n, State S, KParam
                                                        const float* __restrict__ f_nu, const float* __restrict__ f_nut,
                                                        const float* __restrict__ f_tke, const float* __restrict__ f_varts,
                                                        const float2* __restrict__ posf, const int32_t* __restrict__ pcell) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const Lanes<L> ln;
+    const int64_t i = ln.particle();
     if (i >= n) return;
     constexpr bool F32 = sizeof(R) == 4;  // FP32 sums: the per-particle fields come from their FP32 twins
     const uint8_t fi = S.flags[i];
@@ -946,76 +947,85 @@ __global__ void __launch_bounds__(NB_BLOCK) k_int_vel(int64_t n, State S, KParam
         const R varts_i = to_r<R>(S.varts[i]);
         const R inv_w0 = (R)K.inv_w0;
         const R eps6 = (R)(double)1e-6f;
-        R ax = 0, ay = 0, kx = 0, ky = 0;  // kx, ky: the SPS sum, scaled by (2/3) n_i once
+        R sum[4] = {0, 0, 0, 0};  // the acceleration's two and the SPS sum's, scaled by (2/3) n_i once
         const int m = cnt[i];
         // FP32 sums: four entries' gathers in flight (measured 3-7 % faster)
         #pragma unroll(sizeof(R) == 4 ? 4 : 1)
-        for (int k = 0; k < m; ++k) {
-            const int64_t e = ell(i, k, K.kmax);
-            const int j = nbr[e];
-            const auto g = gw[e];
-            const bool fluid_j = S.tid[j] == BSC_TID_FLUID;
-            R cmu;
-            if (fluid_j) {
-                const R nuj = F32 ? (R)f_nu[j] : (R)nu[j];
-                cmu = !F32 && nuj == nui ? cmui : (R)2 * nui * nuj / (nui + nuj);
-            } else {
-                cmu = nui;
+        for (int k0 = 0; k0 < m; k0 += L) {
+            const int k = k0 + ln.sub;
+            R ta[4] = {0, 0, 0, 0}, tb[4] = {0, 0, 0, 0};  // their terms' factors
+            if (L == 1 || k < m) {
+                const int64_t e = ell(i, k, K.kmax);
+                const int j = nbr[e];
+                const auto g = gw[e];
+                const bool fluid_j = S.tid[j] == BSC_TID_FLUID;
+                R cmu;
+                if (fluid_j) {
+                    const R nuj = F32 ? (R)f_nu[j] : (R)nu[j];
+                    cmu = !F32 && nuj == nui ? cmui : (R)2 * nui * nuj / (nui + nuj);
+                } else {
+                    cmu = nui;
+                }
+                R fx, fy, r2;
+                [[maybe_unused]] double dx = 0.0, dy = 0.0;
+                if constexpr (F32) {
+                    const float2 pfj = posf[j];
+                    const int cj = pcell[j], cxj = cj / K.ny, cyj = cj - cxj * K.ny;
+                    fx = (pfi.x - pfj.x) + (float)(cxi - cxj) * csf;
+                    fy = (pfi.y - pfj.y) + (float)(cyi - cyj) * csf;
+                    r2 = fx * fx + fy * fy;
+                } else {
+                    dx = xi - S.x[j];
+                    dy = yi - S.y[j];
+                    fx = dx;
+                    fy = dy;
+                    r2 = dx * dx + dy * dy;
+                }
+                R vart = 0;
+                if (free_i) {
+                    vart = varts_i;
+                } else if ((S.flags[j] & BSC_FLAG_FREE) && !(fi & BSC_FLAG_BUFFER)) {
+                    R r;
+                    if constexpr (F32)
+                        r = sqrtf(r2);
+                    else
+                        r = sqrt(dx * dx + dy * dy);
+                    vart = kern_w<R>(K, r) * (F32 ? (R)f_varts[j] : (R)S.varts[j]) * inv_w0;
+                }
+                const R pvol = F32 ? (R)f_vol[j] : (R)S.vol[j];
+                const R p_dist = (R)1 / (r2 + (R)K.lam);
+                const R gx = L0 * g.x + L1 * g.y, gy = L2 * g.x + L3 * g.y;
+                const R geo = (R)2 * pvol * (fx * gx + fy * gy) * p_dist;
+                R dvx, dvy;
+                if constexpr (F32) {
+                    dvx = vxif - f32_of(S.vx[j]);
+                    dvy = vyif - f32_of(S.vy[j]);
+                } else {
+                    dvx = vxi - S.vx[j];
+                    dvy = vyi - S.vy[j];
+                }
+                R visc = cmu + vart;
+                if (fluid_j) {
+                    const R nutj = F32 ? (R)f_nut[j] : (R)S.nut[j];
+                    if (nuti < eps6 && nutj < eps6) visc += (nuti + nutj) * (R)0.5;
+                    else visc += ((R)2 * nuti * nutj) / (nuti + nutj);
+                }
+                ta[0] = geo * dvx;
+                ta[1] = geo * dvy;
+                tb[0] = tb[1] = visc;
+                // SPS turbulence (:645-666): -(2/3) n_i sum_j V_j (k_j - k_i) L grad W
+                const R dk = pvol * ((F32 ? (R)f_tke[j] : (R)S.tke[j]) - tkei);
+                ta[2] = ta[3] = dk;
+                tb[2] = gx;
+                tb[3] = gy;
             }
-            R fx, fy, r2;
-            [[maybe_unused]] double dx = 0.0, dy = 0.0;
-            if constexpr (F32) {
-                const float2 pfj = posf[j];
-                const int cj = pcell[j], cxj = cj / K.ny, cyj = cj - cxj * K.ny;
-                fx = (pfi.x - pfj.x) + (float)(cxi - cxj) * csf;
-                fy = (pfi.y - pfj.y) + (float)(cyi - cyj) * csf;
-                r2 = fx * fx + fy * fy;
-            } else {
-                dx = xi - S.x[j];
-                dy = yi - S.y[j];
-                fx = dx;
-                fy = dy;
-                r2 = dx * dx + dy * dy;
-            }
-            R vart = 0;
-            if (free_i) {
-                vart = varts_i;
-            } else if ((S.flags[j] & BSC_FLAG_FREE) && !(fi & BSC_FLAG_BUFFER)) {
-                R r;
-                if constexpr (F32)
-                    r = sqrtf(r2);
-                else
-                    r = sqrt(dx * dx + dy * dy);
-                vart = kern_w<R>(K, r) * (F32 ? (R)f_varts[j] : (R)S.varts[j]) * inv_w0;
-            }
-            const R pvol = F32 ? (R)f_vol[j] : (R)S.vol[j];
-            const R p_dist = (R)1 / (r2 + (R)K.lam);
-            const R gx = L0 * g.x + L1 * g.y, gy = L2 * g.x + L3 * g.y;
-            const R geo = (R)2 * pvol * (fx * gx + fy * gy) * p_dist;
-            R dvx, dvy;
-            if constexpr (F32) {
-                dvx = vxif - f32_of(S.vx[j]);
-                dvy = vyif - f32_of(S.vy[j]);
-            } else {
-                dvx = vxi - S.vx[j];
-                dvy = vyi - S.vy[j];
-            }
-            R visc = cmu + vart;
-            if (fluid_j) {
-                const R nutj = F32 ? (R)f_nut[j] : (R)S.nut[j];
-                if (nuti < eps6 && nutj < eps6) visc += (nuti + nutj) * (R)0.5;
-                else visc += ((R)2 * nuti * nutj) / (nuti + nutj);
-            }
-            ax += geo * dvx * visc;
-            ay += geo * dvy * visc;
-            // SPS turbulence (:645-666): -(2/3) n_i sum_j V_j (k_j - k_i) L grad W
-            const R dk = pvol * ((F32 ? (R)f_tke[j] : (R)S.tke[j]) - tkei);
-            kx += dk * gx;
-            ky += dk * gy;
+            ln.ordered(sum, ta, tb);
         }
+        if (ln.sub != 0) return;
+        R ax = sum[0], ay = sum[1];
         const R sps = ni * (R)2 / (R)3;
-        ax -= kx * sps;
-        ay -= ky * sps;
+        ax -= sum[2] * sps;
+        ay -= sum[3] * sps;
         const double nn = S.por[i], R_ = S.resist[i];
         double vxs, vys;
         if constexpr (F32) {
@@ -1031,7 +1041,7 @@ __global__ void __launch_bounds__(NB_BLOCK) k_int_vel(int64_t n, State S, KParam
         S.vxs[i] = vxs;
         S.vys[i] = vys;
     }
-    if (fi & BSC_FLAG_BUFFER) {  // :691-698
+    if (ln.sub == 0 && (fi & BSC_FLAG_BUFFER)) {  // :691-698
         S.vxs[i] = S.vx[i];
         S.vys[i] = K.g * S.por[i] * dt;
     }
@@ -1072,13 +1082,15 @@ int op_int_vel(Ctx* c, const double* d_umax) {
     BSC_LAUNCH(c);
     StageTimer tk(c, BSC_T_K_INT_VEL);
     if (mx)
-        k_int_vel<float><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->gwf, c->cnt, nu, c->dt,
+        k_int_vel<float, 1><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->gwf, c->cnt, nu, c->dt,
                                                         c->f_vol, c->f_nu, c->f_nut, c->f_tke, c->f_varts, c->posf,
                                                         c->pcell);
     else
-        k_int_vel<double><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->gw, c->cnt, nu, c->dt,
-                                                         nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                                                         nullptr);
+        with_pair_lanes(c->n, [&](auto L) {
+            k_int_vel<double, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
+                c->n, c->S, c->K, c->nbr, c->gw, c->cnt, nu, c->dt, nullptr, nullptr, nullptr, nullptr, nullptr,
+                nullptr, nullptr);
+        });
     BSC_LAUNCH(c);
     return BSC_OK;
 }
@@ -1099,42 +1111,51 @@ __global__ void k_rho_over_por(int64_t n, State S, double* __restrict__ q, float
     }
 }
 
-template <typename R>
+template <typename R, int L>
 __global__ void __launch_bounds__(NB_BLOCK) k_comp_vel(int64_t n, State S, KParams K, const int32_t* __restrict__ nbr,
                                                         const typename Vec2<R>::type* __restrict__ gw,
                                                         const int32_t* __restrict__ cnt,
                                                         const double* __restrict__ q, double dt) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const Lanes<L> ln;
+    const int64_t i = ln.particle();
     if (i >= n) return;
     const uint8_t fi = S.flags[i];
     if (S.tid[i] == BSC_TID_FLUID && !(fi & (BSC_FLAG_BUFFER | BSC_FLAG_DEAD))) {
         const R L0 = to_r<R>(S.L0[i]), L1 = to_r<R>(S.L1[i]), L2 = to_r<R>(S.L2[i]), L3 = to_r<R>(S.L3[i]);
         const R ni = (R)S.por[i], rhoi = (R)S.rho[i], pi = (R)S.p[i], qi = (R)q[i];
         const R c0 = ni * ni / rhoi;
-        R wgx = 0, wgy = 0;  // sums of w grad W; the row's L is applied after them
+        R sum[2] = {0, 0};  // sums of w grad W; the row's L is applied after them
         const int m = cnt[i];
-        for (int k = 0; k < m; ++k) {
-            const int64_t e = ell(i, k, K.kmax);
-            const int j = nbr[e];
-            const auto g = gw[e];
-            const R vj = (R)S.vol[j], pj = (R)S.p[j];
-            R w;
-            if (S.tid[j] == BSC_TID_FLUID) {
-                const R qj = (R)q[j];
-                w = (R)2 * vj * c0 * (pj * qi + pi * qj) / (qi + qj);
-            } else {
-                w = vj * c0 * (pj + pi);
+        for (int k0 = 0; k0 < m; k0 += L) {
+            const int k = k0 + ln.sub;
+            R w[2] = {0, 0}, gr[2] = {0, 0};
+            if (L == 1 || k < m) {
+                const int64_t e = ell(i, k, K.kmax);
+                const int j = nbr[e];
+                const auto g = gw[e];
+                const R vj = (R)S.vol[j], pj = (R)S.p[j];
+                if (S.tid[j] == BSC_TID_FLUID) {
+                    const R qj = (R)q[j];
+                    w[0] = (R)2 * vj * c0 * (pj * qi + pi * qj) / (qi + qj);
+                } else {
+                    w[0] = vj * c0 * (pj + pi);
+                }
+                w[1] = w[0];
+                gr[0] = g.x;
+                gr[1] = g.y;
             }
-            wgx += w * g.x;
-            wgy += w * g.y;
+            ln.ordered(sum, w, gr);
         }
+        const R wgx = sum[0], wgy = sum[1];
         const R ax = L0 * wgx + L1 * wgy, ay = L2 * wgx + L3 * wgy;
+        if (ln.sub != 0) return;
         const double vx = S.vxs[i] - dt * (double)ax;
         const double vy = S.vys[i] - dt * (double)ay;
         S.vx[i] = vx;
         S.vy[i] = vy;
         S.vel[i] = sqrt(vx * vx + vy * vy) / S.por[i];
     }
+    if (ln.sub != 0) return;
     if (fi & BSC_FLAG_BUFFER) {
         S.vx[i] = S.vxs[i];
         S.vy[i] = 0.0;
@@ -1214,7 +1235,10 @@ int op_comp_vel(Ctx* c) {
         k_comp_vel_mixed<<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->gwf, c->gwl, c->cnt, c->f_q,
                                                         c->f_vol, c->f_vol_lo, c->dt);
     else
-        k_comp_vel<double><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->gw, c->cnt, q, c->dt);
+        with_pair_lanes(c->n, [&](auto L) {
+            k_comp_vel<double, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
+                c->n, c->S, c->K, c->nbr, c->gw, c->cnt, q, c->dt);
+        });
     BSC_LAUNCH(c);
     return BSC_OK;
 }

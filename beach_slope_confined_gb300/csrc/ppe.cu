@@ -39,7 +39,8 @@ namespace bsc {
 // FAST (the mixed path): the per-pair and per-row quotients by rcp_nr, a
 // Newton-Raphson reciprocal within ~2^-46 of the FP64 quotient.  The FP64
 // path divides (correctly rounded, as the reference).
-template <typename R, bool FAST>
+// L lanes per row (lanes_for), the sums in list order.
+template <typename R, bool FAST, int L>
 __global__ void __launch_bounds__(NB_BLOCK) k_assemble(int64_t n, State S, KParams K, const int32_t* __restrict__ nbr,
                                                         const typename Vec2<R>::type* __restrict__ gw,
                                                         const int32_t* __restrict__ cnt, R* __restrict__ aval,
@@ -47,7 +48,8 @@ __global__ void __launch_bounds__(NB_BLOCK) k_assemble(int64_t n, State S, KPara
                                                         double* __restrict__ b, const double* __restrict__ q,
                                                         const double* __restrict__ usx, const double* __restrict__ usy,
                                                         double dt) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const Lanes<L> ln;
+    const int64_t i = ln.particle();
     if (i >= n) return;
     const int tid_i = S.tid[i];
     const bool free_i = S.flags[i] & BSC_FLAG_FREE;
@@ -72,73 +74,81 @@ __global__ void __launch_bounds__(NB_BLOCK) k_assemble(int64_t n, State S, KPara
         vyi_n = quot(S.vys[i], (double)ni);
     }
     const int m = cnt[i];
-    R dia = 0, fv = 0;
-    for (int k = 0; k < m; ++k) {
-        const int64_t e = ell(i, k, K.kmax);
-        const int j = nbr[e];
-        const auto g = gw[e];
-        const int tid_j = S.tid[j];
-        const double dx = xi - S.x[j], dy = yi - S.y[j];
-        const R p_dist = (R)quot(1.0, (R)(dx * dx + dy * dy) + (R)K.lam);
-        const R pvol = (R)S.vol[j];
-        R val = 0;
-        if (tid_i == BSC_TID_FLUID) {
-            const R lamp = (free_i && tid_j == BSC_TID_FLUID) ? (R)1 + (R)S.oden[j] * lamp_f : (R)1;
-            const R gx = L0 * g.x + L1 * g.y, gy = L2 * g.x + L3 * g.y;
-            const R t = (R)2 * pvol * ((R)dx * gx + (R)dy * gy) * p_dist;
-            val = -t;
-            dia += t * lamp;
-            // divergence of the porous-weighted predicted velocity (:241-270)
-            R ddx, ddy;
-            if (tid_j == BSC_TID_FLUID) {
-                // 2 rho_i rho_j / (n_i n_j (rho_i/n_i + rho_j/n_j)) = 2 q_i q_j / (q_i + q_j)
-                const R qj = (R)q[j];
-                const R rho_ij = qj == qi ? rho_ii : (R)quot((R)2 * qi * qj, qi + qj);
-                ddx = rho_ij * (R)(usx[j] - usxi);
-                ddy = rho_ij * (R)(usy[j] - usyi);
-            } else {
-                ddx = qi * ((R)(S.vxs[j] - S.vxs[i]) * inv_ni);
-                ddy = qi * ((R)(S.vys[j] - S.vys[i]) * inv_ni);
-            }
-            fv += pvol * (ddx * gx + ddy * gy);
-        } else if (tid_i == BSC_TID_GHOST) {
-            if (tid_j <= 2) {
-                const R t = (R)2 * pvol * ((R)dx * g.x + (R)dy * g.y) * p_dist;
+    R sum[2] = {0, 0};  // the diagonal, and the right-hand side's divergence
+    for (int k0 = 0; k0 < m; k0 += L) {
+        const int k = k0 + ln.sub;
+        R ta[2] = {0, 0}, tb[2] = {1, 0};  // their terms' factors
+        if (L == 1 || k < m) {
+            const int64_t e = ell(i, k, K.kmax);
+            const int j = nbr[e];
+            const auto g = gw[e];
+            const int tid_j = S.tid[j];
+            const double dx = xi - S.x[j], dy = yi - S.y[j];
+            const R p_dist = (R)quot(1.0, (R)(dx * dx + dy * dy) + (R)K.lam);
+            const R pvol = (R)S.vol[j];
+            R val = 0;
+            if (tid_i == BSC_TID_FLUID) {
+                const R lamp = (free_i && tid_j == BSC_TID_FLUID) ? (R)1 + (R)S.oden[j] * lamp_f : (R)1;
+                const R gx = L0 * g.x + L1 * g.y, gy = L2 * g.x + L3 * g.y;
+                const R t = (R)2 * pvol * ((R)dx * gx + (R)dy * gy) * p_dist;
                 val = -t;
-                dia += t;
+                ta[0] = t;
+                tb[0] = lamp;
+                // divergence of the porous-weighted predicted velocity (:241-270)
+                R ddx, ddy;
+                if (tid_j == BSC_TID_FLUID) {
+                    // 2 rho_i rho_j / (n_i n_j (rho_i/n_i + rho_j/n_j)) = 2 q_i q_j / (q_i + q_j)
+                    const R qj = (R)q[j];
+                    const R rho_ij = qj == qi ? rho_ii : (R)quot((R)2 * qi * qj, qi + qj);
+                    ddx = rho_ij * (R)(usx[j] - usxi);
+                    ddy = rho_ij * (R)(usy[j] - usyi);
+                } else {
+                    ddx = qi * ((R)(S.vxs[j] - S.vxs[i]) * inv_ni);
+                    ddy = qi * ((R)(S.vys[j] - S.vys[i]) * inv_ni);
+                }
+                ta[1] = pvol;
+                tb[1] = ddx * gx + ddy * gy;
+            } else if (tid_i == BSC_TID_GHOST) {
+                if (tid_j <= 2) {
+                    const R t = (R)2 * pvol * ((R)dx * g.x + (R)dy * g.y) * p_dist;
+                    val = -t;
+                    ta[0] = t;
+                }
+            } else if (tid_i == BSC_TID_WALL) {
+                if (tid_j == BSC_TID_FLUID) {
+                    const R Lj0 = (R)S.L0[j], Lj1 = (R)S.L1[j], Lj2 = (R)S.L2[j], Lj3 = (R)S.L3[j];
+                    const R gx = Lj0 * g.x + Lj1 * g.y, gy = Lj2 * g.x + Lj3 * g.y;
+                    const R t = (R)2 * mi_over_rhoi * ((R)dx * gx + (R)dy * gy) * p_dist;
+                    val = -t;
+                    ta[0] = t;
+                    const R qj = (R)q[j];
+                    const R ddx = qj * (R)(usx[j] - vxi_n);
+                    const R ddy = qj * (R)(usy[j] - vyi_n);
+                    ta[1] = mi_over_rhoi;
+                    tb[1] = ddx * gx + ddy * gy;
+                } else {
+                    const R t = (R)2 * pvol * ((R)dx * g.x + (R)dy * g.y) * p_dist;
+                    val = -t;
+                    ta[0] = t;
+                }
             }
-        } else if (tid_i == BSC_TID_WALL) {
-            if (tid_j == BSC_TID_FLUID) {
-                const R Lj0 = (R)S.L0[j], Lj1 = (R)S.L1[j], Lj2 = (R)S.L2[j], Lj3 = (R)S.L3[j];
-                const R gx = Lj0 * g.x + Lj1 * g.y, gy = Lj2 * g.x + Lj3 * g.y;
-                const R t = (R)2 * mi_over_rhoi * ((R)dx * gx + (R)dy * gy) * p_dist;
-                val = -t;
-                dia += t;
-                const R qj = (R)q[j];
-                const R ddx = qj * (R)(usx[j] - vxi_n);
-                const R ddy = qj * (R)(usy[j] - vyi_n);
-                fv += mi_over_rhoi * (ddx * gx + ddy * gy);
-            } else {
-                const R t = (R)2 * pvol * ((R)dx * g.x + (R)dy * g.y) * p_dist;
-                val = -t;
-                dia += t;
-            }
+            aval[e] = val;
         }
-        aval[e] = val;
+        ln.ordered(sum, ta, tb);
     }
-    const double d = (double)dia;
+    const double d = (double)sum[0];
     if (d == 0.0 || !isfinite(d)) {
         // zero-neighbour guard: identity row, b = 0 (the reference divides by 0)
-        for (int k = 0; k < m; ++k) {
+        for (int k = ln.sub; k < m; k += L) {
             aval[ell(i, k, K.kmax)] = 0;
             if (ellf) ellf[ell(i, k, K.kmax)] = make_int2(nbr[ell(i, k, K.kmax)], 0);
             if (avalh) avalh[ell(i, k, K.kmax)] = __float2half_rn(0.f);
         }
-        b[i] = 0.0;
+        if (ln.sub == 0) b[i] = 0.0;
         return;
     }
     const R inv = (R)(1.0 / d);
-    for (int k = 0; k < m; ++k) {
+    for (int k = ln.sub; k < m; k += L) {
         const int64_t e = ell(i, k, K.kmax);
         const R v = aval[e] * inv;
         aval[e] = v;
@@ -148,7 +158,7 @@ __global__ void __launch_bounds__(NB_BLOCK) k_assemble(int64_t n, State S, KPara
             avalh[e] = __float2half_rn(vf);
         }
     }
-    b[i] = ((double)fv / dt) / d;
+    if (ln.sub == 0) b[i] = ((double)sum[1] / dt) / d;
 }
 
 // ---- the mixed path's assembly in double-float arithmetic (dfloat.cuh) -------------
@@ -350,12 +360,14 @@ int op_ppe_assemble(Ctx* c) {
     } else {
         StageTimer tk(c, BSC_T_K_ASSEMBLE);
         if (c->mixed && !c->exact_div)
-            k_assemble<double, true><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->gw, c->cnt, c->aval,
+            k_assemble<double, true, 1><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->gw, c->cnt, c->aval,
                                                                     c->ellf, c->avalh, c->b, q, ux, uy, c->dt);
         else
-            k_assemble<double, false><<<g, NB_BLOCK, 0, c->stream>>>(
-                c->n, c->S, c->K, c->nbr, c->gw, c->cnt, c->aval, c->mixed ? c->ellf : nullptr,
-                c->mixed ? c->avalh : nullptr, c->b, q, ux, uy, c->dt);
+            with_pair_lanes(c->n, [&](auto L) {
+                k_assemble<double, false, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
+                    c->n, c->S, c->K, c->nbr, c->gw, c->cnt, c->aval, c->mixed ? c->ellf : nullptr,
+                    c->mixed ? c->avalh : nullptr, c->b, q, ux, uy, c->dt);
+            });
         BSC_LAUNCH(c);
     }
     if (c->mixed) {
