@@ -57,7 +57,8 @@ struct Lanes {
         for (int u = 0; u < L; ++u)
 #pragma unroll
             for (int q = 0; q < N; ++q)
-                acc[q] = fma(L == 1 ? a[q] : __shfl_sync(mask, a[q], u, L), L == 1 ? b[q] : __shfl_sync(mask, b[q], u, L), acc[q]);
+                acc[q] = fma(L == 1 ? a[q] : __shfl_sync(mask, a[q], u, L),
+                             L == 1 ? b[q] : __shfl_sync(mask, b[q], u, L), acc[q]);
     }
     // the place of this lane's kept item among the particle's, after `count`
     // of them; count moves past them
@@ -83,10 +84,14 @@ void with_lanes(int lanes, F f) {
     }
 }
 
-// the FP64 step's pair sums, whose rounds cost more than WCSPH's: one lane or four
+// The FP64 step's pair sums: four lanes, their terms added up in list order
+// (Lanes::ordered).  Measured, the step's five pair kernels together with one
+// and four lanes: 418 and 361 us at 21490 particles, 472 and 428 at 25881,
+// 470 and 519 at 35943 (at 3816: 278 and 113).
+inline bool pair_lanes(int64_t n) { return n <= 30000; }
 template <typename F>
 void with_pair_lanes(int64_t n, F f) {
-    if (lanes_for(n) > 1) f(std::integral_constant<int, 4>{});
+    if (pair_lanes(n)) f(std::integral_constant<int, 4>{});
     else f(std::integral_constant<int, 1>{});
 }
 

@@ -430,8 +430,8 @@ __global__ void __launch_bounds__(NB_BLOCK) k_neighbour_lists(
     cnt[i] = count;
 }
 
-static void launch_lists(Ctx* c) {
-    with_lanes(lanes_for(c->n), [&](auto L) {
+static void launch_lists(Ctx* c, int lanes) {
+    with_lanes(lanes, [&](auto L) {
         k_neighbour_lists<L.value><<<blocks_for(c->n * L.value, NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
             c->n, c->S.x, c->S.y, c->K, c->cell_start, c->cell_count, c->sorted, c->pcell, c->posf, c->nbr, c->cnt,
             c->d_flag);
@@ -442,7 +442,7 @@ int op_neighbour_lists(Ctx* c) {
     k_posf<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->S.x, c->S.y, c->pcell, c->K, c->posf, c->S.vol,
                                                          nullptr, nullptr, nullptr);
     BSC_LAUNCH(c);
-    launch_lists(c);
+    launch_lists(c, lanes_for(c->n));
     BSC_LAUNCH(c);
     return BSC_OK;
 }
@@ -535,8 +535,8 @@ int op_neighbour(Ctx* c) {
         k_neighbour<float><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->cell_start, c->cell_count, c->sorted,
                                                           c->pcell, c->posf, c->posd, c->nbr, gw64, c->gwf, c->gwl,
                                                           c->f_vol, c->ndist, c->cnt, c->d_flag);
-    else if (lanes_for(c->n) > 1) {
-        launch_lists(c);
+    else if (pair_lanes(c->n)) {
+        launch_lists(c, std::max(4, lanes_for(c->n)));
         BSC_LAUNCH(c);
         k_neighbour_rows<<<blocks_for(c->n * 4, NB_BLOCK), NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->cnt,
                                                                                   c->gw, c->ndist);

@@ -35,3 +35,26 @@ def test_lanes_per_row(dx, length, kernel):
     for prec in ("fp64", "mixed"):
         p = pressure(spec, precision=prec, **mg)[1]
         assert np.linalg.norm(p - want) <= 600 * 2e-10 * np.linalg.norm(want), prec
+
+
+@pytest.mark.parametrize("kernel", [0, 1])
+@pytest.mark.parametrize("dx", [0.0068, 0.0064])
+def test_lanes_per_particle_keep_the_bits(dx, kernel, monkeypatch):
+    """The FP64 search by lanes and the one-thread FP64 phase over the
+    warp-per-cell search's lists write the same lists and fields (a tank on
+    each side of the 30000 particles up to which lanes share a particle)."""
+    spec = sc.TankSpec(dx=dx, kernel=kernel, piston_ramp=0.0)
+    scen = sc.build(spec)
+    assert (scen.n <= 30000) == (dx > 0.0066)
+    out = []
+    for variant in ("thread", "warpcell"):
+        monkeypatch.setenv("BSC_NEIGHBOUR", variant)
+        g = Solver(sc.make_params(spec, scen.bounds, solver="fgmres", precond="mg", tol=1e-8, maxit=2000))
+        setup_tank(g, scen)
+        g.step(1)
+        out.append((g.download_state(), g.get_neighbors()))
+        g.close()
+    (a, la), (b, lb) = out
+    assert np.array_equal(la[0], lb[0]) and np.array_equal(la[1], lb[1])
+    for f in ("x", "y", "vx", "vy", "p", "nut", "porosity", "L"):
+        assert np.array_equal(a[f], b[f]), f
