@@ -88,10 +88,14 @@ void with_lanes(int lanes, F f) {
 // (Lanes::ordered).  Measured, the step's five pair kernels together with one
 // and four lanes: 418 and 361 us at 21490 particles, 472 and 428 at 25881,
 // 470 and 519 at 35943 (at 3816: 278 and 113).
-inline bool pair_lanes(int64_t n) { return n <= 30000; }
+// The lighter ones (eddyvis, varts, shift, freesurf, and the mixed path's FP32
+// sums) gain nothing above PAIR_LANES_LIGHT: the routine sequence at 23441
+// particles 2.35 ms with one lane there, 2.39 with four.
+constexpr int64_t PAIR_LANES = 30000, PAIR_LANES_LIGHT = 20000;
+inline bool pair_lanes(int64_t n) { return n <= PAIR_LANES; }
 template <typename F>
-void with_pair_lanes(int64_t n, F f) {
-    if (pair_lanes(n)) f(std::integral_constant<int, 4>{});
+void with_pair_lanes(int64_t n, F f, int64_t most = PAIR_LANES) {
+    if (n <= most) f(std::integral_constant<int, 4>{});
     else f(std::integral_constant<int, 1>{});
 }
 

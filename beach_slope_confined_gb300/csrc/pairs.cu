@@ -553,21 +553,27 @@ int op_neighbour(Ctx* c) {
 // vicinity_j |= (exists neighbour i: fluid, not buffer, tr M_i <= threshold).
 // The neighbour relation is symmetric, so j's own list enumerates the i that
 // would have scattered to it; this removes the reference's racy scatter.
+template <int L>
 __global__ void k_freesurf(int64_t n, State S, KParams K, const int32_t* __restrict__ nbr,
                            const int32_t* __restrict__ cnt) {
-    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const Lanes<L> ln;
+    const int64_t j = ln.particle();
     if (j >= n) return;
     const int m = cnt[j];
     bool hit = false;
-    for (int k = 0; k < m && !hit; ++k) {
+    for (int k = ln.sub; k < m && !hit; k += L) {
         const int i = nbr[ell(j, k, K.kmax)];
         hit = (S.tid[i] == BSC_TID_FLUID) && !(S.flags[i] & BSC_FLAG_BUFFER) && (S.gradvx[i] <= K.free_thr);
     }
-    if (hit) S.flags[j] |= BSC_FLAG_VICINITY;
+    if (L > 1) hit = __ballot_sync(ln.mask, hit) & ln.mask;
+    if (ln.sub == 0 && hit) S.flags[j] |= BSC_FLAG_VICINITY;
 }
 
 int op_freesurf(Ctx* c) {
-    k_freesurf<<<blocks_for(c->n, NB_BLOCK), NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->cnt);
+    with_pair_lanes(c->n, [&](auto L) {
+        k_freesurf<L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr,
+                                                                                     c->cnt);
+    }, PAIR_LANES_LIGHT);
     BSC_LAUNCH(c);
     return BSC_OK;
 }
@@ -794,47 +800,57 @@ __device__ __forceinline__ float2 udf_diff(float4 uj, float4 ui) {
 }
 
 // ---- turbulence.f90:12-110 eddyvis -----------------------------------------------
-template <typename R>
+template <typename R, int L>
 __global__ void __launch_bounds__(NB_BLOCK) k_eddyvis(int64_t n, State S, KParams K, const int32_t* __restrict__ nbr,
                                                        const typename Vec2<R>::type* __restrict__ gw,
                                                        const int32_t* __restrict__ cnt, const double* __restrict__ ux,
                                                        const double* __restrict__ uy, const float* __restrict__ f_vol,
                                                        const float4* __restrict__ udf) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const Lanes<L> ln;
+    const int64_t i = ln.particle();
     if (i >= n || S.tid[i] != BSC_TID_FLUID) return;
     const R L0 = to_r<R>(S.L0[i]), L1 = to_r<R>(S.L1[i]), L2 = to_r<R>(S.L2[i]), L3 = to_r<R>(S.L3[i]);
     const double uxi = ux[i], uyi = uy[i];
     [[maybe_unused]] const float4 udi = sizeof(R) == 4 ? udf[i] : float4{};
-    R t1 = 0, t2 = 0, t3 = 0;
+    R sum[3] = {0, 0, 0};
     const int m = cnt[i];
     // FP32 sums: four entries' gathers in flight (measured 3-7 % faster)
     #pragma unroll(sizeof(R) == 4 ? 4 : 1)
-    for (int k = 0; k < m; ++k) {
-        const int64_t e = ell(i, k, K.kmax);
-        const int j = nbr[e];
-        const auto g = gw[e];
-        R vj;
-        if constexpr (sizeof(R) == 4)
-            vj = f_vol[j];
-        else
-            vj = S.vol[j];
-        // differences in FP64 (they cancel); for R = float in double-float
-        // arithmetic, rounded
-        R du, dv;
-        if constexpr (sizeof(R) == 4) {
-            const float2 d = udf_diff(udf[j], udi);
-            du = d.x;
-            dv = d.y;
-        } else {
-            du = ux[j] - uxi;
-            dv = uy[j] - uyi;
+    for (int k0 = 0; k0 < m; k0 += L) {
+        const int k = k0 + ln.sub;
+        R ta[3] = {0, 0, 0}, tb[3] = {0, 0, 0};  // the terms' factors
+        if (L == 1 || k < m) {
+            const int64_t e = ell(i, k, K.kmax);
+            const int j = nbr[e];
+            const auto g = gw[e];
+            R vj;
+            if constexpr (sizeof(R) == 4)
+                vj = f_vol[j];
+            else
+                vj = S.vol[j];
+            // differences in FP64 (they cancel); for R = float in double-float
+            // arithmetic, rounded
+            R du, dv;
+            if constexpr (sizeof(R) == 4) {
+                const float2 d = udf_diff(udf[j], udi);
+                du = d.x;
+                dv = d.y;
+            } else {
+                du = ux[j] - uxi;
+                dv = uy[j] - uyi;
+            }
+            const R gx = L0 * g.x + L1 * g.y, gy = L2 * g.x + L3 * g.y;
+            ta[0] = vj * du;
+            tb[0] = gx;
+            ta[1] = vj * dv;
+            tb[1] = gy;
+            ta[2] = (R)0.5 * vj;
+            tb[2] = du * gy + dv * gx;
         }
-        const R gx = L0 * g.x + L1 * g.y, gy = L2 * g.x + L3 * g.y;
-        t1 += vj * du * gx;
-        t2 += vj * dv * gy;
-        t3 += (R)0.5 * vj * (du * gy + dv * gx);
+        ln.ordered(sum, ta, tb);
     }
-    const double T1 = t1, T2 = t2, T3 = t3;
+    if (ln.sub != 0) return;
+    const double T1 = sum[0], T2 = sum[1], T3 = sum[2];
     const double t4 = sqrt(2 * (T1 * T1 + T2 * T2) + (2 * T3) * (2 * T3));
     const double csdl = K.eddy_cs * K.dl, dlt = K.dl * t4;
     S.nut[i] = (csdl * csdl) * t4;
@@ -847,55 +863,66 @@ int op_eddyvis(Ctx* c) {
     k_vel_over_por<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->S, ux, uy, c->mixed ? c->f_vol : nullptr,
                                                                  c->mixed ? c->udf : nullptr);
     BSC_LAUNCH(c);
-    const unsigned g = blocks_for(c->n, NB_BLOCK);
     if (c->mixed)
-        k_eddyvis<float><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->gwf, c->cnt, ux, uy, c->f_vol,
-                                                        c->udf);
+        with_pair_lanes(c->n, [&](auto L) {
+            k_eddyvis<float, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
+                c->n, c->S, c->K, c->nbr, c->gwf, c->cnt, ux, uy, c->f_vol, c->udf);
+        }, PAIR_LANES_LIGHT);
     else
-        k_eddyvis<double><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->gw, c->cnt, ux, uy, nullptr,
-                                                         nullptr);
+        with_pair_lanes(c->n, [&](auto L) {
+            k_eddyvis<double, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
+                c->n, c->S, c->K, c->nbr, c->gw, c->cnt, ux, uy, nullptr, nullptr);
+        }, PAIR_LANES_LIGHT);
     BSC_LAUNCH(c);
     return BSC_OK;
 }
 
 // ---- integrator.f90:458-713 int_vel ------------------------------------------------
 // pass 1: free-surface artificial viscosity (:467-506)
-template <typename R>
+template <typename R, int L>
 __global__ void __launch_bounds__(NB_BLOCK) k_varts(int64_t n, State S, KParams K, const int32_t* __restrict__ nbr,
                                                      const typename Vec2<R>::type* __restrict__ gw,
                                                      const int32_t* __restrict__ cnt, const double* __restrict__ ux,
                                                      const double* __restrict__ uy, const double* __restrict__ umax,
                                                      const float* __restrict__ f_vol, float* __restrict__ f_varts,
                                                      const float4* __restrict__ udf) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const Lanes<L> ln;
+    const int64_t i = ln.particle();
     if (i >= n || !(S.flags[i] & BSC_FLAG_FREE)) return;
     const R L0 = to_r<R>(S.L0[i]), L1 = to_r<R>(S.L1[i]), L2 = to_r<R>(S.L2[i]), L3 = to_r<R>(S.L3[i]);
     const double uxi = ux[i], uyi = uy[i];
     [[maybe_unused]] const float4 udi = sizeof(R) == 4 ? udf[i] : float4{};
-    R t1 = 0, t2 = 0;
+    R sum[2] = {0, 0};
     const int m = cnt[i];
-    for (int k = 0; k < m; ++k) {
-        const int64_t e = ell(i, k, K.kmax);
-        const int j = nbr[e];
-        const auto g = gw[e];
-        R vj;
-        if constexpr (sizeof(R) == 4)
-            vj = f_vol[j];
-        else
-            vj = S.vol[j];
-        R du, dv;
-        if constexpr (sizeof(R) == 4) {
-            const float2 d = udf_diff(udf[j], udi);
-            du = d.x;
-            dv = d.y;
-        } else {
-            du = ux[j] - uxi;
-            dv = uy[j] - uyi;
+    for (int k0 = 0; k0 < m; k0 += L) {
+        const int k = k0 + ln.sub;
+        R ta[2] = {0, 0}, tb[2] = {0, 0};  // the terms' factors
+        if (L == 1 || k < m) {
+            const int64_t e = ell(i, k, K.kmax);
+            const int j = nbr[e];
+            const auto g = gw[e];
+            R vj;
+            if constexpr (sizeof(R) == 4)
+                vj = f_vol[j];
+            else
+                vj = S.vol[j];
+            R du, dv;
+            if constexpr (sizeof(R) == 4) {
+                const float2 d = udf_diff(udf[j], udi);
+                du = d.x;
+                dv = d.y;
+            } else {
+                du = ux[j] - uxi;
+                dv = uy[j] - uyi;
+            }
+            ta[0] = du * (L0 * g.x + L1 * g.y);
+            ta[1] = dv * (L2 * g.x + L3 * g.y);
+            tb[0] = tb[1] = vj;
         }
-        t1 += du * (L0 * g.x + L1 * g.y) * vj;
-        t2 += dv * (L2 * g.x + L3 * g.y) * vj;
+        ln.ordered(sum, ta, tb);
     }
-    const double T1 = t1, T2 = t2, vx = S.vx[i], vy = S.vy[i];
+    if (ln.sub != 0) return;
+    const double T1 = sum[0], T2 = sum[1], vx = S.vx[i], vy = S.vy[i];
     const double va = K.varts_ps * (K.dl * K.dl) * sqrt(T1 * T1 + T2 * T2) * sqrt(vx * vx + vy * vy) /
                       ((*umax + (double)1e-6f) * S.por[i]);
     S.varts[i] = va;
@@ -1065,26 +1092,31 @@ __global__ void k_kin_visc(int64_t n, State S, double* __restrict__ nu, float* _
 int op_int_vel(Ctx* c, const double* d_umax) {
     if (!c->have_lists) return set_err(c, BSC_E_INVALID, "int_vel before neighbour");
     double *ux = c->r, *uy = c->rh, *nu = c->pd;
-    const unsigned g = blocks_for(c->n, NB_BLOCK);
     const bool mx = c->mixed;
     k_vel_over_por<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->S, ux, uy, mx ? c->f_vol : nullptr,
                                                                  mx ? c->udf : nullptr);
     BSC_LAUNCH(c);
     if (mx)
-        k_varts<float><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->gwf, c->cnt, ux, uy, d_umax,
-                                                      c->f_vol, c->f_varts, c->udf);
+        with_pair_lanes(c->n, [&](auto L) {
+            k_varts<float, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
+                c->n, c->S, c->K, c->nbr, c->gwf, c->cnt, ux, uy, d_umax, c->f_vol, c->f_varts, c->udf);
+        }, PAIR_LANES_LIGHT);
     else
-        k_varts<double><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->gw, c->cnt, ux, uy, d_umax,
-                                                       nullptr, nullptr, nullptr);
+        with_pair_lanes(c->n, [&](auto L) {
+            k_varts<double, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
+                c->n, c->S, c->K, c->nbr, c->gw, c->cnt, ux, uy, d_umax, nullptr, nullptr, nullptr);
+        }, PAIR_LANES_LIGHT);
     BSC_LAUNCH(c);
     k_kin_visc<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->S, nu, mx ? c->f_nu : nullptr,
                                                              mx ? c->f_nut : nullptr, mx ? c->f_tke : nullptr);
     BSC_LAUNCH(c);
     StageTimer tk(c, BSC_T_K_INT_VEL);
     if (mx)
-        k_int_vel<float, 1><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->gwf, c->cnt, nu, c->dt,
-                                                        c->f_vol, c->f_nu, c->f_nut, c->f_tke, c->f_varts, c->posf,
-                                                        c->pcell);
+        with_pair_lanes(c->n, [&](auto L) {
+            k_int_vel<float, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
+                c->n, c->S, c->K, c->nbr, c->gwf, c->cnt, nu, c->dt, c->f_vol, c->f_nu, c->f_nut, c->f_tke,
+                c->f_varts, c->posf, c->pcell);
+        }, PAIR_LANES_LIGHT);
     else
         with_pair_lanes(c->n, [&](auto L) {
             k_int_vel<double, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
@@ -1257,15 +1289,16 @@ int op_comp_vel(Ctx* c) {
 // of the velocities (taken on the integer pipe) and the FP32 grad W (an
 // error of ~1e-8 of v in the correction), so the kernel issues no FP64
 // operation per pair (ten on the FP64 path).
-template <typename R>
+template <typename R, int L>
 __global__ void __launch_bounds__(NB_BLOCK) k_shift(int64_t n, State S, KParams K, const int32_t* __restrict__ nbr,
                                                      const double2* __restrict__ gw, const float2* __restrict__ gwf,
                                                      const float2* __restrict__ gwl, const float* __restrict__ f_vol,
                                                      const float* __restrict__ f_vol_lo,
                                                      const int32_t* __restrict__ cnt, int8_t* __restrict__ mark) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const Lanes<L> ln;
+    const int64_t i = ln.particle();
     if (i >= n) return;
-    mark[i] = 0;
+    if (ln.sub == 0) mark[i] = 0;
     const uint8_t fi = S.flags[i];
     if (!(S.tid[i] == BSC_TID_FLUID && !(fi & (BSC_FLAG_BUFFER | BSC_FLAG_DEAD)))) return;
     const int m = cnt[i];
@@ -1276,45 +1309,49 @@ __global__ void __launch_bounds__(NB_BLOCK) k_shift(int64_t n, State S, KParams 
     // the corrected gradient L grad W enters linearly and L is the row's own,
     // so L is applied once to the four sums of grad W (dv V) rather than per
     // pair
-    double sx = 0, sy = 0;
     [[maybe_unused]] df2 sxd{0.f, 0.f}, syd{0.f, 0.f};
     [[maybe_unused]] const float vxif = f32_of(vxi), vyif = f32_of(vyi);
-    R ax = 0, bx = 0, ay = 0, by = 0;
+    R sum[6] = {0, 0, 0, 0, 0, 0};  // FP64: the shift's two; then grad W (dv V)
     // FP32 sums: four entries' gathers in flight (measured 3-7 % faster)
     #pragma unroll(sizeof(R) == 4 ? 4 : 1)
-    for (int k = 0; k < m; ++k) {
-        const int64_t e = ell(i, k, K.kmax);
-        const int j = nbr[e];
-        R gx, gy, dvx, dvy;
-        if constexpr (F32) {
-            const float2 gf = gwf[e], gl = gwl[e];
-            const float vf = f_vol[j];
-            const df2 vjd{vf, f_vol_lo[j]};
-            sxd = df_add(sxd, df_mul(df2{gf.x, gl.x}, vjd));
-            syd = df_add(syd, df_mul(df2{gf.y, gl.y}, vjd));
-            gx = gf.x;
-            gy = gf.y;
-            dvx = (f32_of(S.vx[j]) - vxif) * vf;
-            dvy = (f32_of(S.vy[j]) - vyif) * vf;
-        } else {
-            const double2 g = gw[e];
-            const double vj = S.vol[j];
-            sx += g.x * vj;
-            sy += g.y * vj;
-            gx = g.x;
-            gy = g.y;
-            dvx = (S.vx[j] - vxi) * vj;
-            dvy = (S.vy[j] - vyi) * vj;
+    for (int k0 = 0; k0 < m; k0 += L) {
+        const int k = k0 + ln.sub;
+        R gx = 0, gy = 0, dvx = 0, dvy = 0, vj = 0;
+        if (L == 1 || k < m) {
+            const int64_t e = ell(i, k, K.kmax);
+            const int j = nbr[e];
+            if constexpr (F32) {
+                const float2 gf = gwf[e], gl = gwl[e];
+                const float vf = f_vol[j];
+                const df2 vjd{vf, f_vol_lo[j]};
+                sxd = df_add(sxd, df_mul(df2{gf.x, gl.x}, vjd));
+                syd = df_add(syd, df_mul(df2{gf.y, gl.y}, vjd));
+                gx = gf.x;
+                gy = gf.y;
+                dvx = (f32_of(S.vx[j]) - vxif) * vf;
+                dvy = (f32_of(S.vy[j]) - vyif) * vf;
+            } else {
+                const double2 g = gw[e];
+                vj = S.vol[j];
+                gx = g.x;
+                gy = g.y;
+                dvx = (S.vx[j] - vxi) * vj;
+                dvy = (S.vy[j] - vyi) * vj;
+            }
         }
-        ax += gx * dvx;
-        bx += gy * dvx;
-        ay += gx * dvy;
-        by += gy * dvy;
+        if constexpr (F32) {
+            sum[2] += gx * dvx;
+            sum[3] += gy * dvx;
+            sum[4] += gx * dvy;
+            sum[5] += gy * dvy;
+        } else {
+            const R ta[6] = {gx, gy, gx, gy, gx, gy}, tb[6] = {vj, vj, dvx, dvx, dvy, dvy};
+            ln.ordered(sum, ta, tb);
+        }
     }
-    if constexpr (F32) {
-        sx = df_to_double(sxd);
-        sy = df_to_double(syd);
-    }
+    if (ln.sub != 0) return;
+    const double sx = F32 ? df_to_double(sxd) : (double)sum[0], sy = F32 ? df_to_double(syd) : (double)sum[1];
+    const R ax = sum[2], bx = sum[3], ay = sum[4], by = sum[5];
     const R tx1 = L0 * ax + L1 * bx, tx2 = L2 * ax + L3 * bx;
     const R ty1 = L0 * ay + L1 * by, ty2 = L2 * ay + L3 * by;
     const double frac = (fi & BSC_FLAG_FREE) ? 0.01 : 1.0;
@@ -1352,11 +1389,13 @@ int op_opt2_shift(Ctx* c) {
     {
         StageTimer tk(c, BSC_T_K_SHIFT);
         if (c->mixed)
-            k_shift<float><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, nullptr, c->gwf, c->gwl,
+            k_shift<float, 1><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, nullptr, c->gwf, c->gwl,
                                                           c->f_vol, c->f_vol_lo, c->cnt, mark);
         else
-            k_shift<double><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->gw, nullptr, nullptr,
-                                                           nullptr, nullptr, c->cnt, mark);
+            with_pair_lanes(c->n, [&](auto L) {
+                k_shift<double, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
+                    c->n, c->S, c->K, c->nbr, c->gw, nullptr, nullptr, nullptr, nullptr, c->cnt, mark);
+            }, PAIR_LANES_LIGHT);
         BSC_LAUNCH(c);
     }
     k_shift_apply<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->S, mark);
