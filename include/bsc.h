@@ -184,7 +184,8 @@ enum {
     BSC_T_EFFPOR, BSC_T_EDDYVIS, BSC_T_INT_VEL, BSC_T_PPE_ASSEMBLE,
     BSC_T_PPE_SOLVE, BSC_T_COMP_VEL, BSC_T_COMP_POS, BSC_T_FREESURF,
     BSC_T_SHIFT, BSC_T_TIMESTEP, BSC_T_PISTON, BSC_T_STEP,
-    BSC_T_SPMV, BSC_T_UPLOAD, BSC_T_DOWNLOAD,
+    BSC_T_SPMV, BSC_T_UPLOAD, BSC_T_DOWNLOAD, /* SPMV: one product per FGMRES cycle, or per batch of the
+                                               * five-kernel BiCGSTAB */
     /* with the BSC_PROFILE_ITER=1 environment variable: the five kernels of
      * one BiCGSTAB iteration per batch; with the multigrid preconditioner,
      * the phases of every FGMRES iteration instead: fine-level pre-smoothing
