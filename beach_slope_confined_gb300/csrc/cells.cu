@@ -5,7 +5,7 @@
 // renumbers them serially (resetid, isph.f90:88-113).  Here the whole list is
 // rebuilt by a counting sort every cell shift: one key per particle, an
 // atomic histogram, an exclusive scan over cells taken in Morton order, a
-// scatter, and a per-cell sort of the slots so the order inside a cell is
+// scatter, and a ranking of each cell's slots so the order inside a cell is
 // deterministic.  Every `reorder_every` shifts the state itself is gathered
 // into that order (the "Morton reorder"), so neighbours sit close in memory.
 #include <algorithm>

@@ -48,6 +48,15 @@ struct Lanes {
         for (int o = L / 2; o > 0; o >>= 1) x += __shfl_xor_sync(mask, x, o);
         return x;
     }
+    // lane u's x, a double-float
+    template <typename X>
+    __device__ __forceinline__ X from(X x, int u) const {
+        if (L > 1) {
+            x.hi = __shfl_sync(mask, x.hi, u, L);
+            x.lo = __shfl_sync(mask, x.lo, u, L);
+        }
+        return x;
+    }
     // acc[q] += a[q] b[q] over the particle's lanes in turn, in each of them: the
     // bits of one thread's fused sums over the same terms (a lane past the end
     // of the list hands in zeros)

@@ -13,7 +13,8 @@
 //    neighbour of a particle lies in the 3x3 cells around it, so the Galerkin
 //    operator P^T A P is a 9-point stencil on the cell grid;
 //  - level l+1: 2x2 blocks of level-l cells, again a 9-point stencil;
-//  - the coarsest level (<= mg_coarse_max cells) is inverted densely.
+//  - the coarsest level (<= mg_coarse_max cells) is inverted densely; with two
+//    sweeps each way the small levels above it become one dense operator.
 // Every coarse operator is summed by one thread per coarse cell in a fixed
 // order, so the hierarchy is deterministic.
 //

@@ -447,38 +447,103 @@ int op_neighbour_lists(Ctx* c) {
     return BSC_OK;
 }
 
-// The rest of the FP64 search on small tanks, over those lists: grad W, the
-// distances, the M sums and what follows from them (the end of k_neighbour),
+// The rest of the search on small tanks, over those lists: grad W, the
+// distances, the M sums and what follows from them (the pair work and the end
+// of k_neighbour, whose lists these are whichever arithmetic decides them),
 // four lanes to a particle.  A round takes four pairs, and lane a then adds
 // their terms of M_a in list order: the bits of the one-thread sums.
+// Search at 3816 particles FP64 53 us with one thread per particle, 25 with
+// the two kernels; at 13599 mixed 50 and 33.
+template <typename R>
 __global__ void __launch_bounds__(NB_BLOCK) k_neighbour_rows(int64_t n, State S, KParams K,
+                                                              const int32_t* __restrict__ pcell,
+                                                              const float2* __restrict__ posf,
+                                                              const float4* __restrict__ posd,
                                                               const int32_t* __restrict__ nbr,
                                                               const int32_t* __restrict__ cnt,
-                                                              double2* __restrict__ gw, double* __restrict__ ndist) {
+                                                              double2* __restrict__ gw, float2* __restrict__ gwf,
+                                                              float2* __restrict__ gwl,
+                                                              const float* __restrict__ f_vol,
+                                                              double* __restrict__ ndist) {
     constexpr int L = 4;
+    constexpr bool F32 = sizeof(R) == 4;
+    using R2 = typename Vec2<R>::type;
     const Lanes<L> ln;
     const int64_t i = ln.particle();
     if (i >= n) return;
-    __shared__ double2 sg[NB_BLOCK], sr[NB_BLOCK];
-    const double* g = reinterpret_cast<const double*>(sg + (threadIdx.x & ~(L - 1))) + (ln.sub & 1);
-    const double* d = reinterpret_cast<const double*>(sr + (threadIdx.x & ~(L - 1))) + (ln.sub >> 1);
+    __shared__ R2 sg[NB_BLOCK], sr[NB_BLOCK];
+    const R* g = reinterpret_cast<const R*>(sg + (threadIdx.x & ~(L - 1))) + (ln.sub & 1);
+    const R* d = reinterpret_cast<const R*>(sr + (threadIdx.x & ~(L - 1))) + (ln.sub >> 1);
     const double xi = S.x[i], yi = S.y[i];
     const int count = cnt[i];
-    double m = 0.0;  // M_sub: gx rx, gy rx, gx ry, gy ry
+    [[maybe_unused]] const float csf = (float)K.cs;
+    [[maybe_unused]] bool use_df = false;
+    [[maybe_unused]] int cx = 0, cy = 0;
+    [[maybe_unused]] df2 oxi{0.f, 0.f}, oyi{0.f, 0.f}, cs_df{0.f, 0.f}, hih{0.f, 0.f}, mwF{0.f, 0.f};
+    if constexpr (F32) {
+        use_df = posd && K.kernel == BSC_KERNEL_WENDLAND_C2 && pre_ok(posf[i], csf);
+        if (use_df) {
+            const int c = pcell[i];
+            cx = c / K.ny;
+            cy = c - cx * K.ny;
+            const float4 oi = posd[i];
+            oxi = {oi.x, oi.y};
+            oyi = {oi.z, oi.w};
+            cs_df = df_of(K.cs);
+            hih = df_of(K.half_inv_h);
+            mwF = df_of(-K.wend_F);
+        }
+    }
+    R m = 0;  // M_sub: gx rx, gy rx, gx ry, gy ry
     for (int k0 = 0; k0 < count; k0 += L) {
         const int k = k0 + ln.sub;
-        double2 gxy = {0.0, 0.0}, rxy = {0.0, 0.0};
+        R2 gxy{0, 0}, rxy{0, 0};  // m_j (x_j - x_i) / rho_j in rxy
         if (k < count) {
             const int64_t e = ell(i, k, K.kmax);
             const int j = nbr[e];
-            const double dx = xi - S.x[j], dy = yi - S.y[j];
-            const double r = __dsqrt_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
-            const double F = grad_factor<double>(K, r);
-            gxy = {F * dx, F * dy};
-            gw[e] = gxy;
-            if (ndist) ndist[e] = r;
-            const double vj = S.vol[j];
-            rxy = {-vj * dx, -vj * dy};  // m_j (x_j - x_i) / rho_j
+            bool done = false;
+            if constexpr (F32) {
+                const float4 oj = use_df ? posd[j] : float4{};
+                if (use_df && pre_ok(make_float2(oj.x, oj.z), csf)) {
+                    const int cj = pcell[j], cxj = cj / K.ny, cyj = cj - cxj * K.ny;
+                    const df2 ddx = df_pair_offset(oxi, make_float2(oj.x, oj.y), cx - cxj, cs_df);
+                    const df2 ddy = df_pair_offset(oyi, make_float2(oj.z, oj.w), cy - cyj, cs_df);
+                    const df2 r2 = df_add(df_sqr(ddx), df_sqr(ddy));
+                    const df2 r = r2.hi > 0.f ? df_sqrt(r2) : df2{0.f, 0.f};
+                    const df2 w = df_sub(df2{1.f, 0.f}, df_mul(r, hih));
+                    const df2 F = df_mul(df_mul(mwF, w), df_sqr(w));  // -F_W (1 - r/2h)^3
+                    const df2 gx = df_mul(F, ddx), gy = df_mul(F, ddy);
+                    if (gw) gw[e] = {df_to_double(gx), df_to_double(gy)};
+                    gwf[e] = {gx.hi, gy.hi};
+                    if (gwl) gwl[e] = {gx.lo, gy.lo};
+                    if (ndist) ndist[e] = df_to_double(r);
+                    const float vj = f_vol[j];
+                    gxy = {gx.hi, gy.hi};
+                    rxy = {-vj * ddx.hi, -vj * ddy.hi};
+                    done = true;
+                }
+            }
+            if (!done) {
+                const double dx = xi - S.x[j], dy = yi - S.y[j];
+                const double d2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
+                const double r = F32 ? (__double_as_longlong(d2) != 0 ? sqrt_nr(d2) : 0.0) : __dsqrt_rn(d2);
+                const double F = grad_factor<double>(K, r);
+                const double gx64 = F * dx, gy64 = F * dy;
+                const R gx = F32 ? (R)f32_of(gx64) : (R)gx64, gy = F32 ? (R)f32_of(gy64) : (R)gy64;
+                if (gw) gw[e] = {gx64, gy64};
+                if (gwl) {
+                    const df2 ax = df_of(gx64), ay = df_of(gy64);
+                    gwf[e] = {ax.hi, ay.hi};
+                    gwl[e] = {ax.lo, ay.lo};
+                } else if (gwf) {
+                    gwf[e] = {(float)gx, (float)gy};
+                }
+                if (ndist) ndist[e] = r;
+                const R vj = F32 ? (R)f_vol[j] : (R)S.vol[j];
+                const R fdx = F32 ? (R)f32_of(dx) : (R)dx, fdy = F32 ? (R)f32_of(dy) : (R)dy;
+                gxy = {gx, gy};
+                rxy = {-vj * fdx, -vj * fdy};
+            }
         }
         ln.sync();
         sg[threadIdx.x] = gxy;
@@ -531,16 +596,23 @@ int op_neighbour(Ctx* c) {
             k_neighbour<double, true><<<g, NB_BLOCK, 0, c->stream>>>(
                 c->n, c->S, c->K, c->cell_start, c->cell_count, c->sorted, c->pcell, c->posf, nullptr, c->nbr, c->gw,
                 nullptr, nullptr, nullptr, c->ndist, c->cnt, c->d_flag, c->cand_nc);
+    } else if (pair_lanes(c->n)) {
+        launch_lists(c, std::max(4, lanes_for(c->n)));
+        BSC_LAUNCH(c);
+        const unsigned gr = blocks_for(c->n * 4, NB_BLOCK);
+        if (c->mixed)
+            k_neighbour_rows<float><<<gr, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->pcell, c->posf, c->posd,
+                                                                     c->nbr, c->cnt, gw64, c->gwf, c->gwl, c->f_vol,
+                                                                     c->ndist);
+        else
+            k_neighbour_rows<double><<<gr, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->pcell, c->posf, nullptr,
+                                                                      c->nbr, c->cnt, c->gw, nullptr, nullptr,
+                                                                      nullptr, c->ndist);
     } else if (c->mixed)
         k_neighbour<float><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->cell_start, c->cell_count, c->sorted,
                                                           c->pcell, c->posf, c->posd, c->nbr, gw64, c->gwf, c->gwl,
                                                           c->f_vol, c->ndist, c->cnt, c->d_flag);
-    else if (pair_lanes(c->n)) {
-        launch_lists(c, std::max(4, lanes_for(c->n)));
-        BSC_LAUNCH(c);
-        k_neighbour_rows<<<blocks_for(c->n * 4, NB_BLOCK), NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->cnt,
-                                                                                  c->gw, c->ndist);
-    } else
+    else
         k_neighbour<double><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->cell_start, c->cell_count,
                                                            c->sorted, c->pcell, c->posf, nullptr, c->nbr, c->gw,
                                                            nullptr, nullptr, nullptr, c->ndist, c->cnt, c->d_flag);

@@ -13,7 +13,9 @@
 // with classical Gram-Schmidt and one re-orthogonalisation pass.  All scalars
 // live on the device; each kernel starts by checking the `done` flag so the
 // host can queue a batch of iterations and test convergence once per batch.
-// Reductions are two-stage with a fixed grid, hence deterministic.
+// Reductions are two-stage on a grid that depends on n alone, hence
+// deterministic.  bicg_coop.cuh runs whole batches of BiCGSTAB iterations in one
+// launch.
 //
 // Mixed precision: the matrix is assembled in FP64 in both paths and the
 // mixed path keeps an FP32 copy of it.  Its solve is FGMRES-IR: a flexible
@@ -187,6 +189,9 @@ __global__ void k_asm_df_pre(int64_t n, State S, KParams K, const int32_t* __res
     pre[4 * n + i] = df_pack(df_of(1.0 + S.oden[i] * K.inv_rho_sea));
 }
 
+// L lanes per row, the sums in list order: 76 us at 13.6k particles with one
+// lane, 27 with four.
+template <int L>
 __global__ void __launch_bounds__(NB_BLOCK) k_assemble_df(int64_t n, State S, KParams K,
                                                            const int32_t* __restrict__ nbr,
                                                            const float2* __restrict__ gwf,
@@ -198,7 +203,8 @@ __global__ void __launch_bounds__(NB_BLOCK) k_assemble_df(int64_t n, State S, KP
                                                            double* __restrict__ b, const double* __restrict__ q,
                                                            const double* __restrict__ usx,
                                                            const double* __restrict__ usy, double dt) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const Lanes<L> ln;
+    const int64_t i = ln.particle();
     if (i >= n) return;
     const float2* __restrict__ pox = pre;
     const float2* __restrict__ poy = pre + n;
@@ -222,80 +228,89 @@ __global__ void __launch_bounds__(NB_BLOCK) k_assemble_df(int64_t n, State S, KP
     const double vxi_n = tid_i == BSC_TID_WALL ? vxsi / ni64 : 0.0, vyi_n = tid_i == BSC_TID_WALL ? vysi / ni64 : 0.0;
     const int m = cnt[i];
     df2 dia{0.0f, 0.0f}, fv{0.0f, 0.0f};
-    for (int k = 0; k < m; ++k) {
-        const int64_t e = ell(i, k, K.kmax);
-        const int j = nbr[e];
-        // grad W as the neighbour search left it, a double-float
-        const float2 gh = gwf[e], gl = gwl[e];
-        const df2 gxr{gh.x, gl.x}, gyr{gh.y, gl.y};
-        const int tid_j = S.tid[j];
-        const int cj = pcell[j], cxj = cj / K.ny, cyj = cj - cxj * K.ny;
-        const df2 dx = df_pair_offset(oxi, pox[j], cxi - cxj, cs);
-        const df2 dy = df_pair_offset(oyi, poy[j], cyi - cyj, cs);
-        const df2 p_dist = df_rcp(df_add(df_add(df_sqr(dx), df_sqr(dy)), lam));
-        const df2 pvol = df_unpack(pvl[j]);
-        df2 val{0.0f, 0.0f};
-        if (tid_i == BSC_TID_FLUID) {
-            const df2 gx = df_add(df_mul(L0, gxr), df_mul(L1, gyr));
-            const df2 gy = df_add(df_mul(L2, gxr), df_mul(L3, gyr));
-            const df2 t = df_mul(df_mul(df_twice(pvol), df_add(df_mul(dx, gx), df_mul(dy, gy))), p_dist);
-            val = df_neg(t);
-            dia = df_add(dia, (free_i && tid_j == BSC_TID_FLUID) ? df_mul(t, df_unpack(plamp[j])) : t);
-            // divergence of the porous-weighted predicted velocity (:241-270)
-            df2 ddx, ddy;
-            if (tid_j == BSC_TID_FLUID) {
-                // 2 q_i q_j / (q_i + q_j), q = rho / n
-                const df2 qj = df_unpack(pq[j]);
-                const df2 rho_ij = df_mul(df_twice(df_mul(qi, qj)), df_rcp(df_add(qi, qj)));
-                ddx = df_mul(rho_ij, df_of(usx[j] - usxi));
-                ddy = df_mul(rho_ij, df_of(usy[j] - usyi));
-            } else {
-                ddx = df_mul(qi, df_mul(df_of(S.vxs[j] - vxsi), inv_ni));
-                ddy = df_mul(qi, df_mul(df_of(S.vys[j] - vysi), inv_ni));
-            }
-            fv = df_add(fv, df_mul(pvol, df_add(df_mul(ddx, gx), df_mul(ddy, gy))));
-        } else if (tid_i == BSC_TID_GHOST) {
-            if (tid_j <= 2) {
-                const df2 t = df_mul(df_mul(df_twice(pvol), df_add(df_mul(dx, gxr), df_mul(dy, gyr))), p_dist);
+    for (int k0 = 0; k0 < m; k0 += L) {
+        const int k = k0 + ln.sub;
+        df2 td{0.0f, 0.0f}, tf{0.0f, 0.0f};  // the sums' terms (a zero leaves a sum as it is)
+        if (L == 1 || k < m) {
+            const int64_t e = ell(i, k, K.kmax);
+            const int j = nbr[e];
+            // grad W as the neighbour search left it, a double-float
+            const float2 gh = gwf[e], gl = gwl[e];
+            const df2 gxr{gh.x, gl.x}, gyr{gh.y, gl.y};
+            const int tid_j = S.tid[j];
+            const int cj = pcell[j], cxj = cj / K.ny, cyj = cj - cxj * K.ny;
+            const df2 dx = df_pair_offset(oxi, pox[j], cxi - cxj, cs);
+            const df2 dy = df_pair_offset(oyi, poy[j], cyi - cyj, cs);
+            const df2 p_dist = df_rcp(df_add(df_add(df_sqr(dx), df_sqr(dy)), lam));
+            const df2 pvol = df_unpack(pvl[j]);
+            df2 val{0.0f, 0.0f};
+            if (tid_i == BSC_TID_FLUID) {
+                const df2 gx = df_add(df_mul(L0, gxr), df_mul(L1, gyr));
+                const df2 gy = df_add(df_mul(L2, gxr), df_mul(L3, gyr));
+                const df2 t = df_mul(df_mul(df_twice(pvol), df_add(df_mul(dx, gx), df_mul(dy, gy))), p_dist);
                 val = df_neg(t);
-                dia = df_add(dia, t);
+                td = (free_i && tid_j == BSC_TID_FLUID) ? df_mul(t, df_unpack(plamp[j])) : t;
+                // divergence of the porous-weighted predicted velocity (:241-270)
+                df2 ddx, ddy;
+                if (tid_j == BSC_TID_FLUID) {
+                    // 2 q_i q_j / (q_i + q_j), q = rho / n
+                    const df2 qj = df_unpack(pq[j]);
+                    const df2 rho_ij = df_mul(df_twice(df_mul(qi, qj)), df_rcp(df_add(qi, qj)));
+                    ddx = df_mul(rho_ij, df_of(usx[j] - usxi));
+                    ddy = df_mul(rho_ij, df_of(usy[j] - usyi));
+                } else {
+                    ddx = df_mul(qi, df_mul(df_of(S.vxs[j] - vxsi), inv_ni));
+                    ddy = df_mul(qi, df_mul(df_of(S.vys[j] - vysi), inv_ni));
+                }
+                tf = df_mul(pvol, df_add(df_mul(ddx, gx), df_mul(ddy, gy)));
+            } else if (tid_i == BSC_TID_GHOST) {
+                if (tid_j <= 2) {
+                    const df2 t = df_mul(df_mul(df_twice(pvol), df_add(df_mul(dx, gxr), df_mul(dy, gyr))), p_dist);
+                    val = df_neg(t);
+                    td = t;
+                }
+            } else if (tid_i == BSC_TID_WALL) {
+                if (tid_j == BSC_TID_FLUID) {
+                    const df2 Lj0 = df_of(S.L0[j]), Lj1 = df_of(S.L1[j]), Lj2 = df_of(S.L2[j]), Lj3 = df_of(S.L3[j]);
+                    const df2 gx = df_add(df_mul(Lj0, gxr), df_mul(Lj1, gyr));
+                    const df2 gy = df_add(df_mul(Lj2, gxr), df_mul(Lj3, gyr));
+                    const df2 t =
+                        df_mul(df_mul(df_twice(mi_over_rhoi), df_add(df_mul(dx, gx), df_mul(dy, gy))), p_dist);
+                    val = df_neg(t);
+                    td = t;
+                    // q_j (v*_j/n_j - v*_i/n_i), the wall row's v*_i/n_i in FP64
+                    const df2 qj = df_unpack(pq[j]);
+                    const df2 ddx = df_mul(qj, df_of(usx[j] - vxi_n));
+                    const df2 ddy = df_mul(qj, df_of(usy[j] - vyi_n));
+                    tf = df_mul(mi_over_rhoi, df_add(df_mul(ddx, gx), df_mul(ddy, gy)));
+                } else {
+                    const df2 t = df_mul(df_mul(df_twice(pvol), df_add(df_mul(dx, gxr), df_mul(dy, gyr))), p_dist);
+                    val = df_neg(t);
+                    td = t;
+                }
             }
-        } else if (tid_i == BSC_TID_WALL) {
-            if (tid_j == BSC_TID_FLUID) {
-                const df2 Lj0 = df_of(S.L0[j]), Lj1 = df_of(S.L1[j]), Lj2 = df_of(S.L2[j]), Lj3 = df_of(S.L3[j]);
-                const df2 gx = df_add(df_mul(Lj0, gxr), df_mul(Lj1, gyr));
-                const df2 gy = df_add(df_mul(Lj2, gxr), df_mul(Lj3, gyr));
-                const df2 t =
-                    df_mul(df_mul(df_twice(mi_over_rhoi), df_add(df_mul(dx, gx), df_mul(dy, gy))), p_dist);
-                val = df_neg(t);
-                dia = df_add(dia, t);
-                // q_j (v*_j/n_j - v*_i/n_i), the wall row's v*_i/n_i in FP64
-                const df2 qj = df_unpack(pq[j]);
-                const df2 ddx = df_mul(qj, df_of(usx[j] - vxi_n));
-                const df2 ddy = df_mul(qj, df_of(usy[j] - vyi_n));
-                fv = df_add(fv, df_mul(mi_over_rhoi, df_add(df_mul(ddx, gx), df_mul(ddy, gy))));
-            } else {
-                const df2 t = df_mul(df_mul(df_twice(pvol), df_add(df_mul(dx, gxr), df_mul(dy, gyr))), p_dist);
-                val = df_neg(t);
-                dia = df_add(dia, t);
-            }
+            vdf[e] = df_pack(val);
         }
-        vdf[e] = df_pack(val);
+#pragma unroll
+        for (int u = 0; u < L; ++u) {
+            dia = df_add(dia, ln.from(td, u));
+            fv = df_add(fv, ln.from(tf, u));
+        }
     }
     const double d = df_to_double(dia);
     if (d == 0.0 || !isfinite(d)) {
         // zero-neighbour guard: identity row, b = 0 (the reference divides by 0)
-        for (int k = 0; k < m; ++k) {
+        for (int k = ln.sub; k < m; k += L) {
             const int64_t e = ell(i, k, K.kmax);
             aval[e] = 0.0;
             ellf[e] = make_int2(nbr[e], 0);
             avalh[e] = __float2half_rn(0.f);
         }
-        b[i] = 0.0;
+        if (ln.sub == 0) b[i] = 0.0;
         return;
     }
     const df2 inv = df_rcp(dia);
-    for (int k = 0; k < m; ++k) {
+    for (int k = ln.sub; k < m; k += L) {
         const int64_t e = ell(i, k, K.kmax);
         const df2 v = df_mul(df_unpack(vdf[e]), inv);
         aval[e] = df_to_double(v);
@@ -304,7 +319,7 @@ __global__ void __launch_bounds__(NB_BLOCK) k_assemble_df(int64_t n, State S, KP
         ellf[e] = make_int2(nbr[e], __float_as_int(v.hi));
         avalh[e] = __float2half_rn(v.hi);
     }
-    b[i] = df_to_double(df_mul(df_mul(fv, df_rcp(df_of(dt))), inv));
+    if (ln.sub == 0) b[i] = df_to_double(df_mul(df_mul(fv, df_rcp(df_of(dt))), inv));
 }
 
 __global__ void k_vs_over_por(int64_t n, State S, double* __restrict__ q, double* __restrict__ ux,
@@ -354,8 +369,11 @@ int op_ppe_assemble(Ctx* c) {
         k_asm_df_pre<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->S, c->K, c->pcell, q, c->asm_df);
         BSC_LAUNCH(c);
         StageTimer tk(c, BSC_T_K_ASSEMBLE);
-        k_assemble_df<<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->gwf, c->gwl, c->cnt, c->pcell,
-                                                      c->asm_df, c->aval, c->ellf, c->avalh, c->b, q, ux, uy, c->dt);
+        with_pair_lanes(c->n, [&](auto L) {
+            k_assemble_df<L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
+                c->n, c->S, c->K, c->nbr, c->gwf, c->gwl, c->cnt, c->pcell, c->asm_df, c->aval, c->ellf, c->avalh,
+                c->b, q, ux, uy, c->dt);
+        });
         BSC_LAUNCH(c);
     } else {
         StageTimer tk(c, BSC_T_K_ASSEMBLE);
