@@ -240,8 +240,8 @@ def spmv_bytes(nnz: int, n: int, fp32: bool) -> int:
 
 def spmv_mg_bytes(nnz: int, n: int, fp32: bool) -> int:
     """Algorithmic bytes of the SpMV w = A z of one multigrid-preconditioned
-    FGMRES iteration: k_spmv_f (FP32 operator and vectors, the mixed path's
-    inner solve) or k_spmv_z<double> (FP64).  Per stored entry the value and
+    FGMRES iteration: k_spmv<float> (FP32 operator and vectors, the mixed path's
+    inner solve) or k_spmv<double> (FP64).  Per stored entry the value and
     the column; per row the count, z_i and w_i.  Neighbour values z_j come
     from cache."""
     if fp32:
@@ -1041,7 +1041,7 @@ def main():
     mg = args.precond == "mg"
     if mg:
         byts = spmv_mg_bytes(m["nnz"], m["n"], fp32=True)
-        kname = "k_spmv_f (FP32 ELL SpMV of the inner FGMRES)"
+        kname = "k_spmv<float> (FP32 ELL SpMV of the inner FGMRES)"
         tpr = traffic_per_row("spmv_f_fp32")
     else:
         byts = spmv_bytes(m["nnz"], m["n"], fp32=True)
@@ -1085,7 +1085,7 @@ def main():
         fp64 = {"value": f["value"], "ms_per_step": f["ms_per_step"], "ppe_iterations": [i[0] for i in f["iters"]],
                 "solve_ms_per_step": f["solve_ms"], "kernels": f["kernels"],
                 "roofline_spmv": {"bound": "hbm",
-                                  "kernel": "k_spmv_z<double>" if mg else "k_bicg_1<EllOp<double>,double>",
+                                  "kernel": "k_spmv<double>" if mg else "k_bicg_1<EllOp<double>,double>",
                                   "achieved": a64,
                                   "peak": hbm, "unit": "GB/s", "frac": (a64 / hbm) if a64 else None,
                                   "traffic": (t64 * f["n"]) if t64 else None}}
