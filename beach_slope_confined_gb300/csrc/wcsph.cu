@@ -860,8 +860,9 @@ Keep seg_keep(WcState* w, int q, int64_t n, int64_t slots) {
 // kept buffers (the context's own are pointed there for the step), and the
 // per-particle quotients, per-pair kernel values and porosity derivatives
 // are kept too.  The step reads the lists only; `last` (the last step that a
-// call runs) takes the full search, which leaves the context's grad W, L and
-// flags as those of the state it ends on.
+// call runs) takes the full search, and its lists and cells are copied to the
+// context's own buffers: the lists, grad W, L and flags that a call leaves are
+// those of its last step's search.
 int wc_step(Ctx* c, WcState* w, double* nbuf, double* Pbuf, const Keep* keep, bool last) {
     const int64_t n = c->n;
     c->t += w->K.dt;
@@ -909,7 +910,17 @@ int wc_step(Ctx* c, WcState* w, double* nbuf, double* Pbuf, const Keep* keep, bo
     c->nbr = own_nbr;
     c->cnt = own_cnt;
     c->pcell = own_cell;
-    if (rc) return rc;
+    c->have_csr = false;  // the lists that an earlier PPE matrix was laid out on are gone
+    if (rc) {
+        c->have_lists = false;
+        return rc;
+    }
+    if (keep && last) {  // into the context's own buffers: have_lists speaks for those
+        BSC_CUDA(c, cudaMemcpyAsync(own_nbr, keep->nbr, sizeof(int32_t) * list_slots(c), cudaMemcpyDeviceToDevice,
+                                    c->stream));
+        BSC_CUDA(c, cudaMemcpyAsync(own_cnt, keep->cnt, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, c->stream));
+        BSC_CUDA(c, cudaMemcpyAsync(own_cell, keep->cell, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, c->stream));
+    }
     // the next state becomes the state
     return wc_copy(c, st_of(w->nxt, n), st_ctx(c));
 }
