@@ -22,7 +22,9 @@
 // 125k rows of 21 entries: 48.8 us with a partial per warp and two rows per
 // thread, 33.5 us here.
 // The grid is launched cooperatively (all blocks resident), and every wait is
-// bounded.
+// bounded: where one runs out the launch ends without its results, and the host
+// goes on with the five kernels from x as it is (rows of blocks that had got to
+// the end may be new, the others old: any x will do to restart from).
 #pragma once
 
 #include "bsc_internal.cuh"
@@ -38,11 +40,10 @@ namespace bsc {
 // steps of 3.8k to 51k rows 5 to 7 % longer (one fence after relaxed polls:
 // the same).  A word per block, each watched by every block, took 14000: the
 // watching slows the words' stores.
-constexpr unsigned GRID_SPIN_LIMIT = 1u << 21;  // polls of ~0.5 us
-
 struct GridBarrier {
     unsigned* count;
     double* err;
+    unsigned limit;  // polls (~0.5 us each) before a wait gives up
     unsigned target = 0;
     // every thread of every block; false (in all threads of the block) if some
     // block never arrived: the caller returns
@@ -56,7 +57,7 @@ struct GridBarrier {
                 unsigned v;
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
                 if (v >= target) break;
-                if (spins >= GRID_SPIN_LIMIT) {
+                if (spins >= limit) {
                     *err = 1.0;
                     fine = 0;
                     break;
@@ -140,7 +141,7 @@ __device__ __forceinline__ double eight_sum(const double (&q)[8], int nwarps) {
 template <typename Op, bool MERGE, int K, int THREADS, int G>
 __global__ void __launch_bounds__(THREADS, 1)
     k_bicg_coop(int64_t n, Op A, double* x, double* r, const double* rh, double* p, double* v, double* s, double* p2,
-                double* v2, double* part, Scalars* sc, unsigned* count, int iters, int cap) {
+                double* v2, double* part, Scalars* sc, unsigned* count, unsigned polls, int iters, int cap) {
     static_assert(G == 1 || K == 1, "G > 1: one row per thread");
     extern __shared__ __align__(16) unsigned char coop_sm[];
     double* sval = reinterpret_cast<double*>(coop_sm);
@@ -300,7 +301,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     int it = sc->it, state = 0;
     bool first = true;
     __syncthreads();  // the units' matrix entries
-    GridBarrier grid{count, &sc->tmp[7]};
+    GridBarrier grid{count, &sc->tmp[7], polls};
     double *pold = p, *pnew = p2, *vold = v, *vnew = MERGE ? v2 : v;
     double* part1 = part + stride;      // each reduction its own partials: a block may still
     double* part2 = part + 3 * stride;  // read one while another writes the next

@@ -546,6 +546,7 @@ __global__ void k_bicg_restart(const double* __restrict__ part, int nb, Scalars*
         sc->rr = v[0];
         sc->rho = v[0];
         sc->k5 = 0;
+        sc->tmp[7] = 0.0;
         sc->done = (sqrt(v[0]) <= sc->target) ? 1 : 0;
         sc->breakdown = (v[0] == 0.0 && !sc->done) ? 1 : 0;
     }
@@ -1060,7 +1061,8 @@ cudaError_t bicg_coop_launch(Ctx* c, int64_t n, Op A, Work<double> w, int iters,
     int cap = P.cap;
     const double* rh = w.rh;
     // MERGE: p and v double-buffered, their second halves in s and t
-    void* args[] = {&n, &A, &w.x, &w.r, &rh, &w.p, &w.v, &w.s, &w.s, &w.t, &c->part, &c->sc, &count, &iters, &cap};
+    void* args[] = {&n,   &A,   &w.x,     &w.r,   &rh,    &w.p, &w.v, &w.s, &w.s,
+                    &w.t, &c->part, &c->sc, &count, &c->barrier_polls, &iters, &cap};
     c->launches++;
     return cudaLaunchCooperativeKernel(P.kernel, dim3(P.blocks), dim3(P.threads), args, (size_t)P.smem, c->stream);
 }
@@ -1112,9 +1114,12 @@ int run_bicgstab(Ctx* c, int64_t n, const Op& A, Work<T> w, double tol, int rel_
         int rc = fetch_scalars(c);
         if (rc) return rc;
         const Scalars& h = *c->h_sc;
-        if (h.breakdown && !h.done && h.it < maxit && restarts < kMaxRestarts) {
-            // rho or omega vanished: restart from x with a fresh shadow residual
-            ++restarts;
+        const bool gave_up = h.tmp[7] != 0.0;  // a wait of the cooperative launch ran out
+        if (gave_up || (h.breakdown && !h.done && h.it < maxit && restarts < kMaxRestarts)) {
+            // rho or omega vanished: restart from x with a fresh shadow residual;
+            // likewise, with the kernels below, after a launch that gave up
+            if (gave_up) coop.blocks = 0;
+            else ++restarts;
             k_bicg_init<Op, T><<<G, B, 0, c->stream>>>(n, A, w.x, w.b, w.r, w.rh, w.p, c->part);
             BSC_LAUNCH(c);
             k_bicg_restart<<<1, B, 0, c->stream>>>(c->part, G, c->sc);
@@ -1123,7 +1128,6 @@ int run_bicgstab(Ctx* c, int64_t n, const Op& A, Work<T> w, double tol, int rel_
             continue;
         }
         if (coop.blocks > 0) {  // the scalars carry on from launch to launch
-            if (h.tmp[7] != 0.0) return set_err(c, BSC_E_CUDA, "BiCGSTAB: a grid barrier's wait ran out");
             if (h.done || h.breakdown || h.it >= maxit) break;
             cudaError_t e = cudaSuccess;
             if constexpr (sizeof(T) == 8)
