@@ -1174,9 +1174,9 @@ int run_bicgstab(Ctx* c, int64_t n, const Op& A, Work<T> w, double tol, int rel_
             for (int q = 0; q < nb; ++q) one();
         }
         c->launches += 5 * nb;
+        BSC_CUDA(c, cudaGetLastError());  // before the poll, whose queries clear it
         if (launched == 0 && c->timing) timing_poll(c);  // while the first batch runs
         launched += nb;
-        BSC_CUDA(c, cudaGetLastError());
     }
     *iters = c->h_sc->it;
     if (xbest) {
