@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         m[q] = act ? A.len(i) : 0;
         const int mw = __reduce_max_sync(0xffffffffu, m[q]);
         int o = 0;
-        if (lane == 0) o = atomicAdd(&used, mw);
+        if (lane == 0) o = mw <= cap ? atomicAdd(&used, mw) : cap;  // (the sum stays far from overflow)
         o = __shfl_sync(0xffffffffu, o, 0);
         off[q] = o + mw <= cap ? o : -1;
         if (MERGE) {

@@ -409,7 +409,7 @@ struct CsrOp {
     const double* val;
     const void* key() const { return val; }
     static constexpr bool UNIT_DIAG = false;
-    __device__ __forceinline__ int len(int64_t i) const { return rp[i + 1] - rp[i]; }
+    __device__ __forceinline__ int len(int64_t i) const { return max(rp[i + 1] - rp[i], 0); }  // as row()'s loop takes it
     __device__ __forceinline__ int64_t at(int64_t i, int k) const { return rp[i] + k; }
     __device__ __forceinline__ int32_t col_at(int64_t e) const { return col[e]; }
     __device__ __forceinline__ double val_at(int64_t e) const { return val[e]; }
