@@ -351,7 +351,7 @@ struct Ctx {
     int32_t* nbr = nullptr;
     double2* gw = nullptr;        // FP64 grad W (the FP64 path; the mixed path's FP64 assembly variants)
     double* ndist = nullptr;      // pair distance per slot (salinity: scalart's radial)
-    double* sdisp = nullptr;      // salinity: D_x, D_y, Dm + nu_t/Sc, 1/n per particle (4n)
+    double* sdisp = nullptr;      // salinity: D_x, D_y, Dm + nu_t/Sc, 1/n, c or NaN per particle (5n)
     // mixed path: grad W as a double-float, {gwf, gwl} (gwf alone is its FP32
     // rounding, which the FP32 pair sums read)
     float2* gwf = nullptr;

@@ -44,17 +44,25 @@ __device__ __forceinline__ double disp(double Dm, double a1, double a2, double a
 
 // per particle: D_x, D_y and the eddy term Dm + nu_t / Sc, the same values
 // scalart forms for a particle as i and as j (one division and root each,
-// instead of per pair)
+// instead of per pair); and in cs the concentration, or a NaN where a
+// coefficient is zero or not finite: between such particles the flux of a pair
+// of one concentration is not the zero that it is elsewhere, but the
+// reference's 0/0 or NaN
 __global__ void k_scalar_pre(int64_t n, State S, ScalarK C, double* __restrict__ Dx, double* __restrict__ Dy,
-                             double* __restrict__ E, double* __restrict__ inv_n) {
+                             double* __restrict__ E, double* __restrict__ inv_n, double* __restrict__ cs) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double vx = S.vx[i], vy = S.vy[i], v = sqrt(vx * vx + vy * vy), ni = S.por[i];
     const double amx = C.al - C.at;
-    Dx[i] = disp(C.Dm, C.al, C.at, amx, vx, vy, v, ni, C.cap);
-    Dy[i] = disp(C.Dm, C.at, C.al, amx, vx, vy, v, ni, C.cap);
-    E[i] = C.Dm + S.nut[i] / C.tsc;
-    inv_n[i] = 1.0 / ni;
+    const double dx = disp(C.Dm, C.al, C.at, amx, vx, vy, v, ni, C.cap);
+    const double dy = disp(C.Dm, C.at, C.al, amx, vx, vy, v, ni, C.cap), e = C.Dm + S.nut[i] / C.tsc, in = 1.0 / ni;
+    Dx[i] = dx;
+    Dy[i] = dy;
+    E[i] = e;
+    inv_n[i] = in;
+    const bool plain = isfinite(dx) && isfinite(dy) && isfinite(e) && isfinite(in) && isfinite(S.ovol[i]) &&
+                       dx != 0.0 && dy != 0.0 && e != 0.0;
+    cs[i] = plain ? S.con[i] : __longlong_as_double(0x7ff8000000000000LL);
 }
 
 // Bound: the FP64 pipe, an FP64 division being about nine of its
@@ -67,11 +75,12 @@ __global__ void k_scalar_pre(int64_t n, State S, ScalarK C, double* __restrict__
 __global__ void __launch_bounds__(128) k_scalart(int64_t n, State S, KParams K, const int32_t* __restrict__ nbr,
                                                  const double* __restrict__ ndist, const int32_t* __restrict__ cnt,
                                                  const double* __restrict__ Dx, const double* __restrict__ Dy,
-                                                 const double* __restrict__ E, const double* __restrict__ inv_n) {
+                                                 const double* __restrict__ E, const double* __restrict__ inv_n,
+                                                 const double* __restrict__ cs) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     if (S.tid[i] != BSC_TID_FLUID || (S.flags[i] & BSC_FLAG_DEAD)) return;
-    const double con1 = S.con[i], ni = S.por[i], nuti = S.nut[i], oi = S.ovol[i];
+    const double con1 = S.con[i], cs1 = cs[i], ni = S.por[i], nuti = S.nut[i], oi = S.ovol[i];
     const double Dxi = Dx[i], Dyi = Dy[i], Ei = E[i], ini = inv_n[i];
     const double xi = S.x[i], yi = S.y[i];
     double cd = 0.0;
@@ -80,9 +89,9 @@ __global__ void __launch_bounds__(128) k_scalart(int64_t n, State S, KParams K, 
         const int64_t e = ell(i, k, K.kmax);
         const int j = nbr[e];
         if (S.tid[j] != BSC_TID_FLUID || (S.flags[j] & BSC_FLAG_DEAD)) continue;
-        const double con2 = S.con[j];
-        const double dcon = con1 - con2;
+        double dcon = cs1 - cs[j];
         if (dcon == 0.0) continue;
+        if (isnan(dcon)) dcon = con1 - S.con[j];
         const double r = ndist[e];
         const double dx = xi - S.x[j], dy = yi - S.y[j], dx2 = dx * dx, dy2 = dy * dy;
         double den = r * r + K.lam, num;  // num / den: t1x dx^2 + t1y dy^2 over r^2 + lam
@@ -136,11 +145,12 @@ int op_scalart(Ctx* c) {
     if (!c->have_lists) return set_err(c, BSC_E_INVALID, "scalart before neighbour");
     const bsc_params& P = c->P;
     const ScalarK C{P.diffusivity, P.disp_long, P.disp_trans, P.tschmidt, 0.12 * (P.dl * P.dl) / c->dt};
-    double *Dx = c->sdisp, *Dy = c->sdisp + c->n, *E = c->sdisp + 2 * c->n, *inv_n = c->sdisp + 3 * c->n;
-    k_scalar_pre<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->S, C, Dx, Dy, E, inv_n);
+    double *Dx = c->sdisp, *Dy = c->sdisp + c->n, *E = c->sdisp + 2 * c->n, *inv_n = c->sdisp + 3 * c->n,
+           *cs = c->sdisp + 4 * c->n;
+    k_scalar_pre<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->S, C, Dx, Dy, E, inv_n, cs);
     BSC_LAUNCH(c);
     k_scalart<<<blocks_for(c->n, 128), 128, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->ndist, c->cnt, Dx, Dy, E,
-                                                             inv_n);
+                                                             inv_n, cs);
     BSC_LAUNCH(c);
     return BSC_OK;
 }
