@@ -124,6 +124,8 @@ static void derive_kparams(Ctx* c) {
     K.alpha = P.darcy_alpha;
     K.beta = P.forch_beta;
     K.d50 = P.d50;
+    K.plain_drag = std::fabs(K.alpha) < 1e15 && std::fabs(K.beta) < 1e15 && std::fabs(K.d50) > 1e-15 &&
+                   std::fabs(K.d50) < 1e15;
     K.eddy_cs = P.eddy_cs;
     K.eddy_cv = P.eddy_cv;
     K.eddy_ce = P.eddy_ce;

@@ -126,6 +126,16 @@ __device__ __forceinline__ double sqrt_nr(double x) {
 // ten instructions on the pipe that bounds the kernels that take it.
 __device__ __forceinline__ double over_por(double a, double n) { return n == 1.0 ? a : a / n; }
 
+// |a| < 1e15, or 1e-15 <= |a| < 1e15, on the integer pipe (false for a NaN):
+// products of a few such values are finite in FP32 too, so a factor of zero
+// makes them zero
+__device__ __forceinline__ bool moderate(double a) {
+    return (__double2hiint(a) & 0x7fffffff) < 0x430c6bf5;
+}
+__device__ __forceinline__ bool moderate_nonzero(double a) {
+    return moderate(a) && (__double2hiint(a) & 0x7fffffff) >= 0x3cd203b0;
+}
+
 // a < b for non-negative doubles a and b (b finite), on the integer pipe:
 // the bit patterns of non-negative IEEE doubles order like their values, and
 // any a with the sign bit set (only a NaN can have it here) compares as not
@@ -160,6 +170,7 @@ struct KParams {
     int pnx, pny;
     double px0, py0, pdx, pdy;
     const double* pgrid;
+    bool plain_drag;  // the drag's parameters are moderate: its terms are zeros at n = 1
     bool por_le1;  // no porosity of the field (or outside it) above 1: the solid fraction's cap is never below 0
 };
 

@@ -806,8 +806,8 @@ __global__ void __launch_bounds__(NB_BLOCK) k_effpor(int64_t n, State S, KParams
     }
     // Ergun/Darcy-Forchheimer coefficient (porous.f90:192,204-212),
     // Fch*sqrt(lamk) written as beta/sqrt(n^3)
-    if (nn == 1.0 && isfinite(S.vx[i]) && isfinite(S.vy[i])) {
-        S.resist[i] = -0.0;  // both terms carry the factor 1 - n
+    if (nn == 1.0 && K.plain_drag && moderate(S.vx[i]) && moderate(S.vy[i]) && moderate_nonzero(oden)) {
+        S.resist[i] = -0.0;  // both terms carry the factor 1 - n, and the others are finite
         return;
     }
     if constexpr (sizeof(R) == 4) {

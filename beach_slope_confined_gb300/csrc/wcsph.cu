@@ -52,6 +52,7 @@ struct WcK {
     double alpha, beta;
     double inv_h, wend_F, wend_W;
     double gx0, gy0, gdx, gdy, por_default;
+    bool plain_drag;                           // the drag's parameters are moderate: it vanishes at n = 1
     int gnx, gny, kmax, np, gc;  // gc: grid cells one support can overlap
     double R1, depth;                          // probe kernel radius, probe depth
 };
@@ -467,7 +468,7 @@ __global__ void __launch_bounds__(WPB) k_wc_step(int64_t n, State S, WcK K, cons
     const double ax = -ni * Px + vx, ay = -ni * Py + vy + ni * K.g;
     // outside the porous layer (whole warps of it) the drag's quotients and
     // roots, a tenth of this kernel's FP64 work, leave the values as they are
-    const bool clear = ni == 1.0 && isfinite(vxi) && isfinite(vyi);
+    const bool clear = ni == 1.0 && K.plain_drag && moderate(vxi) && moderate(vyi);
     double vxn = vxi + K.dt * ax, vyn = vyi + K.dt * ay, sxn, syn;
     if (clear) {  // n = 1: no drag, and quotients by 1
         sxn = K.dt * vxn;
@@ -798,6 +799,8 @@ namespace {
 int wc_params(Ctx* c, WcState* w, double alpha, double beta, const double* grid) {
     w->K.alpha = alpha;
     w->K.beta = beta;
+    w->K.plain_drag = std::fabs(alpha) < 1e15 && std::fabs(beta) < 1e15 && std::fabs(w->K.nu) < 1e15 &&
+                      std::fabs(w->K.d50) > 1e-15 && std::fabs(w->K.d50) < 1e15;
     if (grid) BSC_CUDA(c, cudaMemcpyAsync(w->theta, grid, sizeof(double) * w->G, cudaMemcpyHostToDevice, c->stream));
     if (w->ns > 0) {
         k_wc_solids<<<blocks_for(w->ns, 256), 256, 0, c->stream>>>(w->ns, c->sx, c->sy, c->svol, w->theta, w->K, w->sw,
