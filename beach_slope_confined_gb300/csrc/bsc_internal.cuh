@@ -537,6 +537,7 @@ int mg_vcycle_f64(Ctx* c, const double* src, double* v, double* z);
 int mg_vcycle_f32(Ctx* c, const float* src, float* v, float* z);
 void mg_free(Ctx* c);
 int fg_layout_size(int m);
+bool csr_bicgstab_load(int dev);
 int csr_solve_device(Ctx* c, int32_t n, const int32_t* rp, const int32_t* col, const double* val,
                      const double* b, double* x, bsc_solve_info* info);
 

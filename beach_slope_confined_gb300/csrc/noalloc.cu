@@ -17,7 +17,8 @@
 // loaded), so an address never outlives the context it came from: after a
 // cudaDeviceReset the module loads again, possibly elsewhere.  Under CUDA's
 // lazy module loading the first call on a device loads this module, which is
-// when the array's memory is committed.  Every call shares the array and
+// when the array's memory is committed, and brings in every kernel that a later
+// call of any size may run.  Every call shares the array and
 // leaves its contents behind, so the ticket and the scalars are cleared at
 // the start of each call; two calls whose work overlaps on the GPU (two
 // streams, or two host threads) race on the array, and on the one host-side
@@ -97,6 +98,7 @@ int bsc_csr_solve_noalloc(const bsc_params* p, int32_t n, const int32_t* rowptr,
     unsigned char* base = nullptr;
     int rc = scratch_address(&base);
     if (rc) return rc;
+    if (!csr_bicgstab_load(dev)) return BSC_E_CUDA;
 
     Ctx c;  // a view on the scratch: owns nothing, frees nothing
     c.P = *p;

@@ -23,6 +23,7 @@
 // preconditioner is a short FP32 BiCGSTAB sweep with FP64 dot products; a
 // breakdown of BiCGSTAB restarts it from the current iterate.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <vector>
@@ -1888,6 +1889,38 @@ int op_ppe_solve(Ctx* c, bsc_solve_info* info) {
 }
 
 // ---- standalone CSR solve (device buffers allocated by the caller context) ----
+// Bring in every kernel that a BiCGSTAB solve of a CSR matrix may run, whatever
+// its size and its course, onto the current device: under lazy module loading a
+// kernel's code takes device memory at its first use, and a host that has given
+// the memory to its own pool has none left by a later call.  Once per device
+// (14 look-ups take ~12 us; after a cudaDeviceReset a kernel is back to loading
+// at its first use).
+bool csr_bicgstab_load(int dev) {
+    static std::atomic<uint64_t> loaded{0};
+    const uint64_t bit = dev < 64 ? uint64_t(1) << dev : 0;
+    if (loaded.load(std::memory_order_relaxed) & bit) return true;
+    const void* kernels[] = {(const void*)k_bicg_init<CsrOp, double>,
+                             (const void*)k_bicg_setup,
+                             (const void*)k_bicg_restart,
+                             (const void*)k_bicg_1<CsrOp, double>,
+                             (const void*)k_bicg_2<double>,
+                             (const void*)k_bicg_3<CsrOp, double>,
+                             (const void*)k_bicg_4<double>,
+                             (const void*)k_bicg_5<double>,
+                             (const void*)k_bicg_coop<CsrOp, true, 1, COOP_BLOCK, 1>,
+                             (const void*)k_bicg_coop<CsrOp, false, 1, COOP_BLOCK, 4>,
+                             (const void*)k_bicg_coop<CsrOp, false, 1, 2 * COOP_BLOCK, 4>,
+                             (const void*)k_bicg_coop<CsrOp, false, 3, COOP_BLOCK, 1>,
+                             (const void*)k_resid<CsrOp, double>,
+                             (const void*)k_ir_norms};
+    for (const void* f : kernels) {
+        cudaFuncAttributes a;
+        if (cudaFuncGetAttributes(&a, f) != cudaSuccess) return (void)cudaGetLastError(), false;
+    }
+    loaded.fetch_or(bit, std::memory_order_relaxed);
+    return true;
+}
+
 int csr_solve_device(Ctx* c, int32_t n, const int32_t* rp, const int32_t* col, const double* val, const double* b,
                      double* x, bsc_solve_info* info) {
     CsrOp A{rp, col, val};

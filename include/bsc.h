@@ -330,7 +330,8 @@ int bsc_csr_solve(const bsc_params* p, int32_t n, const int32_t* rowptr,
  *    device's memory, a solver other than BSC_SOLVER_BICGSTAB, or n <= 0
  *    return BSC_E_INVALID.
  *  - Under CUDA's default lazy module loading the array's memory is
- *    committed by the first call on each device: make that call before the
+ *    committed by the first call on each device, and the code of every kernel
+ *    that a later call of any size runs: make that call before the
  *    host reserves its pool (or set CUDA_MODULE_LOADING=EAGER, which commits
  *    it when the library's device code loads), and before any stream capture
  *    begins.  Each call looks up the array's address on the current device.
