@@ -886,7 +886,9 @@ int bsc_step(bsc_ctx* c, int32_t nsteps, bsc_solve_info* last) {
         if (c->P.salinity) RUN(BSC_T_EDDYVIS, op_eddyvis(c));
 #undef RUN
     }
-    return check_flags(c);
+    const int rc = check_flags(c);
+    if (c->timing) timing_poll(c);  // the stream is idle: nothing is left over for a later call
+    return rc;
 }
 
 int bsc_get_neighbors(bsc_ctx* c, int64_t* offsets, int32_t* ids) {
