@@ -33,17 +33,19 @@
 namespace bsc {
 
 // ---- grid barrier -------------------------------------------------------------------
-// count: arrivals (zero at launch); err: set to 1 once a wait has run out.
+// count: arrivals (zero at launch, or out of reach: bicg_coop_launch); err: set to 1 once a wait has run out.
 // The arrival releases what the block has written (its threads' writes come
 // before it by the block barrier), the polls acquire: with relaxed accesses
 // between __threadfence() calls a barrier took ~3000 clocks on 152 blocks, and
 // steps of 3.8k to 51k rows 5 to 7 % longer (one fence after relaxed polls:
 // the same).  A word per block, each watched by every block, took 14000: the
 // watching slows the words' stores.
+// a constant: as a kernel parameter it cost an iteration 1 % at 4096 rows
+constexpr unsigned GRID_SPIN_LIMIT = 1u << 21;  // polls: a few tenths of a second
+
 struct GridBarrier {
     unsigned* count;
     double* err;
-    unsigned limit;  // polls (~0.5 us each) before a wait gives up
     unsigned target = 0;
     // every thread of every block; false (in all threads of the block) if some
     // block never arrived: the caller returns
@@ -56,8 +58,8 @@ struct GridBarrier {
             for (unsigned spins = 0;; ++spins) {
                 unsigned v;
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
-                if (v >= target) break;
-                if (spins >= limit) {
+                if ((int)(v - target) >= 0) break;
+                if (spins >= GRID_SPIN_LIMIT) {
                     *err = 1.0;
                     fine = 0;
                     break;
@@ -141,7 +143,7 @@ __device__ __forceinline__ double eight_sum(const double (&q)[8], int nwarps) {
 template <typename Op, bool MERGE, int K, int THREADS, int G>
 __global__ void __launch_bounds__(THREADS, 1)
     k_bicg_coop(int64_t n, Op A, double* x, double* r, const double* rh, double* p, double* v, double* s, double* p2,
-                double* v2, double* part, Scalars* sc, unsigned* count, unsigned polls, int iters, int cap) {
+                double* v2, double* part, Scalars* sc, unsigned* count, int iters, int cap) {
     static_assert(G == 1 || K == 1, "G > 1: one row per thread");
     extern __shared__ __align__(16) unsigned char coop_sm[];
     double* sval = reinterpret_cast<double*>(coop_sm);
@@ -301,7 +303,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     int it = sc->it, state = 0;
     bool first = true;
     __syncthreads();  // the units' matrix entries
-    GridBarrier grid{count, &sc->tmp[7], polls};
+    GridBarrier grid{count, &sc->tmp[7]};
     double *pold = p, *pnew = p2, *vold = v, *vnew = MERGE ? v2 : v;
     double* part1 = part + stride;      // each reduction its own partials: a block may still
     double* part2 = part + 3 * stride;  // read one while another writes the next

@@ -42,7 +42,6 @@ struct State {
 };
 constexpr int N_DBL_FIELDS = 28;
 constexpr int TICKET_WORDS = 128;  // Ctx::ticket
-constexpr unsigned GRID_SPIN_LIMIT = 1u << 21;  // polls of a grid barrier: about a second
 
 // ---- neighbour list (ELL, 32-slot slices) ----------------------------------
 __host__ __device__ inline int64_t ell(int64_t i, int k, int kmax) {
@@ -392,7 +391,7 @@ struct Ctx {
     Scalars* sc2 = nullptr;       // FGMRES-IR outer scalars (h_sc[1] mirrors them)
     unsigned* ticket = nullptr;   // TICKET_WORDS: [0] last-block counter of the Krylov reductions (kept at 0
                                   // between launches), [64] the cooperative BiCGSTAB's barrier
-    unsigned barrier_polls = GRID_SPIN_LIMIT;  // BSC_BARRIER_POLLS
+    bool barrier_stuck = false;   // BSC_BARRIER_STUCK: the cooperative launches' waits run out
     int ir_m = 0;
     // instantiated CUDA graphs of one batch of Krylov iterations, keyed by
     // the operator and vectors they were captured with

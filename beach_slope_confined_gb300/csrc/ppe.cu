@@ -1058,12 +1058,12 @@ CoopPlan coop_plan(int64_t n) {
 template <typename Op>
 cudaError_t bicg_coop_launch(Ctx* c, int64_t n, Op A, Work<double> w, int iters, const CoopPlan& P) {
     unsigned* count = c->ticket + COOP_BAR;
-    if (cudaError_t e = cudaMemsetAsync(count, 0, sizeof(unsigned), c->stream)) return e;
+    // (stuck: 2^30 below zero, which no arrivals make up for)
+    if (cudaError_t e = cudaMemsetAsync(count, c->barrier_stuck ? 0xC0 : 0, sizeof(unsigned), c->stream)) return e;
     int cap = P.cap;
     const double* rh = w.rh;
     // MERGE: p and v double-buffered, their second halves in s and t
-    void* args[] = {&n,   &A,   &w.x,     &w.r,   &rh,    &w.p, &w.v, &w.s, &w.s,
-                    &w.t, &c->part, &c->sc, &count, &c->barrier_polls, &iters, &cap};
+    void* args[] = {&n, &A, &w.x, &w.r, &rh, &w.p, &w.v, &w.s, &w.s, &w.t, &c->part, &c->sc, &count, &iters, &cap};
     c->launches++;
     return cudaLaunchCooperativeKernel(P.kernel, dim3(P.blocks), dim3(P.threads), args, (size_t)P.smem, c->stream);
 }
