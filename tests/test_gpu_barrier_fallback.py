@@ -4,8 +4,8 @@ BSC_BARRIER_STUCK=1 starts the barrier's count out of the arrivals' reach: every
 block's first wait runs out (a few tenths of a second) and the launch ends with x as it
 was.  The five kernels that go on from there (their products are timed, those
 of the cooperative form are not) have to give their own run's iterations and
-bits.  The tanks take the merged form, and the forms with one
-and two rows per thread.
+bits, and so does the launch that holds.  The tanks take the merged form, and the
+forms for up to 77824, 155648 and 233472 rows.
 """
 import numpy as np
 import pytest
@@ -31,12 +31,13 @@ def pressure(dx):
     return info.iterations, p, timed
 
 
-@pytest.mark.parametrize("dx", [0.02, 0.0075, 0.0038])
+@pytest.mark.parametrize("dx", [0.02, 0.0075, 0.0038, 0.0025])
 def test_the_kernels_go_on_from_x(dx, monkeypatch):
     monkeypatch.setenv("BSC_PROFILE_ITER", "1")  # the five kernels alone
     it, want, _ = pressure(dx)
     monkeypatch.setenv("BSC_PROFILE_ITER", "0")
-    assert pressure(dx)[2] == 0
+    k, p, timed = pressure(dx)
+    assert timed == 0 and k == it and np.array_equal(p, want)
     monkeypatch.setenv("BSC_BARRIER_STUCK", "1")
     k, p, timed = pressure(dx)
     assert timed > 0 and k == it and np.array_equal(p, want)
