@@ -493,6 +493,7 @@ int bsc_create(const bsc_params* p, bsc_ctx** out) {
     for (int k = 0; k < Ctx::EVPOOL; ++k) cudaEventCreate(&c->evs[k]);
     for (int k = 0; k < 4; ++k) cudaEventCreate(&c->ev_spmv[k]);
     if (const char* e = std::getenv("BSC_GRAPHS")) c->use_graphs = e[0] != '0';
+    if (const char* e = std::getenv("BSC_PAIR_LANES")) c->pair_lanes = std::atoi(e);
     if (const char* e = std::getenv("BSC_BARRIER_STUCK")) c->barrier_stuck = e[0] == '1';
     if (const char* e = std::getenv("BSC_DEBUG")) c->debug = e[0] == '1';
     if (const char* e = std::getenv("BSC_SPMV_UNROLL")) c->spmv_unroll = e[0] == '1';

@@ -391,6 +391,7 @@ struct Ctx {
     Scalars* sc2 = nullptr;       // FGMRES-IR outer scalars (h_sc[1] mirrors them)
     unsigned* ticket = nullptr;   // TICKET_WORDS: [0] last-block counter of the Krylov reductions (kept at 0
                                   // between launches), [64] the cooperative BiCGSTAB's barrier
+    int pair_lanes = 0;           // BSC_PAIR_LANES: lanes per particle of the pair kernels (0: lanes.cuh's rule)
     bool barrier_stuck = false;   // BSC_BARRIER_STUCK: the cooperative launches' waits run out
     int ir_m = 0;
     // instantiated CUDA graphs of one batch of Krylov iterations, keyed by

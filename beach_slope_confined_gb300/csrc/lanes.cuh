@@ -101,10 +101,13 @@ void with_lanes(int lanes, F f) {
 // sums) gain nothing above PAIR_LANES_LIGHT: the routine sequence at 23441
 // particles 2.35 ms with one lane there, 2.39 with four.
 constexpr int64_t PAIR_LANES = 30000, PAIR_LANES_LIGHT = 20000;
-inline bool pair_lanes(int64_t n) { return n <= PAIR_LANES; }
+// (BSC_PAIR_LANES: one or four at any size, for comparing the two)
+inline bool pair_lanes(const Ctx* c, int64_t most = PAIR_LANES) {
+    return c->pair_lanes ? c->pair_lanes > 1 : c->n <= most;
+}
 template <typename F>
-void with_pair_lanes(int64_t n, F f, int64_t most = PAIR_LANES) {
-    if (n <= most) f(std::integral_constant<int, 4>{});
+void with_pair_lanes(const Ctx* c, F f, int64_t most = PAIR_LANES) {
+    if (pair_lanes(c, most)) f(std::integral_constant<int, 4>{});
     else f(std::integral_constant<int, 1>{});
 }
 

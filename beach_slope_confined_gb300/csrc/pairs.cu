@@ -596,7 +596,7 @@ int op_neighbour(Ctx* c) {
             k_neighbour<double, true><<<g, NB_BLOCK, 0, c->stream>>>(
                 c->n, c->S, c->K, c->cell_start, c->cell_count, c->sorted, c->pcell, c->posf, nullptr, c->nbr, c->gw,
                 nullptr, nullptr, nullptr, c->ndist, c->cnt, c->d_flag, c->cand_nc);
-    } else if (pair_lanes(c->n)) {
+    } else if (pair_lanes(c)) {
         launch_lists(c, std::max(4, lanes_for(c->n)));
         BSC_LAUNCH(c);
         const unsigned gr = blocks_for(c->n * 4, NB_BLOCK);
@@ -642,7 +642,7 @@ __global__ void k_freesurf(int64_t n, State S, KParams K, const int32_t* __restr
 }
 
 int op_freesurf(Ctx* c) {
-    with_pair_lanes(c->n, [&](auto L) {
+    with_pair_lanes(c, [&](auto L) {
         k_freesurf<L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr,
                                                                                      c->cnt);
     }, PAIR_LANES_LIGHT);
@@ -838,7 +838,7 @@ int op_effpor(Ctx* c) {
                                                        c->sx, c->sy, c->sposf, c->swf, c->svol, c->spor, c->f_vol,
                                                        c->f_vol_lo);
     else
-        with_pair_lanes(c->n, [&](auto L) {
+        with_pair_lanes(c, [&](auto L) {
             k_effpor<double, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
                 c->n, c->S, c->K, c->pcell, c->scell_start, c->scell_count, c->sx, c->sy, c->sposf, c->swf, c->svol,
                 c->spor);
@@ -936,12 +936,12 @@ int op_eddyvis(Ctx* c) {
                                                                  c->mixed ? c->udf : nullptr);
     BSC_LAUNCH(c);
     if (c->mixed)
-        with_pair_lanes(c->n, [&](auto L) {
+        with_pair_lanes(c, [&](auto L) {
             k_eddyvis<float, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
                 c->n, c->S, c->K, c->nbr, c->gwf, c->cnt, ux, uy, c->f_vol, c->udf);
         }, PAIR_LANES_LIGHT);
     else
-        with_pair_lanes(c->n, [&](auto L) {
+        with_pair_lanes(c, [&](auto L) {
             k_eddyvis<double, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
                 c->n, c->S, c->K, c->nbr, c->gw, c->cnt, ux, uy, nullptr, nullptr);
         }, PAIR_LANES_LIGHT);
@@ -1169,12 +1169,12 @@ int op_int_vel(Ctx* c, const double* d_umax) {
                                                                  mx ? c->udf : nullptr);
     BSC_LAUNCH(c);
     if (mx)
-        with_pair_lanes(c->n, [&](auto L) {
+        with_pair_lanes(c, [&](auto L) {
             k_varts<float, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
                 c->n, c->S, c->K, c->nbr, c->gwf, c->cnt, ux, uy, d_umax, c->f_vol, c->f_varts, c->udf);
         }, PAIR_LANES_LIGHT);
     else
-        with_pair_lanes(c->n, [&](auto L) {
+        with_pair_lanes(c, [&](auto L) {
             k_varts<double, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
                 c->n, c->S, c->K, c->nbr, c->gw, c->cnt, ux, uy, d_umax, nullptr, nullptr, nullptr);
         }, PAIR_LANES_LIGHT);
@@ -1184,13 +1184,13 @@ int op_int_vel(Ctx* c, const double* d_umax) {
     BSC_LAUNCH(c);
     StageTimer tk(c, BSC_T_K_INT_VEL);
     if (mx)
-        with_pair_lanes(c->n, [&](auto L) {
+        with_pair_lanes(c, [&](auto L) {
             k_int_vel<float, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
                 c->n, c->S, c->K, c->nbr, c->gwf, c->cnt, nu, c->dt, c->f_vol, c->f_nu, c->f_nut, c->f_tke,
                 c->f_varts, c->posf, c->pcell);
         }, PAIR_LANES_LIGHT);
     else
-        with_pair_lanes(c->n, [&](auto L) {
+        with_pair_lanes(c, [&](auto L) {
             k_int_vel<double, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
                 c->n, c->S, c->K, c->nbr, c->gw, c->cnt, nu, c->dt, nullptr, nullptr, nullptr, nullptr, nullptr,
                 nullptr, nullptr);
@@ -1339,7 +1339,7 @@ int op_comp_vel(Ctx* c) {
         k_comp_vel_mixed<<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->gwf, c->gwl, c->cnt, c->f_q,
                                                         c->f_vol, c->f_vol_lo, c->dt);
     else
-        with_pair_lanes(c->n, [&](auto L) {
+        with_pair_lanes(c, [&](auto L) {
             k_comp_vel<double, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
                 c->n, c->S, c->K, c->nbr, c->gw, c->cnt, q, c->dt);
         });
@@ -1464,7 +1464,7 @@ int op_opt2_shift(Ctx* c) {
             k_shift<float, 1><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, nullptr, c->gwf, c->gwl,
                                                           c->f_vol, c->f_vol_lo, c->cnt, mark);
         else
-            with_pair_lanes(c->n, [&](auto L) {
+            with_pair_lanes(c, [&](auto L) {
                 k_shift<double, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
                     c->n, c->S, c->K, c->nbr, c->gw, nullptr, nullptr, nullptr, nullptr, c->cnt, mark);
             }, PAIR_LANES_LIGHT);

@@ -372,7 +372,7 @@ int op_ppe_assemble(Ctx* c) {
         k_asm_df_pre<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->S, c->K, c->pcell, q, c->asm_df);
         BSC_LAUNCH(c);
         StageTimer tk(c, BSC_T_K_ASSEMBLE);
-        with_pair_lanes(c->n, [&](auto L) {
+        with_pair_lanes(c, [&](auto L) {
             k_assemble_df<L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
                 c->n, c->S, c->K, c->nbr, c->gwf, c->gwl, c->cnt, c->pcell, c->asm_df, c->aval, c->ellf, c->avalh,
                 c->b, q, ux, uy, c->dt);
@@ -384,7 +384,7 @@ int op_ppe_assemble(Ctx* c) {
             k_assemble<double, true, 1><<<g, NB_BLOCK, 0, c->stream>>>(c->n, c->S, c->K, c->nbr, c->gw, c->cnt, c->aval,
                                                                     c->ellf, c->avalh, c->b, q, ux, uy, c->dt);
         else
-            with_pair_lanes(c->n, [&](auto L) {
+            with_pair_lanes(c, [&](auto L) {
                 k_assemble<double, false, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
                     c->n, c->S, c->K, c->nbr, c->gw, c->cnt, c->aval, c->mixed ? c->ellf : nullptr,
                     c->mixed ? c->avalh : nullptr, c->b, q, ux, uy, c->dt);
