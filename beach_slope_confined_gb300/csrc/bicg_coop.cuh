@@ -80,8 +80,8 @@ constexpr int coop_entry(bool merge) { return 32 * (int)(sizeof(double) + sizeof
 constexpr int COOP_ITERS = 1024;                   // iterations per launch: tens of milliseconds at the largest sizes
 constexpr int COOP_BAR = 64;                       // the barrier's word in the ticket array
 constexpr int COOP_SETS = 5;                       // partials of an iteration's three reductions, a set per value
-// doubles a set takes: a partial per warp of rows
-__host__ __device__ inline int coop_part(int64_t n) { return (int)((n + 255) / 256 * 8); }
+// doubles a set takes at most: a partial per warp of rows
+constexpr int coop_part(int64_t n) { return (int)((n + 255) / 256 * 8); }
 
 // the warp sum over the tree of warp_sum_to_lane0, in every lane
 __device__ __forceinline__ double warp_sum_all(double x) {

@@ -36,7 +36,7 @@ constexpr size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
 // layout of the scratch array, every region on a 256-byte boundary
 constexpr size_t kOffWork = 0;                                        // r rh p v s t (6 vectors)
 constexpr size_t kOffPart = kOffWork + 6 * kVecBytes;                // partials of either BiCGSTAB
-constexpr size_t kOffHd = kOffPart + round256(std::max(8 * RED_GRID, COOP_SETS * (BSC_NOALLOC_MAX_ROWS / 32)) * sizeof(double));  // residual norms
+constexpr size_t kOffHd = kOffPart + round256(std::max(8 * RED_GRID, COOP_SETS * coop_part(BSC_NOALLOC_MAX_ROWS)) * sizeof(double));  // residual norms
 constexpr size_t kOffSc = kOffHd + round256(64 * sizeof(double));    // device scalars
 constexpr size_t kOffTicket = kOffSc + round256(sizeof(Scalars));    // last-block ticket, barrier word
 constexpr size_t kScratchBytes = kOffTicket + round256(TICKET_WORDS * sizeof(unsigned));
