@@ -66,7 +66,7 @@ struct WcState {
     double* mass = nullptr;                    // particle masses rho_init dl^2
     double *theta = nullptr, *sw = nullptr;    // grid porosities; (1 - phi_s) V_s
     int32_t* sg = nullptr;                     // solid -> grid cell or -1
-    double *rt = nullptr, *pp = nullptr, *ex = nullptr, *drh = nullptr;  // per step
+    double *rt = nullptr, *ex = nullptr, *drh = nullptr;  // per step
     double *vol = nullptr, *pr = nullptr;      // m/rt, p/rt^2 (per step)
     double* dpdr = nullptr;                    // dp/drt (per step)
     double* nxt = nullptr;                     // next state (5n)
@@ -168,11 +168,11 @@ __global__ void k_wc_solids(int64_t ns, const double* __restrict__ sx, const dou
     sg[s] = g;
 }
 
-// clamped density, pressure, the density's excess over the hydrostatic one and
+// clamped density, the density's excess over the hydrostatic one and
 // that one's slope, and the per-particle quotients the pair loops read (volume
 // m/rt, p/rt^2)
 struct Pre {
-    double *rt, *pp, *ex, *drh, *vol, *pr, *dpdr;  // dpdr: dp/drt of the EOS
+    double *rt, *ex, *drh, *vol, *pr, *dpdr;  // dpdr: dp/drt of the EOS
 };
 
 // s^(1/m) for a whole m and s > 0 in FP32's range: an FP32 seed, then two
@@ -215,7 +215,6 @@ __global__ void k_wc_pre(int64_t n, const int8_t* __restrict__ tid, const double
     const double ir = 1.0 / r;
     o.dpdr[i] = K.B * K.gam * (qm + 1.0) * ir;  // B gamma (rt/rho0)^(gamma-1) / rho0
     o.rt[i] = r;
-    o.pp[i] = p;
     o.vol[i] = mass[i] * ir;
     o.pr[i] = p * ir * ir;
     const double s = 1.0 + K.grav_c * (K.ys - y[i]);
@@ -662,7 +661,7 @@ __global__ void __launch_bounds__(WB) k_wc_adj_local(int64_t n, const int8_t* __
 template <int L>
 __global__ void __launch_bounds__(WPB) k_wc_adj_pair(
     int64_t n, State S, WcK K, St s0, const int32_t* __restrict__ nbr, const int32_t* __restrict__ cnt, Pre pq,
-    const double* __restrict__ geo, int64_t slots, const double* __restrict__ nbuf, AdjPair ap,
+    const double* __restrict__ geo, int64_t slots, AdjPair ap,
     const double* __restrict__ lD, const double* __restrict__ ln, const double* __restrict__ lvl,
     const double* __restrict__ lrl, St lam_in, St lam_out, const double* __restrict__ dn,
     const int32_t* __restrict__ pgi, const double* __restrict__ pgv, double* __restrict__ part, int pstride) {
@@ -812,7 +811,7 @@ int wc_params(Ctx* c, WcState* w, double alpha, double beta, const double* grid)
 }
 
 // one forward step on c->S; keeps n and P in nbuf, Pbuf
-Pre wc_pre(WcState* w) { return {w->rt, w->pp, w->ex, w->drh, w->vol, w->pr, w->dpdr}; }
+Pre wc_pre(WcState* w) { return {w->rt, w->ex, w->drh, w->vol, w->pr, w->dpdr}; }
 
 // the context's state with the model's masses
 State wc_view(Ctx* c, WcState* w) {
@@ -848,12 +847,12 @@ struct Keep {
 int64_t list_slots(const Ctx* c) { return ((c->n + 31) / 32) * 32 * (int64_t)c->K.kmax; }
 
 Keep seg_keep(WcState* w, int q, int64_t n, int64_t slots) {
-    double* pre = w->segpre + (int64_t)q * 7 * n;
+    double* pre = w->segpre + (int64_t)q * 6 * n;
     const int gc = w->K.gc;
     return {w->segnbr + (int64_t)q * slots,
             w->segcnt + (int64_t)q * n,
             w->segpc + (int64_t)q * n,
-            {pre, pre + n, pre + 2 * n, pre + 3 * n, pre + 4 * n, pre + 5 * n, pre + 6 * n},
+            {pre, pre + n, pre + 2 * n, pre + 3 * n, pre + 4 * n, pre + 5 * n},
             w->seggeo + (int64_t)q * 4 * slots,
             {w->segdn + (int64_t)q * 2 * n, w->segpgi + (int64_t)q * gc * n, w->segpgv + (int64_t)q * gc * n}};
 }
@@ -993,7 +992,7 @@ int bsc_wcsph_setup(bsc_ctx* c, const bsc_wcsph_params* p) {
     if ((rc = wc_alloc(c, w, &w->init, 5 * n)) || (rc = wc_alloc(c, w, &w->mass, n)) ||
         (rc = wc_alloc(c, w, &w->theta, G)) ||
         (rc = wc_alloc(c, w, &w->sw, w->ns)) || (rc = wc_alloc(c, w, &w->sg, w->ns)) ||
-        (rc = wc_alloc(c, w, &w->rt, n)) || (rc = wc_alloc(c, w, &w->pp, n)) || (rc = wc_alloc(c, w, &w->ex, n)) ||
+        (rc = wc_alloc(c, w, &w->rt, n)) || (rc = wc_alloc(c, w, &w->ex, n)) ||
         (rc = wc_alloc(c, w, &w->drh, n)) || (rc = wc_alloc(c, w, &w->vol, n)) || (rc = wc_alloc(c, w, &w->pr, n)) ||
         (rc = wc_alloc(c, w, &w->dpdr, n)) ||
         (rc = wc_alloc(c, w, &w->nxt, 5 * n)) ||
@@ -1042,7 +1041,7 @@ int bsc_wcsph_forward(bsc_ctx* c, int32_t nsteps, int32_t every, double* eta) {
             (rc = wc_alloc(c, w, &w->segnbr, (int64_t)every * slots)) ||
             (rc = wc_alloc(c, w, &w->segcnt, (int64_t)every * n)) ||
             (rc = wc_alloc(c, w, &w->segpc, (int64_t)every * n)) ||
-            (rc = wc_alloc(c, w, &w->segpre, (int64_t)every * 7 * n)) ||
+            (rc = wc_alloc(c, w, &w->segpre, (int64_t)every * 6 * n)) ||
             (rc = wc_alloc(c, w, &w->seggeo, (int64_t)every * 4 * slots)) ||
             (rc = wc_alloc(c, w, &w->segdn, (int64_t)every * 2 * n)) ||
             (rc = wc_alloc(c, w, &w->segpgi, (int64_t)every * gc * n)) ||
@@ -1143,7 +1142,7 @@ int bsc_wcsph_adjoint(bsc_ctx* c, const double* dJ_deta, double* grad) {
             BSC_LAUNCH(c);
             with_lanes(lanes, [&](auto L) {
                 k_wc_adj_pair<decltype(L)::value><<<nbp, WPB, 0, c->stream>>>(
-                    n, S, w->K, st0, kq.nbr, kq.cnt, kq.pre, kq.geo, slots, nq, ap, w->lD, w->ln, w->lvl, w->lrl, lam,
+                    n, S, w->K, st0, kq.nbr, kq.cnt, kq.pre, kq.geo, slots, ap, w->lD, w->ln, w->lvl, w->lrl, lam,
                     lamn, kq.por.dn, kq.por.pgi, kq.por.pgv, w->part, pstride);
             });
             BSC_LAUNCH(c);
