@@ -28,6 +28,7 @@ namespace {
 // the reference's single-precision literals, promoted to FP64
 constexpr double SC_NUT_MIN = (double)1e-6f;  // scalar.f90 `nut < 1e-6`
 constexpr double SC_TOR = 1.0;                // scalar.f90 `tor`
+constexpr long long SC_MARK = 0x7ff8000000000000LL;  // cs of a particle whose pairs are never skipped (a NaN)
 
 struct ScalarK {
     double Dm, al, at, tsc, cap;  // molecular diffusivity, dispersivities, Schmidt number, D cap
@@ -44,10 +45,10 @@ __device__ __forceinline__ double disp(double Dm, double a1, double a2, double a
 
 // per particle: D_x, D_y and the eddy term Dm + nu_t / Sc, the same values
 // scalart forms for a particle as i and as j (one division and root each,
-// instead of per pair); and in cs the concentration, or a NaN where a
-// coefficient is zero or not finite: between such particles the flux of a pair
-// of one concentration is not the zero that it is elsewhere, but the
-// reference's 0/0 or NaN
+// instead of per pair); and in cs the concentration, or SC_MARK where it or a
+// coefficient is not finite or a coefficient is zero: with such a particle the
+// flux of a pair of one concentration is not the zero that it is elsewhere,
+// but the reference's NaN or 0/0
 __global__ void k_scalar_pre(int64_t n, State S, ScalarK C, double* __restrict__ Dx, double* __restrict__ Dy,
                              double* __restrict__ E, double* __restrict__ inv_n, double* __restrict__ cs) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -61,8 +62,8 @@ __global__ void k_scalar_pre(int64_t n, State S, ScalarK C, double* __restrict__
     E[i] = e;
     inv_n[i] = in;
     const bool plain = isfinite(dx) && isfinite(dy) && isfinite(e) && isfinite(in) && isfinite(S.ovol[i]) &&
-                       dx != 0.0 && dy != 0.0 && e != 0.0;
-    cs[i] = plain ? S.con[i] : __longlong_as_double(0x7ff8000000000000LL);
+                       isfinite(S.con[i]) && dx != 0.0 && dy != 0.0 && e != 0.0;
+    cs[i] = plain ? S.con[i] : __longlong_as_double(SC_MARK);
 }
 
 // Bound: the FP64 pipe, an FP64 division being about nine of its
@@ -71,7 +72,8 @@ __global__ void k_scalar_pre(int64_t n, State S, ScalarK C, double* __restrict__
 // the eddy diffusivities is (E_i + E_j) / 2 with E = Dm + nu_t / Sc; and a
 // pair of one concentration, which has no flux, takes none (fresh water away
 // from the front; whole warps).  198k particles: 425 us with three divisions a
-// pair, 226 now.
+// pair, 226 with one; with the concentrations compared as bits instead of
+// subtracted first the call (both kernels, c2) went from 269 to 262.
 __global__ void __launch_bounds__(128) k_scalart(int64_t n, State S, KParams K, const int32_t* __restrict__ nbr,
                                                  const double* __restrict__ ndist, const int32_t* __restrict__ cnt,
                                                  const double* __restrict__ Dx, const double* __restrict__ Dy,
@@ -80,18 +82,20 @@ __global__ void __launch_bounds__(128) k_scalart(int64_t n, State S, KParams K, 
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     if (S.tid[i] != BSC_TID_FLUID || (S.flags[i] & BSC_FLAG_DEAD)) return;
-    const double con1 = S.con[i], cs1 = cs[i], ni = S.por[i], nuti = S.nut[i], oi = S.ovol[i];
+    const double con1 = S.con[i], ni = S.por[i], nuti = S.nut[i], oi = S.ovol[i];
     const double Dxi = Dx[i], Dyi = Dy[i], Ei = E[i], ini = inv_n[i];
     const double xi = S.x[i], yi = S.y[i];
+    // compared as bit patterns, off the FP64 pipe (the other NaN: no cs has it)
+    const long long cs1 = __double_as_longlong(cs[i]), same = cs1 == SC_MARK ? -1LL : cs1;
     double cd = 0.0;
     const int m = cnt[i];
     for (int k = 0; k < m; ++k) {
         const int64_t e = ell(i, k, K.kmax);
         const int j = nbr[e];
         if (S.tid[j] != BSC_TID_FLUID || (S.flags[j] & BSC_FLAG_DEAD)) continue;
-        double dcon = cs1 - cs[j];
-        if (dcon == 0.0) continue;
-        if (isnan(dcon)) dcon = con1 - S.con[j];
+        const long long cs2 = __double_as_longlong(cs[j]);
+        if (cs2 == same) continue;
+        const double dcon = con1 - (cs2 == SC_MARK ? S.con[j] : __longlong_as_double(cs2));
         const double r = ndist[e];
         const double dx = xi - S.x[j], dy = yi - S.y[j], dx2 = dx * dx, dy2 = dy * dy;
         double den = r * r + K.lam, num;  // num / den: t1x dx^2 + t1y dy^2 over r^2 + lam
