@@ -17,8 +17,8 @@
 //    in phases of their own, by all warps of the block into shared memory:
 //    three barriers an iteration instead of five.
 // Per iteration at 7600 rows: 35 us as five kernels in a graph, ~15 us here:
-// three barriers ~1.8 us each, two products ~2.5 us each (28 dependent FP64
-// additions of ~140 clocks), three sums with their quotients ~1.5 us each.
+// three barriers ~1.8 us each, two products ~2.5 us each (28 FP64 FMAs
+// in turn, 64 clocks or more each), three sums with their quotients ~1.5 us each.
 // 125k rows of 21 entries: 48.8 us with a partial per warp and two rows per
 // thread, 33.5 us here.
 // The grid is launched cooperatively (all blocks resident), and every wait is

@@ -191,8 +191,8 @@ struct EllPackF {
 // the row times x in every lane of the row.  With L = 1 the constructor loads
 // the entry count alone and dot() is the operator's own loop.
 // Small systems' passes are the length of one row's chain of rounds (entries,
-// then the gathers they index) and sums, FP64 ones above all (one in flight
-// per warp and ~100 clocks); L lanes shorten it.
+// then the gathers they index) and sums, FP64 ones above all (a warp
+// issues one per 64 clocks); L lanes shorten it.
 template <typename T, typename Op, int L>
 struct RowLanes {
     static constexpr int E = L == 1 ? 1 : 32 / L;

@@ -1,9 +1,9 @@
 // lanes.cuh -- several lanes per particle for the FP64 pair sums.
 //
-// A warp has one FP64 instruction in flight per ~100 clocks on this GPU
-// (dependent or not), and the FP64 pipe takes one per 16: below about eight
-// warps an SM a pair sum's time is the length of a thread's own loop, whatever
-// the particle count.  L lanes of a warp then share a particle: each takes
+// A warp issues one FP64 add, multiply or FMA per 64 clocks on this GPU,
+// dependent or not, and an SM one per 19 (measured, one block, clock64): with
+// fewer than some four warps an SM that have FP64 work at hand, a pair sum's time
+// is the length of a thread's own loop, whatever the particle count.  L lanes of a warp then share a particle: each takes
 // every L-th neighbour, and the sums are added up across them.
 #pragma once
 

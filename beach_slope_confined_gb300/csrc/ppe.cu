@@ -42,7 +42,7 @@ namespace bsc {
 // FAST (the mixed path): the per-pair and per-row quotients by rcp_nr, a
 // Newton-Raphson reciprocal within ~2^-46 of the FP64 quotient.  The FP64
 // path divides (correctly rounded, as the reference).
-// L lanes per row (lanes_for), the sums in list order.
+// L lanes per row (with_pair_lanes), the sums in list order.
 template <typename R, bool FAST, int L>
 __global__ void __launch_bounds__(NB_BLOCK) k_assemble(int64_t n, State S, KParams K, const int32_t* __restrict__ nbr,
                                                         const typename Vec2<R>::type* __restrict__ gw,
@@ -1450,7 +1450,7 @@ int fg_cycle(Ctx* c, int m, int budget, Scalars* h, int* iters, Q queue) {
 // Givens step.  The next basis vector is not written here: the V-cycle's
 // first pass scales w by the reciprocal of the norm (sc->tmp[4]).
 // What bounds them on systems below ~10^5 rows is the chain of dependent
-// steps, FP64 ones above all (~140 clocks each here): hence the finishing
+// steps, FP64 ones above all (64 clocks each at least): hence the finishing
 // block's four partial sums per lane, the earlier rotations of the column in
 // a block of their own beside the update, and one division for the reciprocal
 // of the norm (k_fg_next divided once per thread: 5 us at any size).
@@ -1610,7 +1610,7 @@ __global__ void __launch_bounds__(RED_BLOCK) k_gs_update(int64_t n, const T* V, 
     double v[1];
     reduce_partials<1>(part, rows, v);
     // a square root and a quotient each in three warps (five in a row by one
-    // thread took ~10 instructions of ~100 clocks each): the norm and its
+    // thread: ~10 instructions of 64 clocks or more each): the norm and its
     // reciprocal, the rotation's cosine, its sine sqrt(v / (a^2 + v))
     const double d2 = a * a + v[0];
     if (t == 0) {
