@@ -247,11 +247,14 @@ struct PorKeep {
 // loop ran ~60 candidates' offsets a particle and their kernels at half the
 // lanes; the FP32 pre-test (sph_kernel.cuh) now compacts the survivors, in
 // cell order, into this thread's column of shared memory, and the FP64 terms
-// run over those.  Same terms, same order.  A particle with more survivors
-// than the column holds, or far from its binned cell, takes one pass.
+// run over those, a column at a time.  A particle far from its binned cell
+// takes one pass over all of them, by one lane.
 // The particles with solids are few and sit together, so several lanes share
 // one at any size.  101573 particles: 236 us before, 61 us, with the adjoint's
-// record 106 us.
+// record 106 us.  (With more survivors than the column holds left to one lane
+// of the four, a forward step at 96593 particles took 3590 us where the solids
+// are nine times as many, 2110 with a thread per particle, 1010 so; the scan's
+// loops are kept rolled for the registers, 80 of them instead of 58.)
 constexpr int WP_CAP = 32;
 template <bool KEEP, int L>
 __global__ void __launch_bounds__(WPB, 8) k_wc_por(int64_t n, State S, KParams KP, WcK K, const int32_t* __restrict__ pcell,
@@ -320,19 +323,24 @@ __global__ void __launch_bounds__(WPB, 8) k_wc_por(int64_t n, State S, KParams K
             return W[0];
         };
         using One = std::integral_constant<int, 1>;
+        // windows of WP_CAP survivors, the scan repeated for each; without the
+        // pre-test one scan sums over the cells directly, by one lane
         int nc = 0;
-        // pass 0 compacts the survivors; pass 1 (only if they do not fit, or
-        // without the pre-test) sums over the cells directly, by one lane
-        for (int pass = pre_i ? 0 : 1; pass < 2; ++pass) {
+#pragma unroll 1
+        for (int w0 = 0; w0 == 0 || w0 < nc; w0 += WP_CAP) {
+            nc = 0;
+#pragma unroll 1
             for (int ax = cx - 1; ax <= cx + 1; ++ax) {
                 if (ax < 0 || ax >= KP.nx) continue;
                 const float shx = (float)(ax - cx) * csf;
+#pragma unroll 1
                 for (int ay = cy - 1; ay <= cy + 1; ++ay) {
                     if (ay < 0 || ay >= KP.ny) continue;
                     const float shy = (float)(ay - cy) * csf;
                     const int cc = ax * KP.ny + ay;
                     const int s0 = scs[cc], s1 = s0 + scc[cc];
-                    if (pass == 1) {
+                    if (!pre_i) {
+#pragma unroll 1
                         for (int s = s0; s < s1 && ln.sub == 0; ++s) {
                             const double W = terms(One{}, &s);
                             if (KEEP && L > 1) cell(cell_of(s, W), svol[s] * W);
@@ -349,37 +357,36 @@ __global__ void __launch_bounds__(WPB, 8) k_wc_por(int64_t n, State S, KParams K
                                 keep = !(fdx * fdx + fdy * fdy > H2f);
                             }
                         }
-                        const int at = ln.place(keep, nc);
-                        if (keep && at < WP_CAP) cand[at * NP + p] = q;
+                        const int at = ln.place(keep, nc) - w0;
+                        if (keep && (unsigned)at < (unsigned)WP_CAP) cand[at * NP + p] = q;
                     }
                 }
             }
-            if (pass == 0 && nc <= WP_CAP) {
-                ln.sync();
-                if (L == 1) {
-                    constexpr int U = KEEP ? 2 : 4;
-                    int k = 0;
-                    for (; k + U <= nc; k += U) {
-                        int q[U];
+            ln.sync();
+            const int m = min(nc - w0, WP_CAP);
+            if (L == 1) {
+                constexpr int U = KEEP ? 2 : 4;
+                int k = 0;
+                for (; k + U <= m; k += U) {
+                    int q[U];
 #pragma unroll
-                        for (int u = 0; u < U; ++u) q[u] = cand[(k + u) * NP + p];
-                        terms(std::integral_constant<int, U>{}, q);
-                    }
-                    for (; k < nc; ++k) terms(One{}, &cand[k * NP + p]);
-                } else {
-                    for (int k = ln.sub; k < nc; k += L) {
-                        const double W = terms(One{}, &cand[k * NP + p]);
-                        if (KEEP) {
-                            const int s = cand[k * NP + p];
-                            wval[k * NP + p] = svol[s] * W;
-                            cand[k * NP + p] = cell_of(s, W);  // read by this lane only
-                        }
-                    }
-                    ln.sync();
-                    if (KEEP && ln.sub == 0)
-                        for (int k = 0; k < nc; ++k) cell(cand[k * NP + p], wval[k * NP + p]);
+                    for (int u = 0; u < U; ++u) q[u] = cand[(k + u) * NP + p];
+                    terms(std::integral_constant<int, U>{}, q);
                 }
-                break;
+                for (; k < m; ++k) terms(One{}, &cand[k * NP + p]);
+            } else {
+                for (int k = ln.sub; k < m; k += L) {
+                    const double W = terms(One{}, &cand[k * NP + p]);
+                    if (KEEP) {
+                        const int s = cand[k * NP + p];
+                        wval[k * NP + p] = svol[s] * W;
+                        cand[k * NP + p] = cell_of(s, W);  // read by this lane only
+                    }
+                }
+                ln.sync();
+                if (KEEP && ln.sub == 0)
+                    for (int k = 0; k < m; ++k) cell(cand[k * NP + p], wval[k * NP + p]);
+                ln.sync();
             }
         }
     }
