@@ -19,7 +19,7 @@ struct EllOp {
     int kmax;
     int unroll = 0;  // 1: eight, then four entries per round (that many gathers in flight)
     const void* key() const { return aval; }
-    static constexpr bool UNIT_DIAG = true;
+    static constexpr bool UNIT_DIAG = true, COALESCED = true;
     __device__ __forceinline__ int len(int64_t i) const { return cnt[i]; }
     __device__ __forceinline__ int64_t at(int64_t i, int k) const { return ell(i, k, kmax); }
     __device__ __forceinline__ int32_t col_at(int64_t e) const { return nbr[e]; }

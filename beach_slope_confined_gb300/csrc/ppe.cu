@@ -409,7 +409,7 @@ struct CsrOp {
     const int32_t* col;
     const double* val;
     const void* key() const { return val; }
-    static constexpr bool UNIT_DIAG = false;
+    static constexpr bool UNIT_DIAG = false, COALESCED = false;
     __device__ __forceinline__ int len(int64_t i) const { return max(rp[i + 1] - rp[i], 0); }  // as row()'s loop takes it
     __device__ __forceinline__ int64_t at(int64_t i, int k) const { return rp[i] + k; }
     __device__ __forceinline__ int32_t col_at(int64_t e) const { return col[e]; }
@@ -502,27 +502,29 @@ __device__ __forceinline__ void reduce_partials(const double* __restrict__ part,
 // ============================================================================
 // BiCGSTAB, value type T (double or float), dots accumulated in double
 // ============================================================================
-// r = b - A x; rhat = r; p = r; partials (r.r, b.b)
+// r = b - A x; rhat = r; p = r; partials (r.r, b.b, and in FP64 the entries)
 template <typename Op, typename T>
 __global__ void __launch_bounds__(RED_BLOCK) k_bicg_init(int64_t n, Op A, const T* __restrict__ x,
                                                           const T* __restrict__ b, T* __restrict__ r,
                                                           T* __restrict__ rh, T* __restrict__ p,
                                                           double* __restrict__ part) {
-    double acc[2] = {0.0, 0.0};
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
     GRID_LOOP(i, n) {
         const double ri = (double)b[i] - A.template row<T, double>(i, x);
         const T rt = (T)ri;
         r[i] = rt; rh[i] = rt; p[i] = rt;
         acc[0] += (double)rt * (double)rt;
         acc[1] += (double)b[i] * (double)b[i];
+        if constexpr (sizeof(T) == 8) acc[2] += (double)A.len(i);
     }
-    block_partials<2>(acc, part);
+    block_partials<4>(acc, part);
 }
 
 __global__ void k_bicg_setup(const double* __restrict__ part, int nb, Scalars* sc, double tol, int rel_r0) {
-    double v[2];
-    reduce_partials<2>(part, nb, v);
+    double v[3];
+    reduce_partials<3>(part, nb, v);
     if (threadIdx.x == 0) {
+        sc->tmp[6] = v[2];
         sc->rr = v[0];
         sc->rho = v[0];
         sc->bestb[0] = sqrt(v[0]);
@@ -1006,12 +1008,14 @@ int graph_run(Ctx* c, const void* k0, const void* k1, const void* k2, int64_t n,
 
 // The cooperative BiCGSTAB for n rows: its kernel, blocks (one per SM at
 // most; none where it cannot run: more than three rows per thread, or no
-// resident grid) and shared memory.  Up to there it is the faster at every
-// size; the five kernels keep the larger systems, the FP32 sweeps and the
-// per-kernel profiling.
+// resident grid) and shared memory.  The five kernels keep the larger systems
+// and the wide ones (coop_entries), the FP32 sweeps and the per-kernel
+// profiling.
 struct CoopPlan {
     const void* kernel = nullptr;
-    int blocks = 0, threads = 0, smem = 0, cap = 0;  // cap: entries of 32 rows in shared memory
+    int blocks = 0, threads = 0, smem = 0;
+    int rows = 0, entry = 0;  // rows per block at most, shared memory of an entry of 32 rows
+    bool ready = false;       // coop_entries has seen it
 };
 template <typename Op>
 CoopPlan coop_plan(int64_t n) {
@@ -1051,8 +1055,25 @@ CoopPlan coop_plan(int64_t n) {
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads, smem) != cudaSuccess || per_sm < 1)
         return (void)cudaGetLastError(), P;
-    P = {f, blocks, threads, smem, smem / entry};
+    P = {f, blocks, threads, smem, merge ? 32 * (int)((warps + blocks - 1) / blocks) : threads * (K == 3 ? 3 : 1), entry};
     return P;
+}
+
+// The plan once the entries are counted (k_bicg_setup's tmp[6]).
+// A block whose rows do not fit takes a quarter of the shared memory where the
+// rest of them is read a thread per row uncoalesced: with all of it taken some
+// 29 KB of L1 were left, and those reads missed it (us per iteration, five
+// kernels / all / a quarter: 40000 rows of 301 entries 333 / 591 / 216, 125000
+// of 61 126 / 167 / 74, of 121 216 / 890 / 140, of 81 anywhere 256 / 460 / 173).
+// ELL rows are read in whole lines: no difference.  But three of them per thread
+// keep too few reads in flight beyond 8 M entries (222850 rows of 59: 116 us by
+// the five kernels, 137 here; 170223 of 45: 100 and 77), where CSR rows do well
+// (200000 of 51: 149 and 113).
+template <typename Op>
+void coop_entries(CoopPlan& P, int64_t n, double entries) {
+    P.ready = true;
+    if (Op::COALESCED && n > 2 * (int64_t)P.blocks * COOP_BLOCK && entries > 8e6) P.blocks = 0;
+    if (!Op::COALESCED && entries / (double)n * P.rows * P.entry / 32 > P.smem) P.smem = P.smem / 4 / P.entry * P.entry;
 }
 
 template <typename Op>
@@ -1060,7 +1081,7 @@ cudaError_t bicg_coop_launch(Ctx* c, int64_t n, Op A, Work<double> w, int iters,
     unsigned* count = c->ticket + COOP_BAR;
     // (stuck: 2^30 below zero, which no arrivals make up for)
     if (cudaError_t e = cudaMemsetAsync(count, c->barrier_stuck ? 0xC0 : 0, sizeof(unsigned), c->stream)) return e;
-    int cap = P.cap;
+    int cap = P.smem / P.entry;  // entries of 32 rows
     const double* rh = w.rh;
     // MERGE: p and v double-buffered, their second halves in s and t
     void* args[] = {&n, &A, &w.x, &w.r, &rh, &w.p, &w.v, &w.s, &w.s, &w.t, &c->part, &c->sc, &count, &iters, &cap};
@@ -1128,6 +1149,8 @@ int run_bicgstab(Ctx* c, int64_t n, const Op& A, Work<T> w, double tol, int rel_
             c->launches += 2;
             continue;
         }
+        if constexpr (sizeof(T) == 8)
+            if (coop.blocks > 0 && !coop.ready) coop_entries<Op>(coop, n, h.tmp[6]);
         if (coop.blocks > 0) {  // the scalars carry on from launch to launch
             if (h.done || h.breakdown || h.it >= maxit) break;
             cudaError_t e = cudaSuccess;
