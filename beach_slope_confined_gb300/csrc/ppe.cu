@@ -417,7 +417,25 @@ struct CsrOp {
     template <typename X, typename A>
     __device__ __forceinline__ A row(int64_t i, const X* __restrict__ x) const {
         A s = 0;
-        for (int k = rp[i]; k < rp[i + 1]; ++k) s += (A)val[k] * (A)x[col[k]];
+        const int end = rp[i + 1];
+        int k = rp[i];
+        // eight entries' loads in flight: 235000 rows of 61 entries 224 us an
+        // iteration of the five kernels one at a time, 196 so
+        for (; k + 8 <= end; k += 8) {
+            int32_t c[8];
+            double a[8];
+            X y[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) c[u] = col[k + u];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                a[u] = val[k + u];
+                y[u] = x[c[u]];
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) s += (A)a[u] * (A)y[u];
+        }
+        for (; k < end; ++k) s += (A)val[k] * (A)x[col[k]];
         return s;
     }
 };
