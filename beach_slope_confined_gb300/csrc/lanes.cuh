@@ -94,13 +94,21 @@ void with_lanes(int lanes, F f) {
 }
 
 // The FP64 step's pair sums: four lanes, their terms added up in list order
-// (Lanes::ordered).  Measured, the step's five pair kernels together with one
-// and four lanes: 418 and 361 us at 21490 particles, 472 and 428 at 25881,
-// 470 and 519 at 35943 (at 3816: 278 and 113).
-// The lighter ones (eddyvis, varts, shift, freesurf, and the mixed path's FP32
-// sums) gain nothing above PAIR_LANES_LIGHT: the routine sequence at 23441
-// particles 2.35 ms with one lane there, 2.39 with four.
-constexpr int64_t PAIR_LANES = 30000, PAIR_LANES_LIGHT = 20000;
+// (Lanes::ordered).  Measured with one and four lanes at 8967, 16422, 23441 and
+// 28635 particles (about 20 neighbours), us:
+//   search       53 / 31   54 / 48   67 / 56   67 / 61
+//   effpor       41 / 33   39 / 43   57 / 47   57 / 49
+//   assembly     70 / 35   70 / 49   85 / 60   87 / 74
+//   int_vel      55 / 33   53 / 50   70 / 62   70 / 97: its blocks (86 registers) no longer fit at once
+//   comp_vel     31 / 23   31 / 32   39 / 37   40 / 43
+//   eddyvis      27 / 23   27 / 33   33 / 37   34 / 43  (12931: 26 / 27)
+//   opt2_shift   21 / 19   21 / 31   24 / 37   24 / 45  (12931: 20 / 25)
+// With 40 and 70 neighbours the lines lie in the same places.  On the mixed path
+// the search and the assembly gain as above, int_vel (29 / 17 at 16422) and
+// varts are given the lanes up to PAIR_LANES_LIGHT, eddyvis as in FP64 (19 / 19
+// at 8967, 19 / 21 at 16422).
+constexpr int64_t PAIR_LANES = 30000, PAIR_LANES_VEL = 24000, PAIR_LANES_LIGHT = 20000, PAIR_LANES_EDDY = 12000,
+                  PAIR_LANES_SHIFT = 10000;
 // (BSC_PAIR_LANES: one or four at any size, for comparing the two)
 inline bool pair_lanes(const Ctx* c, int64_t most = PAIR_LANES) {
     return c->pair_lanes ? c->pair_lanes > 1 : c->n <= most;

@@ -948,12 +948,12 @@ int op_eddyvis(Ctx* c) {
         with_pair_lanes(c, [&](auto L) {
             k_eddyvis<float, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
                 c->n, c->S, c->K, c->nbr, c->gwf, c->cnt, ux, uy, c->f_vol, c->udf);
-        }, PAIR_LANES_LIGHT);
+        }, PAIR_LANES_EDDY);
     else
         with_pair_lanes(c, [&](auto L) {
             k_eddyvis<double, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
                 c->n, c->S, c->K, c->nbr, c->gw, c->cnt, ux, uy, nullptr, nullptr);
-        }, PAIR_LANES_LIGHT);
+        }, PAIR_LANES_EDDY);
     BSC_LAUNCH(c);
     return BSC_OK;
 }
@@ -1203,7 +1203,7 @@ int op_int_vel(Ctx* c, const double* d_umax) {
             k_int_vel<double, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
                 c->n, c->S, c->K, c->nbr, c->gw, c->cnt, nu, c->dt, nullptr, nullptr, nullptr, nullptr, nullptr,
                 nullptr, nullptr);
-        });
+        }, PAIR_LANES_VEL);
     BSC_LAUNCH(c);
     return BSC_OK;
 }
@@ -1351,7 +1351,7 @@ int op_comp_vel(Ctx* c) {
         with_pair_lanes(c, [&](auto L) {
             k_comp_vel<double, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
                 c->n, c->S, c->K, c->nbr, c->gw, c->cnt, q, c->dt);
-        });
+        }, PAIR_LANES_VEL);
     BSC_LAUNCH(c);
     return BSC_OK;
 }
@@ -1476,7 +1476,7 @@ int op_opt2_shift(Ctx* c) {
             with_pair_lanes(c, [&](auto L) {
                 k_shift<double, L()><<<blocks_for(c->n * L(), NB_BLOCK), NB_BLOCK, 0, c->stream>>>(
                     c->n, c->S, c->K, c->nbr, c->gw, nullptr, nullptr, nullptr, nullptr, c->cnt, mark);
-            }, PAIR_LANES_LIGHT);
+            }, PAIR_LANES_SHIFT);
         BSC_LAUNCH(c);
     }
     k_shift_apply<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->S, mark);
