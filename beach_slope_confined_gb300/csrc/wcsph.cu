@@ -250,8 +250,8 @@ struct PorKeep {
 // run over those, a column at a time.  A particle far from its binned cell
 // takes one pass over all of them, by one lane.
 // The particles with solids are few and sit together, so several lanes share
-// one at any size.  101573 particles: 236 us before, 61 us, with the adjoint's
-// record 106 us.  (With more survivors than the column holds left to one lane
+// one at any size.  101573 particles: 236 us with a thread each, 64 us, with the adjoint's
+// record 83 us.  (With more survivors than the column holds left to one lane
 // of the four, a forward step at 96593 particles took 3590 us where the solids
 // are nine times as many, 2110 with a thread per particle, 1010 so; the scan's
 // loops are kept rolled for the registers, 80 of them instead of 58.)

@@ -54,26 +54,28 @@ T_STEP, T_PPE_SOLVE, T_SPMV, T_UPLOAD, T_DOWNLOAD, T_SCALAR = 15, 8, 16, 17, 18,
 T_K_NEIGHBOUR, T_K_ASSEMBLE, T_K_INT_VEL, T_K_EFFPOR, T_K_SHIFT = 25, 26, 27, 28, 29
 
 # Algorithmic FP64 flops per pair of the pair kernels, counted from the
-# formulas each kernel evaluates (an FMA is 2 flops; a division or a square
-# root is 1): kernel slot -> (FP64 path, mixed path).  Per neighbour pair:
+# formulas each kernel evaluates for a pair of one density and one porosity
+# (nearly all; an FMA is 2 flops; a division or a square root is 1): kernel
+# slot -> (FP64 path, mixed path).  Per neighbour pair:
 #   k_neighbour: offsets 2, d^2 3, root 1, grad W factor 6, grad W 2, the
 #     moment sum M 10 (mixed: membership, root and grad W on FP32 pairs from
 #     double-float offsets, grad W stored as a double-float; the FP64 test
 #     only inside a 1e-10 band around the threshold, 0 per pair);
 #   k_assemble: offsets 2, 1/(r^2+lam) 5, L grad W 6, the coefficient 6, the
-#     diagonal 2, rho_ij 4, velocity differences 4, divergence 5, the Jacobi
-#     scaling 1 (mixed: k_assemble_df runs that arithmetic on FP32 pairs; its
-#     FP64 work is the two velocity differences and their splits and the
-#     widening of the entry, 5);
-#   k_int_vel: the two harmonic viscosity means and their sum 10, offsets
-#     and r^2 5, 1/(r^2+lam) 2, L grad W 6, the coefficient 6, velocity
-#     differences 2, viscous sums 6, SPS sums 6 (mixed: 0; offsets from the
-#     FP32 cell offsets, velocity differences from FP32 roundings);
+#     diagonal 2, velocity differences 4, divergence 5, the Jacobi scaling 1;
+#     rho_ij, 4 more, once per row (mixed: k_assemble_df runs that arithmetic
+#     on FP32 pairs; its FP64 work is the two velocity differences and their
+#     splits and the widening of the entry, 5);
+#   k_int_vel: the eddy viscosity's harmonic mean and the sum of the two 6 (the
+#     kinematic one's, 4 more, once per particle), offsets and r^2 5,
+#     1/(r^2+lam) 2, L grad W 6, the coefficient 6, velocity differences 2,
+#     viscous sums 6, SPS sums 6 (mixed: 0; offsets from the FP32 cell
+#     offsets, velocity differences from FP32 roundings);
 #   k_shift: 16 (mixed: 0; the position-shift sums run as double-floats,
 #     the velocity-gradient sums in FP32).
 # Per solid pair, k_effpor: offsets 2, d^2 3, root 1, W 9, the weighted sum
 # 4 (mixed: FP32 terms summed as a double-float, 0).
-FP64_FLOPS = {T_K_NEIGHBOUR: (24, 0), T_K_ASSEMBLE: (35, 5), T_K_INT_VEL: (43, 0), T_K_SHIFT: (16, 0),
+FP64_FLOPS = {T_K_NEIGHBOUR: (24, 0), T_K_ASSEMBLE: (31, 5), T_K_INT_VEL: (39, 0), T_K_SHIFT: (16, 0),
               T_K_EFFPOR: (19, 0)}
 # Algorithmic DRAM bytes: (per row, per neighbour entry) for each path, each
 # input read and each output written once (neighbours' particle data counted
@@ -92,13 +94,13 @@ FP64_FLOPS = {T_K_NEIGHBOUR: (24, 0), T_K_ASSEMBLE: (35, 5), T_K_INT_VEL: (43, 0
 HBM_BYTES = {T_K_NEIGHBOUR: ((110, 20), (130, 20)), T_K_ASSEMBLE: ((108, 28), (148, 38)),
              T_K_INT_VEL: ((175, 20), (175, 12)), T_K_SHIFT: ((150, 20), (150, 20)),
              T_K_EFFPOR: ((73, 0), (73, 0))}
-# what ncu shows limits a kernel that neither bound reaches (full captures of
-# one launch each on the c2 tank)
+# what ncu shows limits a kernel that neither bound reaches (one launch each on
+# the c2 tank)
 KERNEL_LIMITER = {
     "k_neighbour<float>": "issue and latency of the double-float chains: 35 % warps active (64 registers), 10 cycles "
-                          "between a warp's instructions; FP64 17 %, FMA 28.5 %, ALU 25 % of their pipes",
-    "k_int_vel<float>": "latency of its per-neighbour gathers (long scoreboard 12.7 per issue), 34 % warps active",
-    "k_assemble_df": "issue and latency: 58 % of issue slots, 29 % warps active (80 registers); FP64 35.5 %, "
+                          "between a warp's instructions; FP64 17 %, FMA 28 %, ALU 24 % of their pipes",
+    "k_int_vel<float>": "latency of its per-neighbour gathers (long scoreboard 11.6 per issue), 34 % warps active",
+    "k_assemble_df": "issue and latency: 55 % of issue slots, 29 % warps active (80 registers); FP64 35.5 %, "
                      "FMA 36.5 %, ALU 26 % of their pipes",
 }
 # the kernel each slot times: (FP64 path, mixed path)
