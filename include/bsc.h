@@ -383,7 +383,9 @@ int bsc_wcsph_setup(bsc_ctx* ctx, const bsc_wcsph_params* w);
 /* New values of the calibrated parameters (grid_por: grid_nx*grid_ny). */
 int bsc_wcsph_set_params(bsc_ctx* ctx, double alpha, double beta, const double* grid_por);
 /* nsteps steps from the initial state, a checkpoint every ckpt_every steps;
- * eta[nsteps * nprobe] receives the probe elevations after each step. */
+ * eta[nsteps * nprobe] receives the probe elevations after each step.  The
+ * context is left with the lists, grad W, L and flags of the last step's search
+ * (so does the adjoint, where it recomputes steps) and without a PPE matrix. */
 int bsc_wcsph_forward(bsc_ctx* ctx, int32_t nsteps, int32_t ckpt_every, double* eta);
 /* Reverse pass through the last forward run: given dJ/deta[nsteps * nprobe],
  * grad[0] = dJ/dalpha, grad[1] = dJ/dbeta, grad[2 + k] = dJ/dpor_k. */
